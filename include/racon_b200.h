@@ -279,7 +279,7 @@ int rb_set_priority(rb_ctx* ctx, int high);
 /* Launch choices of one device, shared by every context on it. None of them
  * changes a result. */
 typedef struct rb_tuning {
-    uint32_t consensus_ctas_per_sm;   /* resident consensus CTAs per SM, 1..3 (4 windows each): windows in flight */
+    uint32_t consensus_ctas_per_sm;   /* resident consensus CTAs per SM, 1..3: windows in flight (4 each; 2 in a batch of few windows) */
     uint32_t consensus_order;         /* queue order: 0 heaviest window first; 1 size buckets interleaved
                                        * (heaviest, lightest, next heaviest, ...) */
     uint32_t alignment_warps_per_sm;  /* resident alignment warps per SM (one pair or split task each): 4..32 */

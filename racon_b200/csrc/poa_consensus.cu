@@ -3,24 +3,23 @@
 // over spoa's partial-order graph (linear-gap NW, match/mismatch/gap from
 // racon's -m/-x/-g, engine built at src/polisher.cpp:181-185).
 //
-// Design (B200, sm_100a). One warp owns one window at a time; warps (4 per
-// CTA, 12 per SM) are persistent and pull windows from a size-sorted queue.
-// Each warp has a slot of global scratch (graph arrays first, then the DP
-// score rows and decision bit-planes) and a 16 KB shared-memory ring.
+// Design (B200, sm_100a). A team of one or four warps owns one window at a
+// time; teams are persistent and pull windows from a size-sorted queue. Each
+// team has a slot of global scratch (graph arrays first, then the DP score
+// rows) and shared memory (the DP's row rings, scratch for the graph steps).
 // * Per layer: the subgraph of a partial layer, row descriptors (first
 //   predecessor ranks, count, sink flag, base), the DP, the end cell, the
-//   traceback and the insertion of the aligned layer, all warp-cooperative.
+//   traceback and the insertion of the aligned layer.
 //   The steps that walk the graph build compact uint16 adjacency lists or
-//   accumulators in the shared ring when they fit, so their dependent steps
+//   accumulators in shared memory when they fit, so their dependent steps
 //   read shared memory; loads of graph arrays go out 128 entries at a time.
 // * The DP runs one row (graph node in a valid topological order kept
-//   incrementally) at a time: lane l owns S consecutive columns, recent rows
-//   sit in the ring, diagonal and vertical terms take the max over the
-//   predecessors (DPX add-max forms), and the in-row gap term H[i][j] =
-//   max(T[j], H[i][j-1] + g) is a max-plus prefix (in-lane sub-chains, warp
-//   scan). Decisions are two bit-planes per lane and row; the walk decides
-//   the rare remaining cells again from the stored scores, in spoa's order
-//   (diagonal through each predecessor, then vertical, then horizontal).
+//   incrementally) at a time, the team's warps side by side on strips of its
+//   columns (dp_strip), on slanted scores H - column * gap, so that the
+//   in-row gap term is a plain running maximum. It keeps no decisions: the
+//   walk back decides at the few hundred cells it visits from the stored
+//   scores, in spoa's order (diagonal through each predecessor, then
+//   vertical, then horizontal).
 // * The NW end cell is the first sink in spoa's topological order with the
 //   best last-column score; spoa's DFS order is built only when tied sinks
 //   belong to aligned groups.
@@ -64,11 +63,6 @@ namespace {
 
 // minus infinity that survives thousands of gap additions without overflow
 constexpr int kNegInf = -(1 << 29);
-// per-warp shared memory: the DP row ring, reused by the other steps
-constexpr int kRingBytesPerWarp = 16384;
-// node ranks held in the ring's shared memory during the descriptor build
-constexpr int kSmemRanks = (kRingBytesPerWarp - 512) / 4;
-
 enum PoaFlag : uint8_t {
     kPolished = 1,
     kChimeric = 2,
@@ -107,7 +101,7 @@ struct Graph {
     int* stack;
     int *pred_off, *pred_idx;
     int4* rowdesc;  // per DP row: first three predecessor ranks (or the list offset) | count, sink, base
-    int *aln_node, *aln_pos;
+    int* aln_node;  // per sequence position of the layer: node on its path, -1 for an inserted base
     long long* bscore;
     int* bpred;
     int* cons;
@@ -115,27 +109,14 @@ struct Graph {
     // its double buffer, per-rank shift counts and the new nodes of a layer
     int *ord, *ord2, *my_rank, *shift, *nw_node, *nw_slot;
     int* H;
-    uint8_t* dec;
     int* lastH;   // per DP row (sinks): score of the last column
     // per-node in-edge and aligned-entry counts, owner node of each aligned
     // entry (for the compact lists built in shared memory)
     int *in_cnt, *al_cnt, *a_owner, *out_cnt;
-    int ncap, ecap, acap, scap, lcap, alncap;
+    int ncap, ecap, acap, scap, lcap;
 };
 
 __host__ __device__ size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
-
-// Decision bytes are stored in tiles of 8 rows x 128 columns (1 KiB): a
-// warp still writes each row as whole 128-byte lines, and the traceback,
-// which walks up and left one cell at a time through nearby rows, stays
-// inside one tile for several steps. lc is a multiple of 128.
-__device__ __forceinline__ size_t dec_at(int i, int j, int lc) {
-    return size_t(i) * size_t(lc) + size_t(j);
-}
-
-// Decision bit-planes of dp_layer_fast: one uint2 per (row, lane), row-major
-// (each row is one coalesced 256-byte store).
-__device__ __forceinline__ size_t bits_at(int i, int lane) { return size_t(i) * 32u + size_t(lane); }
 
 // Row descriptor word w: predecessor count (17 bits) | sink << 17 | base << 24.
 __device__ __forceinline__ int desc_np(int w) { return w & 0x1FFFF; }
@@ -193,14 +174,12 @@ __host__ __device__ size_t walk_layout(int ncap, int ecap, int acap, int lcap, F
     take(N * 4, 43);       // out_cnt
     take((N + 2) * 4, 24); // pred_off
     take((E + N + 2) * 4, 25);  // pred_idx
-    take((N + L + 2) * 4, 26);  // aln_node
-    take((N + L + 2) * 4, 27);  // aln_pos
+    take((L + 2) * 4, 26);  // aln_node
     take(N * 8, 28);       // bscore
     take(N * 4, 29);       // bpred
     take(N * 4, 30);       // cons
     take(S * 4, 23);       // stack
     take((N + 1) * L * 4, 31);  // H
-    take(std::max(((N + 8) & ~size_t(7)) * L, (N + 1) * 256), 32);  // dec: bytes, or 32 uint2 per row
     take((N + 1) * 4, 44);      // lastH: last-column score of each sink row
     // whole 2 MiB pages per slot, so that a slot's graph arrays share one page
     off = (off + (size_t(2) << 20) - 1) & ~((size_t(2) << 20) - 1);
@@ -239,12 +218,10 @@ __device__ Graph make_graph(const PoaArgs& a, uint32_t slot) {
     g.pred_off = (int*)p[24];
     g.pred_idx = (int*)p[25];
     g.aln_node = (int*)p[26];
-    g.aln_pos = (int*)p[27];
     g.bscore = (long long*)p[28];
     g.bpred = (int*)p[29];
     g.cons = (int*)p[30];
     g.H = (int*)p[31];
-    g.dec = (uint8_t*)p[32];
     g.ord = (int*)p[33];
     g.ord2 = (int*)p[34];
     g.my_rank = (int*)p[35];
@@ -262,27 +239,22 @@ __device__ Graph make_graph(const PoaArgs& a, uint32_t slot) {
     g.acap = a.acap;
     g.scap = a.ncap + a.ecap + a.acap + 16;
     g.lcap = a.lcap;
-    g.alncap = a.ncap + a.lcap + 2;
     return g;
 }
 
-// Shared per-CTA state.
-// NW end cell of one layer: first sink row (in the DP order) with the best
-// last-column value, that value, and how many sinks share it.
-struct EndCell {
-    int row, value, ties;
-    int preds;  // predecessor links over the DP rows (edge-cells = |layer| x (rows + preds))
-    bool h16;   // the layer's score rows in global memory are int16
-};
-
+// Shared per-team state.
 struct PoaShared {
     int nnodes, nedges, naligned, nseq;
     int nnew;     // new nodes of the last insertion (g.nw_node / g.nw_slot)
     int nranks;   // entries of rank_to_node (full graph order)
-    int ndp;      // rows of the current DP
     int fail;     // 0 ok, else PoaFlag
-    int iend;     // DP rank of the NW end cell
-    int naln;
+    int ndp;      // rows of the current DP
+    int partial;  // the current layer is aligned to a subgraph
+    int end_value;  // score of the NW end cell of the current layer
+    int preds;    // predecessor links over the DP rows (edge-cells = |layer| x (rows + preds))
+    int scratch_bytes;  // the team's shared memory, scratch between the DPs
+    uint32_t next;      // queue position the team took
+    volatile int done[4];  // per warp: rows it has finished (counting on from pass to pass)
 };
 
 // ---------------- graph primitives (thread 0) ----------------
@@ -453,8 +425,7 @@ __device__ bool build_out_csr(const Graph& g, int N, int E, int lane, void* smem
 // Graph::add_alignment for one layer, by the whole warp. A path visits every
 // node and every aligned group at most once, so the per-position work is
 // independent: classify each aligned base (existing node, new base, new
-// member of an aligned group), number the new nodes in spoa's order (head
-// bases, tail bases, then new aligned bases along the path), then in
+// member of an aligned group), number the new nodes in path order, then in
 // parallel create nodes, aligned-group links, edges P[k-1] -> P[k] with
 // weight w[k-1] + w[k] (every sequence position k owns exactly one path node
 // P[k]) and coverage, and list the new nodes with their order slots (see
@@ -462,11 +433,11 @@ __device__ bool build_out_csr(const Graph& g, int N, int E, int lane, void* smem
 // | aligned-count << 2, [2m,3m) anchor slot, [3m,4m) group start.
 __device__ void add_alignment_warp(const Graph& g, PoaShared& sh, const uint8_t* seq, const uint8_t* qual,
                                    int len, int lane, int4* ring) {
-    const int m = sh.naln;
+    const int m = len;  // the walk gives every position a node or -1
     const int nold = sh.nnodes;
     if (len == 0) return;
-    if (m == 0 || 4 * m + 64 > g.scap) {
-        if (lane == 0) sh.fail = m == 0 ? kFailed : kOverflow;
+    if (4 * m + 64 > g.scap) {
+        if (lane == 0) sh.fail = kOverflow;
         __syncwarp();
         return;
     }
@@ -474,26 +445,23 @@ __device__ void add_alignment_warp(const Graph& g, PoaShared& sh, const uint8_t*
     int* e_kind = g.stack + m;
     int* e_slot = g.stack + 2 * m;
     int* e_start = g.stack + 3 * m;
-    const int first_pos = g.aln_pos[m - 1], last_pos = g.aln_pos[0];
-    const int h = first_pos, tl = len - 1 - last_pos;
     // existing-edge lookups of step 5 from shared memory when they fit
     OutCsr oc;
-    const bool ocsr = build_out_csr(g, nold, sh.nedges, lane, ring, kRingBytesPerWarp, oc);
+    const bool ocsr = build_out_csr(g, nold, sh.nedges, lane, ring, sh.scratch_bytes, oc);
     // 1. classify (reads only the graph as it was before this insertion);
     //    the loads of four 32-entry chunks go out together
     for (int t4 = 0; t4 < m; t4 += 128) {
-        int at[4], pos[4], cd[4], rk[4], ah[4];
+        int at[4], cd[4], rk[4], ah[4];
         uint8_t letter[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int t = t4 + 32 * u + lane;
-            at[u] = t < m ? g.aln_node[m - 1 - t] : -1;
-            pos[u] = t < m ? g.aln_pos[m - 1 - t] : 0;
+            at[u] = t < m ? g.aln_node[t] : -1;
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int t = t4 + 32 * u + lane;
-            letter[u] = t < m ? seq[pos[u]] : 0;
+            letter[u] = t < m ? seq[t] : 0;
             cd[u] = at[u] >= 0 ? g.code[at[u]] : -1;
             rk[u] = at[u] >= 0 ? g.my_rank[at[u]] : 0;
             ah[u] = at[u] >= 0 ? g.al_head[at[u]] : -1;
@@ -535,7 +503,7 @@ __device__ void add_alignment_warp(const Graph& g, PoaShared& sh, const uint8_t*
     }
     __syncwarp();
     // 2. ids of new aligned bases, aligned-pool offsets, order slots
-    const int base_id = nold + h + tl;
+    const int base_id = nold;
     int nnew_e = 0, nal_tot = 0, cur_slot = INT_MIN, first_start = INT_MAX;
     for (int c0 = 0; c0 < m; c0 += 32) {
         const int t = c0 + lane;
@@ -568,7 +536,7 @@ __device__ void add_alignment_warp(const Graph& g, PoaShared& sh, const uint8_t*
         nnew_e += tot;
         nal_tot += atot;
     }
-    const int nnew = h + tl + nnew_e;
+    const int nnew = nnew_e;
     if (nold + nnew > g.ncap || sh.nedges + len + 2 > g.ecap || sh.naligned + nal_tot > g.acap) {
         if (lane == 0) sh.fail = kOverflow;
         __syncwarp();
@@ -576,24 +544,10 @@ __device__ void add_alignment_warp(const Graph& g, PoaShared& sh, const uint8_t*
     }
     __syncwarp();
     // 3. new nodes
-    auto path_node = [&](int k) -> int {
-        if (k < first_pos) return nold + k;
-        if (k > last_pos) return nold + h + (k - last_pos - 1);
-        return e_nid[k - first_pos];
-    };
-    for (int x = lane; x < nnew; x += 32) {
-        int id, k;
-        if (x < h) {
-            id = nold + x;
-            k = x;
-        } else if (x < h + tl) {
-            id = nold + x;
-            k = last_pos + 1 + (x - h);
-        } else {
-            id = nold + x;
-            k = -1;
-        }
-        g.code[id] = k >= 0 ? seq[k] : 0;
+    for (int t = lane; t < m; t += 32) {
+        if ((e_kind[t] & 3) == 0) continue;
+        const int id = e_nid[t];
+        g.code[id] = seq[t];
         g.cov[id] = 0;
         g.in_head[id] = g.in_tail[id] = -1;
         g.out_head[id] = g.out_tail[id] = -1;
@@ -603,15 +557,11 @@ __device__ void add_alignment_warp(const Graph& g, PoaShared& sh, const uint8_t*
         g.out_cnt[id] = 0;
     }
     __syncwarp();
-    for (int t = lane; t < m; t += 32) {
-        if ((e_kind[t] & 3) != 0) g.code[e_nid[t]] = seq[first_pos + t];
-    }
-    __syncwarp();
     // 4. aligned groups: a new base joining the group of `at` links to every
     //    member, then to `at` (spoa's order)
     for (int t = lane; t < m; t += 32) {
         if ((e_kind[t] & 3) != 2) continue;
-        const int at = g.aln_node[m - 1 - t];
+        const int at = g.aln_node[t];
         const int G = e_nid[t];
         int slot = sh.naligned + e_start[t];
         auto link = [&](int v, int y) {
@@ -639,8 +589,8 @@ __device__ void add_alignment_warp(const Graph& g, PoaShared& sh, const uint8_t*
         const int k = c0 + lane;
         int u = -1, v = -1, w = 0, found = -1;
         if (k < len) {
-            u = path_node(k - 1);
-            v = path_node(k);
+            u = e_nid[k - 1];
+            v = e_nid[k];
             w = layer_weight(qual, k - 1) + layer_weight(qual, k);
             if (u < nold && v < nold) {
                 if (ocsr) {
@@ -686,25 +636,15 @@ __device__ void add_alignment_warp(const Graph& g, PoaShared& sh, const uint8_t*
     }
     // 6. coverage: every node of a path with at least two bases
     if (len >= 2)
-        for (int k = lane; k < len; k += 32) g.cov[path_node(k)] += 1;
+        for (int k = lane; k < len; k += 32) g.cov[e_nid[k]] += 1;
     // 7. new nodes with their order slots, in path order
     const int before = first_start == INT_MAX ? nold - 1 : first_start - 1;
-    const int last_slot = cur_slot == INT_MIN ? before : cur_slot;
-    for (int x = lane; x < h; x += 32) {
-        g.nw_node[x] = nold + x;
-        g.nw_slot[x] = before;
-    }
     for (int t = lane; t < m; t += 32) {
         if ((e_kind[t] & 3) == 0) continue;
         const int id = e_nid[t];
-        const int at = id - base_id;  // position among the new aligned bases
         const int sl = e_slot[t];
-        g.nw_node[h + at] = id;
-        g.nw_slot[h + at] = sl == INT_MIN ? before : sl;
-    }
-    for (int x = lane; x < tl; x += 32) {
-        g.nw_node[h + nnew_e + x] = nold + h + x;
-        g.nw_slot[h + nnew_e + x] = last_slot;
+        g.nw_node[id - base_id] = id;
+        g.nw_slot[id - base_id] = sl == INT_MIN ? before : sl;
     }
     __syncwarp();
     if (lane == 0) {
@@ -723,7 +663,7 @@ __device__ void add_alignment_warp(const Graph& g, PoaShared& sh, const uint8_t*
 __device__ void order_insert(const Graph& g, const PoaShared& sh, int nold, int lane, int4* ring) {
     const int nnew = sh.nnew, n = nold + nnew;
     // shift counts in shared memory when they fit (the ring is free here)
-    int* const shift = size_t(nold + 1) * 4 <= size_t(kRingBytesPerWarp) ? reinterpret_cast<int*>(ring) : g.shift;
+    int* const shift = size_t(nold + 1) * 4 <= size_t(sh.scratch_bytes) ? reinterpret_cast<int*>(ring) : g.shift;
     for (int r = lane; r <= nold; r += 32) shift[r] = 0;
     __syncwarp();
     for (int k = lane; k < nnew; k += 32) {
@@ -858,590 +798,633 @@ __device__ __forceinline__ int desc_pred(const Graph& g, const int4& d, int p) {
     return p == 0 ? d.x : (p == 1 ? d.y : d.z);
 }
 
-// ---------------- DP of one layer (one warp) ----------------
+// ---------------- DP of one layer (one team) ----------------
 
-// Columns covered by one warp pass: S cells per lane, S a multiple of 4.
-__host__ __device__ inline int seg_cells(int wc) {
-    const int s = (wc + 31) / 32;
-    return s <= 24 ? ((s + 3) & ~3) : 24;
+// the CTA's dynamic shared memory: WarpMem<NW>::bytes per warp, teams in order
+extern __shared__ int4 g_poa_smem[];
+
+// Shared memory of one warp of a team of NW: the ring of recent DP rows, the
+// staged controls and score words of 32 rows, and the final scores at the
+// right edge of the strip to its left. Between layers the whole team's
+// memory is scratch for the graph steps. One-warp teams run 12 warps to an
+// SM, four-warp teams 24.
+constexpr int kEdgeRows = 64;
+template <int NW>
+struct WarpMem {
+    static constexpr int ring_bytes = NW == 1 ? 17408 : 8064;
+    static constexpr int ctl = ring_bytes;          // uint32_t[32]
+    static constexpr int pool = ctl + 32 * 4;       // uint32_t[32]
+    static constexpr int edge = pool + 32 * 4 + 16; // int[kEdgeRows]
+    static constexpr int bytes = edge + kEdgeRows * 4;
+};
+// rows between two looks at the neighbouring warps' progress
+constexpr int kGroupRows = 8;
+// polls of a wait on another warp of the team (about a second) before the
+// window is given up as failed
+constexpr int kWaitPolls = 1 << 26;
+
+// Barrier of the NW warps of one team (hardware barrier team + 1).
+template <int NW>
+__device__ __forceinline__ void team_sync(int team) {
+    if (NW == 1) {
+        __syncwarp();
+    } else {
+        asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(32 * NW) : "memory");
+    }
 }
-__host__ __device__ inline int row_cover(int wc) {
-    const int s = seg_cells(wc);
-    const int ch = 32 * s;
+
+// Cells per lane for rows of wc columns: the team's NW strips of 32 * S
+// columns cover the row in one pass where that fits in registers (768
+// columns for one warp, 1024 for four), else in passes of the
+// largest S.
+__host__ __device__ inline int seg_cells(int nw, int wc) {
+    if (nw == 4) return wc <= 256 ? 2 : wc <= 512 ? 4 : wc <= 768 ? 6 : 8;
+    return wc <= 256 ? 8 : wc <= 512 ? 16 : 24;
+}
+// Row stride of the score rows: whole passes.
+__host__ __device__ inline int row_cover(int nw, int wc) {
+    const int ch = 32 * nw * seg_cells(nw, wc);
     return ((wc + ch - 1) / ch) * ch;
 }
 
-constexpr uint32_t kNoPred = 0xFFu;
-constexpr uint32_t kEscape = 63u;  // predecessor index >= 63: decide again in the walk
-
-// DP of one layer against rows order[0..ndp) (ranks 1..ndp; rank 0 = empty
-// prefix row). Lane l owns columns [c + l*S, c + l*S + S) of each chunk c of
-// 32*S columns. Per cell it keeps T = max over predecessors of the diagonal
-// and vertical terms, the first predecessor giving T diagonally and the first
-// giving it vertically; the horizontal term is a max-plus scan: in-lane
-// prefix, then a warp shuffle scan of lane aggregates. Decision byte: p
-// (diagonal via predecessor p), 64 + p (vertical), 128 (horizontal), 255
-// (predecessor index >= 63). Returns the rank of the NW end cell (first sink
-// in rank order with the best last-column value).
-template <int S>
-__device__ EndCell dp_layer(const PoaArgs& a, const Graph& g, const int* order, int ndp, const uint8_t* seq, int L,
-                        int lane) {
-    static_assert(S % 4 == 0 && S >= 4 && S <= 32, "segment");
-    constexpr unsigned kFull = 0xffffffffu;
-    const int lc = g.lcap;
-    int* const Hm = g.H;
-    uint8_t* const Dm = g.dec;
-    const int wc = L + 1;
-    const int ch = 32 * S;
-    const int nch = (wc + ch - 1) / ch;
-    const int gap = a.gap, mt = a.match, mm = a.mismatch;
-    // virtual row 0: j * gap
-    for (int j = lane; j < nch * ch; j += 32) Hm[j] = j * gap;
-    __syncwarp();
-    const int lane_l = (L % ch) / S, k_l = L % S, ch_l = L / ch;
-    int best_v = kNegInf, best_r = INT_MAX, ties = 0, npreds = 0;
-    for (int i = 1; i <= ndp; ++i) {
-        const int4 d = g.rowdesc[i - 1];
-        const uint32_t cmask = desc_base(d.w) * 0x01010101u;
-        const int np = desc_np(d.w);
-        npreds += np;
-        const int cnt = np == 0 ? 1 : np;
-        const bool is_sink = desc_sink(d.w);
-        int carry_in = kNegInf;  // final H of the last column of the previous chunk
-        for (int c = 0; c < nch; ++c) {
-            const int j0 = c * ch + lane * S;
-            // sequence chars of columns j0 .. j0+S-1 (column j compares seq[j-1])
-            uint32_t eq[S / 4];
-#pragma unroll
-            for (int q = 0; q < S / 4; ++q) {
-                uint32_t w = 0;
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const int j = j0 + 4 * q + b;
-                    const uint32_t ch8 = (j >= 1 && j <= L) ? uint32_t(seq[j - 1]) : 0u;
-                    w |= ch8 << (8 * b);
-                }
-                eq[q] = __vcmpeq4(w, cmask);
-            }
-            int T[S];
-            uint32_t code[S];
-#pragma unroll
-            for (int k = 0; k < S; ++k) {
-                T[k] = kNegInf;
-                code[k] = 0xFFFFu;
-            }
-            for (int p = 0; p < cnt; ++p) {
-                const int r = desc_pred(g, d, p);
-                const int4* hp4 = reinterpret_cast<const int4*>(Hm + r * lc + j0);
-                int hv[S];
-#pragma unroll
-                for (int q = 0; q < S / 4; ++q) {
-                    const int4 t4 = hp4[q];
-                    hv[4 * q] = t4.x;
-                    hv[4 * q + 1] = t4.y;
-                    hv[4 * q + 2] = t4.z;
-                    hv[4 * q + 3] = t4.w;
-                }
-                int left = __shfl_up_sync(kFull, hv[S - 1], 1);
-                if (lane == 0) left = j0 > 0 ? Hm[r * lc + j0 - 1] : kNegInf;
-                const uint32_t pc = p < int(kEscape) ? uint32_t(p) : kEscape;
-#pragma unroll
-                for (int k = 0; k < S; ++k) {
-                    const int prev = k == 0 ? left : hv[k - 1];
-                    const bool same = (eq[k / 4] >> (8 * (k % 4))) & 1u;
-                    const int dg = prev <= kNegInf / 2 ? kNegInf : prev + (same ? mt : mm);
-                    const int vt = hv[k] + gap;
-                    const int mx = max(dg, vt);
-                    if (mx > T[k]) {
-                        T[k] = mx;
-                        code[k] = (dg == mx ? pc : kNoPred) | ((vt == mx ? pc : kNoPred) << 8);
-                    } else if (mx == T[k]) {
-                        if ((code[k] & 0xFFu) == kNoPred && dg == mx) code[k] = (code[k] & 0xFF00u) | pc;
-                        if ((code[k] >> 8) == kNoPred && vt == mx) code[k] = (code[k] & 0xFFu) | (pc << 8);
-                    }
-                }
-            }
-            // horizontal term: in-lane prefix, warp scan of lane aggregates
-            int hk[S];
-            int run = kNegInf;
-#pragma unroll
-            for (int k = 0; k < S; ++k) {
-                run = max(T[k], run <= kNegInf / 2 ? kNegInf : run + gap);
-                hk[k] = run;
-            }
-            int x = run;
-            if (lane == 0 && carry_in > kNegInf / 2) x = max(x, carry_in + S * gap);
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(kFull, x, o);
-                if (lane >= o && y > kNegInf / 2) x = max(x, y + o * S * gap);
-            }
-            int carry = __shfl_up_sync(kFull, x, 1);
-            if (lane == 0) carry = carry_in;
-            int hrow[S];
-            uint32_t dec4[S / 4];
-#pragma unroll
-            for (int q = 0; q < S / 4; ++q) dec4[q] = 0;
-#pragma unroll
-            for (int k = 0; k < S; ++k) {
-                const int cin = carry <= kNegInf / 2 ? kNegInf : carry + (k + 1) * gap;
-                const int h = max(hk[k], cin);
-                hrow[k] = h;
-                uint32_t d;
-                if (h > T[k]) {
-                    d = 128u;
-                } else if ((code[k] & 0xFFu) != kNoPred) {
-                    d = code[k] & 0xFFu;
-                    if (d == kEscape) d = 255u;
-                } else {
-                    d = (code[k] >> 8);
-                    d = d == kEscape ? 255u : 64u + d;
-                }
-                dec4[k / 4] |= d << (8 * (k % 4));
-            }
-            int4* out4 = reinterpret_cast<int4*>(Hm + i * lc + j0);
-#pragma unroll
-            for (int q = 0; q < S / 4; ++q)
-                out4[q] = make_int4(hrow[4 * q], hrow[4 * q + 1], hrow[4 * q + 2], hrow[4 * q + 3]);
-#pragma unroll
-            for (int q = 0; q < S / 4; ++q) *reinterpret_cast<uint32_t*>(Dm + dec_at(i, j0 + 4 * q, lc)) = dec4[q];
-            if (c == ch_l && lane == lane_l && is_sink) {
-                int val = kNegInf;
-#pragma unroll
-                for (int k = 0; k < S; ++k)
-                    if (k == k_l) val = hrow[k];
-                g.lastH[i] = val;
-                if (val > best_v) {
-                    best_v = val;
-                    best_r = i;
-                    ties = 1;
-                } else if (val == best_v) {
-                    ++ties;
-                }
-            }
-            carry_in = __shfl_sync(kFull, hrow[S - 1], 31);
-        }
-        __syncwarp();
-    }
-    // the owner lane of column L holds the end cell (int32 score rows)
-    return EndCell{__shfl_sync(kFull, best_r, lane_l), __shfl_sync(kFull, best_v, lane_l),
-                   __shfl_sync(kFull, ties, lane_l), npreds, false};
+// Scores are kept slanted: H'[i][j] = H[i][j] - j * gap. A gap along the row
+// is then free (H'[i][j] = max(T'[i][j], H'[i][j-1])), so the in-row term is
+// a plain running maximum, the diagonal step adds s - gap, the vertical step
+// gap, and the empty prefix row is 0. Cells of one column compare as before.
+//
+// The fast form of a layer's DP stores int16 rows and permutes bytes for the
+// substitution scores. It needs a gap not above 0, s - gap in a signed
+// byte, bases A, C, G, T only, and slanted scores that provably fit: H lies
+// between gap x (row + column) (the all-gap path, which the maximum
+// includes) and max(match, 0) x column, so H' lies between gap x row and
+// (max(match, 0) - gap) x column. Other layers take the general form: int32
+// rows, characters compared. The DP is int32 in registers and in the ring
+// either way.
+__device__ __forceinline__ bool fast_scores(int mt, int mm, int gap, int ndp, int L) {
+    return gap <= 0 && max(mt, mm) - gap <= 127 && min(mt, mm) - gap >= -128 &&
+           (long long)ndp * (long long)(-gap) <= 32767 &&
+           ((long long)max(mt, 0) - gap) * (long long)L <= 32767;
 }
-
-// Score rows in global memory (read back for rows beyond the ring and by
-// the walk's re-decisions) are int16 for a layer whose scores provably fit:
-// every score lies between gap x (rows + columns) (the all-gap path, which
-// the maximum includes) and max(match, 0) x columns, so with
-// (ndp + L) x |gap| <= 32767 and max(match, 0) x L <= 32767 no score leaves
-// [-32767, 32767]. Other layers are promoted to int32 rows. Stores saturate,
-// so minus infinity (kNegInf and what is derived from it) becomes -32768,
-// which no score reaches and which reads back as kNegInf. The DP itself
-// stays int32 in registers and in the ring.
-__device__ __forceinline__ bool layer_fits_s16(const PoaArgs& a, int ndp, int L) {
-    return a.gap <= 0 && (long long)(ndp + L) * (long long)(-a.gap) <= 32767 &&
-           (long long)max(int(a.match), 0) * (long long)L <= 32767;
+__device__ __forceinline__ bool acgt_base(uint32_t c) {
+    return ((0x47544341u >> (8 * ((c >> 1) & 3u))) & 0xFFu) == c;
 }
-// two scores in one word, lo in bits 0..15 and hi in bits 16..31, saturated
+// two scores in one word, lo in bits 0..15 and hi in bits 16..31
+// (saturated: only columns past the layer's end can exceed 16 bits)
 __device__ __forceinline__ uint32_t pack_s16(int lo, int hi) {
     uint32_t d;
     asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(d) : "r"(hi), "r"(lo));
     return d;
 }
-__device__ __forceinline__ int s16_score(int v) { return v == -32768 ? kNegInf : v; }
-__device__ __forceinline__ int unpack_lo(uint32_t w) { return s16_score(int(w << 16) >> 16); }
-__device__ __forceinline__ int unpack_hi(uint32_t w) { return s16_score(int(w) >> 16); }
-// score (row r, column j) as the layer stored it
-__device__ __forceinline__ int h_at(const Graph& g, int r, int j, bool h16) {
-    if (h16) return s16_score(reinterpret_cast<const int16_t*>(g.H)[r * g.lcap + j]);
-    return g.H[r * g.lcap + j];
+__device__ __forceinline__ int unpack_lo(uint32_t w) { return int(w << 16) >> 16; }
+__device__ __forceinline__ int unpack_hi(uint32_t w) { return int(w) >> 16; }
+// slanted score (row r, column j) as the layer stored it, rows of lc columns
+template <bool FAST>
+__device__ __forceinline__ int h_at(const uint8_t* Hb, int r, int j, int lc) {
+    if (FAST) return reinterpret_cast<const int16_t*>(Hb)[size_t(r) * lc + j];
+    return reinterpret_cast<const int*>(Hb)[size_t(r) * lc + j];
 }
 
-// last 512 bytes of each warp's ring hold the 32-row descriptor block
-constexpr int kRingDescOffset = (kRingBytesPerWarp - 512) / 16;
+// Byte `sel & 7` (per nibble) of lo, sign extended by the nibble's top bit.
+__device__ __forceinline__ int prmt_score(uint32_t lo, uint32_t sel) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(lo), "r"(0u), "r"(sel));
+    return int(d);
+}
 
-// Single-pass form of dp_layer for rows of at most 32*S columns. A lane only
-// ever reads its own column segment of earlier rows (the left neighbour
-// comes by shuffle), so rows are served without any cross-lane memory
-// ordering: the last R rows sit in a shared-memory ring laid out
-// [row][S/4][lane] (conflict-free int4), older rows come from global memory.
-// Row descriptors are prefetched 32 rows at a time.
-// Per cell: T = max over predecessors of the diagonal (H[p][j-1] + s) and
-// vertical (H[p][j] + g) terms, with the DPX forms max(a + b, c) and
-// max-with-predicate doing the add/max pairs; the horizontal term is a
-// max-plus scan (in-lane prefix as 4 independent sub-chains, warp scan of the
-// lane aggregates, one fix-up per cell). Decisions are two bit-planes per lane
-// and row (one uint2): bit k of .x = horizontal (h > T), bit k of .y = the
-// diagonal through predecessor 0 gives T (spoa tests it first). The walk
-// reads the rest from the row's predecessor count: a single predecessor
-// makes every other cell vertical through it; with several it decides again
-// from H. Requires match >= mismatch and match - mismatch <= 255.
-template <int S, bool H16>
-__device__ EndCell dp_layer_fast(const PoaArgs& a, const Graph& g, const int* order, int ndp, const uint8_t* seq, int L,
-                             int lane, int4* ring) {
-    static_assert(S % 4 == 0 && S >= 4 && S <= 24, "segment");
+// Scores of one row against the four bases as signed bytes, at the base's
+// index (c >> 1) & 3 (A, C, T, G): match at the row's own base.
+__device__ __forceinline__ uint32_t score_pool(uint32_t base, uint32_t mm4, uint32_t flip) {
+    return acgt_base(base) ? mm4 ^ (flip << (8 * ((base >> 1) & 3u))) : mm4;
+}
+
+// DP of one layer against its rows (ranks 1..ndp; rank 0 = empty prefix
+// row), by a team of NW warps. The columns are cut into strips of 32 * S,
+// one per warp (rows longer than a pass take several); lane l owns S
+// consecutive columns of its warp's strip. Each warp goes down the rows on
+// its own, a few rows behind the warp to its left: the only thing it needs
+// from there is each row's final score at the strips' edge, which the left
+// warp leaves in a shared ring, publishing its progress every kGroupRows
+// rows. A row is a chain of dependent steps, and its fixed work
+// (control, in-row scan, stores) is as large as its cells' work: one warp
+// over all columns spends the fewest instructions, several side by side
+// finish a window sooner.
+//
+// The last R rows sit in a shared-memory ring, [unit][lane] and then the
+// score left of each lane's segment (conflict-free, and no lane reads
+// another's words); older rows come from global memory. On this chip a vote
+// with a branch on it costs about 75 cycles, a shuffle 33, so the row is kept
+// nearly free of branches. What a row needs besides its scores is
+// worked out 32 rows at a time, one row per lane: a score word, and a control
+// word with the ring slots of up to 7 predecessors besides the row just
+// computed, which is still in registers. The control goes through a warp
+// reduction, so that branches on it are uniform.
+//
+// Per cell: the elementwise maximum M over the predecessor rows, then
+// T = max(M[j-1] + s - gap, M[j] + gap) (the substitution score comes from one
+// byte permute of the row's four scores), then the running maximum along the
+// row: maxima of groups of cells, a warp scan of the lanes' maxima, and one
+// chain per group from what lies left of it. No decisions are kept: the walk
+// visits a few cells of each row and decides there from the scores, which
+// are stored anyway.
+constexpr unsigned kCtlChain = 8, kCtlSlow = 7;  // control: count (7 = general way) | chain | 7 slot nibbles
+template <int S, int NW, bool FAST, bool LEFT>
+__device__ __noinline__ void dp_strip(const Graph& g, PoaShared& sh, int ndp_, const uint8_t* seq, int L, int mt,
+                                      int mm, int gap, int lane, int w, int team, int pass) {
+    static_assert(S % 2 == 0 && S >= 2 && S <= 24, "segment");
     constexpr unsigned kFull = 0xffffffffu;
-    constexpr int Q = S / 4;
-    constexpr int R = (kRingBytesPerWarp - 512) / (S * 128);
+    using Mem = WarpMem<NW>;
+    constexpr int U = S % 4 == 0 ? 4 : 2;  // cells per ring unit
+    constexpr int Q = S / U;
+    constexpr int RB = S * 128 + 128;      // bytes per ring row
+    constexpr int R = Mem::ring_bytes / RB < 15 ? Mem::ring_bytes / RB : 15;
     static_assert(R >= 2, "ring");
-    const int lc = g.lcap;
-    int* const Hm = g.H;
-    uint2* const D2 = reinterpret_cast<uint2*>(g.dec);
-    const int* const pred_idx = g.pred_idx;
-    const int gap = a.gap, mm = a.mismatch;
-    const uint32_t diff4 = uint32_t(a.match - a.mismatch) * 0x01010101u;
-    const int j0 = lane * S;
-    uint32_t sc[Q];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        uint32_t w = 0;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int j = j0 + 4 * q + b;
-            w |= ((j >= 1 && j <= L) ? uint32_t(seq[j - 1]) : 0u) << (8 * b);
-        }
-        sc[q] = w;
-    }
-    int16_t* const Hs = reinterpret_cast<int16_t*>(g.H);  // the same rows as int16 (H16)
-    // row 0 (empty graph prefix) in global memory for the traceback
+    constexpr int W = 32 * S;
+    constexpr int HB = FAST ? 2 : 4;       // bytes per stored score
+    // uniform registers, by way of warp votes and reductions
+    const int ndp = __reduce_max_sync(kFull, ndp_);
+    const int lc = row_cover(NW, L + 1);
+    const int strip = pass * NW + w;
+    const int tag0 = pass * (ndp + 1);
+    const int c0 = strip * W;
+    const int j0 = c0 + lane * S;
+    uint8_t* const Hb = reinterpret_cast<uint8_t*>(g.H);
+    const int4* const rowdesc = g.rowdesc;
+    uint8_t* const mine = reinterpret_cast<uint8_t*>(g_poa_smem) + (team * NW + w) * Mem::bytes;
+    uint8_t* const ring = mine + lane * (U * 4);              // the lane's first unit of row 0
+    uint8_t* const ring_left = mine + S * 128 + lane * 4;
+    uint32_t* const cblk = reinterpret_cast<uint32_t*>(mine + Mem::ctl);
+    uint32_t* const pblk = reinterpret_cast<uint32_t*>(mine + Mem::pool);
+    volatile int* const ein = reinterpret_cast<volatile int*>(mine + Mem::edge);
+    // another warp takes this strip's edge, from the last lane
+    const bool feeds = __any_sync(kFull, w + 1 < NW && c0 + W <= L);
+    const bool waits = __any_sync(kFull, LEFT && w > 0);
+    const bool feed_lane = feeds && lane == 31;
+    const int dmt = mt - gap, dmm = mm - gap;
+    const uint32_t mm4 = uint32_t(uint8_t(dmm)) * 0x01010101u;
+    const uint32_t flip = uint32_t(uint8_t(dmt)) ^ uint32_t(uint8_t(dmm));
+    // per cell: the permute selector of its base, or its character
+    uint32_t sel[S];
 #pragma unroll
     for (int k = 0; k < S; ++k) {
-        if (H16) {
-            Hs[j0 + k] = int16_t((j0 + k) * gap);
+        const int j = j0 + k;
+        const uint32_t c = (j >= 1 && j <= L) ? uint32_t(seq[j - 1]) : 0u;
+        sel[k] = FAST ? ((c >> 1) & 3u) * 0x1111u + 0x8880u : c;
+    }
+    // row 0 (empty graph prefix) in global memory for the walk
+#pragma unroll
+    for (int k = 0; k < S; ++k) {
+        if (FAST) {
+            reinterpret_cast<int16_t*>(Hb)[j0 + k] = 0;
         } else {
-            Hm[j0 + k] = (j0 + k) * gap;
+            reinterpret_cast<int*>(Hb)[j0 + k] = 0;
         }
     }
-    const int lane_l = L / S, k_l = L % S;
-    int best_v = kNegInf, best_r = INT_MAX, ties = 0, npreds = 0;
-    int4* const dblk = ring + kRingDescOffset;
-    const int4* const rowdesc = g.rowdesc;
+    // score rows, at the lane's segment of the row being computed
+    uint8_t* hrow = Hb + (size_t(lc) + j0) * HB;
+    const size_t hstep = size_t(lc) * HB;
     int4 pre = lane < ndp ? rowdesc[lane] : make_int4(0, 0, 0, 0);
     // hv holds the previous row's final scores between iterations (row 0
-    // first), and left_prev that row's score left of the lane's segment: a
-    // row whose first predecessor is the row just computed (the common
-    // chain) reads both from registers instead of the ring and a shuffle
+    // first), and left that row's score left of the lane's segment
     int hv[S];
 #pragma unroll
-    for (int k = 0; k < S; ++k) hv[k] = (j0 + k) * gap;
-    int left_prev = lane == 0 ? kNegInf : (j0 - 1) * gap;
-    // the next row's descriptor is read while this row's scan and stores
-    // are in flight (from the staged block, or from `pre` at a block edge)
-    int4 dnext = make_int4(__shfl_sync(kFull, pre.x, 0), __shfl_sync(kFull, pre.y, 0),
-                           __shfl_sync(kFull, pre.z, 0), __shfl_sync(kFull, pre.w, 0));
-    for (int i = 1; i <= ndp; ++i) {
-        const int bi = (i - 1) & 31;
-        if (bi == 0) {
-            __syncwarp();
-            dblk[lane] = pre;
-            __syncwarp();
-            const int nx = i - 1 + 32 + lane;
-            pre = nx < ndp ? rowdesc[nx] : make_int4(0, 0, 0, 0);
-        }
-        const int4 d = dnext;
-        const int np = desc_np(d.w);
-        npreds += np;
-        const bool is_sink = desc_sink(d.w);
-        const uint32_t cmask = desc_base(d.w) * 0x01010101u;
-        const int p0 = np > 3 ? d.y : d.x;
-        // per cell: match - mismatch where the base matches, else 0 (bytes)
-        uint32_t sw[Q];
-#pragma unroll
-        for (int q = 0; q < Q; ++q) sw[q] = __vcmpeq4(sc[q], cmask) & diff4;
-        int T[S];
-        uint32_t dbit = 0;
-        // row r's scores of the lane's segment into dst
-        auto load_row = [&](int r, int (&dst)[S]) {
-            if (r == 0) {
-#pragma unroll
-                for (int k = 0; k < S; ++k) dst[k] = (j0 + k) * gap;
-            } else if (i - r <= R) {
-                // separate shared and global paths (warp-uniform branch), so
-                // the ring is read with shared-memory loads, not generic ones
-                const int4* src = ring + (r % R) * Q * 32 + lane;
-#pragma unroll
-                for (int q = 0; q < Q; ++q) {
-                    const int4 t4 = src[q * 32];
-                    dst[4 * q] = t4.x;
-                    dst[4 * q + 1] = t4.y;
-                    dst[4 * q + 2] = t4.z;
-                    dst[4 * q + 3] = t4.w;
-                }
-            } else if (H16) {
-                const uint2* src = reinterpret_cast<const uint2*>(Hs + r * lc + j0);
-#pragma unroll
-                for (int q = 0; q < Q; ++q) {
-                    const uint2 t2 = src[q];
-                    dst[4 * q] = unpack_lo(t2.x);
-                    dst[4 * q + 1] = unpack_hi(t2.x);
-                    dst[4 * q + 2] = unpack_lo(t2.y);
-                    dst[4 * q + 3] = unpack_hi(t2.y);
-                }
-            } else {
-                const int4* src = reinterpret_cast<const int4*>(Hm + r * lc + j0);
-#pragma unroll
-                for (int q = 0; q < Q; ++q) {
-                    const int4 t4 = src[q];
-                    dst[4 * q] = t4.x;
-                    dst[4 * q + 1] = t4.y;
-                    dst[4 * q + 2] = t4.z;
-                    dst[4 * q + 3] = t4.w;
-                }
-            }
-        };
-        auto sbyte = [&](int k) -> int { return int((sw[k >> 2] >> (8 * (k & 3))) & 0xFFu); };
+    for (int k = 0; k < S; ++k) hv[k] = 0;
+    int left = j0 == 0 ? kNegInf : 0;
+    int wofs = RB;  // ring offset of the row being computed: (row % R) * RB, R >= 2
+    for (int i0 = 0; i0 < ndp; i0 += 32) {
+        __syncwarp();
         {
-            const int r0 = np == 0 ? 0 : p0;
-            int left = left_prev;
-            if (r0 != i - 1) {
-                load_row(r0, hv);
-                left = __shfl_up_sync(kFull, hv[S - 1], 1);
-                if (lane == 0) left = kNegInf;
-            }
-            // Several predecessors: the maximum over them of the diagonal
-            // (H[p][j-1] + s) and vertical (H[p][j] + g) terms is the
-            // diagonal and vertical term of their elementwise maximum row M,
-            // so each further row costs one max per cell. hv and left become
-            // M; p0m / p0left mark the columns where the first predecessor
-            // holds M, which is where its diagonal can give T.
-            uint32_t p0m = ~0u;
-            bool p0left = true;
-            for (int p = 1; p < np; ++p) {
-                load_row(np > 3 ? pred_idx[d.x + p] : (p == 1 ? d.y : d.z), T);
-                int lft = __shfl_up_sync(kFull, T[S - 1], 1);
-                if (lane == 0) lft = kNegInf;
-                uint32_t lq[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-                for (int k = 0; k < S; ++k) {
-                    bool keep;
-                    hv[k] = __vibmax_s32(hv[k], T[k], &keep);
-                    lq[k & 3] |= uint32_t(!keep) << k;
+            // controls of rows i0 + 1 .. i0 + 32, one per lane
+            const int r = i0 + 1 + lane;
+            const int np = desc_np(pre.w);
+            uint32_t ctl = 0, n = 0;
+            bool slow = np > 8 || (np == 0 && r > 1);
+            if (np == 0) ctl = kCtlChain;
+            if (!slow)
+                for (int q = 0; q < np; ++q) {
+                    const int p = np > 3 ? (q == 0 ? pre.y : g.pred_idx[pre.x + q]) : q == 0 ? pre.x : q == 1 ? pre.y : pre.z;
+                    if (p == r - 1) {
+                        ctl |= kCtlChain;
+                    } else {
+                        slow |= r - p > R || n == 6;
+                        ctl |= n < 6 ? uint32_t(p % R) << (4 + 4 * n) : 0u;
+                        ++n;
+                    }
                 }
-                bool keepl;
-                left = __vibmax_s32(left, lft, &keepl);
-                p0left = p0left && keepl;
-                p0m &= ~((lq[0] | lq[1]) | (lq[2] | lq[3]));
-            }
-            // T = max(M[j-1] + s, M[j] + g); the diagonal of predecessor 0
-            // gives T where it holds M[j-1] and the diagonal is not below the
-            // vertical. Decision bits gathered in four independent words.
-            uint32_t dq[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-            for (int k = 0; k < S; ++k) {
-                const int pv = k == 0 ? left : hv[k - 1];
-                const int dg = pv + mm + sbyte(k);
-                bool dge;
-                T[k] = __vibmax_s32(dg, hv[k] + gap, &dge);
-                dq[k & 3] |= uint32_t(dge) << k;
-            }
-            dbit = ((dq[0] | dq[1]) | (dq[2] | dq[3])) & ((p0m << 1) | (p0left ? 1u : 0u));
-        }
-        // horizontal term
-        constexpr int C = S / 4;  // cells per sub-chain
-        int agg[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            int run = T[c * C];
-            hv[c * C] = run;
-#pragma unroll
-            for (int k = c * C + 1; k < (c + 1) * C; ++k) {
-                run = __viaddmax_s32(run, gap, T[k]);
-                hv[k] = run;
-            }
-            agg[c] = run;
-        }
-        int x = agg[0];
-#pragma unroll
-        for (int c = 1; c < 4; ++c) x = __viaddmax_s32(x, C * gap, agg[c]);
-        // max-plus prefix of the lane aggregates (penalty S * gap per lane),
-        // rounds of offset 1, 2, 4, 8, 16, stopping at the first round in
-        // which no lane changes: with a uniform penalty per lane, a round of
-        // offset o that changes nothing means x_(l-o) + o S gap <= x_l for
-        // every l, so x_(l-2o) + 2o S gap <= x_(l-o) + o S gap <= x_l and no
-        // later round can change anything either. Horizontal runs rarely
-        // cross a whole lane segment, so most rows stop after one round; a
-        // run across many lanes takes at most five.
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int y = __shfl_up_sync(kFull, x, o);
-            if (lane < o) y = kNegInf;
-            const int nx = __viaddmax_s32(y, o * S * gap, x);
-            const bool changed = nx != x;
-            x = nx;
-            if (!__any_sync(kFull, changed)) break;
-        }
-        int cin = __shfl_up_sync(kFull, x, 1);  // final value left of the segment
-        if (lane == 0) cin = kNegInf;
-        left_prev = cin;
-        if (i < ndp) {
-            const int bn = i & 31;  // slot of row i + 1 in the staged block
-            if (bn == 0) {
-                dnext = make_int4(__shfl_sync(kFull, pre.x, 0), __shfl_sync(kFull, pre.y, 0),
-                                  __shfl_sync(kFull, pre.z, 0), __shfl_sync(kFull, pre.w, 0));
-            } else {
-                dnext = dblk[bn];
+            cblk[lane] = slow ? kCtlSlow : ctl | n;
+            pblk[lane] = FAST ? score_pool(desc_base(pre.w), mm4, flip) : desc_base(pre.w);
+            if (LEFT && w == 0 && r <= ndp) {
+                // the first strip of a later pass: the edge of the strip
+                // to its left is in the score rows of the pass before
+                ein[(r - 1) & (kEdgeRows - 1)] = h_at<FAST>(Hb, r, c0 - 1, lc);
             }
         }
-        uint32_t hq[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int next = __viaddmax_s32(cin, C * gap, agg[c]);
-#pragma unroll
-            for (int k = c * C; k < (c + 1) * C; ++k) {
-                hv[k] = __viaddmax_s32(cin, (k - c * C + 1) * gap, hv[k]);
-                hq[k & 3] |= uint32_t(hv[k] > T[k]) << k;
+        __syncwarp();
+        const int nx = i0 + 32 + lane;
+        pre = nx < ndp ? rowdesc[nx] : make_int4(0, 0, 0, 0);
+        const int cnt = min(32, ndp - i0);
+        volatile int* const ein_b = ein + (i0 & (kEdgeRows - 1));
+        unsigned cnext = __reduce_or_sync(kFull, cblk[0]);
+        uint32_t pnext = pblk[0];
+        for (int b0 = 0; b0 < cnt; b0 += kGroupRows) {
+        const int bend = min(b0 + kGroupRows, cnt);
+        if (NW > 1) {
+            // the left neighbour is past these rows; the right one is at
+            // most the edge ring behind
+            if (waits) {
+                for (int polls = 0; __any_sync(kFull, sh.done[w - 1] < tag0 + i0 + bend); ++polls)
+                    if (polls > kWaitPolls) {
+                        sh.fail = kFailed;
+                        break;
+                    }
+                __threadfence_block();
             }
-            cin = next;
+            if (feeds) {
+                for (int polls = 0; __any_sync(kFull, sh.done[w + 1] < tag0 + i0 + bend - kEdgeRows); ++polls)
+                    if (polls > kWaitPolls) {
+                        sh.fail = kFailed;
+                        break;
+                    }
+            }
         }
-        const uint32_t hbit = (hq[0] | hq[1]) | (hq[2] | hq[3]);
-        int4* dst_g = reinterpret_cast<int4*>(Hm + i * lc + j0);
-        uint2* dst_s = reinterpret_cast<uint2*>(Hs + i * lc + j0);
-        int4* dst_r = ring + (i % R) * Q * 32 + lane;
+#pragma unroll 1
+        for (int b = b0; b < bend; ++b) {
+            unsigned ctl = cnext;
+            const uint32_t pool = pnext;
+            // next row's (one past the block at its end: unused)
+            cnext = __reduce_or_sync(kFull, cblk[b + 1]);
+            pnext = pblk[b + 1];
+            int bx = kNegInf;  // final score of this row left of the strip, at lane 0
+            if (LEFT) {
+                const int e = ein_b[b];
+                bx = lane == 0 ? e : kNegInf;
+            }
+            if ((ctl & 15u) != kCtlChain) {
+                // ring row at byte offset o; returns its score left of the segment
+                auto ring_row = [&](int o, int (&dst)[S]) -> int {
 #pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            const int4 v4 = make_int4(hv[4 * q], hv[4 * q + 1], hv[4 * q + 2], hv[4 * q + 3]);
+                    for (int q = 0; q < Q; ++q) {
+                        if constexpr (U == 4) {
+                            const int4 t = *reinterpret_cast<const int4*>(ring + o + q * 512);
+                            dst[4 * q] = t.x;
+                            dst[4 * q + 1] = t.y;
+                            dst[4 * q + 2] = t.z;
+                            dst[4 * q + 3] = t.w;
+                        } else {
+                            const int2 t = *reinterpret_cast<const int2*>(ring + o + q * 256);
+                            dst[2 * q] = t.x;
+                            dst[2 * q + 1] = t.y;
+                        }
+                    }
+                    return *reinterpret_cast<const int*>(ring_left + o);
+                };
+                int t[S];
+                auto merge = [&](int lft) {
+#pragma unroll
+                    for (int k = 0; k < S; ++k) hv[k] = max(hv[k], t[k]);
+                    left = max(left, lft);
+                };
+                if ((ctl & 7u) != kCtlSlow) {
+                    if (!(ctl & kCtlChain)) {
+                        // the row just computed is no predecessor: start from the first
+                        left = ring_row(((ctl >> 4) & 15u) * RB, hv);
+                        ctl = ((ctl >> 4) & ~15u) | ((ctl & 7u) - 1u);
+                    }
+#pragma unroll 1
+                    for (unsigned n = ctl & 7u; n > 0; --n) {
+                        ctl >>= 4;
+                        merge(ring_row((ctl & 15u) * RB, t));
+                    }
+                } else {
+                    // general row: any number of predecessors at any distance
+                    const int i = i0 + 1 + b;
+                    const int4 d = rowdesc[i - 1];
+                    const int np = desc_np(d.w);
+#pragma unroll
+                    for (int k = 0; k < S; ++k) hv[k] = INT_MIN;
+                    left = INT_MIN;
+#pragma unroll 1
+                    for (int p = 0; p < max(np, 1); ++p) {
+                        const int r = desc_pred(g, d, p);
+                        int lft;
+                        if (r == 0) {
+                            lft = j0 == 0 ? kNegInf : 0;
+#pragma unroll
+                            for (int k = 0; k < S; ++k) t[k] = 0;
+                        } else if (i - r <= R) {
+                            lft = ring_row((r % R) * RB, t);
+                        } else {
+                            const uint8_t* const src = Hb + (size_t(r) * lc + j0) * HB;
+                            if constexpr (FAST) {
+                                uint32_t v[S / 2];
+                                if constexpr (S % 8 == 0) {
+#pragma unroll
+                                    for (int q = 0; q < S / 8; ++q)
+                                        *reinterpret_cast<uint4*>(v + 4 * q) = reinterpret_cast<const uint4*>(src)[q];
+                                } else if constexpr (S % 4 == 0) {
+#pragma unroll
+                                    for (int q = 0; q < S / 4; ++q)
+                                        *reinterpret_cast<uint2*>(v + 2 * q) = reinterpret_cast<const uint2*>(src)[q];
+                                } else {
+#pragma unroll
+                                    for (int q = 0; q < S / 2; ++q) v[q] = reinterpret_cast<const uint32_t*>(src)[q];
+                                }
+#pragma unroll
+                                for (int q = 0; q < S / 2; ++q) {
+                                    t[2 * q] = unpack_lo(v[q]);
+                                    t[2 * q + 1] = unpack_hi(v[q]);
+                                }
+                            } else {
+#pragma unroll
+                                for (int q = 0; q < S / 2; ++q) {
+                                    const int2 v2 = reinterpret_cast<const int2*>(src)[q];
+                                    t[2 * q] = v2.x;
+                                    t[2 * q + 1] = v2.y;
+                                }
+                            }
+                            lft = __shfl_up_sync(kFull, t[S - 1], 1);
+                            int e = kNegInf;
+                            if (LEFT) e = h_at<FAST>(Hb, r, c0 - 1, lc);
+                            if (lane == 0) lft = e;
+                        }
+                        merge(lft);
+                    }
+                }
+            }
+            // T = max(M[j-1] + s - gap, M[j] + gap), in place from the right
+#pragma unroll
+            for (int k = S - 1; k >= 0; --k) {
+                const int s = FAST ? prmt_score(pool, sel[k]) : (sel[k] == pool ? dmt : dmm);
+                const int dg = (k == 0 ? left : hv[k - 1]) + s;
+                hv[k] = __viaddmax_s32(hv[k], gap, dg);
+            }
+            // running maximum along the row: C groups of K cells
+            constexpr int K = S % 4 == 0 ? 4 : S % 3 == 0 ? 3 : 2;
+            constexpr int C = S / K;
+            int tot[C];
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                tot[c] = K == 2 ? max(hv[c * K], hv[c * K + 1])
+                                : __vimax3_s32(hv[c * K], hv[c * K + 1], hv[c * K + 2]);
+                if (K == 4) tot[c] = max(tot[c], hv[c * K + 3]);
+                if (c > 0) tot[c] = max(tot[c], tot[c - 1]);
+            }
+            // prefix maximum over the lanes by fours: three shuffles of one
+            // value cost little more than one (a lane that a shuffle does not
+            // reach gets its own value back)
+            int x = LEFT ? max(tot[C - 1], bx) : tot[C - 1];
+            {
+                const int s1 = __shfl_up_sync(kFull, x, 1), s2 = __shfl_up_sync(kFull, x, 2);
+                const int s3 = __shfl_up_sync(kFull, x, 3);
+                x = max(__vimax3_s32(x, s1, s2), s3);
+                const int t1 = __shfl_up_sync(kFull, x, 4), t2 = __shfl_up_sync(kFull, x, 8);
+                const int t3 = __shfl_up_sync(kFull, x, 12);
+                x = max(__vimax3_s32(x, t1, t2), t3);
+                x = max(x, __shfl_up_sync(kFull, x, 16));
+            }
+            left = __shfl_up_sync(kFull, x, 1);  // final value left of the segment
+            if (lane == 0) left = bx;
+#pragma unroll
+            for (int c = 0; c < C; ++c) hv[c * K] = max(hv[c * K], c == 0 ? left : max(left, tot[c - 1]));
+#pragma unroll
+            for (int k = 1; k < K; ++k)
+#pragma unroll
+                for (int c = 0; c < C; ++c) hv[c * K + k] = max(hv[c * K + k], hv[c * K + k - 1]);
+            if (feed_lane)
+                reinterpret_cast<volatile int*>(mine + Mem::bytes + Mem::edge)[(i0 + b) & (kEdgeRows - 1)] = hv[S - 1];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                if constexpr (U == 4) {
+                    *reinterpret_cast<int4*>(ring + wofs + q * 512) =
+                        make_int4(hv[4 * q], hv[4 * q + 1], hv[4 * q + 2], hv[4 * q + 3]);
+                } else {
+                    *reinterpret_cast<int2*>(ring + wofs + q * 256) = make_int2(hv[2 * q], hv[2 * q + 1]);
+                }
+            }
+            *reinterpret_cast<int*>(ring_left + wofs) = left;
+            wofs = wofs == (R - 1) * RB ? 0 : wofs + RB;
             // streamed: keep the graph arrays in L2
-            if (H16) {
-                __stcs(dst_s + q, make_uint2(pack_s16(v4.x, v4.y), pack_s16(v4.z, v4.w)));
-            } else {
-                __stcs(dst_g + q, v4);
-            }
-            dst_r[q * 32] = v4;
-        }
-        __stcs(D2 + bits_at(i, lane), make_uint2(hbit, dbit));
-        if (lane == lane_l && is_sink) {
-            int val = kNegInf;
+            if constexpr (FAST) {
+                uint32_t pk[S / 2];
 #pragma unroll
-            for (int k = 0; k < S; ++k)
-                if (k == k_l) val = hv[k];
-            g.lastH[i] = val;
-            if (val > best_v) {
-                best_v = val;
-                best_r = i;
-                ties = 1;
-            } else if (val == best_v) {
-                ++ties;
+                for (int q = 0; q < S / 2; ++q) pk[q] = pack_s16(hv[2 * q], hv[2 * q + 1]);
+                if constexpr (S % 8 == 0) {
+#pragma unroll
+                    for (int q = 0; q < S / 8; ++q)
+                        __stcs(reinterpret_cast<uint4*>(hrow) + q,
+                               make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]));
+                } else if constexpr (S % 4 == 0) {
+#pragma unroll
+                    for (int q = 0; q < S / 4; ++q)
+                        __stcs(reinterpret_cast<uint2*>(hrow) + q, make_uint2(pk[2 * q], pk[2 * q + 1]));
+                } else {
+#pragma unroll
+                    for (int q = 0; q < S / 2; ++q) __stcs(reinterpret_cast<uint32_t*>(hrow) + q, pk[q]);
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < S / 2; ++q)
+                    __stcs(reinterpret_cast<int2*>(hrow) + q, make_int2(hv[2 * q], hv[2 * q + 1]));
             }
+            hrow += hstep;
+        }
+        if (NW > 1) {
+            // lane 31 wrote the strip's edge; its stores come before the count
+            __threadfence_block();
+            if (lane == 31) sh.done[w] = tag0 + i0 + bend;
+        }
         }
     }
     __syncwarp();
-    return EndCell{__shfl_sync(kFull, best_r, lane_l), __shfl_sync(kFull, best_v, lane_l),
-                   __shfl_sync(kFull, ties, lane_l), npreds, H16};
 }
 
-// True when the layer's DP runs in dp_layer_fast (bit-plane decisions).
-__device__ __forceinline__ bool fast_dp(const PoaArgs& a, int L) {
-    return L + 1 <= 32 * 24 && a.match >= a.mismatch && a.match - a.mismatch <= 255;
-}
-
-__device__ EndCell dp_dispatch(const PoaArgs& a, const Graph& g, const int* order, int ndp, const uint8_t* seq, int L,
-                           int lane, int4* ring) {
-    if (fast_dp(a, L)) {
-        if (layer_fits_s16(a, ndp, L)) {
-            switch (seg_cells(L + 1)) {
-                case 4: return dp_layer_fast<4, true>(a, g, order, ndp, seq, L, lane, ring);
-                case 8: return dp_layer_fast<8, true>(a, g, order, ndp, seq, L, lane, ring);
-                case 12: return dp_layer_fast<12, true>(a, g, order, ndp, seq, L, lane, ring);
-                case 16: return dp_layer_fast<16, true>(a, g, order, ndp, seq, L, lane, ring);
-                case 20: return dp_layer_fast<20, true>(a, g, order, ndp, seq, L, lane, ring);
-                default: return dp_layer_fast<24, true>(a, g, order, ndp, seq, L, lane, ring);
-            }
-        }
-        switch (seg_cells(L + 1)) {
-            case 4: return dp_layer_fast<4, false>(a, g, order, ndp, seq, L, lane, ring);
-            case 8: return dp_layer_fast<8, false>(a, g, order, ndp, seq, L, lane, ring);
-            case 12: return dp_layer_fast<12, false>(a, g, order, ndp, seq, L, lane, ring);
-            case 16: return dp_layer_fast<16, false>(a, g, order, ndp, seq, L, lane, ring);
-            case 20: return dp_layer_fast<20, false>(a, g, order, ndp, seq, L, lane, ring);
-            default: return dp_layer_fast<24, false>(a, g, order, ndp, seq, L, lane, ring);
-        }
-    }
-    return dp_layer<24>(a, g, order, ndp, seq, L, lane);
-}
-
-// Walk back from (iend, L) over the decision bytes (lane 0). Writes the
-// sequence-consuming steps of the alignment (node id or -1 for an inserted
-// base, sequence position), end of path first; vertical steps (a graph node
-// against a gap) consume no position and add nothing to the graph. Each step
-// loads the cell's decision byte and its row's descriptor (independent
-// loads); the next row comes from the descriptor. Used for the byte
-// decisions of the chunked dp_layer (rows over 768 columns).
-__device__ bool traceback(const PoaArgs& a, const Graph& g, PoaShared& sh, const int* order, const uint8_t* seq,
-                          int L, int iend) {
-    const int lc = g.lcap;
-    int i = iend, j = L, n = 0;
-    if (iend == INT_MAX || iend < 1) return false;
-    while (!(i == 0 && j == 0)) {
-        if (n >= g.alncap) return false;
-        if (i == 0) {
-            g.aln_node[n] = -1;
-            g.aln_pos[n] = j - 1;
-            ++n;
-            --j;
-            continue;
-        }
-        const int4 d = g.rowdesc[i - 1];
-        const int v = order[i - 1];
-        const int np = desc_np(d.w);
-        uint32_t code = g.dec[dec_at(i, j, lc)];
-        if (code == 255u) {  // decide again from H: diagonal, then vertical, preds in order
-            const int h = g.H[i * lc + j];
-            const int s = j > 0 ? (uint32_t(seq[j - 1]) == desc_base(d.w) ? a.match : a.mismatch) : 0;
-            const int cnt = np == 0 ? 1 : np;
-            code = 128u;
-            int pick = -1;
-            if (cnt <= 3) {
-                // all candidate values loaded at once (independent loads)
-                int hd[3], hvv[3];
-#pragma unroll
-                for (int p = 0; p < 3; ++p) {
-                    const int r = p < cnt ? desc_pred(g, d, p) : 0;
-                    hd[p] = (p < cnt && j > 0) ? g.H[r * lc + j - 1] : kNegInf;
-                    hvv[p] = p < cnt ? g.H[r * lc + j] : kNegInf;
-                }
-#pragma unroll
-                for (int p = 2; p >= 0; --p)
-                    if (j > 0 && hd[p] + s == h) pick = p;
-                if (pick >= 0) {
-                    code = 1000u + uint32_t(pick);
-                } else {
-#pragma unroll
-                    for (int p = 2; p >= 0; --p)
-                        if (hvv[p] + a.gap == h) pick = p;
-                    if (pick >= 0) code = 2000u + uint32_t(pick);
-                }
+// One layer's DP, all passes.
+template <int S, int NW>
+__device__ __forceinline__ void dp_layer(const Graph& g, PoaShared& sh, int ndp, const uint8_t* seq, int L, int mt,
+                                         int mm, int gap, int lane, int w, int team, bool fast) {
+    constexpr int W = 32 * S;
+    const int nstrips = (L + W) / W;
+    if (lane == 0) sh.done[w] = 0;
+    for (int pass = 0; pass * NW < nstrips; ++pass) {
+        team_sync<NW>(team);
+        const int strip = pass * NW + w;
+        if (strip >= nstrips) continue;
+        if (fast) {
+            if (strip == 0) {
+                dp_strip<S, NW, true, false>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, pass);
             } else {
-                if (j > 0)
-                    for (int p = 0; p < cnt && pick < 0; ++p)
-                        if (g.H[desc_pred(g, d, p) * lc + j - 1] + s == h) pick = p;
-                if (pick >= 0) {
-                    code = 1000u + uint32_t(pick);
-                } else {
-                    for (int p = 0; p < cnt && pick < 0; ++p)
-                        if (g.H[desc_pred(g, d, p) * lc + j] + a.gap == h) pick = p;
-                    if (pick >= 0) code = 2000u + uint32_t(pick);
-                }
+                dp_strip<S, NW, true, true>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, pass);
+            }
+        } else {
+            if (strip == 0) {
+                dp_strip<S, NW, false, false>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, pass);
+            } else {
+                dp_strip<S, NW, false, true>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, pass);
             }
         }
-        if (code < 64u || (code >= 1000u && code < 2000u)) {
-            const int p = code < 64u ? int(code) : int(code - 1000u);
-            g.aln_node[n] = v;
-            g.aln_pos[n] = j - 1;
-            ++n;
-            i = desc_pred(g, d, p);
-            --j;
-        } else if (code < 128u || code >= 2000u) {
-            const int p = code < 128u ? int(code - 64u) : int(code - 2000u);
-            i = desc_pred(g, d, p);  // vertical: no sequence position
-        } else {
-            if (j == 0) return false;
-            g.aln_node[n] = -1;
-            g.aln_pos[n] = j - 1;
-            ++n;
-            --j;
+    }
+}
+
+template <int NW>
+__device__ void dp_dispatch(const Graph& g, PoaShared& sh, int ndp, const uint8_t* seq, int L, int mt, int mm,
+                            int gap, int lane, int w, int team, bool fast) {
+    const int s = seg_cells(NW, L + 1);
+    if constexpr (NW == 4) {
+        switch (s) {
+            case 2: return dp_layer<2, NW>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, fast);
+            case 4: return dp_layer<4, NW>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, fast);
+            case 6: return dp_layer<6, NW>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, fast);
+            default: return dp_layer<8, NW>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, fast);
+        }
+    } else {
+        switch (s) {
+            case 8: return dp_layer<8, NW>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, fast);
+            case 16: return dp_layer<16, NW>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, fast);
+            default: return dp_layer<24, NW>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, fast);
         }
     }
-    sh.naln = n;
-    return true;
+}
+
+// The walk back from (iend, L) over the stored scores, by one warp. At a
+// cell with slanted score h it takes spoa's first way to h: the diagonal through the
+// predecessors in order, then the vertical through them, then left. The walk
+// is a chain of dependent steps through nearby rows and columns, so the warp
+// stages a tile of score rows, descriptors and node ids in shared memory and
+// one lane walks through it, loading all candidates of a step at once and
+// choosing among them without branches (votes and shuffles between lanes
+// would cost more than the whole step). A predecessor above the tile is read
+// from global memory; a step that leaves the tile ends the lane's run and
+// the warp stages the next one. Writes the node of every sequence position
+// (-1 for an inserted base) to g.aln_node; a vertical step consumes no
+// position and adds nothing to the graph. Returns false on a broken walk.
+constexpr int kTileRows = 96;
+constexpr int kTilePitch = 128;  // bytes per row: 64 int16 or 32 int32 columns
+constexpr int kTileBytes = kTileRows * kTilePitch;
+constexpr int kTileSmem = kTileBytes + kTileRows * 20 + 64;
+static_assert(kTileSmem <= 4 * WarpMem<4>::bytes && kTileSmem <= WarpMem<1>::bytes, "the tile fits every team's memory");
+template <bool FAST>
+__device__ __noinline__ bool traceback_warp(const Graph& g, const int* order, const uint8_t* seq, int L, int iend,
+                                            int hend, int mt, int mm, int gap, int lane, int smem_off, int lc) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr int HB = FAST ? 2 : 4;              // bytes per score
+    constexpr int kCols = kTilePitch / HB;       // tile columns
+    constexpr int kUnit = 16 / HB;               // columns per 16-byte chunk
+    constexpr int kChunks = kTilePitch / 16;
+    uint8_t* const tile = reinterpret_cast<uint8_t*>(g_poa_smem) + smem_off;
+    // per tile row: byte offsets of the predecessors' tile rows (-1: outside,
+    // or more than three) | base
+    int4* const w_desc = reinterpret_cast<int4*>(tile + kTileBytes);
+    int* const w_node = reinterpret_cast<int*>(tile + kTileBytes + kTileRows * 16);
+    uint8_t* const w_seq = tile + kTileBytes + kTileRows * 20;
+    const uint8_t* const Hb = reinterpret_cast<const uint8_t*>(g.H);
+    const int4* const rowdesc = g.rowdesc;
+    const int* const pred_idx = g.pred_idx;
+    int* const path = g.aln_node;
+    int i = iend, j = L, h = hend;
+    if (iend == INT_MAX || iend < 1) return false;
+    auto score = [&](const uint8_t* p) -> int {
+        return FAST ? int(*reinterpret_cast<const int16_t*>(p)) : *reinterpret_cast<const int*>(p);
+    };
+    const int dmt = mt - gap, dmm = mm - gap;
+    bool ok = true;
+    while (i > 0 && ok) {
+        // rows (i - kTileRows, i], columns up to j
+        const int wlo = max(0, i - (kTileRows - 1));
+        const int clo = max(0, (j / kUnit + 1) * kUnit - kCols);
+        const int rows = i - wlo + 1;
+        int4* const t4 = reinterpret_cast<int4*>(tile);
+        __syncwarp();
+#pragma unroll 12
+        for (int q = lane; q < kTileRows * kChunks; q += 32) {
+            const int tr = q / kChunks, tc = q % kChunks;
+            if (tr < rows && clo + tc * kUnit < lc)
+                t4[q] = *reinterpret_cast<const int4*>(Hb + (size_t(wlo + tr) * lc + clo) * HB + tc * 16);
+        }
+#pragma unroll
+        for (int o = lane; o < kTileRows; o += 32) {
+            const int r = wlo + o;
+            if (r >= 1 && r <= i) {
+                int4 d = rowdesc[r - 1];
+                w_node[o] = order[r - 1];
+                const int np = desc_np(d.w);
+                // absent predecessors repeat the first
+                if (np == 0) d.x = 0;
+                if (np < 2) d.y = d.x;
+                if (np < 3) d.z = d.x;
+                const bool inside = np <= 3 && min(d.x, min(d.y, d.z)) >= wlo;
+                w_desc[o] = make_int4(inside ? (d.x - wlo) * kTilePitch : -1, (d.y - wlo) * kTilePitch,
+                                      (d.z - wlo) * kTilePitch, int(desc_base(d.w)));
+            }
+        }
+        for (int c = lane; c < kCols; c += 32) w_seq[c] = (clo + c >= 1 && clo + c <= L) ? seq[clo + c - 1] : 0;
+        __syncwarp();
+        if (lane == 0) {
+            int oi = (i - wlo) * kTilePitch, cj = j - clo;  // the cell in the tile
+            const int cmin = clo > 0 ? 1 : 0;               // the walk needs column cj - 1 unless it is before the first
+            do {
+                const int4 d = w_desc[oi / kTilePitch];
+                const int v = w_node[oi / kTilePitch];
+                const int s = uint32_t(w_seq[cj]) == uint32_t(d.w) ? dmt : dmm;
+                const bool col = cj > 0;
+                const uint8_t* const tj = tile + cj * HB;
+                const uint8_t* const tl = tile + (col ? cj - 1 : 0) * HB;
+                int no = oi, nh = score(tl + oi), node = -1;  // left
+                bool step = true;
+                if (d.x >= 0) {
+                    const int a0 = score(tl + d.x), a1 = score(tl + d.y), a2 = score(tl + d.z);
+                    const int b0 = score(tj + d.x), b1 = score(tj + d.y), b2 = score(tj + d.z);
+                    const int hd = col ? h - s : INT_MIN, hu = h - gap;
+                    const bool up = b0 == hu || b1 == hu || b2 == hu;
+                    const bool dg = a0 == hd || a1 == hd || a2 == hd;
+                    const int ou = b0 == hu ? d.x : b1 == hu ? d.y : d.z;
+                    const int od = a0 == hd ? d.x : a1 == hd ? d.y : d.z;
+                    no = dg ? od : up ? ou : oi;
+                    nh = dg ? hd : up ? hu : nh;
+                    node = dg ? v : -1;
+                    step = dg || !up;
+                } else {
+                    // long list, or a predecessor above the tile: the first
+                    // diagonal, else the first vertical
+                    const int4 e = rowdesc[wlo + oi / kTilePitch - 1];
+                    const int np = desc_np(e.w);
+                    int vr = -1, dr = -1;
+                    for (int p = 0; p < max(np, 1) && dr < 0; ++p) {
+                        const int r = np == 0 ? 0 : np > 3 ? (p == 0 ? e.y : pred_idx[e.x + p]) : p == 0 ? e.x : p == 1 ? e.y : e.z;
+                        const uint8_t* const pr = Hb + (size_t(r) * lc + clo + cj) * HB;
+                        if (col && score(pr - HB) == h - s) dr = r;
+                        if (vr < 0 && score(pr) == h - gap) vr = r;
+                    }
+                    const int nr = dr >= 0 ? dr : vr;
+                    if (nr >= 0) {
+                        no = (nr - wlo) * kTilePitch;
+                        nh = dr >= 0 ? h - s : h - gap;
+                        node = dr >= 0 ? v : -1;
+                        step = dr >= 0;
+                    }
+                }
+                if (step) {
+                    if (!col) {
+                        ok = false;
+                        break;
+                    }
+                    --cj;
+                    path[clo + cj] = node;
+                }
+                oi = no;
+                h = nh;
+            } while (oi >= (wlo == 0 ? kTilePitch : 0) && cj >= cmin);
+            // rank 0 (oi == 0 with wlo == 0) ends the walk
+            i = wlo + (oi >= 0 ? oi / kTilePitch : -((-oi) / kTilePitch));
+            j = clo + cj;
+        }
+        i = __shfl_sync(kFull, i, 0);
+        j = __shfl_sync(kFull, j, 0);
+        h = __shfl_sync(kFull, h, 0);
+        ok = __shfl_sync(kFull, ok ? 1 : 0, 0) != 0;
+    }
+    if (ok)
+        for (int k = lane; k < j; k += 32) path[k] = -1;
+    __syncwarp();
+    return ok;
 }
 
 // ---------------- compact adjacency in shared memory ----------------
@@ -1631,7 +1614,7 @@ __device__ int topo_sort_warp(const Graph& g, PoaShared& sh, bool all_nodes, int
     const int N = sh.nnodes;
     SmemCsr c;
     int nr = 0;
-    if (build_csr(g, sh, lane, ring, kRingBytesPerWarp, c)) {
+    if (build_csr(g, sh, lane, ring, sh.scratch_bytes, c)) {
         for (int i = lane; i < N; i += 32) c.flag[i] = uint8_t(4 | (all_nodes || g.member[i] ? 8 : 0));
         __syncwarp();
         if (lane == 0) nr = g_topo_sort_csr(g, c, N, all_nodes, out);
@@ -1658,7 +1641,7 @@ __device__ bool mark_subgraph_warp(const Graph& g, PoaShared& sh, int begin_node
     }
     SmemCsr c;
     bool ok = true;
-    if (build_csr(g, sh, lane, ring, kRingBytesPerWarp, c)) {
+    if (build_csr(g, sh, lane, ring, sh.scratch_bytes, c)) {
         for (int i = lane; i < N; i += 32) c.flag[i] = 0;
         __syncwarp();
         if (lane == 0) {
@@ -1700,11 +1683,11 @@ __device__ bool mark_subgraph_warp(const Graph& g, PoaShared& sh, int begin_node
 // arrays are issued four 32-element chunks at a time, so one memory latency
 // covers 128 edges or rows. Same order rules as the global form below.
 // Returns false, building nothing, when the graph does not fit.
-__device__ bool descriptors_smem(const Graph& g, const PoaShared& sh, const int* order, int N, int ndp, int lane,
+__device__ bool descriptors_smem(const Graph& g, PoaShared& sh, const int* order, int N, int ndp, int lane,
                                  int4* ring) {
     constexpr unsigned kFull = 0xffffffffu;
     const size_t rk_bytes = size_t((N + 3) / 4) * 8;
-    if (ndp >= 32768 || sh.nseq >= 65535 || rk_bytes + size_t(8) * ndp > size_t(kRingBytesPerWarp)) return false;
+    if (ndp >= 32768 || sh.nseq >= 65535 || rk_bytes + size_t(8) * ndp > size_t(sh.scratch_bytes)) return false;
     uint16_t* const rk = reinterpret_cast<uint16_t*>(ring);
     ushort4* const acc = reinterpret_cast<ushort4*>(reinterpret_cast<uint8_t*>(ring) + rk_bytes);
     for (int i = lane; i < N; i += 32) rk[i] = 0;
@@ -1761,7 +1744,7 @@ __device__ bool descriptors_smem(const Graph& g, const PoaShared& sh, const int*
         }
     }
     any_long = __any_sync(kFull, any_long);
-    int list_base = 0;
+    int list_base = 0, preds = 0;
     for (int c0 = 0; c0 < ndp; c0 += 128) {
         int v[4], code[4];
 #pragma unroll
@@ -1777,6 +1760,7 @@ __device__ bool descriptors_smem(const Graph& g, const PoaShared& sh, const int*
             const int i = c0 + 32 * u + lane;
             const ushort4 dd = i < ndp ? acc[i] : make_ushort4(0, 0, 0, 0);
             const int np = dd.w;
+            preds += np;
             int off = 0;
             if (any_long) {
                 int tot = 0;
@@ -1794,6 +1778,8 @@ __device__ bool descriptors_smem(const Graph& g, const PoaShared& sh, const int*
             }
         }
     }
+    preds = __reduce_add_sync(kFull, preds);
+    if (lane == 0) sh.preds = preds;
     __syncwarp();
     if (any_long) {
         for (int c0 = 0; c0 < E; c0 += 32) {
@@ -1843,7 +1829,7 @@ __device__ int heaviest_bundle_warp(const Graph& g, PoaShared& sh, int lane, int
     int* const sv = reinterpret_cast<int*>(su + 32 * D);                      // [32] node
     int* const sd = sv + 32;                                                  // [32] degree, D + 1 = more
     const size_t need = st_off + 32 * D * 6 + 32 * 8;
-    const bool fits = N < 65535 && need <= size_t(kRingBytesPerWarp) &&
+    const bool fits = N < 65535 && need <= size_t(sh.scratch_bytes) &&
                       double(sh.nseq + 1) * 186.0 * double(N + 1) < 2.0e9;
     if (!fits) {
         int len = 0;
@@ -1963,167 +1949,272 @@ __device__ int heaviest_bundle_warp(const Graph& g, PoaShared& sh, int lane, int
     return __shfl_sync(0xffffffffu, len, 0);
 }
 
-// Escape decision from H for a row of several predecessors (warp, uniform
-// arguments): the first predecessor whose diagonal gives H[i][j],
-// else the first whose vertical does, else horizontal. Returns 1000 + p,
-// 2000 + p or 128. Lanes load the candidates of 32 predecessors at a time.
-__device__ uint32_t decide_from_h(const PoaArgs& a, const Graph& g, const int4& d, const uint8_t* seq, int i, int j,
-                                  int lane, bool h16) {
-    const int np = desc_np(d.w);
-    const int h = h_at(g, i, j, h16);
-    const int s = j > 0 ? (uint32_t(seq[j - 1]) == desc_base(d.w) ? a.match : a.mismatch) : 0;
-    const int cnt = np == 0 ? 1 : np;
-    int vpick = -1;
-    for (int p0 = 0; p0 < cnt; p0 += 32) {
-        const int p = p0 + lane;
-        bool dm = false, vm = false;
-        if (p < cnt) {
-            const int r = desc_pred(g, d, p);
-            dm = j > 0 && h_at(g, r, j - 1, h16) + s == h;
-            vm = h_at(g, r, j, h16) + a.gap == h;
-        }
-        const unsigned bd = __ballot_sync(0xffffffffu, dm);
-        if (bd) return 1000u + uint32_t(p0 + __ffs(bd) - 1);
-        const unsigned bv = __ballot_sync(0xffffffffu, vm);
-        if (bv && vpick < 0) vpick = p0 + __ffs(bv) - 1;
-    }
-    return vpick >= 0 ? 2000u + uint32_t(vpick) : 128u;
-}
-
-// Warp form of the walk over dp_layer_fast's bit-plane decisions. The walk is
-// a chain of dependent steps through nearby rows and columns, so the warp
-// stages a window in shared memory with one parallel load: descriptors,
-// node ids and the decision words of rows [wlo, wlo + 64) in column segments
-// wseg and wseg - 1. Every lane then runs the same walk over the window
-// (uniform control flow); lane 0 writes the alignment. A step that leaves
-// the window reloads it. Decoding: horizontal plane, else the diagonal of
-// predecessor 0; rows of one predecessor are otherwise vertical through it,
-// rows of several decide again from H. Returns false on a broken walk.
-__device__ bool traceback_warp(const PoaArgs& a, const Graph& g, PoaShared& sh, const int* order, const uint8_t* seq,
-                               int L, int iend, int lane, int4* ring, bool h16) {
-    constexpr int W = 64;
-    const int S = seg_cells(L + 1);
-    int4* const w_desc = ring;                                           // [W]
-    int* const w_node = reinterpret_cast<int*>(ring + W);               // [W]
-    uint2* const w_bits = reinterpret_cast<uint2*>(ring + W + W / 4);   // [2][W]
-    const uint2* const D2 = reinterpret_cast<const uint2*>(g.dec);
-    int i = iend, j = L, n = 0;
-    if (iend == INT_MAX || iend < 1) return false;
-    int seg = L / S, k = L % S;
-    int wlo = INT_MAX, wseg = -1;
-    bool ok = true;
-    auto step_left = [&]() {
-        --j;
-        if (k == 0) {
-            k = S - 1;
-            --seg;
-        } else {
-            --k;
-        }
-    };
-    while (!(i == 0 && j == 0)) {
-        if (n >= g.alncap) {
-            ok = false;
-            break;
-        }
-        if (i == 0) {
-            if (lane == 0) {
-                g.aln_node[n] = -1;
-                g.aln_pos[n] = j - 1;
-            }
-            ++n;
-            step_left();
-            continue;
-        }
-        if (i < wlo || seg < wseg - 1 || seg > wseg) {
-            // stage rows [i - 63, i] (clamped at 1) for segments seg, seg - 1
-            __syncwarp();
-            wlo = max(1, i - (W - 1));
-            wseg = seg;
-#pragma unroll
-            for (int h = 0; h < W / 32; ++h) {
-                const int o = h * 32 + lane;
-                const int r = wlo + o;
-                if (r <= i) {
-                    w_desc[o] = g.rowdesc[r - 1];
-                    w_node[o] = order[r - 1];
-                    w_bits[o] = D2[bits_at(r, seg)];
-                    w_bits[W + o] = seg > 0 ? D2[bits_at(r, seg - 1)] : make_uint2(0, 0);
-
-                }
-            }
-            __syncwarp();
-        }
-        const int o = i - wlo;
-        const int4 d = w_desc[o];
-        const int v = w_node[o];
-        const uint2 w = w_bits[(seg == wseg ? 0 : W) + o];
-        const int np = desc_np(d.w);
-        uint32_t code;
-        if ((w.x >> k) & 1u) {
-            code = 128u;
-        } else if ((w.y >> k) & 1u) {
-            code = 0u;  // diagonal through predecessor 0
-        } else if (np <= 1) {
-            code = 64u;  // vertical through the only predecessor
-        } else {
-            code = decide_from_h(a, g, d, seq, i, j, lane, h16);
-        }
-        if (code < 64u || (code >= 1000u && code < 2000u)) {
-            const int p = code < 64u ? int(code) : int(code - 1000u);
-            if (lane == 0) {
-                g.aln_node[n] = v;
-                g.aln_pos[n] = j - 1;
-            }
-            ++n;
-            i = desc_pred(g, d, p);
-            step_left();
-        } else if (code < 128u || code >= 2000u) {
-            const int p = code < 128u ? int(code - 64u) : int(code - 2000u);
-            i = desc_pred(g, d, p);  // vertical: no sequence position
-        } else {
-            if (j == 0) {
-                ok = false;
-                break;
-            }
-            if (lane == 0) {
-                g.aln_node[n] = -1;
-                g.aln_pos[n] = j - 1;
-            }
-            ++n;
-            step_left();
-        }
-    }
+// Rows of one layer's DP (warp): marks the subgraph of a partial layer, lists
+// its rows (the incremental order, restricted to the subgraph) and builds
+// their descriptors. sh.ndp rows, or sh.fail.
+__device__ void layer_rows(const Graph& g, PoaShared& sh, const int* order, bool full, int begin, int end, int lane,
+                           int4* ring) {
+    const int N = sh.nnodes;
+    for (int i = lane; i < N; i += 32) g.member[i] = full ? 1 : 0;
     __syncwarp();
-    if (lane == 0) sh.naln = n;
-    return ok;
+    if (!full && !mark_subgraph_warp(g, sh, begin, end, lane, ring) && lane == 0) sh.fail = kOverflow;
+    __syncwarp();
+    if (sh.fail) return;
+            // DP rows: the incremental order, restricted to the subgraph for a
+            // partial layer (any topological order gives the same DP values)
+            int ndp = N;
+                    if (!full) {
+                // compaction of the member nodes in order; the loads of four
+                // 32-entry chunks go out together
+                int base = 0;
+                for (int c4 = 0; c4 < N; c4 += 128) {
+                    int vv[4];
+                    bool in[4];
+    #pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int r = c4 + 32 * u + lane;
+                        vv[u] = r < N ? g.ord[r] : 0;
+                    }
+    #pragma unroll
+                    for (int u = 0; u < 4; ++u) in[u] = c4 + 32 * u + lane < N && g.member[vv[u]];
+    #pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const unsigned m = __ballot_sync(0xffffffffu, in[u]);
+                        if (in[u]) g.dporder[base + __popc(m & ((1u << lane) - 1u))] = vv[u];
+                        base += __popc(m);
+                    }
+                }
+                ndp = base;
+                        __syncwarp();
+            }
+            // Row descriptors: shared-memory accumulators when the graph fits,
+            // else the global form below.
+            if (!descriptors_smem(g, sh, order, N, ndp, lane, ring)) {
+                // Row descriptors. DP ranks of the nodes live in shared memory (the
+                // row ring is free until the DP) when they fit, else in global
+                // scratch; bit 31 marks a node with a successor among the rows.
+                int* const dpr = 4 * N <= sh.scratch_bytes ? reinterpret_cast<int*>(ring) : g.dprank;
+                for (int i = lane; i < N; i += 32) dpr[i] = 0;
+                __syncwarp();
+                for (int i = lane; i < ndp; i += 32) dpr[order[i]] = i + 1;
+                __syncwarp();
+                // Predecessors by one pass over the edges in id order. A node's
+                // in-edge list is in edge-id order (each layer adds at most one edge
+                // into a node, with a fresh, larger id), which is spoa's predecessor
+                // order. Lanes take 32 consecutive edges; edges into the same row
+                // are ranked by lane, so the order is deterministic. rowdesc[r - 1]
+                // collects the first three predecessor ranks (x, y, z) and the count
+                // (w) of row r; bit 31 of dpr marks a node with a successor row.
+                for (int i = lane; i < ndp; i += 32) g.rowdesc[i] = make_int4(0, 0, 0, 0);
+                __syncwarp();
+                const int E = sh.nedges;
+                const unsigned below = (1u << lane) - 1u;
+                bool any_long = false;
+                for (int c0 = 0; c0 < E; c0 += 32) {
+                    const int e = c0 + lane;
+                    int rs = 0, rd = 0, src = 0;
+                    if (e < E) {
+                        src = g.e_src[e];
+                        const int dst = g.e_dst[e];
+                        rs = dpr[src] & 0x7FFFFFFF;
+                        rd = rs > 0 ? dpr[dst] & 0x7FFFFFFF : 0;
+                    }
+                    const bool q = rs > 0 && rd > 0;
+                    const unsigned grp = __match_any_sync(0xffffffffu, q ? rd : -1 - lane);
+                    int cnt = 0;
+                    if (q) {
+                        atomicOr(reinterpret_cast<unsigned*>(&dpr[src]), 0x80000000u);
+                        cnt = g.rowdesc[rd - 1].w;
+                    }
+                    __syncwarp();
+                    if (q) {
+                        const int pos = cnt + __popc(grp & below);
+                        int* rdw = reinterpret_cast<int*>(&g.rowdesc[rd - 1]);
+                        if (pos < 3) rdw[pos] = rs;
+                        if ((grp & below) == 0) {
+                            const int tot = cnt + __popc(grp);
+                            rdw[3] = tot;
+                            any_long |= tot > 3;
+                        }
+                    }
+                    __syncwarp();
+                }
+                any_long = __any_sync(0xffffffffu, any_long);
+                // final descriptors; rows with more than three predecessors get their
+                // full list in pred_idx at an offset from a warp prefix of the counts
+                int list_base = 0, preds = 0;
+                for (int c0 = 0; c0 < ndp; c0 += 32) {
+                    const int i = c0 + lane;
+                    int4 dd = i < ndp ? g.rowdesc[i] : make_int4(0, 0, 0, 0);
+                    const int v = i < ndp ? order[i] : 0;
+                    int off = 0;
+                preds += dd.w;
+                    if (any_long) {
+                        int tot = 0;
+                        const int cntl = (i < ndp && dd.w > 3) ? dd.w : 0;
+                        off = list_base + warp_excl(cntl, lane, tot);
+                        list_base += tot;
+                        if (cntl) g.bpred[v] = off;  // list cursor of the node
+                    }
+                    if (i < ndp) {
+                        const bool sink = (dpr[v] & 0x80000000) == 0;
+                        g.sink[i] = sink ? 1 : 0;
+                        // long rows: x = list offset, y = first predecessor
+                        g.rowdesc[i] = make_int4(dd.w > 3 ? off : dd.x, dd.w > 3 ? dd.x : dd.y, dd.z,
+                                                 int(uint32_t(dd.w) | (uint32_t(sink) << 17) | (uint32_t(g.code[v]) << 24)));
+                    }
+                }
+                preds = __reduce_add_sync(0xffffffffu, preds);
+        if (lane == 0) sh.preds = preds;
+        __syncwarp();
+                if (any_long) {
+                    // second pass over the edges for the long lists, same ranking
+                    for (int c0 = 0; c0 < E; c0 += 32) {
+                        const int e = c0 + lane;
+                        int rs = 0, dst = 0;
+                        bool q = false;
+                        if (e < E) {
+                            dst = g.e_dst[e];
+                            const int rd = dpr[dst] & 0x7FFFFFFF;
+                            if (rd > 0 && desc_np(g.rowdesc[rd - 1].w) > 3) {
+                                rs = dpr[g.e_src[e]] & 0x7FFFFFFF;
+                                q = rs > 0;
+                            }
+                        }
+                        const unsigned grp = __match_any_sync(0xffffffffu, q ? dst : -1 - lane);
+                        int cur = 0;
+                        if (q) cur = g.bpred[dst];
+                        __syncwarp();
+                        if (q) {
+                            g.pred_idx[cur + __popc(grp & below)] = rs;
+                            if ((grp & below) == 0) g.bpred[dst] = cur + __popc(grp);
+                        }
+                        __syncwarp();
+                    }
+                }
+                __syncwarp();
+            }
+    if (lane == 0) sh.ndp = ndp;
+    __syncwarp();
 }
 
-// ---------------- one window (one warp) ----------------
+// NW end row of the layer (warp): the first sink row with the best
+// last-column score, or, when several sinks share it, spoa's first among
+// them. Sets sh.end_value.
+template <bool FAST>
+__device__ int end_row(const Graph& g, PoaShared& sh, const int* order, int ndp, int L, int lc, bool full, int lane,
+                       int4* ring) {
+    const uint8_t* const Hb = reinterpret_cast<const uint8_t*>(g.H);
+    int best = INT_MIN, iend = INT_MAX, ties = 0;
+    for (int i = 1 + lane; i <= ndp; i += 32) {
+        if (!g.sink[i - 1]) continue;
+        const int v = h_at<FAST>(Hb, i, L, lc);
+        g.lastH[i] = v;
+        ties = v > best ? 1 : ties + (v == best ? 1 : 0);
+        iend = v > best ? i : iend;
+        best = max(best, v);
+    }
+    sh.end_value = __reduce_max_sync(0xffffffffu, best);
+    __syncwarp();
+    if (best != sh.end_value) {
+        ties = 0;
+        iend = INT_MAX;
+    }
+    iend = __reduce_min_sync(0xffffffffu, iend);
+    ties = __reduce_add_sync(0xffffffffu, ties);
+    if (ties > 1) {
+                // several sinks share the best last-column value: spoa takes the
+                // first in its own topological order of the aligned (sub)graph.
+                // A sink outside every aligned group is reached by spoa's DFS
+                // only as a root (no member lists it as an in-edge tail, and
+                // aligned links are symmetric), so such sinks are ranked by node
+                // id; only a tie that involves an aligned sink needs the DFS.
+                int low_id = INT_MAX, low_i = iend;
+                bool grouped = false;
+                for (int i = 1 + lane; i <= ndp; i += 32) {
+                    if (!g.sink[i - 1] || g.lastH[i] != sh.end_value) continue;
+                    const int v = order[i - 1];
+                    grouped |= g.al_cnt[v] != 0;
+                    if (v < low_id) {
+                        low_id = v;
+                        low_i = i;
+                    }
+                }
+    #pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    const int ov = __shfl_xor_sync(0xffffffffu, low_id, o);
+                    const int oi = __shfl_xor_sync(0xffffffffu, low_i, o);
+                    if (ov < low_id) {
+                        low_id = ov;
+                        low_i = oi;
+                    }
+                }
+                grouped = __any_sync(0xffffffffu, grouped);
+                const int nr = grouped ? topo_sort_warp(g, sh, full, g.rank_to_node, lane, ring) : 0;
+                if (!grouped) {
+                    iend = low_i;
+                } else if (nr < 0) {
+                    if (lane == 0) sh.fail = kOverflow;
+                } else {
+                    for (int r = lane; r < nr; r += 32) g.node_rank[g.rank_to_node[r]] = r;
+                    __syncwarp();
+                    // the tied sink of lowest rank (ranks are distinct)
+                    int best = INT_MAX, bi = iend;
+                    for (int i = 1 + lane; i <= ndp; i += 32) {
+                        if (!g.sink[i - 1] || g.lastH[i] != sh.end_value) continue;
+                        const int rr = g.node_rank[order[i - 1]];
+                        if (rr < best) {
+                            best = rr;
+                            bi = i;
+                        }
+                    }
+    #pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        const int ob = __shfl_xor_sync(0xffffffffu, best, o);
+                        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                        if (ob < best) {
+                            best = ob;
+                            bi = oi;
+                        }
+                    }
+                    iend = bi;
+                }
+                __syncwarp();
+            }
+    return iend;
+}
 
-__device__ void poa_window(const PoaArgs& a, const Graph& g, PoaShared& sh, uint32_t wi, int lane, int4* ring) {
+// ---------------- one window (one team) ----------------
+
+// The team's warps share the set-up and the DPs; warp 0 does the graph steps
+// between them. Every thread of the team returns together.
+template <int NW>
+__device__ void poa_window(const PoaArgs& a, const Graph& g, PoaShared& sh, uint32_t wi, int lane, int w, int team) {
+    constexpr int NT = 32 * NW;
+    const int tid = 32 * w + lane;
+    int4* const ring = g_poa_smem + team * (NW * WarpMem<NW>::bytes / 16);
     const PoaWinDev W = a.wins[wi];
     const uint8_t* bb = a.in + W.bb_off;
     const uint8_t* bq = W.bq_off == kNoQual ? nullptr : a.in + W.bq_off;
     uint8_t* outp = reinterpret_cast<uint8_t*>(a.out) + W.out_off;
     const int B = int(W.bb_len);
     if (W.n_layers < 2) {
-        for (int i = lane; i < B; i += 32) outp[i] = bb[i];
-        if (lane == 0) {
+        for (int i = tid; i < B; i += NT) outp[i] = bb[i];
+        if (tid == 0) {
             a.out_len[wi] = uint32_t(B);
             a.flags[wi] = 0;
         }
         return;
     }
     if (B > g.ncap) {
-        if (lane == 0) {
+        if (tid == 0) {
             a.flags[wi] = kOverflow;
             a.out_len[wi] = 0;
         }
         return;
     }
     // backbone: chain of B nodes, edge weights from quality (0 with the dummy)
-    for (int i = lane; i < B; i += 32) {
+    for (int i = tid; i < B; i += NT) {
         g.code[i] = bb[i];
         g.cov[i] = B >= 2 ? 1u : 0u;
         g.al_head[i] = g.al_tail[i] = -1;
@@ -2150,15 +2241,16 @@ __device__ void poa_window(const PoaArgs& a, const Graph& g, PoaShared& sh, uint
         g.al_cnt[i] = 0;
         g.out_cnt[i] = i + 1 < B ? 1 : 0;
     }
-    if (lane == 0) {
+    if (tid == 0) {
         sh.nnodes = B;
         sh.nedges = B - 1;
         sh.naligned = 0;
         sh.nseq = 1;
         sh.nranks = B;
         sh.fail = 0;
+        sh.scratch_bytes = NW * WarpMem<NW>::bytes;
     }
-    __syncwarp();
+    team_sync<NW>(team);
     unsigned long long cells = 0, edge_cells = 0;
 
     for (uint32_t li = 0; li < W.n_layers; ++li) {
@@ -2167,225 +2259,41 @@ __device__ void poa_window(const PoaArgs& a, const Graph& g, PoaShared& sh, uint
         const uint8_t* qual = Lr.qual_off == kNoQual ? nullptr : a.in + Lr.qual_off;
         const int L = int(Lr.len);
         const bool full = Lr.begin < W.offset && Lr.end > uint32_t(B) - W.offset;
-        const int N = sh.nnodes;
-        for (int i = lane; i < N; i += 32) {
-            g.member[i] = full ? 1 : 0;
+        const int* const order = full ? g.ord : g.dporder;
+        if (w == 0 && !sh.fail) {
+            // subgraph, DP rows and their descriptors
+            layer_rows(g, sh, order, full, int(Lr.begin), int(Lr.end), lane, ring);
+            if (lane == 0 && !sh.fail && row_cover(NW, L + 1) > g.lcap) sh.fail = kOverflow;
         }
-        __syncwarp();
-        if (!full && !mark_subgraph_warp(g, sh, int(Lr.begin), int(Lr.end), lane, ring) && lane == 0)
-            sh.fail = kOverflow;
-        __syncwarp();
-        if (lane == 0 && !sh.fail && row_cover(L + 1) > g.lcap) sh.fail = kOverflow;
-        __syncwarp();
+        team_sync<NW>(team);
         if (sh.fail) break;
-        // DP rows: the incremental order, restricted to the subgraph for a
-        // partial layer (any topological order gives the same DP values)
-        int ndp = N;
-        const int* order = g.ord;
-        if (!full) {
-            // compaction of the member nodes in order; the loads of four
-            // 32-entry chunks go out together
-            int base = 0;
-            for (int c4 = 0; c4 < N; c4 += 128) {
-                int vv[4];
-                bool in[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int r = c4 + 32 * u + lane;
-                    vv[u] = r < N ? g.ord[r] : 0;
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) in[u] = c4 + 32 * u + lane < N && g.member[vv[u]];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const unsigned m = __ballot_sync(0xffffffffu, in[u]);
-                    if (in[u]) g.dporder[base + __popc(m & ((1u << lane) - 1u))] = vv[u];
-                    base += __popc(m);
-                }
+        const int ndp = sh.ndp;
+        bool fast = fast_scores(a.match, a.mismatch, a.gap, ndp, L);
+        for (int k = lane; k < L; k += 32) fast = fast && acgt_base(seq[k]);
+        fast = __all_sync(0xffffffffu, fast);
+        dp_dispatch<NW>(g, sh, ndp, seq, L, a.match, a.mismatch, a.gap, lane, w, team, fast);
+        team_sync<NW>(team);
+        if (w == 0) {
+            cells += (unsigned long long)ndp * (unsigned long long)L;
+            edge_cells += (unsigned long long)(ndp + sh.preds) * (unsigned long long)L;
+            const int N = sh.nnodes;
+            const int off = team * (NW * WarpMem<NW>::bytes), lc = row_cover(NW, L + 1);
+            const int iend = fast ? end_row<true>(g, sh, order, ndp, L, lc, full, lane, ring)
+                                  : end_row<false>(g, sh, order, ndp, L, lc, full, lane, ring);
+            if (!sh.fail) {
+                const bool ok = fast ? traceback_warp<true>(g, order, seq, L, iend, sh.end_value, a.match, a.mismatch,
+                                                           a.gap, lane, off, lc)
+                                    : traceback_warp<false>(g, order, seq, L, iend, sh.end_value, a.match, a.mismatch,
+                                                            a.gap, lane, off, lc);
+                if (!ok && lane == 0) sh.fail = kFailed;
             }
-            ndp = base;
-            order = g.dporder;
             __syncwarp();
+            if (!sh.fail) add_alignment_warp(g, sh, seq, qual, L, lane, ring);
+            if (!sh.fail) order_insert(g, sh, N, lane, ring);
         }
-        // Row descriptors: shared-memory accumulators when the graph fits,
-        // else the global form below.
-        if (!descriptors_smem(g, sh, order, N, ndp, lane, ring)) {
-            // Row descriptors. DP ranks of the nodes live in shared memory (the
-            // row ring is free until the DP) when they fit, else in global
-            // scratch; bit 31 marks a node with a successor among the rows.
-            int* const dpr = N <= kSmemRanks ? reinterpret_cast<int*>(ring) : g.dprank;
-            for (int i = lane; i < N; i += 32) dpr[i] = 0;
-            __syncwarp();
-            for (int i = lane; i < ndp; i += 32) dpr[order[i]] = i + 1;
-            __syncwarp();
-            // Predecessors by one pass over the edges in id order. A node's
-            // in-edge list is in edge-id order (each layer adds at most one edge
-            // into a node, with a fresh, larger id), which is spoa's predecessor
-            // order. Lanes take 32 consecutive edges; edges into the same row
-            // are ranked by lane, so the order is deterministic. rowdesc[r - 1]
-            // collects the first three predecessor ranks (x, y, z) and the count
-            // (w) of row r; bit 31 of dpr marks a node with a successor row.
-            for (int i = lane; i < ndp; i += 32) g.rowdesc[i] = make_int4(0, 0, 0, 0);
-            __syncwarp();
-            const int E = sh.nedges;
-            const unsigned below = (1u << lane) - 1u;
-            bool any_long = false;
-            for (int c0 = 0; c0 < E; c0 += 32) {
-                const int e = c0 + lane;
-                int rs = 0, rd = 0, src = 0;
-                if (e < E) {
-                    src = g.e_src[e];
-                    const int dst = g.e_dst[e];
-                    rs = dpr[src] & 0x7FFFFFFF;
-                    rd = rs > 0 ? dpr[dst] & 0x7FFFFFFF : 0;
-                }
-                const bool q = rs > 0 && rd > 0;
-                const unsigned grp = __match_any_sync(0xffffffffu, q ? rd : -1 - lane);
-                int cnt = 0;
-                if (q) {
-                    atomicOr(reinterpret_cast<unsigned*>(&dpr[src]), 0x80000000u);
-                    cnt = g.rowdesc[rd - 1].w;
-                }
-                __syncwarp();
-                if (q) {
-                    const int pos = cnt + __popc(grp & below);
-                    int* rdw = reinterpret_cast<int*>(&g.rowdesc[rd - 1]);
-                    if (pos < 3) rdw[pos] = rs;
-                    if ((grp & below) == 0) {
-                        const int tot = cnt + __popc(grp);
-                        rdw[3] = tot;
-                        any_long |= tot > 3;
-                    }
-                }
-                __syncwarp();
-            }
-            any_long = __any_sync(0xffffffffu, any_long);
-            // final descriptors; rows with more than three predecessors get their
-            // full list in pred_idx at an offset from a warp prefix of the counts
-            int list_base = 0;
-            for (int c0 = 0; c0 < ndp; c0 += 32) {
-                const int i = c0 + lane;
-                int4 dd = i < ndp ? g.rowdesc[i] : make_int4(0, 0, 0, 0);
-                const int v = i < ndp ? order[i] : 0;
-                int off = 0;
-                if (any_long) {
-                    int tot = 0;
-                    const int cntl = (i < ndp && dd.w > 3) ? dd.w : 0;
-                    off = list_base + warp_excl(cntl, lane, tot);
-                    list_base += tot;
-                    if (cntl) g.bpred[v] = off;  // list cursor of the node
-                }
-                if (i < ndp) {
-                    const bool sink = (dpr[v] & 0x80000000) == 0;
-                    g.sink[i] = sink ? 1 : 0;
-                    // long rows: x = list offset, y = first predecessor
-                    g.rowdesc[i] = make_int4(dd.w > 3 ? off : dd.x, dd.w > 3 ? dd.x : dd.y, dd.z,
-                                             int(uint32_t(dd.w) | (uint32_t(sink) << 17) | (uint32_t(g.code[v]) << 24)));
-                }
-            }
-            __syncwarp();
-            if (any_long) {
-                // second pass over the edges for the long lists, same ranking
-                for (int c0 = 0; c0 < E; c0 += 32) {
-                    const int e = c0 + lane;
-                    int rs = 0, dst = 0;
-                    bool q = false;
-                    if (e < E) {
-                        dst = g.e_dst[e];
-                        const int rd = dpr[dst] & 0x7FFFFFFF;
-                        if (rd > 0 && desc_np(g.rowdesc[rd - 1].w) > 3) {
-                            rs = dpr[g.e_src[e]] & 0x7FFFFFFF;
-                            q = rs > 0;
-                        }
-                    }
-                    const unsigned grp = __match_any_sync(0xffffffffu, q ? dst : -1 - lane);
-                    int cur = 0;
-                    if (q) cur = g.bpred[dst];
-                    __syncwarp();
-                    if (q) {
-                        g.pred_idx[cur + __popc(grp & below)] = rs;
-                        if ((grp & below) == 0) g.bpred[dst] = cur + __popc(grp);
-                    }
-                    __syncwarp();
-                }
-            }
-            __syncwarp();
-        }
-        const EndCell ec = dp_dispatch(a, g, order, ndp, seq, L, lane, ring);
-        cells += (unsigned long long)ndp * (unsigned long long)L;
-        edge_cells += (unsigned long long)(ndp + ec.preds) * (unsigned long long)L;
-        int iend = ec.row;
-        if (ec.ties > 1) {
-            // several sinks share the best last-column value: spoa takes the
-            // first in its own topological order of the aligned (sub)graph.
-            // A sink outside every aligned group is reached by spoa's DFS
-            // only as a root (no member lists it as an in-edge tail, and
-            // aligned links are symmetric), so such sinks are ranked by node
-            // id; only a tie that involves an aligned sink needs the DFS.
-            int low_id = INT_MAX, low_i = iend;
-            bool grouped = false;
-            for (int i = 1 + lane; i <= ndp; i += 32) {
-                if (!g.sink[i - 1] || g.lastH[i] != ec.value) continue;
-                const int v = order[i - 1];
-                grouped |= g.al_cnt[v] != 0;
-                if (v < low_id) {
-                    low_id = v;
-                    low_i = i;
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const int ov = __shfl_xor_sync(0xffffffffu, low_id, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, low_i, o);
-                if (ov < low_id) {
-                    low_id = ov;
-                    low_i = oi;
-                }
-            }
-            grouped = __any_sync(0xffffffffu, grouped);
-            const int nr = grouped ? topo_sort_warp(g, sh, full, g.rank_to_node, lane, ring) : 0;
-            if (!grouped) {
-                iend = low_i;
-            } else if (nr < 0) {
-                if (lane == 0) sh.fail = kOverflow;
-            } else {
-                for (int r = lane; r < nr; r += 32) g.node_rank[g.rank_to_node[r]] = r;
-                __syncwarp();
-                // the tied sink of lowest rank (ranks are distinct)
-                int best = INT_MAX, bi = iend;
-                for (int i = 1 + lane; i <= ndp; i += 32) {
-                    if (!g.sink[i - 1] || g.lastH[i] != ec.value) continue;
-                    const int rr = g.node_rank[order[i - 1]];
-                    if (rr < best) {
-                        best = rr;
-                        bi = i;
-                    }
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const int ob = __shfl_xor_sync(0xffffffffu, best, o);
-                    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                    if (ob < best) {
-                        best = ob;
-                        bi = oi;
-                    }
-                }
-                iend = bi;
-            }
-            __syncwarp();
-        }
-        if (fast_dp(a, L)) {
-            if (!sh.fail && !traceback_warp(a, g, sh, order, seq, L, iend, lane, ring, ec.h16) && lane == 0)
-                sh.fail = kFailed;
-        } else if (lane == 0 && !sh.fail && !traceback(a, g, sh, order, seq, L, iend)) {
-            sh.fail = kFailed;
-        }
-        __syncwarp();
-        if (sh.fail) break;
-        add_alignment_warp(g, sh, seq, qual, L, lane, ring);
-        if (sh.fail) break;
-        order_insert(g, sh, N, lane, ring);
     }
+    team_sync<NW>(team);
+    if (w != 0) return;
     // spoa's topological order of the final graph for the consensus
     if (!sh.fail) {
         const int nr = topo_sort_warp(g, sh, true, g.rank_to_node, lane, ring);
@@ -2454,46 +2362,48 @@ __device__ void poa_window(const PoaArgs& a, const Graph& g, PoaShared& sh, uint
     __syncwarp();
 }
 
-constexpr int kWarpsPerCta = 4;
-// resident CTAs per SM the register budget is sized for
+// Warps of a full CTA (teams of NW): three CTAs fill an SM's registers and
+// shared memory, with 12 one-warp teams or 24 warps of larger teams.
+__host__ __device__ constexpr int cta_warps(int nw) { return nw == 1 ? 4 : 8; }
+__host__ __device__ constexpr int warp_smem(int nw) { return nw == 1 ? WarpMem<1>::bytes : WarpMem<4>::bytes; }
 constexpr int kCtasPerSm = 3;
 
-__global__ void __launch_bounds__(32 * kWarpsPerCta, kCtasPerSm) poa_kernel(PoaArgs a) {
-    __shared__ PoaShared sh_all[kWarpsPerCta];
-    // the per-warp view of its scratch slot lives in shared memory so the
+template <int NW>
+__global__ void __launch_bounds__(32 * cta_warps(NW), kCtasPerSm) poa_kernel(PoaArgs a) {
+    __shared__ PoaShared sh_all[cta_warps(NW) / NW];
+    // each team's view of its scratch slot lives in shared memory so the
     // ~35 array pointers are not held in registers across the DP
-    __shared__ Graph g_all[kWarpsPerCta];
-    extern __shared__ int4 ring_all[];
+    __shared__ Graph g_all[cta_warps(NW) / NW];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int4* ring = ring_all + wid * (kRingBytesPerWarp / 16);
-    PoaShared& sh = sh_all[wid];
-    const uint32_t slot = blockIdx.x * kWarpsPerCta + wid;
-    if (lane == 0) g_all[wid] = make_graph(a, slot);
-    __syncwarp();
-    const Graph& g = g_all[wid];
-    // with a cap the CTA retires after that many windows per warp, so other
+    const int team = wid / NW, w = wid % NW;
+    PoaShared& sh = sh_all[team];
+    const uint32_t slot = blockIdx.x * (blockDim.x / (32 * NW)) + team;
+    if (w == 0 && lane == 0) g_all[team] = make_graph(a, slot);
+    const Graph& g = g_all[team];
+    // with a cap the CTA retires after that many windows per team, so other
     // streams' kernels get SMs between launches (the host launches enough)
     for (uint32_t done = 0; a.per_warp_cap == 0 || done < a.per_warp_cap; ++done) {
-        unsigned k = 0;
-        if (lane == 0) k = atomicAdd(&a.counters[0], 1u);
-        k = __shfl_sync(0xffffffffu, k, 0);
+        if (w == 0 && lane == 0) sh.next = atomicAdd(&a.counters[0], 1u);
+        team_sync<NW>(team);
+        const uint32_t k = sh.next;
         if (k >= a.nwin) break;
-        poa_window(a, g, sh, a.order[k], lane, ring);
+        poa_window<NW>(a, g, sh, a.order[k], lane, w, team);
+        team_sync<NW>(team);
     }
 }
 
-// Plain comparison form: one window per one-warp block, block b takes window
+// Plain comparison form: one window per one-team block, block b takes window
 // order[b] with scratch slot b, one launch per batch, no work queue. Same
 // per-window code as poa_kernel, so results are identical.
-__global__ void __launch_bounds__(32 * kWarpsPerCta, kCtasPerSm) poa_plain_kernel(PoaArgs a) {
+constexpr int kPlainWarps = 1;
+__global__ void __launch_bounds__(32 * cta_warps(kPlainWarps), kCtasPerSm) poa_plain_kernel(PoaArgs a) {
     __shared__ PoaShared sh;
     __shared__ Graph g;
-    extern __shared__ int4 ring_all[];
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (blockIdx.x >= a.nwin) return;
-    if (lane == 0) g = make_graph(a, blockIdx.x);
-    __syncwarp();
-    poa_window(a, g, sh, a.order[blockIdx.x], lane, ring_all);
+    if (threadIdx.x == 0) g = make_graph(a, blockIdx.x);
+    team_sync<kPlainWarps>(0);
+    poa_window<kPlainWarps>(a, g, sh, a.order[blockIdx.x], lane, w, 0);
 }
 
 // ---------------- shared queue (serving) ----------------
@@ -2506,60 +2416,65 @@ struct PoaSvcArgs {
     SvcQueueDev q;
 };
 
-// Persistent consensus over the shared queue: each warp owns one scratch
+// Persistent consensus over the shared queue: each team owns one scratch
 // slot and takes windows of any job until the queue stays empty. Sized for
 // at most kSvcCtasPerSm resident CTAs per SM, so that the rest of each SM
 // stays free for the alignment and layer kernels of newly admitted jobs.
 constexpr int kSvcCtasPerSm = 3;
-__global__ void __launch_bounds__(32 * kWarpsPerCta, kSvcCtasPerSm) poa_service_kernel(PoaSvcArgs s) {
-    __shared__ PoaShared sh_all[kWarpsPerCta];
-    __shared__ Graph g_all[kWarpsPerCta];
-    __shared__ PoaArgs a_all[kWarpsPerCta];
-    extern __shared__ int4 ring_all[];
+constexpr int kSvcTeamWarps = 1;
+__global__ void __launch_bounds__(32 * cta_warps(kSvcTeamWarps), kSvcCtasPerSm) poa_service_kernel(PoaSvcArgs s) {
+    constexpr int NW = kSvcTeamWarps, T = cta_warps(NW) / NW;
+    __shared__ PoaShared sh_all[T];
+    __shared__ Graph g_all[T];
+    __shared__ PoaArgs a_all[T];
+    __shared__ unsigned long long item_all[T];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int4* ring = ring_all + wid * (kRingBytesPerWarp / 16);
-    PoaShared& sh = sh_all[wid];
-    const uint32_t slot = blockIdx.x * kWarpsPerCta + wid;
-    if (lane == 0) g_all[wid] = make_graph(s.base, slot);
-    __syncwarp();
+    const int team = wid / NW, w = wid % NW;
+    PoaShared& sh = sh_all[team];
+    const uint32_t slot = blockIdx.x * T + team;
+    if (w == 0 && lane == 0) g_all[team] = make_graph(s.base, slot);
     for (;;) {
-        unsigned long long it = 0;
-        if (lane == 0) it = svc_claim(s.q, slot);
-        it = __shfl_sync(0xffffffffu, it, 0);
-        if (it == ~0ull) break;
-        const uint32_t job = uint32_t(it >> 32), win = uint32_t(it);
         uint32_t total = 0, gen = 0;
-        if (lane == 0) {
-            // the record is rewritten for every batch that reuses the slot:
-            // read it past L1
-            const volatile PoaJobDev& J = s.jobs[job];
-            PoaArgs a = s.base;
-            a.in = const_cast<const uint8_t*>(J.in);
-            a.wins = const_cast<const PoaWinDev*>(J.wins);
-            a.layers = const_cast<const PoaLayerDev*>(J.layers);
-            a.out = const_cast<char*>(J.out);
-            a.out_len = const_cast<uint32_t*>(J.out_len);
-            a.flags = const_cast<uint8_t*>(J.flags);
-            a.trim = J.trim;
-            a.cells = const_cast<unsigned long long*>(J.cells);
-            total = J.head.total;
-            gen = J.head.generation;
-            a.nwin = total;
-            a_all[wid] = a;
+        if (w == 0 && lane == 0) {
+            const unsigned long long it = svc_claim(s.q, slot);
+            item_all[team] = it;
+            if (it != ~0ull) {
+                // the record is rewritten for every batch that reuses the slot:
+                // read it past L1
+                const volatile PoaJobDev& J = s.jobs[uint32_t(it >> 32)];
+                PoaArgs a = s.base;
+                a.in = const_cast<const uint8_t*>(J.in);
+                a.wins = const_cast<const PoaWinDev*>(J.wins);
+                a.layers = const_cast<const PoaLayerDev*>(J.layers);
+                a.out = const_cast<char*>(J.out);
+                a.out_len = const_cast<uint32_t*>(J.out_len);
+                a.flags = const_cast<uint8_t*>(J.flags);
+                a.trim = J.trim;
+                a.cells = const_cast<unsigned long long*>(J.cells);
+                total = J.head.total;
+                gen = J.head.generation;
+                a.nwin = total;
+                a_all[team] = a;
+            }
         }
-        __syncwarp();
-        poa_window(a_all[wid], g_all[wid], sh, win, lane, ring);
+        team_sync<NW>(team);
+        const unsigned long long it = item_all[team];
+        if (it == ~0ull) break;
+        poa_window<NW>(a_all[team], g_all[team], sh, uint32_t(it), lane, w, team);
         __threadfence();
-        __syncwarp();
-        if (lane == 0) svc_item_done(s.q, job, total, gen);
+        team_sync<NW>(team);
+        if (w == 0 && lane == 0) svc_item_done(s.q, uint32_t(it >> 32), total, gen);
     }
 }
 
 }  // namespace
 
+// Row stride that holds rows of wc columns in every team form.
+static int max_cover(int wc) { return std::max(row_cover(1, wc), row_cover(4, wc)); }
+
 size_t PoaEngine::slot_bytes_for(uint32_t max_layer_length) {
     const int ncap = 4096;
-    return walk_layout(ncap, 2 * ncap, ncap, row_cover(int(max_layer_length) + 1), [](int, size_t) {});
+    return walk_layout(ncap, 2 * ncap, ncap, max_cover(int(max_layer_length) + 1), [](int, size_t) {});
 }
 
 PoaEngine::PoaEngine(const DeviceInfo& dev, cudaStream_t stream, int8_t m, int8_t x, int8_t g)
@@ -2568,7 +2483,8 @@ PoaEngine::PoaEngine(const DeviceInfo& dev, cudaStream_t stream, int8_t m, int8_
     check_cuda(cudaEventCreate(&ev1_), "cudaEventCreate");
     check_cuda(cudaEventCreate(&ev2_), "cudaEventCreate");
     check_cuda(cudaEventCreate(&ev3_), "cudaEventCreate");
-    prefer_max_shared(reinterpret_cast<const void*>(poa_kernel));
+    prefer_max_shared(reinterpret_cast<const void*>(poa_kernel<1>));
+    prefer_max_shared(reinterpret_cast<const void*>(poa_kernel<4>));
     prefer_max_shared(reinterpret_cast<const void*>(poa_plain_kernel));
 }
 
@@ -2818,25 +2734,36 @@ void PoaEngine::run_list(std::vector<uint32_t> todo, int ncap, bool plain) {
     float total_ms = 0;
     // DP row width: every layer's columns rounded up to whole warp passes
     const uint32_t* lens_max = &max_len_;
-    const int lcap = row_cover(int(*lens_max) + 1);
+    const int lcap = max_cover(int(*lens_max) + 1);
     while (!todo.empty()) {
         const int ecap = 2 * ncap, acap = ncap;
         const size_t slot = walk_layout(ncap, ecap, acap, lcap, [](int, size_t) {});
-        // resident windows (one warp each): enough to fill the SMs, bounded by
+        // Warps per window. Four warps side by side finish a window sooner
+        // (150 windows of 1000 bases at 20x: 55 ms against 85 ms), one warp
+        // spends the fewest instructions (2001 windows of 500 bases at 50x:
+        // 139 ms against 211 ms). The line lies at four windows per SM,
+        // where four-warp teams no longer all run at once.
+        const int nw = plain ? kPlainWarps : todo.size() <= 4 * size_t(dev_.sm_count) ? 4 : 1;
+        const size_t teams = size_t(cta_warps(nw)) / nw;  // per full CTA
+        // resident windows (one team each): enough to fill the SMs, bounded by
         // a scratch budget
         const size_t budget = scratch_budget_;
         // resident windows: the device's tuned CTAs per SM on the context's
         // share of the SMs (all by default)
         const uint32_t cps = std::min<uint32_t>(kCtasPerSm, tuning_get(dev_.device).consensus_ctas_per_sm);
-        const size_t resident = std::max<size_t>(
-            kWarpsPerCta, size_t(dev_.sm_count) * kWarpsPerCta * cps * sm_share_pct_ / 100);
+        const size_t resident =
+            std::max<size_t>(teams, size_t(dev_.sm_count) * teams * cps * sm_share_pct_ / 100);
         size_t slots = std::min<size_t>(todo.size(), plain ? todo.size() : resident);
         // RB_POA_SLOTS caps the resident windows (smaller scratch, e.g. for
         // profiler captures); results do not depend on it
         if (const char* e = getenv("RB_POA_SLOTS"))
             slots = std::max<size_t>(1, std::min<size_t>(slots, strtoull(e, nullptr, 10)));
         while (slots > 1 && slots * slot > budget) slots /= 2;
-        if (!plain) slots = (slots + kWarpsPerCta - 1) / kWarpsPerCta * kWarpsPerCta;
+        // teams per CTA: one while that still leaves SMs free, so that a small
+        // batch spreads over all of them
+        const size_t per_cta =
+            std::max<size_t>(1, std::min<size_t>(teams, slots / std::max<size_t>(1, size_t(dev_.sm_count) * sm_share_pct_ / 100)));
+        if (!plain) slots = (slots + per_cta - 1) / per_cta * per_cta;
         d_graph_.reserve(slots * slot);
         DevBuf& d_todo = d_dp_;
         d_todo.reserve(todo.size() * 4);
@@ -2868,19 +2795,21 @@ void PoaEngine::run_list(std::vector<uint32_t> todo, int ncap, bool plain) {
         check_cuda(cudaEventRecord(ev0_, stream_), "cudaEventRecord");
         if (plain) {
             // one launch per batch of `slots` windows
-            check_cuda(cudaFuncSetAttribute(poa_plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            kRingBytesPerWarp),
+            const int smem = kPlainWarps * warp_smem(kPlainWarps);
+            check_cuda(cudaFuncSetAttribute(poa_plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                        "cudaFuncSetAttribute");
             for (size_t b0 = 0; b0 < todo.size(); b0 += slots) {
                 PoaArgs ab = a;
                 ab.order = a.order + b0;
                 ab.nwin = uint32_t(std::min(slots, todo.size() - b0));
-                poa_plain_kernel<<<int(ab.nwin), 32, kRingBytesPerWarp, stream_>>>(ab);
+                poa_plain_kernel<<<int(ab.nwin), 32 * kPlainWarps, smem, stream_>>>(ab);
                 ++stats_.launches;
             }
         } else {
-            const int smem = kWarpsPerCta * kRingBytesPerWarp;
-            check_cuda(cudaFuncSetAttribute(poa_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+            void (*const kernel)(PoaArgs) = nw == 4 ? poa_kernel<4> : poa_kernel<1>;
+            const int smem = int(per_cta) * nw * warp_smem(nw);
+            check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            cta_warps(nw) * warp_smem(nw)),
                        "cudaFuncSetAttribute");
             // persistent by default; with a per-warp cap, enough launches
             // back to back that every window is taken
@@ -2890,7 +2819,7 @@ void PoaEngine::run_list(std::vector<uint32_t> todo, int ncap, bool plain) {
                 launches = (todo.size() + slots * yield_windows_ - 1) / (slots * yield_windows_);
             }
             for (size_t l = 0; l < launches; ++l) {
-                poa_kernel<<<int(slots / kWarpsPerCta), 32 * kWarpsPerCta, smem, stream_>>>(a);
+                kernel<<<int(slots / per_cta), int(per_cta) * nw * 32, smem, stream_>>>(a);
                 ++stats_.launches;
             }
         }
@@ -2976,7 +2905,8 @@ struct PoaSvcState {
 namespace {
 cudaError_t launch_poa_service(cudaStream_t stream, void* user) {
     const PoaSvcState* S = static_cast<const PoaSvcState*>(user);
-    poa_service_kernel<<<S->grid, 32 * kWarpsPerCta, kWarpsPerCta * kRingBytesPerWarp, stream>>>(S->args);
+    poa_service_kernel<<<S->grid, 32 * cta_warps(kSvcTeamWarps), cta_warps(kSvcTeamWarps) * warp_smem(kSvcTeamWarps),
+                         stream>>>(S->args);
     return cudaGetLastError();
 }
 }  // namespace
@@ -2991,13 +2921,14 @@ PoaService::PoaService(int device, int8_t m, int8_t x, int8_t g, uint32_t window
     // slot layout for layers up to three window lengths; longer ones (and
     // graphs over 4096 nodes) overflow and run again in the job's own engine
     const int ncap = 4096, ecap = 2 * ncap, acap = ncap;
-    const int lcap = row_cover(int(std::max<uint32_t>(window_length, 1)) * 3 + 1);
+    const int lcap = row_cover(kSvcTeamWarps, int(std::max<uint32_t>(window_length, 1)) * 3 + 1);
+    const size_t teams = cta_warps(kSvcTeamWarps) / kSvcTeamWarps;
     const size_t slot = walk_layout(ncap, ecap, acap, lcap, [](int, size_t) {});
     const uint32_t cps = std::max<uint32_t>(1, std::min<uint32_t>(ctas_per_sm, kSvcCtasPerSm));
-    size_t slots = size_t(sm_count) * cps * kWarpsPerCta;
-    while (slots > kWarpsPerCta && slots * slot > scratch_budget) slots -= kWarpsPerCta;
+    size_t slots = size_t(sm_count) * cps * teams;
+    while (slots > teams && slots * slot > scratch_budget) slots -= teams;
     S->slots = uint32_t(slots);
-    S->grid = uint32_t(slots / kWarpsPerCta);
+    S->grid = uint32_t(slots / teams);
     check_cuda(cudaMalloc(&S->d_scratch, slots * slot), "cudaMalloc service scratch");
     PoaSvcArgs& A = S->args;
     memset(&A, 0, sizeof(A));
@@ -3014,7 +2945,7 @@ PoaService::PoaService(int device, int8_t m, int8_t x, int8_t g, uint32_t window
     A.jobs = static_cast<const PoaJobDev*>(S->ring.records());
     A.q = S->ring.queue();
     check_cuda(cudaFuncSetAttribute(poa_service_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kWarpsPerCta * kRingBytesPerWarp),
+                                    cta_warps(kSvcTeamWarps) * warp_smem(kSvcTeamWarps)),
                "cudaFuncSetAttribute");
     prefer_max_shared(reinterpret_cast<const void*>(poa_service_kernel));
     st_ = S.release();
