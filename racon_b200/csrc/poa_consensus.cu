@@ -7,12 +7,14 @@
 // time; teams are persistent and pull windows from a size-sorted queue. Each
 // team has a slot of global scratch (graph arrays first, then the DP score
 // rows) and shared memory (the DP's row rings, scratch for the graph steps).
-// * Per layer: the subgraph of a partial layer, row descriptors (first
-//   predecessor ranks, count, sink flag, base), the DP, the end cell, the
-//   traceback and the insertion of the aligned layer.
-//   The steps that walk the graph build compact uint16 adjacency lists or
-//   accumulators in shared memory when they fit, so their dependent steps
-//   read shared memory; loads of graph arrays go out 128 entries at a time.
+// * In-edges are kept with their node, in the order in which they were added,
+//   the first eight in two 16-byte words each for sources and weights, so that
+//   building a layer's rows and adding its edges are independent per node.
+// * Per layer: the subgraph of a partial layer, row descriptors (predecessor
+//   ranks, count, base), the DP, the end cell, the traceback and the insertion
+//   of the aligned layer. Per-node and per-position steps run on the whole
+//   team with four entries per thread in flight; the few serial ones (subgraph
+//   sweep, DFS, bundle scores) run on one lane over shared memory.
 // * The DP runs one row (graph node in a valid topological order kept
 //   incrementally) at a time, the team's warps side by side on strips of its
 //   columns (dp_strip), on slanted scores H - column * gap, so that the
@@ -21,10 +23,10 @@
 //   scores, in spoa's order (diagonal through each predecessor, then
 //   vertical, then horizontal).
 // * The NW end cell is the first sink in spoa's topological order with the
-//   best last-column score; spoa's DFS order is built only when tied sinks
-//   belong to aligned groups.
-// * After the last layer: spoa's topological order, heaviest bundle (scores
-//   in shared memory), branch completion, coverages and trimming.
+//   best last-column score; spoa's DFS order is built only when that cannot be
+//   told from node ids (end_row).
+// * After the last layer: heaviest bundle (scores in shared memory, spoa's
+//   topological order only for ties), branch completion, coverages, trimming.
 // Exact int32 arithmetic throughout; results are byte-identical to the CPU
 // algorithm by construction.
 #include <cuda_runtime.h>
@@ -37,6 +39,7 @@
 #include <cstdlib>
 #include <memory>
 #include <numeric>
+#include <type_traits>
 
 #include "rb_internal.hpp"
 #include "ring_queue.cuh"
@@ -90,97 +93,57 @@ struct PoaArgs {
 };
 
 // Per-slot scratch view.
+constexpr int kInline = 8;  // in-edges kept with their node
+constexpr int kGraphArrays = 39;
 struct Graph {
-    uint8_t* code;
+    // nodes
+    uint8_t *code, *flag;
     uint32_t* cov;
-    int *in_head, *in_tail, *out_head, *out_tail, *al_head, *al_tail;
-    uint8_t *mark, *prim, *member, *sink;
-    int *dprank, *rank_to_node, *dporder, *node_rank;
-    int *e_src, *e_dst, *e_w, *e_next_in, *e_next_out;
-    int *a_node, *a_next;
-    int* stack;
-    int *pred_off, *pred_idx;
-    int4* rowdesc;  // per DP row: first three predecessor ranks (or the list offset) | count, sink, base
-    int* aln_node;  // per sequence position of the layer: node on its path, -1 for an inserted base
-    long long* bscore;
-    int* bpred;
-    int* cons;
+    int *in_cnt, *out_cnt, *al_cnt;
+    int4 *in_src, *in_w;    // [N][2]: the first kInline in-edges' sources and weights
+    int *ov_head, *ov_tail; // list of the further ones
+    int4* al4;              // the first four aligned nodes
+    int *al_head, *al_tail; // list of the further ones
+    int *e_src, *e_w, *e_next;  // in-edges past kInline
+    int *a_node, *a_next;       // aligned entries past four
     // valid topological order kept incrementally (rank -> node, node -> rank),
-    // its double buffer, per-rank shift counts and the new nodes of a layer
-    int *ord, *ord2, *my_rank, *shift, *nw_node, *nw_slot;
+    // its double buffer, per-rank shift counts
+    int *ord, *ord2, *rank, *shift;
+    int *dporder, *sub_rank;  // rows of a partial layer, node -> row (0: none)
+    int *dfs, *dfs_rank;      // spoa's DFS order and its inverse
+    int* stack;
+    int4* rowdesc;            // per DP row (build_rows)
+    int* pred_idx;
+    int *sink_rows, *sink_h;  // sink rows and their last-column scores
+    // per sequence position of the layer: node on its path (-1 for an
+    // inserted base), node id, order slot; order slots of the new nodes
+    int *path, *nid, *slot, *new_slot;
+    long long* bscore;
+    int *bpred, *cons;
     int* H;
-    int* lastH;   // per DP row (sinks): score of the last column
-    // per-node in-edge and aligned-entry counts, owner node of each aligned
-    // entry (for the compact lists built in shared memory)
-    int *in_cnt, *al_cnt, *a_owner, *out_cnt;
     int ncap, ecap, acap, scap, lcap;
 };
 
 __host__ __device__ size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
-// Row descriptor word w: predecessor count (17 bits) | sink << 17 | base << 24.
-__device__ __forceinline__ int desc_np(int w) { return w & 0x1FFFF; }
-__device__ __forceinline__ bool desc_sink(int w) { return (w >> 17) & 1; }
-__device__ __forceinline__ uint32_t desc_base(int w) { return uint32_t(w) >> 24; }
-
-struct SlotLayout {
-    size_t bytes;
-};
-
+// Offsets of the slot's arrays: f(pointer to the Graph member's place, offset).
 template <class F>
 __host__ __device__ size_t walk_layout(int ncap, int ecap, int acap, int lcap, F&& f) {
     size_t off = 0;
-    auto take = [&](size_t bytes, int id) {
-        f(id, off);
-        off += align256(bytes);
-    };
     const size_t N = size_t(ncap), E = size_t(ecap), A = size_t(acap), L = size_t(lcap);
     const size_t S = N + E + A + 16;
     // graph arrays (touched by the pointer-walking steps) first, packed;
-    // the DP matrices, streamed once per layer, last
-    take(N, 0);            // code
-    take(N * 4, 1);        // cov
-    take(N * 4, 2);        // in_head
-    take(N * 4, 3);        // in_tail
-    take(N * 4, 4);        // out_head
-    take(N * 4, 5);        // out_tail
-    take(N * 4, 6);        // al_head
-    take(N * 4, 7);        // al_tail
-    take(N, 8);            // mark
-    take(N, 9);            // prim
-    take(N, 10);           // member
-    take(N, 11);           // sink
-    take(N * 4, 12);       // dprank
-    take(N * 4, 13);       // rank_to_node
-    take(N * 4, 14);       // dporder
-    take(N * 4, 15);       // node_rank
-    take(E * 4, 16);       // e_src
-    take(E * 4, 17);       // e_dst
-    take(E * 4, 18);       // e_w
-    take(E * 4, 19);       // e_next_in
-    take(E * 4, 20);       // e_next_out
-    take(A * 4, 21);       // a_node
-    take(A * 4, 22);       // a_next
-    take(N * 4, 33);       // ord
-    take(N * 4, 34);       // ord2
-    take(N * 4, 35);       // my_rank
-    take((N + 2) * 4, 36); // shift
-    take(N * 4, 37);       // nw_node
-    take(N * 4, 38);       // nw_slot
-    take((N + 32) * 16, 39);  // rowdesc
-    take(N * 4, 40);       // in_cnt
-    take(N * 4, 41);       // al_cnt
-    take(A * 4, 42);       // a_owner
-    take(N * 4, 43);       // out_cnt
-    take((N + 2) * 4, 24); // pred_off
-    take((E + N + 2) * 4, 25);  // pred_idx
-    take((L + 2) * 4, 26);  // aln_node
-    take(N * 8, 28);       // bscore
-    take(N * 4, 29);       // bpred
-    take(N * 4, 30);       // cons
-    take(S * 4, 23);       // stack
-    take((N + 1) * L * 4, 31);  // H
-    take((N + 1) * 4, 44);      // lastH: last-column score of each sink row
+    // the DP matrix, streamed once per layer, last
+    const size_t bytes[kGraphArrays] = {
+        N,       N + 8,   N * 4,   N * 4,   N * 4,   N * 4,    N * 32,  N * 32,        N * 4,   N * 4,
+        N * 16,  N * 4,   N * 4,   E * 4,   E * 4,   E * 4,    A * 4,   A * 4,         N * 4,   N * 4,
+        N * 4,   (N + 2) * 4,      N * 4,   N * 4,   N * 4,    N * 4,   S * 4,         (N + 32) * 16,
+        (N * kInline + E + 2) * 4, N * 4,   N * 4,   (L + 2) * 4, (L + 2) * 4, (L + 2) * 4, N * 4, N * 8,
+        N * 4,   N * 4,   (N + 1) * L * 4};
+    for (int id = 0; id < kGraphArrays; ++id) {
+        f(id, off);
+        off += align256(bytes[id]);
+    }
     // whole 2 MiB pages per slot, so that a slot's graph arrays share one page
     off = (off + (size_t(2) << 20) - 1) & ~((size_t(2) << 20) - 1);
     return off;
@@ -189,51 +152,16 @@ __host__ __device__ size_t walk_layout(int ncap, int ecap, int acap, int lcap, F
 __device__ Graph make_graph(const PoaArgs& a, uint32_t slot) {
     uint8_t* base = a.scratch + size_t(slot) * a.slot_bytes;
     Graph g;
-    void* p[45];
+    void* p[kGraphArrays];
     walk_layout(a.ncap, a.ecap, a.acap, a.lcap, [&](int id, size_t off) { p[id] = base + off; });
-    g.code = (uint8_t*)p[0];
-    g.cov = (uint32_t*)p[1];
-    g.in_head = (int*)p[2];
-    g.in_tail = (int*)p[3];
-    g.out_head = (int*)p[4];
-    g.out_tail = (int*)p[5];
-    g.al_head = (int*)p[6];
-    g.al_tail = (int*)p[7];
-    g.mark = (uint8_t*)p[8];
-    g.prim = (uint8_t*)p[9];
-    g.member = (uint8_t*)p[10];
-    g.sink = (uint8_t*)p[11];
-    g.dprank = (int*)p[12];
-    g.rank_to_node = (int*)p[13];
-    g.dporder = (int*)p[14];
-    g.node_rank = (int*)p[15];
-    g.e_src = (int*)p[16];
-    g.e_dst = (int*)p[17];
-    g.e_w = (int*)p[18];
-    g.e_next_in = (int*)p[19];
-    g.e_next_out = (int*)p[20];
-    g.a_node = (int*)p[21];
-    g.a_next = (int*)p[22];
-    g.stack = (int*)p[23];
-    g.pred_off = (int*)p[24];
-    g.pred_idx = (int*)p[25];
-    g.aln_node = (int*)p[26];
-    g.bscore = (long long*)p[28];
-    g.bpred = (int*)p[29];
-    g.cons = (int*)p[30];
-    g.H = (int*)p[31];
-    g.ord = (int*)p[33];
-    g.ord2 = (int*)p[34];
-    g.my_rank = (int*)p[35];
-    g.shift = (int*)p[36];
-    g.nw_node = (int*)p[37];
-    g.nw_slot = (int*)p[38];
-    g.rowdesc = (int4*)p[39];
-    g.in_cnt = (int*)p[40];
-    g.al_cnt = (int*)p[41];
-    g.a_owner = (int*)p[42];
-    g.out_cnt = (int*)p[43];
-    g.lastH = (int*)p[44];
+    int id = 0;
+    auto set = [&](auto*& m) { m = static_cast<std::remove_reference_t<decltype(m)>>(p[id++]); };
+    set(g.code), set(g.flag), set(g.cov), set(g.in_cnt), set(g.out_cnt), set(g.al_cnt), set(g.in_src), set(g.in_w);
+    set(g.ov_head), set(g.ov_tail), set(g.al4), set(g.al_head), set(g.al_tail);
+    set(g.e_src), set(g.e_w), set(g.e_next), set(g.a_node), set(g.a_next);
+    set(g.ord), set(g.ord2), set(g.rank), set(g.shift), set(g.dporder), set(g.sub_rank), set(g.dfs), set(g.dfs_rank);
+    set(g.stack), set(g.rowdesc), set(g.pred_idx), set(g.sink_rows), set(g.sink_h);
+    set(g.path), set(g.nid), set(g.slot), set(g.new_slot), set(g.bscore), set(g.bpred), set(g.cons), set(g.H);
     g.ncap = a.ncap;
     g.ecap = a.ecap;
     g.acap = a.acap;
@@ -244,561 +172,20 @@ __device__ Graph make_graph(const PoaArgs& a, uint32_t slot) {
 
 // Shared per-team state.
 struct PoaShared {
-    int nnodes, nedges, naligned, nseq;
-    int nnew;     // new nodes of the last insertion (g.nw_node / g.nw_slot)
-    int nranks;   // entries of rank_to_node (full graph order)
-    int fail;     // 0 ok, else PoaFlag
-    int ndp;      // rows of the current DP
-    int partial;  // the current layer is aligned to a subgraph
-    int end_value;  // score of the NW end cell of the current layer
-    int preds;    // predecessor links over the DP rows (edge-cells = |layer| x (rows + preds))
-    int scratch_bytes;  // the team's shared memory, scratch between the DPs
-    uint32_t next;      // queue position the team took
+    int nnodes, nseq;
+    int nedges, naligned;  // entries of the overflow pools in use
+    int nnew;              // new nodes of the last insertion
+    int fail;              // 0 ok, else PoaFlag
+    int ndp;               // rows of the current DP
+    int nsinks, nlisted;   // sink rows; entries of pred_idx in use
+    int preds;             // predecessor links over the DP rows (edge-cells = |layer| x (rows + preds))
+    int end_value;         // score of the NW end cell of the current layer
+    int scratch_bytes;     // the team's shared memory, scratch between the DPs
+    uint32_t next;         // queue position the team took
     volatile int done[4];  // per warp: rows it has finished (counting on from pass to pass)
 };
 
-// ---------------- graph primitives (thread 0) ----------------
-
-// spoa's DFS topological order over the nodes with member flag set (all nodes
-// when all_nodes). Writes the order to out; returns its length, -1 on overflow.
-__device__ int g_topo_sort(const Graph& g, PoaShared& sh, bool all_nodes, int* out) {
-    const int N = sh.nnodes;
-    int nr = 0;
-    int sp = 0;
-    for (int i = 0; i < N; ++i) {
-        if (!all_nodes && !g.member[i]) continue;
-        if (g.mark[i] != 0) continue;
-        g.stack[sp++] = i;
-        while (sp > 0) {
-            const int v = g.stack[sp - 1];
-            bool valid = true;
-            if (g.mark[v] != 2) {
-                for (int e = g.in_head[v]; e != -1; e = g.e_next_in[e]) {
-                    const int u = g.e_src[e];
-                    if (!all_nodes && !g.member[u]) continue;
-                    if (g.mark[u] != 2) {
-                        if (sp >= g.scap) return -1;
-                        g.stack[sp++] = u;
-                        valid = false;
-                    }
-                }
-                if (g.prim[v]) {
-                    for (int x = g.al_head[v]; x != -1; x = g.a_next[x]) {
-                        const int y = g.a_node[x];
-                        if (!all_nodes && !g.member[y]) continue;
-                        if (g.mark[y] != 2) {
-                            if (sp >= g.scap) return -1;
-                            g.stack[sp++] = y;
-                            g.prim[y] = 0;
-                            valid = false;
-                        }
-                    }
-                }
-                if (valid) {
-                    g.mark[v] = 2;
-                    if (g.prim[v]) {
-                        out[nr++] = v;
-                        for (int x = g.al_head[v]; x != -1; x = g.a_next[x]) {
-                            const int y = g.a_node[x];
-                            if (!all_nodes && !g.member[y]) continue;
-                            out[nr++] = y;
-                        }
-                    }
-                } else {
-                    g.mark[v] = 1;
-                }
-            }
-            if (valid) --sp;
-        }
-    }
-    return nr;
-}
-
-// Nodes reachable backwards (in-edges and aligned groups) from end_node whose
-// id is not below begin_node (spoa's subgraph node set).
-__device__ bool g_mark_subgraph(const Graph& g, PoaShared& sh, int begin_node, int end_node) {
-    if (end_node < 0 || end_node >= sh.nnodes) {
-        sh.fail = kFailed;
-        return true;
-    }
-    int sp = 0;
-    g.stack[sp++] = end_node;
-    while (sp > 0) {
-        const int v = g.stack[--sp];
-        if (!g.member[v] && v >= begin_node) {
-            for (int e = g.in_head[v]; e != -1; e = g.e_next_in[e]) {
-                if (sp >= g.scap) return false;
-                g.stack[sp++] = g.e_src[e];
-            }
-            for (int x = g.al_head[v]; x != -1; x = g.a_next[x]) {
-                if (sp >= g.scap) return false;
-                g.stack[sp++] = g.a_node[x];
-            }
-            g.member[v] = 1;
-        }
-    }
-    return true;
-}
-
-__device__ int layer_weight(const uint8_t* qual, int k) { return qual ? int(qual[k]) - 33 : 1; }
-
-// Warp prefix helpers: exclusive prefix of v over lanes, and the total.
-__device__ __forceinline__ int warp_excl(int v, int lane, int& total) {
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    total = __shfl_sync(0xffffffffu, x, 31);
-    return x - v;
-}
-
-// Out-edges of nodes [0, N) as uint16 lists in shared memory: destination and
-// edge id, grouped by source (order within a source is irrelevant: the lists
-// answer "does u -> v exist, and which edge is it"). Loads of the edge
-// arrays go four 32-edge chunks at a time. Returns false, building nothing,
-// when the lists do not fit in `cap` bytes or 16-bit indices.
-struct OutCsr {
-    uint16_t* off;  // [N + 1]
-    uint16_t* dst;  // [E]
-    uint16_t* eid;  // [E]
-};
-__device__ bool build_out_csr(const Graph& g, int N, int E, int lane, void* smem, int cap, OutCsr& c) {
-    if (N >= 65535 || E >= 65535 || 2 * (size_t(N) + 1) + 4 * size_t(E) > size_t(cap)) return false;
-    c.off = reinterpret_cast<uint16_t*>(smem);
-    c.dst = c.off + (N + 1);
-    c.eid = c.dst + E;
-    int b = 0;
-    for (int c4 = 0; c4 < N; c4 += 128) {
-        int cn[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int v = c4 + 32 * u + lane;
-            cn[u] = v < N ? g.out_cnt[v] : 0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int v = c4 + 32 * u + lane;
-            int t = 0;
-            const int x = warp_excl(cn[u], lane, t);
-            if (v < N) c.off[v] = uint16_t(b + x);
-            b += t;
-        }
-    }
-    if (lane == 0) c.off[N] = uint16_t(E);
-    __syncwarp();
-    const unsigned below = (1u << lane) - 1u;
-    for (int c4 = 0; c4 < E; c4 += 128) {
-        int ss[4], ds[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int e = c4 + 32 * u + lane;
-            ss[u] = e < E ? g.e_src[e] : -1 - lane;
-            ds[u] = e < E ? g.e_dst[e] : 0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int src = ss[u];
-            const unsigned grp = __match_any_sync(0xffffffffu, src);
-            const int cur = src >= 0 ? c.off[src] : 0;
-            __syncwarp();
-            if (src >= 0) {
-                const int q = cur + __popc(grp & below);
-                c.dst[q] = uint16_t(ds[u]);
-                c.eid[q] = uint16_t(c4 + 32 * u + lane);
-                if ((grp & below) == 0) c.off[src] = uint16_t(cur + __popc(grp));
-            }
-            __syncwarp();
-        }
-    }
-    for (int c0 = ((N - 1) / 32) * 32; c0 >= 0; c0 -= 32) {
-        const int v = c0 + lane;
-        const uint16_t pv = (v < N && v > 0) ? c.off[v - 1] : uint16_t(0);
-        __syncwarp();
-        if (v < N) c.off[v] = pv;
-        __syncwarp();
-    }
-    return true;
-}
-
-// Graph::add_alignment for one layer, by the whole warp. A path visits every
-// node and every aligned group at most once, so the per-position work is
-// independent: classify each aligned base (existing node, new base, new
-// member of an aligned group), number the new nodes in path order, then in
-// parallel create nodes, aligned-group links, edges P[k-1] -> P[k] with
-// weight w[k-1] + w[k] (every sequence position k owns exactly one path node
-// P[k]) and coverage, and list the new nodes with their order slots (see
-// order_insert). Per-entry scratch lives in g.stack: [0,m) node, [m,2m) kind
-// | aligned-count << 2, [2m,3m) anchor slot, [3m,4m) group start.
-__device__ void add_alignment_warp(const Graph& g, PoaShared& sh, const uint8_t* seq, const uint8_t* qual,
-                                   int len, int lane, int4* ring) {
-    const int m = len;  // the walk gives every position a node or -1
-    const int nold = sh.nnodes;
-    if (len == 0) return;
-    if (4 * m + 64 > g.scap) {
-        if (lane == 0) sh.fail = kOverflow;
-        __syncwarp();
-        return;
-    }
-    int* e_nid = g.stack;
-    int* e_kind = g.stack + m;
-    int* e_slot = g.stack + 2 * m;
-    int* e_start = g.stack + 3 * m;
-    // existing-edge lookups of step 5 from shared memory when they fit
-    OutCsr oc;
-    const bool ocsr = build_out_csr(g, nold, sh.nedges, lane, ring, sh.scratch_bytes, oc);
-    // 1. classify (reads only the graph as it was before this insertion);
-    //    the loads of four 32-entry chunks go out together
-    for (int t4 = 0; t4 < m; t4 += 128) {
-        int at[4], cd[4], rk[4], ah[4];
-        uint8_t letter[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int t = t4 + 32 * u + lane;
-            at[u] = t < m ? g.aln_node[t] : -1;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int t = t4 + 32 * u + lane;
-            letter[u] = t < m ? seq[t] : 0;
-            cd[u] = at[u] >= 0 ? g.code[at[u]] : -1;
-            rk[u] = at[u] >= 0 ? g.my_rank[at[u]] : 0;
-            ah[u] = at[u] >= 0 ? g.al_head[at[u]] : -1;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int t = t4 + 32 * u + lane;
-            if (t >= m) continue;
-            int kind = 1, nid = -1, nal = 0, slot = INT_MIN, start = INT_MAX;
-            if (at[u] != -1) {
-                // the rank extent, in the incremental order, of v's aligned
-                // group among the nodes that existed before this insertion
-                slot = start = rk[u];
-                const bool same = cd[u] == int(letter[u]);
-                for (int x = ah[u]; x != -1; x = g.a_next[x]) {
-                    const int y = g.a_node[x];
-                    if (y < nold) {
-                        const int ry = g.my_rank[y];
-                        slot = max(slot, ry);
-                        start = min(start, ry);
-                    }
-                    if (!same) {
-                        ++nal;
-                        if (nid == -1 && g.code[y] == letter[u]) nid = y;
-                    }
-                }
-                if (same) {
-                    kind = 0;
-                    nid = at[u];
-                } else {
-                    kind = nid == -1 ? 2 : 0;
-                }
-            }
-            e_nid[t] = nid;
-            e_kind[t] = kind | (kind == 2 ? nal << 2 : 0);
-            e_slot[t] = slot;
-            e_start[t] = start;
-        }
-    }
-    __syncwarp();
-    // 2. ids of new aligned bases, aligned-pool offsets, order slots
-    const int base_id = nold;
-    int nnew_e = 0, nal_tot = 0, cur_slot = INT_MIN, first_start = INT_MAX;
-    for (int c0 = 0; c0 < m; c0 += 32) {
-        const int t = c0 + lane;
-        const int kd = t < m ? e_kind[t] : 0;
-        const int kind = kd & 3;
-        const bool is_new = t < m && kind != 0;
-        int tot;
-        const int pre = warp_excl(is_new ? 1 : 0, lane, tot);
-        int atot;
-        const int apre = warp_excl(kind == 2 ? 2 * (kd >> 2) + 2 : 0, lane, atot);
-        // last anchor slot up to t (anchors: kind 0 or 2), carried over chunks
-        int sl = (t < m && kind != 1) ? e_slot[t] : INT_MIN;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, sl, o);
-            if (lane >= o) sl = max(sl, y);
-        }
-        sl = max(sl, cur_slot);
-        int st = (t < m && kind != 1) ? e_start[t] : INT_MAX;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) st = min(st, __shfl_xor_sync(0xffffffffu, st, o));
-        if (first_start == INT_MAX) first_start = st;
-        if (t < m) {
-            if (is_new) e_nid[t] = base_id + nnew_e + pre;
-            // kind 2: own group slot; kind 1: last anchor before it (INT_MIN: none yet)
-            e_slot[t] = kind == 2 ? e_slot[t] : sl;
-            e_start[t] = nal_tot + apre;  // aligned-pool offset (kind 2)
-        }
-        cur_slot = __shfl_sync(0xffffffffu, sl, 31);
-        nnew_e += tot;
-        nal_tot += atot;
-    }
-    const int nnew = nnew_e;
-    if (nold + nnew > g.ncap || sh.nedges + len + 2 > g.ecap || sh.naligned + nal_tot > g.acap) {
-        if (lane == 0) sh.fail = kOverflow;
-        __syncwarp();
-        return;
-    }
-    __syncwarp();
-    // 3. new nodes
-    for (int t = lane; t < m; t += 32) {
-        if ((e_kind[t] & 3) == 0) continue;
-        const int id = e_nid[t];
-        g.code[id] = seq[t];
-        g.cov[id] = 0;
-        g.in_head[id] = g.in_tail[id] = -1;
-        g.out_head[id] = g.out_tail[id] = -1;
-        g.al_head[id] = g.al_tail[id] = -1;
-        g.in_cnt[id] = 0;
-        g.al_cnt[id] = 0;
-        g.out_cnt[id] = 0;
-    }
-    __syncwarp();
-    // 4. aligned groups: a new base joining the group of `at` links to every
-    //    member, then to `at` (spoa's order)
-    for (int t = lane; t < m; t += 32) {
-        if ((e_kind[t] & 3) != 2) continue;
-        const int at = g.aln_node[t];
-        const int G = e_nid[t];
-        int slot = sh.naligned + e_start[t];
-        auto link = [&](int v, int y) {
-            g.a_node[slot] = y;
-            g.a_owner[slot] = v;
-            g.al_cnt[v] += 1;  // one group per node and layer: no other lane links v
-            g.a_next[slot] = -1;
-            if (g.al_tail[v] == -1) g.al_head[v] = slot;
-            else g.a_next[g.al_tail[v]] = slot;
-            g.al_tail[v] = slot;
-            ++slot;
-        };
-        for (int x = g.al_head[at]; x != -1; x = g.a_next[x]) {
-            const int y = g.a_node[x];
-            link(G, y);
-            link(y, G);
-        }
-        link(G, at);
-        link(at, G);
-    }
-    __syncwarp();
-    // 5. edges P[k-1] -> P[k]: existing ones gain weight, new ones are appended
-    int new_edges = 0;
-    for (int c0 = 1; c0 < len; c0 += 32) {
-        const int k = c0 + lane;
-        int u = -1, v = -1, w = 0, found = -1;
-        if (k < len) {
-            u = e_nid[k - 1];
-            v = e_nid[k];
-            w = layer_weight(qual, k - 1) + layer_weight(qual, k);
-            if (u < nold && v < nold) {
-                if (ocsr) {
-                    for (int q = oc.off[u], qe = oc.off[u + 1]; q < qe; ++q)
-                        if (oc.dst[q] == v) {
-                            found = oc.eid[q];
-                            break;
-                        }
-                } else {
-                    for (int e = g.out_head[u]; e != -1; e = g.e_next_out[e])
-                        if (g.e_dst[e] == v) {
-                            found = e;
-                            break;
-                        }
-                }
-            }
-        }
-        int tot;
-        const int pre = warp_excl((k < len && found < 0) ? 1 : 0, lane, tot);
-        __syncwarp();
-        if (k < len) {
-            if (found >= 0) {
-                g.e_w[found] += w;
-            } else {
-                const int id = sh.nedges + new_edges + pre;
-                g.e_src[id] = u;
-                g.e_dst[id] = v;
-                g.e_w[id] = w;
-                g.e_next_in[id] = -1;
-                g.e_next_out[id] = -1;
-                if (g.out_tail[u] == -1) g.out_head[u] = id;
-                else g.e_next_out[g.out_tail[u]] = id;
-                g.out_tail[u] = id;
-                if (g.in_tail[v] == -1) g.in_head[v] = id;
-                else g.e_next_in[g.in_tail[v]] = id;
-                g.in_tail[v] = id;
-                g.in_cnt[v] += 1;  // at most one new edge into v per layer
-                g.out_cnt[u] += 1;  // and at most one out of u
-            }
-        }
-        new_edges += tot;
-        __syncwarp();
-    }
-    // 6. coverage: every node of a path with at least two bases
-    if (len >= 2)
-        for (int k = lane; k < len; k += 32) g.cov[e_nid[k]] += 1;
-    // 7. new nodes with their order slots, in path order
-    const int before = first_start == INT_MAX ? nold - 1 : first_start - 1;
-    for (int t = lane; t < m; t += 32) {
-        if ((e_kind[t] & 3) == 0) continue;
-        const int id = e_nid[t];
-        const int sl = e_slot[t];
-        g.nw_node[id - base_id] = id;
-        g.nw_slot[id - base_id] = sl == INT_MIN ? before : sl;
-    }
-    __syncwarp();
-    if (lane == 0) {
-        sh.nnodes = nold + nnew;
-        sh.nedges += new_edges;
-        sh.naligned += nal_tot;
-        sh.nnew = nnew;
-        sh.nseq += 1;
-    }
-    __syncwarp();
-}
-
-// Splices the new nodes of the last insertion into the incremental order
-// (warp): an old node at rank r moves up by the number of new nodes with slot
-// < r, the k-th new node (slots sorted) lands at slot + 1 + k.
-__device__ void order_insert(const Graph& g, const PoaShared& sh, int nold, int lane, int4* ring) {
-    const int nnew = sh.nnew, n = nold + nnew;
-    // shift counts in shared memory when they fit (the ring is free here)
-    int* const shift = size_t(nold + 1) * 4 <= size_t(sh.scratch_bytes) ? reinterpret_cast<int*>(ring) : g.shift;
-    for (int r = lane; r <= nold; r += 32) shift[r] = 0;
-    __syncwarp();
-    for (int k = lane; k < nnew; k += 32) {
-        const int at = g.nw_slot[k] + 1;
-        if (at < nold) atomicAdd(&shift[at], 1);
-    }
-    __syncwarp();
-    int base = 0;
-    for (int c4 = 0; c4 < nold; c4 += 128) {
-        int ov[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int r = c4 + 32 * u + lane;
-            ov[u] = r < nold ? g.ord[r] : 0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int r = c4 + 32 * u + lane;
-            int v = r < nold ? shift[r] : 0;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, v, o);
-                if (lane >= o) v += y;
-            }
-            if (r < nold) g.ord2[r + base + v] = ov[u];
-            base += __shfl_sync(0xffffffffu, v, 31);
-        }
-    }
-    for (int k = lane; k < nnew; k += 32) g.ord2[g.nw_slot[k] + 1 + k] = g.nw_node[k];
-    __syncwarp();
-    for (int x4 = 0; x4 < n; x4 += 128) {
-        int vv[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int x = x4 + 32 * u + lane;
-            vv[u] = x < n ? g.ord2[x] : 0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int x = x4 + 32 * u + lane;
-            if (x < n) {
-                g.ord[x] = vv[u];
-                g.my_rank[vv[u]] = x;
-            }
-        }
-    }
-    __syncwarp();
-}
-
-__device__ int g_branch_completion(const Graph& g, PoaShared& sh, int rank) {
-    const int v0 = g.rank_to_node[rank];
-    for (int e = g.out_head[v0]; e != -1; e = g.e_next_out[e]) {
-        const int d = g.e_dst[e];
-        for (int oe = g.in_head[d]; oe != -1; oe = g.e_next_in[oe]) {
-            if (g.e_src[oe] != v0) g.bscore[g.e_src[oe]] = -1;
-        }
-    }
-    long long best = 0;
-    int best_id = 0;
-    for (int r = rank + 1; r < sh.nranks; ++r) {
-        const int v = g.rank_to_node[r];
-        g.bscore[v] = -1;
-        g.bpred[v] = -1;
-        for (int e = g.in_head[v]; e != -1; e = g.e_next_in[e]) {
-            const int u = g.e_src[e];
-            if (g.bscore[u] == -1) continue;
-            const long long w = g.e_w[e];
-            if (g.bscore[v] < w ||
-                (g.bscore[v] == w && g.bpred[v] != -1 && g.bscore[g.bpred[v]] <= g.bscore[u])) {
-                g.bscore[v] = w;
-                g.bpred[v] = u;
-            }
-        }
-        if (g.bpred[v] != -1) g.bscore[v] += g.bscore[g.bpred[v]];
-        if (best < g.bscore[v]) {
-            best = g.bscore[v];
-            best_id = v;
-        }
-    }
-    return best_id;
-}
-
-// Heaviest bundle over the full graph in rank order; writes the path to
-// g.cons and returns its length (-1 on failure).
-__device__ int g_heaviest_bundle(const Graph& g, PoaShared& sh) {
-    const int N = sh.nnodes;
-    int best_id = 0;
-    for (int r = 0; r < sh.nranks; ++r) {
-        const int v = g.rank_to_node[r];
-        for (int e = g.in_head[v]; e != -1; e = g.e_next_in[e]) {
-            const int u = g.e_src[e];
-            const long long w = g.e_w[e];
-            if (g.bscore[v] < w ||
-                (g.bscore[v] == w && g.bpred[v] != -1 && g.bscore[g.bpred[v]] <= g.bscore[u])) {
-                g.bscore[v] = w;
-                g.bpred[v] = u;
-            }
-        }
-        if (g.bpred[v] != -1) g.bscore[v] += g.bscore[g.bpred[v]];
-        if (g.bscore[best_id] < g.bscore[v]) best_id = v;
-    }
-    if (g.out_head[best_id] != -1) {
-        for (int r = 0; r < sh.nranks; ++r) g.node_rank[g.rank_to_node[r]] = r;
-        int guard = 0;
-        while (g.out_head[best_id] != -1) {
-            best_id = g_branch_completion(g, sh, g.node_rank[best_id]);
-            if (++guard > N + 1) return -1;
-        }
-    }
-    int len = 0;
-    while (g.bpred[best_id] != -1) {
-        g.cons[len++] = best_id;
-        best_id = g.bpred[best_id];
-        if (len > N) return -1;
-    }
-    g.cons[len++] = best_id;
-    // reverse in place
-    for (int i = 0, j = len - 1; i < j; ++i, --j) {
-        const int t = g.cons[i];
-        g.cons[i] = g.cons[j];
-        g.cons[j] = t;
-    }
-    return len;
-}
-
-// Predecessor p (in in-edge order) of a DP row from its descriptor: DP rank
-// (0 = the empty prefix row when the row has no predecessor).
-__device__ __forceinline__ int desc_pred(const Graph& g, const int4& d, int p) {
-    const int np = desc_np(d.w);
-    if (np == 0) return 0;
-    if (np > 3) return p == 0 ? d.y : g.pred_idx[d.x + p];
-    return p == 0 ? d.x : (p == 1 ? d.y : d.z);
-}
-
-// ---------------- DP of one layer (one team) ----------------
+// ---------------- team memory ----------------
 
 // the CTA's dynamic shared memory: WarpMem<NW>::bytes per warp, teams in order
 extern __shared__ int4 g_poa_smem[];
@@ -832,6 +219,1040 @@ __device__ __forceinline__ void team_sync(int team) {
         asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(32 * NW) : "memory");
     }
 }
+
+// slanted score (row r, column j) as the layer stored it, rows of lc columns
+template <bool FAST>
+__device__ __forceinline__ int h_at(const uint8_t* Hb, int r, int j, int lc) {
+    if (FAST) return reinterpret_cast<const int16_t*>(Hb)[size_t(r) * lc + j];
+    return reinterpret_cast<const int*>(Hb)[size_t(r) * lc + j];
+}
+
+// ---------------- graph primitives ----------------
+
+// In-edges of node v in spoa's order (the order in which they were added):
+// f(source, weight); f returns false to stop.
+template <class F>
+__device__ __forceinline__ void for_in_edges(const Graph& g, int v, F&& f) {
+    const int n = g.in_cnt[v];
+    const int* s = reinterpret_cast<const int*>(g.in_src + 2 * size_t(v));
+    const int* wt = reinterpret_cast<const int*>(g.in_w + 2 * size_t(v));
+    for (int q = 0; q < min(n, kInline); ++q)
+        if (!f(s[q], wt[q])) return;
+    if (n > kInline)
+        for (int e = g.ov_head[v]; e != -1; e = g.e_next[e])
+            if (!f(g.e_src[e], g.e_w[e])) return;
+}
+
+// Nodes aligned to v, in the order in which they were linked: f(node) as above.
+template <class F>
+__device__ __forceinline__ void for_aligned(const Graph& g, int v, F&& f) {
+    const int n = g.al_cnt[v];
+    const int* s = reinterpret_cast<const int*>(g.al4 + v);
+    for (int q = 0; q < min(n, 4); ++q)
+        if (!f(s[q])) return;
+    if (n > 4)
+        for (int x = g.al_head[v]; x != -1; x = g.a_next[x])
+            if (!f(g.a_node[x])) return;
+}
+
+// Links node y to v's aligned list. Only one thread of the team touches v's
+// group during an insertion.
+__device__ __forceinline__ void link_aligned(const Graph& g, PoaShared& sh, int v, int y) {
+    const int n = g.al_cnt[v];
+    g.al_cnt[v] = n + 1;
+    if (n < 4) {
+        reinterpret_cast<int*>(g.al4 + v)[n] = y;
+        return;
+    }
+    const int x = atomicAdd(&sh.naligned, 1);
+    if (x >= g.acap) {
+        sh.fail = kOverflow;
+        return;
+    }
+    g.a_node[x] = y;
+    g.a_next[x] = -1;
+    if (n == 4) {
+        g.al_head[v] = x;
+    } else {
+        g.a_next[g.al_tail[v]] = x;
+    }
+    g.al_tail[v] = x;
+}
+
+__device__ int layer_weight(const uint8_t* qual, int k) { return qual ? int(qual[k]) - 33 : 1; }
+
+// Warp prefix helpers: exclusive prefix of v over lanes, and the total.
+__device__ __forceinline__ int warp_excl(int v, int lane, int& total) {
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    total = __shfl_sync(0xffffffffu, x, 31);
+    return x - v;
+}
+
+// ---------------- rows of one layer's DP ----------------
+
+// Row descriptor: word w holds the predecessor count (17 bits) and the base
+// (<< 24). Up to kPacked predecessors' ranks sit in x, y, z as 16-bit halves;
+// more of them, or any in a graph of 65536 rows or more (kWide), in pred_idx
+// from x on.
+constexpr int kPacked = 6;
+constexpr int kWide = 1 << 17;
+__device__ __forceinline__ int desc_np(int w) { return w & 0x1FFFF; }
+__device__ __forceinline__ uint32_t desc_base(int w) { return uint32_t(w) >> 24; }
+__device__ __forceinline__ bool desc_listed(int w) { return desc_np(w) > kPacked || (w & kWide) != 0; }
+// Packed predecessor p (in in-edge order).
+__device__ __forceinline__ int desc_packed(const int4& d, int p) {
+    const int q = p < 2 ? d.x : p < 4 ? d.y : d.z;
+    return (p & 1) ? int(unsigned(q) >> 16) : q & 0xFFFF;
+}
+// Predecessor p of a row: DP rank (0 = the empty prefix row when the row has
+// no predecessor).
+__device__ __forceinline__ int desc_pred(const int* pred_idx, const int4& d, int p) {
+    if (desc_np(d.w) == 0) return 0;
+    return desc_listed(d.w) ? pred_idx[d.x + p] : desc_packed(d, p);
+}
+
+// Descriptors of rows order[0 .. ndp), ranks 1 .. ndp, and the list of sink
+// rows (no successor row), by the team, four rows per thread at a time so
+// that one memory latency covers them. rk(v) is node v's DP rank, 0 when it
+// is no row; the ranks go to shared memory as 16-bit words when they fit. With
+// `partial` predecessors outside the rows are dropped and a row is a sink when
+// no row lists it; otherwise a sink is a node without out-edges.
+template <int NW>
+__device__ void build_rows(const Graph& g, PoaShared& sh, const int* order, int ndp, bool partial, int tid, int team,
+                           uint8_t* smem) {
+    constexpr int NT = 32 * NW;
+    const int N = sh.nnodes;
+    const int* const grk = partial ? g.sub_rank : g.rank;
+    const int up = partial ? 0 : 1;  // g.rank counts from 0
+    const size_t rk_bytes = (2 * size_t(N) + 3) & ~size_t(3);
+    const bool in_smem = N < 65535 && rk_bytes + (partial ? size_t(ndp) + 1 : 0) <= size_t(sh.scratch_bytes);
+    uint16_t* const rk16 = reinterpret_cast<uint16_t*>(smem);
+    uint8_t* const succ = in_smem ? smem + rk_bytes : g.flag;
+    const bool wide = ndp >= 65536;
+    if (in_smem)
+        for (int c0 = tid; c0 < N; c0 += 4 * NT) {
+            int r[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) r[u] = c0 + u * NT < N ? grk[c0 + u * NT] : 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (c0 + u * NT < N) rk16[c0 + u * NT] = uint16_t(r[u] + up);
+        }
+    if (partial)
+        for (int i = tid; i <= ndp; i += NT) succ[i] = 0;
+    if (tid == 0) {
+        sh.nsinks = 0;
+        sh.preds = 0;
+        sh.nlisted = 0;
+    }
+    team_sync<NW>(team);
+    auto rk = [&](int v) -> int { return in_smem ? int(rk16[v]) : grk[v] + up; };
+    int preds = 0;
+    for (int c0 = tid; c0 < ndp; c0 += 4 * NT) {
+        int v[4], cnt[4], oc[4];
+        uint8_t code[4];
+        int4 s0[4], s1[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = c0 + u * NT < ndp ? order[c0 + u * NT] : 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            cnt[u] = g.in_cnt[v[u]];
+            oc[u] = partial ? 1 : g.out_cnt[v[u]];
+            code[u] = g.code[v[u]];
+            s0[u] = g.in_src[2 * size_t(v[u])];
+            s1[u] = g.in_src[2 * size_t(v[u]) + 1];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = c0 + u * NT;
+            if (i >= ndp) continue;
+            int np = 0;
+            int4 d = make_int4(0, 0, 0, 0);
+            auto add = [&](int src) {
+                const int r = rk(src);
+                if (r == 0) return;
+                const int h = r << (16 * (np & 1));
+                if (np < 2) d.x |= h;
+                else if (np < 4) d.y |= h;
+                else if (np < 6) d.z |= h;
+                ++np;
+                if (partial) succ[r] = 1;  // every writer stores the same value
+            };
+            const int c = cnt[u];
+            if (c > 0) add(s0[u].x);
+            if (c > 1) add(s0[u].y);
+            if (c > 2) add(s0[u].z);
+            if (c > 3) add(s0[u].w);
+            if (c > 4) {
+                add(s1[u].x);
+                if (c > 5) add(s1[u].y);
+                if (c > 6) add(s1[u].z);
+                if (c > 7) add(s1[u].w);
+                if (c > kInline)
+                    for (int e = g.ov_head[v[u]]; e != -1; e = g.e_next[e]) add(g.e_src[e]);
+            }
+            if (np > kPacked || (wide && np > 0)) {
+                const int off = atomicAdd(&sh.nlisted, np);
+                int k = off;
+                for_in_edges(g, v[u], [&](int src, int) {
+                    const int r = rk(src);
+                    if (r != 0) g.pred_idx[k++] = r;
+                    return true;
+                });
+                d = make_int4(off, 0, 0, wide ? kWide : 0);
+            }
+            d.w |= np | int(uint32_t(code[u]) << 24);
+            g.rowdesc[i] = d;
+            preds += np;
+            if (!partial && oc[u] == 0) g.sink_rows[atomicAdd(&sh.nsinks, 1)] = i + 1;
+        }
+    }
+    preds = __reduce_add_sync(0xffffffffu, preds);
+    if ((tid & 31) == 0 && preds) atomicAdd(&sh.preds, preds);
+    if (partial) {
+        team_sync<NW>(team);
+        for (int i = 1 + tid; i <= ndp; i += NT)
+            if (!succ[i]) g.sink_rows[atomicAdd(&sh.nsinks, 1)] = i;
+    }
+    team_sync<NW>(team);
+}
+
+// spoa's subgraph of a partial layer: the nodes reached from end_node
+// backwards over in-edges and aligned links, going on only from nodes whose id
+// is not below begin_node. One sweep down the incremental order, in which
+// every aligned group is contiguous and a group's successors all come after
+// it: when the sweep reaches a group's last row, all links into the group
+// are known. The descriptors of the whole graph (just built) are staged 64
+// rows at a time and one lane sweeps them. Leaves the rows in g.dporder
+// (sh.ndp of them) and every node's DP rank (0: none) in g.sub_rank. Warp 0.
+__device__ void mark_subgraph(const Graph& g, PoaShared& sh, int begin_node, int end_node, int lane, uint8_t* smem) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr int CH = 64, LOW = 8;
+    const int N = sh.nnodes;
+    if (end_node < 0 || end_node >= N) {
+        if (lane == 0) sh.fail = kFailed;
+        __syncwarp();
+        return;
+    }
+    int4* const s_desc = reinterpret_cast<int4*>(smem);              // [CH]
+    int* const s_start = reinterpret_cast<int*>(s_desc + CH);        // [CH] first row of the row's group
+    int* const s_id = s_start + CH;                                  // [LOW + CH] node of rows base - LOW ..
+    uint8_t* const rest = reinterpret_cast<uint8_t*>(s_id + LOW + CH);
+    const size_t used = size_t(rest - smem);
+    // reached flag of every row (by rank, from 0)
+    uint8_t* const flag = used + size_t(N) <= size_t(sh.scratch_bytes) ? rest : g.flag;
+    for (int r = lane; r < N; r += 32) flag[r] = 0;
+    int top = g.rank[end_node];
+    for_aligned(g, end_node, [&](int y) {
+        top = max(top, g.rank[y]);
+        return true;
+    });
+    __syncwarp();
+    if (lane == 0) flag[g.rank[end_node]] = 1;
+    for (int base = top / CH * CH; base >= 0; base -= CH) {
+        __syncwarp();
+        for (int o = lane; o < CH + LOW; o += 32) {
+            const int r = base - LOW + o;
+            const int v = r >= 0 && r < N ? g.ord[r] : 0;
+            s_id[o] = v;
+            if (o >= LOW && r < N) {
+                s_desc[o - LOW] = g.rowdesc[r];
+                int st = r;
+                for_aligned(g, v, [&](int y) {
+                    st = min(st, g.rank[y]);
+                    return true;
+                });
+                // only a group's last row starts its check
+                bool last = true;
+                for_aligned(g, v, [&](int y) {
+                    last = last && g.rank[y] < r;
+                    return last;
+                });
+                s_start[o - LOW] = last ? st : r;
+            }
+        }
+        __syncwarp();
+        if (lane == 0) {
+            for (int r = min(top, base + CH - 1); r >= base; --r) {
+                const int st = s_start[r - base];
+                if (st < r) {
+                    bool any = false;
+                    for (int x = st; x <= r; ++x) {
+                        const int id = x >= base - LOW ? s_id[x - base + LOW] : g.ord[x];
+                        any |= flag[x] != 0 && id >= begin_node;
+                    }
+                    if (any)
+                        for (int x = st; x <= r; ++x) flag[x] = 1;
+                }
+                if (!flag[r] || s_id[r - base + LOW] < begin_node) continue;
+                const int4 d = s_desc[r - base];
+                const int np = desc_np(d.w);
+                for (int p = 0; p < np; ++p) flag[desc_pred(g.pred_idx, d, p) - 1] = 1;
+            }
+        }
+    }
+    __syncwarp();
+    // the rows, in order; the loads of four 32-row chunks go out together
+    int cnt = 0;
+    for (int c4 = 0; c4 < N; c4 += 128) {
+        int vv[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) vv[u] = c4 + 32 * u + lane < N ? g.ord[c4 + 32 * u + lane] : -1;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int r = c4 + 32 * u + lane;
+            const bool in = vv[u] >= begin_node && flag[r] != 0;
+            const unsigned m = __ballot_sync(kFull, in && r < N);
+            const int k = cnt + __popc(m & ((1u << lane) - 1u));
+            if (vv[u] >= 0) g.sub_rank[vv[u]] = in ? k + 1 : 0;
+            if (in) g.dporder[k] = vv[u];
+            cnt += __popc(m);
+        }
+    }
+    if (lane == 0) sh.ndp = cnt;
+    __syncwarp();
+}
+
+// ---------------- spoa's depth-first topological order ----------------
+
+// spoa's DFS order over the nodes x with member(x), written to out; returns
+// its length, -1 when the stack (cap entries) overflows. ins(v, f) and als(v,
+// f) go through v's in-edge sources and aligned nodes; state(x) is a byte per
+// node, cleared: bits 0-1 mark, bit 2 set once x is no primary of its group.
+template <class Ins, class Als, class Mem, class Stack>
+__device__ int dfs_order(int N, Ins&& ins, Als&& als, Mem&& member, uint8_t* state, Stack* stack, int cap, int* out) {
+    int nr = 0, sp = 0;
+    for (int i = 0; i < N; ++i) {
+        if (!member(i) || (state[i] & 3) != 0) continue;
+        stack[sp++] = Stack(i);
+        while (sp > 0) {
+            const int v = stack[sp - 1];
+            const int sv = state[v];
+            bool valid = true, room = true;
+            if ((sv & 3) != 2) {
+                ins(v, [&](int u) {
+                    if (!member(u) || (state[u] & 3) == 2) return true;
+                    room = sp < cap;
+                    if (room) stack[sp++] = Stack(u);
+                    valid = false;
+                    return room;
+                });
+                if (!(sv & 4))
+                    als(v, [&](int y) {
+                        if (!member(y) || (state[y] & 3) == 2) return true;
+                        room = room && sp < cap;
+                        if (room) stack[sp++] = Stack(y);
+                        state[y] |= 4;
+                        valid = false;
+                        return room;
+                    });
+                if (!room) return -1;
+                if (valid) {
+                    state[v] = uint8_t((sv & ~3) | 2);
+                    if (!(sv & 4)) {
+                        out[nr++] = v;
+                        als(v, [&](int y) {
+                            if (member(y)) out[nr++] = y;
+                            return true;
+                        });
+                    }
+                } else {
+                    state[v] = uint8_t((sv & ~3) | 1);
+                }
+            }
+            if (valid) --sp;
+        }
+    }
+    return nr;
+}
+
+// spoa's topological order of the whole graph (g.sub_rank unused) or of the
+// rows of a partial layer, into g.dfs; its inverse into g.dfs_rank. In-edge
+// and aligned lists, states and the stack sit in shared memory as 16-bit
+// words when they fit, else the lists are walked in global memory. Warp 0; the
+// count is returned on every lane (-1: stack overflow).
+__device__ int topo_sort_warp(const Graph& g, PoaShared& sh, bool partial, int lane, uint8_t* smem) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const int N = sh.nnodes;
+    auto member = [&](int x) { return !partial || g.sub_rank[x] != 0; };
+    // list offsets by warp prefix of the counts
+    uint16_t* const in_off = reinterpret_cast<uint16_t*>(smem);
+    uint16_t* const al_off = in_off + (N + 1);
+    bool fits = N < 65535 && 5 * size_t(N) + 8 <= size_t(sh.scratch_bytes);
+    int E = 0, A = 0;
+    if (fits) {
+        for (int c4 = 0; c4 < N; c4 += 128) {
+            int ci[4], ca[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int v = c4 + 32 * u + lane;
+                ci[u] = v < N ? g.in_cnt[v] : 0;
+                ca[u] = v < N ? g.al_cnt[v] : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int v = c4 + 32 * u + lane;
+                int ti = 0, ta = 0;
+                const int xi = warp_excl(ci[u], lane, ti), xa = warp_excl(ca[u], lane, ta);
+                if (v < N) {
+                    in_off[v] = uint16_t(E + xi);
+                    al_off[v] = uint16_t(A + xa);
+                }
+                E += ti;
+                A += ta;
+            }
+        }
+        // lists, a state byte per node, and a stack of at least N + 64 entries
+        fits = E < 65535 && A < 65535 &&
+               2 * (size_t(N) + 1) * 2 + 2 * size_t(E) + 2 * size_t(A) + size_t(N) + 2 * (size_t(N) + 64) <=
+                   size_t(sh.scratch_bytes);
+    }
+    int nr = -1;
+    if (fits) {
+        if (lane == 0) {
+            in_off[N] = uint16_t(E);
+            al_off[N] = uint16_t(A);
+        }
+        uint16_t* const in_src = al_off + (N + 1);
+        uint16_t* const al_x = in_src + E;
+        uint16_t* const stack = al_x + A;
+        uint8_t* const end = smem + sh.scratch_bytes;
+        uint8_t* const state = end - N;
+        const int cap = int((state - reinterpret_cast<uint8_t*>(stack)) / 2);
+        __syncwarp();
+        for (int v = lane; v < N; v += 32) {
+            int q = in_off[v], x = al_off[v];
+            for_in_edges(g, v, [&](int s, int) {
+                in_src[q++] = uint16_t(s);
+                return true;
+            });
+            for_aligned(g, v, [&](int y) {
+                al_x[x++] = uint16_t(y);
+                return true;
+            });
+            // nodes outside the subgraph count as done and are never roots
+            state[v] = member(v) ? 0 : 2;
+        }
+        __syncwarp();
+        if (lane == 0)
+            nr = dfs_order(
+                N,
+                [&](int v, auto&& f) {
+                    for (int q = in_off[v], qe = in_off[v + 1]; q < qe; ++q)
+                        if (!f(int(in_src[q]))) return;
+                },
+                [&](int v, auto&& f) {
+                    for (int q = al_off[v], qe = al_off[v + 1]; q < qe; ++q)
+                        if (!f(int(al_x[q]))) return;
+                },
+                [&](int) { return true; }, state, stack, cap, g.dfs);
+        // members of a group outside the subgraph were listed with it
+        if (partial) {
+            nr = __shfl_sync(kFull, nr, 0);
+            int k = 0;
+            for (int c0 = 0; c0 < nr; c0 += 32) {
+                const int v = c0 + lane < nr ? g.dfs[c0 + lane] : -1;
+                const bool in = v >= 0 && member(v);
+                const unsigned m = __ballot_sync(kFull, in);
+                __syncwarp();
+                if (in) g.dfs[k + __popc(m & ((1u << lane) - 1u))] = v;
+                k += __popc(m);
+                __syncwarp();
+            }
+            nr = nr < 0 ? nr : k;
+        }
+        nr = __shfl_sync(kFull, nr, 0);
+    }
+    if (nr < 0) {
+        __syncwarp();
+        for (int v = lane; v < N; v += 32) g.flag[v] = 0;
+        __syncwarp();
+        if (lane == 0)
+            nr = dfs_order(
+                N,
+                [&](int v, auto&& f) { for_in_edges(g, v, [&](int s, int) { return f(s); }); },
+                [&](int v, auto&& f) { for_aligned(g, v, f); }, member, g.flag, g.stack, g.scap, g.dfs);
+        nr = __shfl_sync(kFull, nr, 0);
+    }
+    __syncwarp();
+    for (int r = lane; r < nr; r += 32) g.dfs_rank[g.dfs[r]] = r;
+    __syncwarp();
+    return nr;
+}
+
+// ---------------- NW end row ----------------
+
+// The first sink row with the best last-column score, or, when several sinks
+// share it, the first of them in spoa's topological order of the (sub)graph.
+// Sets sh.end_value. Warp 0.
+//
+// spoa's order lists nodes by the root of the DFS that reaches them, roots in
+// ascending id. Three facts order nearly all tied sinks without the DFS:
+// a sink outside every aligned group is its own root (nothing else leads to
+// it); a group with a backbone node x (id below B) is reached from root x,
+// no earlier (every earlier root precedes x on the backbone, so the group is
+// none of its ancestors; B is the backbone's length); and x, the group's
+// first visited node, is listed first and then its aligned list in order. Only
+// a tied sink in a group without a backbone node needs the DFS itself.
+template <bool FAST>
+__device__ int end_row(const Graph& g, PoaShared& sh, const int* order, int L, int lc, bool partial, int begin_node,
+                       int B, int lane, uint8_t* smem) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const uint8_t* const Hb = reinterpret_cast<const uint8_t*>(g.H);
+    const int ns = sh.nsinks;
+    int best = INT_MIN, low = INT_MAX, ties = 0;
+    for (int k = lane; k < ns; k += 32) {
+        const int i = g.sink_rows[k];
+        const int v = h_at<FAST>(Hb, i, L, lc);
+        g.sink_h[k] = v;
+        ties = v > best ? 1 : ties + (v == best ? 1 : 0);
+        low = v > best ? i : v == best ? min(low, i) : low;
+        best = max(best, v);
+    }
+    const int top = __reduce_max_sync(kFull, best);
+    if (best != top) {
+        ties = 0;
+        low = INT_MAX;
+    }
+    int iend = __reduce_min_sync(kFull, low);
+    ties = __reduce_add_sync(kFull, ties);
+    if (lane == 0) sh.end_value = top;
+    __syncwarp();
+    if (ties <= 1) return iend;
+    // key: root id, then the place in the group's listing
+    bool open = false;
+    unsigned root = ~0u, place = ~0u;
+    int row = iend;
+    for (int k = lane; k < ns; k += 32) {
+        if (g.sink_h[k] != top) continue;
+        const int i = g.sink_rows[k];
+        const int v = order[i - 1];
+        int x = v;
+        for_aligned(g, v, [&](int y) {
+            if (y >= begin_node) x = min(x, y);
+            return true;
+        });
+        unsigned pl = 0;
+        if (g.al_cnt[v] != 0) {
+            open |= x >= B;
+            if (x != v) {
+                unsigned at = 1;
+                for_aligned(g, x, [&](int y) {
+                    if (y == v) pl = at;
+                    ++at;
+                    return y != v;
+                });
+            }
+        }
+        if (unsigned(x) < root || (unsigned(x) == root && pl < place)) {
+            root = unsigned(x);
+            place = pl;
+            row = i;
+        }
+    }
+    if (!__any_sync(kFull, open)) {
+        const unsigned r0 = __reduce_min_sync(kFull, root);
+        const unsigned p0 = __reduce_min_sync(kFull, root == r0 ? place : ~0u);
+        return __reduce_min_sync(kFull, unsigned(root == r0 && place == p0 ? row : INT_MAX));
+    }
+    const int nr = topo_sort_warp(g, sh, partial, lane, smem);
+    if (nr < 0) {
+        if (lane == 0) sh.fail = kOverflow;
+        __syncwarp();
+        return iend;
+    }
+    int first = INT_MAX, fi = iend;
+    for (int k = lane; k < ns; k += 32) {
+        if (g.sink_h[k] != top) continue;
+        const int i = g.sink_rows[k];
+        const int rr = g.dfs_rank[order[i - 1]];
+        if (rr < first) {
+            first = rr;
+            fi = i;
+        }
+    }
+    const int f0 = __reduce_min_sync(kFull, first);
+    return __reduce_min_sync(kFull, first == f0 ? fi : INT_MAX);
+}
+
+// ---------------- adding a layer ----------------
+
+// Graph::add_alignment for one layer, by the team. A path visits every node
+// and every aligned group at most once, so the per-position work is
+// independent: classify each base (existing node, new base, new member of an
+// aligned group), number the new nodes in path order, then in parallel
+// create nodes, aligned-group links, edges P[k-1] -> P[k] with weight w[k-1] +
+// w[k] (every sequence position k owns exactly one path node P[k]) and
+// coverage. In-edges sit with their node (kInline of them in two 16-byte
+// words), so that finding or adding an edge reads only its head. Leaves the
+// new nodes' order slots (see order_insert) in g.new_slot.
+template <int NW>
+__device__ void add_layer(const Graph& g, PoaShared& sh, const uint8_t* seq, const uint8_t* qual, int len, int lane,
+                          int w, int team, uint8_t* smem) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr int NT = 32 * NW;
+    const int tid = 32 * w + lane;
+    const int nold = sh.nnodes;
+    const bool in_smem = 8 * size_t(len) <= size_t(sh.scratch_bytes);
+    int* const nid = in_smem ? reinterpret_cast<int*>(smem) : g.nid;  // node of position t, -1 until numbered
+    int* const slot = in_smem ? nid + len : g.slot;                   // last rank of the position's group
+    const int* const path = g.path;
+    // 1. classify (reads only the graph as it was before this insertion)
+    for (int t4 = tid; t4 < len; t4 += 4 * NT) {
+        int at[4], ac[4], rk[4];
+        uint8_t cd[4], ch[4];
+        int4 al[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) at[u] = t4 + u * NT < len ? path[t4 + u * NT] : -1;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int v = max(at[u], 0);
+            ch[u] = t4 + u * NT < len ? seq[t4 + u * NT] : 0;
+            cd[u] = g.code[v];
+            ac[u] = g.al_cnt[v];
+            rk[u] = g.rank[v];
+            al[u] = g.al4[v];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int t = t4 + u * NT;
+            if (t >= len) continue;
+            int n = -1, sl = INT_MIN;
+            if (at[u] >= 0) {
+                sl = rk[u];
+                if (cd[u] == ch[u]) n = at[u];
+                if (ac[u] > 0) {
+                    const int ys[4] = {al[u].x, al[u].y, al[u].z, al[u].w};
+                    int yr[4];
+                    uint8_t yc[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int y = q < ac[u] ? ys[q] : at[u];
+                        yr[q] = g.rank[y];
+                        yc[q] = g.code[y];
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        sl = max(sl, yr[q]);
+                        if (n < 0 && q < ac[u] && yc[q] == ch[u]) n = ys[q];
+                    }
+                    if (ac[u] > 4)
+                        for_aligned(g, at[u], [&](int y) {
+                            sl = max(sl, g.rank[y]);
+                            if (n < 0 && g.code[y] == ch[u]) n = y;
+                            return true;
+                        });
+                }
+            }
+            nid[t] = n;
+            slot[t] = sl;
+        }
+    }
+    team_sync<NW>(team);
+    // 2. ids and order slots of the new nodes: a new member of a group goes
+    //    behind the group, an inserted base behind the last anchor before it
+    //    (anchors: positions on existing groups, whose ranks rise along the
+    //    path), those before the first anchor in front of its group
+    if (w == 0) {
+        int nnew = 0, carry = INT_MIN;
+        for (int c0 = 0; c0 < len; c0 += 32) {
+            const int t = c0 + lane;
+            const bool on = t < len;
+            const int n = on ? nid[t] : 0, s = on ? slot[t] : INT_MIN;
+            const unsigned ba = __ballot_sync(kFull, s != INT_MIN);
+            if (carry == INT_MIN && ba != 0) {
+                // the first anchor: the slot in front of its group
+                const int v = path[c0 + __ffs(ba) - 1];
+                int st = g.rank[v];
+                for_aligned(g, v, [&](int y) {
+                    st = min(st, g.rank[y]);
+                    return true;
+                });
+                carry = st - 1;
+                // bases inserted so far were given the slot "before" below
+                for (int k = lane; k < nnew; k += 32) g.new_slot[k] = carry;
+            }
+            const unsigned bn = __ballot_sync(kFull, on && n < 0);
+            const unsigned upto = ba & (0xffffffffu >> (31 - lane));
+            const int sl = __shfl_sync(kFull, s, upto ? 31 - __clz(upto) : 0);
+            if (on && n < 0) {
+                const int k = nnew + __popc(bn & ((1u << lane) - 1u));
+                if (nold + k < g.ncap) g.new_slot[k] = upto ? sl : carry == INT_MIN ? nold - 1 : carry;
+                nid[t] = nold + k;
+            }
+            if (ba) carry = __shfl_sync(kFull, s, 31 - __clz(ba));
+            nnew += __popc(bn);
+        }
+        if (lane == 0) {
+            const bool room = nold + nnew <= g.ncap;
+            sh.nnew = room ? nnew : -1;
+            if (!room) sh.fail = kOverflow;
+        }
+        __syncwarp();
+    }
+    team_sync<NW>(team);
+    // (not sh.fail, which a faster thread may set below while a slower one
+    // still reads it here: all threads have to take the same way)
+    if (sh.nnew < 0) return;
+    // 3. new nodes, and their aligned groups: a new base joining the group of
+    //    `at` links to every member, then to `at` (spoa's order)
+    for (int t = tid; t < len; t += NT) {
+        const int G = nid[t];
+        if (G < nold) continue;
+        g.code[G] = seq[t];
+        g.cov[G] = 0;
+        g.in_cnt[G] = 0;
+        g.out_cnt[G] = 0;
+        g.al_cnt[G] = 0;
+        const int at = path[t];
+        if (at >= 0) {
+            for_aligned(g, at, [&](int y) {
+                link_aligned(g, sh, G, y);
+                link_aligned(g, sh, y, G);
+                return true;
+            });
+            link_aligned(g, sh, G, at);
+            link_aligned(g, sh, at, G);
+        }
+    }
+    team_sync<NW>(team);
+    // 4. edges P[k-1] -> P[k]: existing ones gain weight, new ones are
+    //    appended (each node is head and tail of at most one of them);
+    //    coverage of every node of a path with at least two bases
+    for (int k = tid; k < len; k += NT) {
+        const int v = nid[k];
+        if (len >= 2) g.cov[v] += 1;
+        if (k == 0) continue;
+        const int u = nid[k - 1];
+        const int wt = layer_weight(qual, k - 1) + layer_weight(qual, k);
+        const int n = g.in_cnt[v];
+        const int4 a = g.in_src[2 * size_t(v)], b = g.in_src[2 * size_t(v) + 1];
+        int* const wv = reinterpret_cast<int*>(g.in_w + 2 * size_t(v));
+        int q = -1;
+        if (n > 7 && b.w == u) q = 7;
+        if (n > 6 && b.z == u) q = 6;
+        if (n > 5 && b.y == u) q = 5;
+        if (n > 4 && b.x == u) q = 4;
+        if (n > 3 && a.w == u) q = 3;
+        if (n > 2 && a.z == u) q = 2;
+        if (n > 1 && a.y == u) q = 1;
+        if (n > 0 && a.x == u) q = 0;
+        if (q >= 0) {
+            wv[q] += wt;
+            continue;
+        }
+        if (n > kInline) {
+            int e = g.ov_head[v];
+            while (e != -1 && g.e_src[e] != u) e = g.e_next[e];
+            if (e != -1) {
+                g.e_w[e] += wt;
+                continue;
+            }
+        }
+        if (n < kInline) {
+            reinterpret_cast<int*>(g.in_src + 2 * size_t(v))[n] = u;
+            wv[n] = wt;
+        } else {
+            const int e = atomicAdd(&sh.nedges, 1);
+            if (e >= g.ecap) {
+                sh.fail = kOverflow;
+                continue;
+            }
+            g.e_src[e] = u;
+            g.e_w[e] = wt;
+            g.e_next[e] = -1;
+            if (n == kInline) {
+                g.ov_head[v] = e;
+            } else {
+                g.e_next[g.ov_tail[v]] = e;
+            }
+            g.ov_tail[v] = e;
+        }
+        g.in_cnt[v] = n + 1;
+        g.out_cnt[u] += 1;
+    }
+    team_sync<NW>(team);
+    if (tid == 0) {
+        sh.nnodes = nold + sh.nnew;
+        sh.nseq += 1;
+    }
+}
+
+// Splices the new nodes of the last insertion into the incremental order
+// (team): an old node at rank r moves up by the number of new nodes with slot
+// < r, the k-th new node (slots rise along the path) lands at slot + 1 + k.
+template <int NW>
+__device__ void order_insert(Graph& g, PoaShared& sh, int lane, int w, int team, uint8_t* smem) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr int NT = 32 * NW;
+    const int tid = 32 * w + lane;
+    const int nnew = sh.nnew;
+    team_sync<NW>(team);  // sh.nnodes is the new count on every thread
+    const int nold = sh.nnodes - nnew;
+    if (nnew == 0) return;
+    int* const shift = (size_t(nold) + 1) * 4 <= size_t(sh.scratch_bytes) ? reinterpret_cast<int*>(smem) : g.shift;
+    for (int r = tid; r <= nold; r += NT) shift[r] = 0;
+    team_sync<NW>(team);
+    for (int k = tid; k < nnew; k += NT) {
+        const int at = g.new_slot[k] + 1;
+        if (at < nold) atomicAdd(&shift[at], 1);
+    }
+    team_sync<NW>(team);
+    if (w == 0) {
+        // inclusive prefix, four independent 32-rank chunks at a time
+        int base = 0;
+        for (int c4 = 0; c4 < nold; c4 += 128) {
+            int x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] = c4 + 32 * u + lane < nold ? shift[c4 + 32 * u + lane] : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int y = __shfl_up_sync(kFull, x[u], o);
+                    if (lane >= o) x[u] += y;
+                }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (c4 + 32 * u + lane < nold) shift[c4 + 32 * u + lane] = base + x[u];
+                base += __shfl_sync(kFull, x[u], 31);
+            }
+        }
+        __syncwarp();
+    }
+    team_sync<NW>(team);
+    for (int c0 = tid; c0 < nold; c0 += 4 * NT) {
+        int v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = c0 + u * NT < nold ? g.ord[c0 + u * NT] : -1;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (v[u] >= 0) {
+                const int r = c0 + u * NT + shift[c0 + u * NT];
+                g.ord2[r] = v[u];
+                g.rank[v[u]] = r;
+            }
+    }
+    for (int k = tid; k < nnew; k += NT) {
+        const int r = g.new_slot[k] + 1 + k;
+        g.ord2[r] = nold + k;
+        g.rank[nold + k] = r;
+    }
+    team_sync<NW>(team);
+    if (tid == 0) {
+        int* const t = g.ord;
+        g.ord = g.ord2;
+        g.ord2 = t;
+    }
+    team_sync<NW>(team);
+}
+
+// ---------------- consensus ----------------
+
+// Heaviest bundle over the nodes in the order given (any topological order
+// gives the same scores and predecessors), 64-bit, in global memory (lane 0).
+__device__ void bundle_scores(const Graph& g, const int* order, int N) {
+    for (int r = 0; r < N; ++r) {
+        const int v = order[r];
+        long long s = -1;
+        int p = -1;
+        for_in_edges(g, v, [&](int u, int wt) {
+            const long long x = wt;
+            if (s < x || (s == x && p != -1 && g.bscore[p] <= g.bscore[u])) {
+                s = x;
+                p = u;
+            }
+            return true;
+        });
+        g.bscore[v] = p != -1 ? s + g.bscore[p] : s;
+        g.bpred[v] = p;
+    }
+}
+
+// spoa's branch completion from DFS rank `rank` (lane 0).
+__device__ int g_branch_completion(const Graph& g, int N, int rank) {
+    const int v0 = g.dfs[rank];
+    // heads of v0's out-edges, found from their in-lists
+    for (int d = 0; d < N; ++d) {
+        bool head = false;
+        for_in_edges(g, d, [&](int s, int) {
+            head = s == v0;
+            return !head;
+        });
+        if (head)
+            for_in_edges(g, d, [&](int s, int) {
+                if (s != v0) g.bscore[s] = -1;
+                return true;
+            });
+    }
+    long long best = 0;
+    int best_id = 0;
+    for (int r = rank + 1; r < N; ++r) {
+        const int v = g.dfs[r];
+        long long s = -1;
+        int p = -1;
+        for_in_edges(g, v, [&](int u, int wt) {
+            if (g.bscore[u] == -1) return true;
+            const long long x = wt;
+            if (s < x || (s == x && p != -1 && g.bscore[p] <= g.bscore[u])) {
+                s = x;
+                p = u;
+            }
+            return true;
+        });
+        if (p != -1) s += g.bscore[p];
+        g.bscore[v] = s;
+        g.bpred[v] = p;
+        if (best < s) {
+            best = s;
+            best_id = v;
+        }
+    }
+    return best_id;
+}
+
+// spoa's heaviest bundle: scores in topological order, the first node of the
+// best score in spoa's DFS order, completed while it has out-edges, and the
+// path back from it into g.cons (in reverse); returns the path length (-1 on
+// failure) on every lane. Scores do not depend on which topological order
+// they are computed in, so the incremental one serves, and the DFS order is
+// only built when several nodes share the best score or the best has
+// out-edges. Scores, predecessors and the ranks of 32 staged nodes' in-edges
+// sit in shared memory when they fit (scores are bounded by sequences x 186 x
+// nodes: two Phred values per sequence and edge, summed along a path). Warp 0.
+__device__ int heaviest_bundle_warp(const Graph& g, PoaShared& sh, int lane, uint8_t* smem) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const int N = sh.nnodes;
+    int* const bs = reinterpret_cast<int*>(smem);                                // [N] by rank
+    uint16_t* const bp = reinterpret_cast<uint16_t*>(smem + 4 * size_t(N));      // [N] by rank, 0xFFFF = none
+    const size_t st_off = (6 * size_t(N) + 15) & ~size_t(15);
+    int* const sw = reinterpret_cast<int*>(smem + st_off);                       // [32][kInline] weights
+    uint16_t* const su = reinterpret_cast<uint16_t*>(sw + 32 * kInline);         // [32][kInline] source ranks
+    int* const sd = reinterpret_cast<int*>(su + 32 * kInline);                   // [32] degree
+    const size_t need = st_off + 32 * kInline * 6 + 32 * 4;
+    const bool fits = N < 65535 && need <= size_t(sh.scratch_bytes) &&
+                      double(sh.nseq + 1) * 186.0 * double(N + 1) < 2.0e9;
+    int best_id = 0, ties = 0;
+    if (fits) {
+        int best = INT_MIN, best_r = 0;
+        for (int r0 = 0; r0 < N; r0 += 32) {
+            const int r = r0 + lane;
+            int deg = 0;
+            if (r < N) {
+                const int v = g.ord[r];
+                deg = g.in_cnt[v];
+                const int* s = reinterpret_cast<const int*>(g.in_src + 2 * size_t(v));
+                const int* wt = reinterpret_cast<const int*>(g.in_w + 2 * size_t(v));
+                for (int q = 0; q < min(deg, kInline); ++q) {
+                    su[lane * kInline + q] = uint16_t(g.rank[s[q]]);
+                    sw[lane * kInline + q] = wt[q];
+                }
+            }
+            sd[lane] = deg;
+            __syncwarp();
+            if (lane == 0) {
+                const int cnt = min(32, N - r0);
+                for (int t = 0; t < cnt; ++t) {
+                    const int d = sd[t];
+                    int s = -1, p = -1, sp = 0;
+                    auto consider = [&](int u, int wt) {
+                        const int su_ = bs[u];
+                        if (s < wt || (s == wt && p != -1 && sp <= su_)) {
+                            s = wt;
+                            p = u;
+                            sp = su_;
+                        }
+                    };
+                    for (int q = 0; q < min(d, kInline); ++q) consider(su[t * kInline + q], sw[t * kInline + q]);
+                    if (d > kInline)
+                        for (int e = g.ov_head[g.ord[r0 + t]]; e != -1; e = g.e_next[e])
+                            consider(g.rank[g.e_src[e]], g.e_w[e]);
+                    if (p != -1) s += sp;
+                    bs[r0 + t] = s;
+                    bp[r0 + t] = p < 0 ? uint16_t(0xFFFF) : uint16_t(p);
+                    if (s > best) {
+                        best = s;
+                        best_r = r0 + t;
+                        ties = 1;
+                    } else if (s == best) {
+                        ++ties;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        best = __shfl_sync(kFull, best, 0);
+        best_r = __shfl_sync(kFull, best_r, 0);
+        ties = __shfl_sync(kFull, ties, 0);
+        best_id = g.ord[best_r];
+        if (ties == 1 && best > -1 && g.out_cnt[best_id] == 0) {
+            int len = 0;
+            if (lane == 0) {
+                int r = best_r;
+                for (; bp[r] != 0xFFFF; r = bp[r]) bs[len++] = r;  // in place of the scores
+                bs[len++] = r;
+            }
+            len = __shfl_sync(kFull, len, 0);
+            __syncwarp();
+            for (int k = lane; k < len; k += 32) g.cons[k] = g.ord[bs[k]];
+            __syncwarp();
+            return len;
+        }
+        for (int r = lane; r < N; r += 32) {
+            const int v = g.ord[r];
+            g.bscore[v] = bs[r];
+            g.bpred[v] = bp[r] == 0xFFFF ? -1 : g.ord[bp[r]];
+        }
+        __syncwarp();
+    } else {
+        if (lane == 0) bundle_scores(g, g.ord, N);
+        __syncwarp();
+    }
+    // the general way: spoa's own order
+    const int nr = topo_sort_warp(g, sh, false, lane, smem);
+    if (nr < 0) {
+        if (lane == 0) sh.fail = kOverflow;
+        __syncwarp();
+        return 0;
+    }
+    int len = 0;
+    if (lane == 0) {
+        // spoa starts from node 0, whose score counts as -1 until its turn
+        long long best = -1;
+        best_id = 0;
+        for (int r = 0; r < N; ++r) {
+            const int v = g.dfs[r];
+            if (best < g.bscore[v] || (v == 0 && best_id == 0)) {
+                best = g.bscore[v];
+                best_id = v;
+            }
+        }
+        int guard = 0;
+        while (g.out_cnt[best_id] != 0 && len >= 0) {
+            best_id = g_branch_completion(g, N, g.dfs_rank[best_id]);
+            if (++guard > N + 1) len = -1;
+        }
+        if (len == 0) {
+            int v = best_id;
+            for (; g.bpred[v] != -1 && len <= N; v = g.bpred[v]) g.cons[len++] = v;
+            if (len > N) {
+                len = -1;
+            } else {
+                g.cons[len++] = v;
+            }
+        }
+    }
+    len = __shfl_sync(kFull, len, 0);
+    __syncwarp();
+    return len;
+}
+
+// ---------------- DP of one layer (one team) ----------------
 
 // Cells per lane for rows of wc columns: the team's NW strips of 32 * S
 // columns cover the row in one pass where that fits in registers (768
@@ -877,13 +1298,6 @@ __device__ __forceinline__ uint32_t pack_s16(int lo, int hi) {
 }
 __device__ __forceinline__ int unpack_lo(uint32_t w) { return int(w << 16) >> 16; }
 __device__ __forceinline__ int unpack_hi(uint32_t w) { return int(w) >> 16; }
-// slanted score (row r, column j) as the layer stored it, rows of lc columns
-template <bool FAST>
-__device__ __forceinline__ int h_at(const uint8_t* Hb, int r, int j, int lc) {
-    if (FAST) return reinterpret_cast<const int16_t*>(Hb)[size_t(r) * lc + j];
-    return reinterpret_cast<const int*>(Hb)[size_t(r) * lc + j];
-}
-
 // Byte `sel & 7` (per nibble) of lo, sign extended by the nibble's top bit.
 __device__ __forceinline__ int prmt_score(uint32_t lo, uint32_t sel) {
     uint32_t d;
@@ -915,7 +1329,7 @@ __device__ __forceinline__ uint32_t score_pool(uint32_t base, uint32_t mm4, uint
 // with a branch on it costs about 75 cycles, a shuffle 33, so the row is kept
 // nearly free of branches. What a row needs besides its scores is
 // worked out 32 rows at a time, one row per lane: a score word, and a control
-// word with the ring slots of up to 7 predecessors besides the row just
+// word with the ring slots of up to 6 predecessors besides the row just
 // computed, which is still in registers. The control goes through a warp
 // reduction, so that branches on it are uniform.
 //
@@ -926,7 +1340,7 @@ __device__ __forceinline__ uint32_t score_pool(uint32_t base, uint32_t mm4, uint
 // chain per group from what lies left of it. No decisions are kept: the walk
 // visits a few cells of each row and decides there from the scores, which
 // are stored anyway.
-constexpr unsigned kCtlChain = 8, kCtlSlow = 7;  // control: count (7 = general way) | chain | 7 slot nibbles
+constexpr unsigned kCtlChain = 8, kCtlSlow = 7;  // control: count (7 = general way) | chain | 6 slot nibbles
 template <int S, int NW, bool FAST, bool LEFT>
 __device__ __noinline__ void dp_strip(const Graph& g, PoaShared& sh, int ndp_, const uint8_t* seq, int L, int mt,
                                       int mm, int gap, int lane, int w, int team, int pass) {
@@ -949,6 +1363,7 @@ __device__ __noinline__ void dp_strip(const Graph& g, PoaShared& sh, int ndp_, c
     const int j0 = c0 + lane * S;
     uint8_t* const Hb = reinterpret_cast<uint8_t*>(g.H);
     const int4* const rowdesc = g.rowdesc;
+    const int* const pred_idx = g.pred_idx;
     uint8_t* const mine = reinterpret_cast<uint8_t*>(g_poa_smem) + (team * NW + w) * Mem::bytes;
     uint8_t* const ring = mine + lane * (U * 4);              // the lane's first unit of row 0
     uint8_t* const ring_left = mine + S * 128 + lane * 4;
@@ -996,20 +1411,20 @@ __device__ __noinline__ void dp_strip(const Graph& g, PoaShared& sh, int ndp_, c
             // controls of rows i0 + 1 .. i0 + 32, one per lane
             const int r = i0 + 1 + lane;
             const int np = desc_np(pre.w);
-            uint32_t ctl = 0, n = 0;
-            bool slow = np > 8 || (np == 0 && r > 1);
-            if (np == 0) ctl = kCtlChain;
-            if (!slow)
-                for (int q = 0; q < np; ++q) {
-                    const int p = np > 3 ? (q == 0 ? pre.y : g.pred_idx[pre.x + q]) : q == 0 ? pre.x : q == 1 ? pre.y : pre.z;
-                    if (p == r - 1) {
-                        ctl |= kCtlChain;
-                    } else {
-                        slow |= r - p > R || n == 6;
-                        ctl |= n < 6 ? uint32_t(p % R) << (4 + 4 * n) : 0u;
-                        ++n;
-                    }
+            uint32_t ctl = np == 0 ? kCtlChain : 0, n = 0;
+            bool slow = desc_listed(pre.w) || (np == 0 && r > 1);
+#pragma unroll
+            for (int q = 0; q < kPacked; ++q) {
+                const int p = desc_packed(pre, q);
+                if (q >= np) continue;
+                if (p == r - 1) {
+                    ctl |= kCtlChain;
+                } else {
+                    slow |= r - p > R;
+                    ctl |= uint32_t(p % R) << (4 + 4 * n);
+                    ++n;
                 }
+            }
             cblk[lane] = slow ? kCtlSlow : ctl | n;
             pblk[lane] = FAST ? score_pool(desc_base(pre.w), mm4, flip) : desc_base(pre.w);
             if (LEFT && w == 0 && r <= ndp) {
@@ -1104,7 +1519,7 @@ __device__ __noinline__ void dp_strip(const Graph& g, PoaShared& sh, int ndp_, c
                     left = INT_MIN;
 #pragma unroll 1
                     for (int p = 0; p < max(np, 1); ++p) {
-                        const int r = desc_pred(g, d, p);
+                        const int r = desc_pred(pred_idx, d, p);
                         int lft;
                         if (r == 0) {
                             lft = j0 == 0 ? kNegInf : 0;
@@ -1294,12 +1709,12 @@ __device__ void dp_dispatch(const Graph& g, PoaShared& sh, int ndp, const uint8_
 // would cost more than the whole step). A predecessor above the tile is read
 // from global memory; a step that leaves the tile ends the lane's run and
 // the warp stages the next one. Writes the node of every sequence position
-// (-1 for an inserted base) to g.aln_node; a vertical step consumes no
+// (-1 for an inserted base) to g.path; a vertical step consumes no
 // position and adds nothing to the graph. Returns false on a broken walk.
 constexpr int kTileRows = 96;
 constexpr int kTilePitch = 128;  // bytes per row: 64 int16 or 32 int32 columns
 constexpr int kTileBytes = kTileRows * kTilePitch;
-constexpr int kTileSmem = kTileBytes + kTileRows * 20 + 64;
+constexpr int kTileSmem = kTileBytes + kTileRows * 36 + 64;
 static_assert(kTileSmem <= 4 * WarpMem<4>::bytes && kTileSmem <= WarpMem<1>::bytes, "the tile fits every team's memory");
 template <bool FAST>
 __device__ __noinline__ bool traceback_warp(const Graph& g, const int* order, const uint8_t* seq, int L, int iend,
@@ -1313,12 +1728,13 @@ __device__ __noinline__ bool traceback_warp(const Graph& g, const int* order, co
     // per tile row: byte offsets of the predecessors' tile rows (-1: outside,
     // or more than three) | base
     int4* const w_desc = reinterpret_cast<int4*>(tile + kTileBytes);
-    int* const w_node = reinterpret_cast<int*>(tile + kTileBytes + kTileRows * 16);
-    uint8_t* const w_seq = tile + kTileBytes + kTileRows * 20;
+    int4* const w_raw = w_desc + kTileRows;
+    int* const w_node = reinterpret_cast<int*>(w_raw + kTileRows);
+    uint8_t* const w_seq = reinterpret_cast<uint8_t*>(w_node + kTileRows);
     const uint8_t* const Hb = reinterpret_cast<const uint8_t*>(g.H);
     const int4* const rowdesc = g.rowdesc;
     const int* const pred_idx = g.pred_idx;
-    int* const path = g.aln_node;
+    int* const path = g.path;
     int i = iend, j = L, h = hend;
     if (iend == INT_MAX || iend < 1) return false;
     auto score = [&](const uint8_t* p) -> int {
@@ -1343,16 +1759,15 @@ __device__ __noinline__ bool traceback_warp(const Graph& g, const int* order, co
         for (int o = lane; o < kTileRows; o += 32) {
             const int r = wlo + o;
             if (r >= 1 && r <= i) {
-                int4 d = rowdesc[r - 1];
+                const int4 d = rowdesc[r - 1];
                 w_node[o] = order[r - 1];
+                w_raw[o] = d;
                 const int np = desc_np(d.w);
                 // absent predecessors repeat the first
-                if (np == 0) d.x = 0;
-                if (np < 2) d.y = d.x;
-                if (np < 3) d.z = d.x;
-                const bool inside = np <= 3 && min(d.x, min(d.y, d.z)) >= wlo;
-                w_desc[o] = make_int4(inside ? (d.x - wlo) * kTilePitch : -1, (d.y - wlo) * kTilePitch,
-                                      (d.z - wlo) * kTilePitch, int(desc_base(d.w)));
+                const int p0 = desc_packed(d, 0), p1 = np > 1 ? desc_packed(d, 1) : p0, p2 = np > 2 ? desc_packed(d, 2) : p0;
+                const bool inside = np <= 3 && !desc_listed(d.w) && min(p0, min(p1, p2)) >= wlo;
+                w_desc[o] = make_int4(inside ? (p0 - wlo) * kTilePitch : -1, (p1 - wlo) * kTilePitch,
+                                      (p2 - wlo) * kTilePitch, int(desc_base(d.w)));
             }
         }
         for (int c = lane; c < kCols; c += 32) w_seq[c] = (clo + c >= 1 && clo + c <= L) ? seq[clo + c - 1] : 0;
@@ -1384,12 +1799,13 @@ __device__ __noinline__ bool traceback_warp(const Graph& g, const int* order, co
                 } else {
                     // long list, or a predecessor above the tile: the first
                     // diagonal, else the first vertical
-                    const int4 e = rowdesc[wlo + oi / kTilePitch - 1];
+                    const int4 e = w_raw[oi / kTilePitch];
                     const int np = desc_np(e.w);
                     int vr = -1, dr = -1;
                     for (int p = 0; p < max(np, 1) && dr < 0; ++p) {
-                        const int r = np == 0 ? 0 : np > 3 ? (p == 0 ? e.y : pred_idx[e.x + p]) : p == 0 ? e.x : p == 1 ? e.y : e.z;
-                        const uint8_t* const pr = Hb + (size_t(r) * lc + clo + cj) * HB;
+                        const int r = desc_pred(pred_idx, e, p);
+                        const uint8_t* const pr = r >= wlo ? tj + (r - wlo) * kTilePitch
+                                                           : Hb + (size_t(r) * lc + clo + cj) * HB;  // generic address
                         if (col && score(pr - HB) == h - s) dr = r;
                         if (vr < 0 && score(pr) == h - gap) vr = r;
                     }
@@ -1427,772 +1843,15 @@ __device__ __noinline__ bool traceback_warp(const Graph& g, const int* order, co
     return ok;
 }
 
-// ---------------- compact adjacency in shared memory ----------------
-
-// In-edge sources and aligned nodes of every node as uint16 CSR lists in a
-// warp's shared memory, in the graph's own list order (in-edges by edge id,
-// aligned entries by slot: both are append-only), plus one flag byte per
-// node. The DFS steps then read shared memory instead of chasing linked
-// lists through global memory.
-struct SmemCsr {
-    uint16_t* in_off;  // [N + 1]
-    uint16_t* al_off;  // [N + 1]
-    uint16_t* in_src;  // [E]
-    uint16_t* al_x;    // [A]
-    uint8_t* flag;     // [N]: mark (bits 0-1), primary (bit 2), member (bit 3)
-};
-
-__device__ __forceinline__ size_t csr_bytes(int N, int E, int A) {
-    return 2 * (size_t(N) + 1) * 2 + 2 * size_t(E) + 2 * size_t(A) + size_t(N);
-}
-
-// Builds the lists (warp). Returns false, building nothing, when the graph
-// does not fit in `cap` bytes or 16-bit indices.
-__device__ bool build_csr(const Graph& g, const PoaShared& sh, int lane, void* smem, int cap, SmemCsr& c) {
-    const int N = sh.nnodes, E = sh.nedges, A = sh.naligned;
-    if (N >= 65535 || E >= 65535 || A >= 65535 || csr_bytes(N, E, A) > size_t(cap)) return false;
-    uint16_t* base = reinterpret_cast<uint16_t*>(smem);
-    c.in_off = base;
-    c.al_off = base + (N + 1);
-    c.in_src = base + 2 * (N + 1);
-    c.al_x = c.in_src + E;
-    c.flag = reinterpret_cast<uint8_t*>(c.al_x + A);
-    // starts: exclusive prefix of the counts
-    // (graph-array loads are issued four 32-element chunks at a time)
-    int bi = 0, ba = 0;
-    for (int c4 = 0; c4 < N; c4 += 128) {
-        int ci[4], ca[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int v = c4 + 32 * u + lane;
-            ci[u] = v < N ? g.in_cnt[v] : 0;
-            ca[u] = v < N ? g.al_cnt[v] : 0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int v = c4 + 32 * u + lane;
-            int ti = 0, ta = 0;
-            const int xi = warp_excl(ci[u], lane, ti);
-            const int xa = warp_excl(ca[u], lane, ta);
-            if (v < N) {
-                c.in_off[v] = uint16_t(bi + xi);
-                c.al_off[v] = uint16_t(ba + xa);
-            }
-            bi += ti;
-            ba += ta;
-        }
-    }
-    if (lane == 0) {
-        c.in_off[N] = uint16_t(E);
-        c.al_off[N] = uint16_t(A);
-    }
-    __syncwarp();
-    // stable fill by owner: the offsets serve as cursors and end up at the
-    // next node's start
-    const unsigned below = (1u << lane) - 1u;
-    for (int c4 = 0; c4 < E; c4 += 128) {
-        int ds[4], ss[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int e = c4 + 32 * u + lane;
-            ds[u] = e < E ? g.e_dst[e] : -1 - lane;
-            ss[u] = e < E ? g.e_src[e] : 0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int dst = ds[u];
-            const unsigned grp = __match_any_sync(0xffffffffu, dst);
-            const int cur = dst >= 0 ? c.in_off[dst] : 0;
-            __syncwarp();
-            if (dst >= 0) {
-                c.in_src[cur + __popc(grp & below)] = uint16_t(ss[u]);
-                if ((grp & below) == 0) c.in_off[dst] = uint16_t(cur + __popc(grp));
-            }
-            __syncwarp();
-        }
-    }
-    for (int c4 = 0; c4 < A; c4 += 128) {
-        int os[4], ys[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int x = c4 + 32 * u + lane;
-            os[u] = x < A ? g.a_owner[x] : -1 - lane;
-            ys[u] = x < A ? g.a_node[x] : 0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int own = os[u];
-            const unsigned grp = __match_any_sync(0xffffffffu, own);
-            const int cur = own >= 0 ? c.al_off[own] : 0;
-            __syncwarp();
-            if (own >= 0) {
-                c.al_x[cur + __popc(grp & below)] = uint16_t(ys[u]);
-                if ((grp & below) == 0) c.al_off[own] = uint16_t(cur + __popc(grp));
-            }
-            __syncwarp();
-        }
-    }
-    // shift the cursors back to starts (off[v] = end of v - 1), top chunk first
-    for (int c0 = ((N - 1) / 32) * 32; c0 >= 0; c0 -= 32) {
-        const int v = c0 + lane;
-        uint16_t pi = 0, pa = 0;
-        if (v < N && v > 0) {
-            pi = c.in_off[v - 1];
-            pa = c.al_off[v - 1];
-        }
-        __syncwarp();
-        if (v < N) {
-            c.in_off[v] = pi;
-            c.al_off[v] = pa;
-        }
-        __syncwarp();
-    }
-    return true;
-}
-
-// g_topo_sort over the shared-memory lists (lane 0; flags initialised by the
-// caller: mark 0, primary set, member bit for the nodes taking part).
-__device__ int g_topo_sort_csr(const Graph& g, const SmemCsr& c, int N, bool all_nodes, int* out) {
-    int nr = 0;
-    int sp = 0;
-    auto member = [&](int x) { return all_nodes || (c.flag[x] & 8); };
-    auto mark = [&](int x) { return c.flag[x] & 3; };
-    auto set_mark = [&](int x, int m) { c.flag[x] = uint8_t((c.flag[x] & ~3) | m); };
-    for (int i = 0; i < N; ++i) {
-        if (!member(i) || mark(i) != 0) continue;
-        g.stack[sp++] = i;
-        while (sp > 0) {
-            const int v = g.stack[sp - 1];
-            bool valid = true;
-            if (mark(v) != 2) {
-                for (int q = c.in_off[v], qe = c.in_off[v + 1]; q < qe; ++q) {
-                    const int u = c.in_src[q];
-                    if (!member(u)) continue;
-                    if (mark(u) != 2) {
-                        if (sp >= g.scap) return -1;
-                        g.stack[sp++] = u;
-                        valid = false;
-                    }
-                }
-                if (c.flag[v] & 4) {
-                    for (int q = c.al_off[v], qe = c.al_off[v + 1]; q < qe; ++q) {
-                        const int y = c.al_x[q];
-                        if (!member(y)) continue;
-                        if (mark(y) != 2) {
-                            if (sp >= g.scap) return -1;
-                            g.stack[sp++] = y;
-                            c.flag[y] &= uint8_t(~4);
-                            valid = false;
-                        }
-                    }
-                }
-                if (valid) {
-                    set_mark(v, 2);
-                    if (c.flag[v] & 4) {
-                        out[nr++] = v;
-                        for (int q = c.al_off[v], qe = c.al_off[v + 1]; q < qe; ++q) {
-                            const int y = c.al_x[q];
-                            if (!member(y)) continue;
-                            out[nr++] = y;
-                        }
-                    }
-                } else {
-                    set_mark(v, 1);
-                }
-            }
-            if (valid) --sp;
-        }
-    }
-    return nr;
-}
-
-// spoa's topological order of the graph (all_nodes) or of the member nodes,
-// into out; shared-memory lists when they fit in the warp's ring, else the
-// global-memory walk. Warp-collective; the count is returned on every lane
-// (-1 on stack overflow).
-__device__ int topo_sort_warp(const Graph& g, PoaShared& sh, bool all_nodes, int* out, int lane, int4* ring) {
-    const int N = sh.nnodes;
-    SmemCsr c;
-    int nr = 0;
-    if (build_csr(g, sh, lane, ring, sh.scratch_bytes, c)) {
-        for (int i = lane; i < N; i += 32) c.flag[i] = uint8_t(4 | (all_nodes || g.member[i] ? 8 : 0));
-        __syncwarp();
-        if (lane == 0) nr = g_topo_sort_csr(g, c, N, all_nodes, out);
-    } else {
-        for (int i = lane; i < N; i += 32) {
-            g.mark[i] = 0;
-            g.prim[i] = 1;
-        }
-        __syncwarp();
-        if (lane == 0) nr = g_topo_sort(g, sh, all_nodes, out);
-    }
-    return __shfl_sync(0xffffffffu, nr, 0);
-}
-
-// spoa's subgraph node set (g_mark_subgraph) into g.member, over the
-// shared-memory lists when they fit. Warp-collective; false on stack
-// overflow (on every lane).
-__device__ bool mark_subgraph_warp(const Graph& g, PoaShared& sh, int begin_node, int end_node, int lane, int4* ring) {
-    const int N = sh.nnodes;
-    if (end_node < 0 || end_node >= N) {
-        if (lane == 0) sh.fail = kFailed;
-        __syncwarp();
-        return true;
-    }
-    SmemCsr c;
-    bool ok = true;
-    if (build_csr(g, sh, lane, ring, sh.scratch_bytes, c)) {
-        for (int i = lane; i < N; i += 32) c.flag[i] = 0;
-        __syncwarp();
-        if (lane == 0) {
-            int sp = 0;
-            g.stack[sp++] = end_node;
-            while (sp > 0 && ok) {
-                const int v = g.stack[--sp];
-                if (!(c.flag[v] & 8) && v >= begin_node) {
-                    for (int q = c.in_off[v], qe = c.in_off[v + 1]; q < qe; ++q) {
-                        if (sp >= g.scap) {
-                            ok = false;
-                            break;
-                        }
-                        g.stack[sp++] = c.in_src[q];
-                    }
-                    for (int q = c.al_off[v], qe = c.al_off[v + 1]; q < qe && ok; ++q) {
-                        if (sp >= g.scap) {
-                            ok = false;
-                            break;
-                        }
-                        g.stack[sp++] = c.al_x[q];
-                    }
-                    c.flag[v] |= 8;
-                }
-            }
-        }
-        __syncwarp();
-        for (int i = lane; i < N; i += 32) g.member[i] = (c.flag[i] & 8) ? 1 : 0;
-    } else if (lane == 0) {
-        ok = g_mark_subgraph(g, sh, begin_node, end_node);
-    }
-    __syncwarp();
-    return __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-}
-
-// Row descriptors with shared-memory accumulators (the ring is free until the
-// DP): node ranks as uint16 (bit 15 marks a node with a successor row) and,
-// per row, the first three predecessor ranks and the count. Loads of graph
-// arrays are issued four 32-element chunks at a time, so one memory latency
-// covers 128 edges or rows. Same order rules as the global form below.
-// Returns false, building nothing, when the graph does not fit.
-__device__ bool descriptors_smem(const Graph& g, PoaShared& sh, const int* order, int N, int ndp, int lane,
-                                 int4* ring) {
-    constexpr unsigned kFull = 0xffffffffu;
-    const size_t rk_bytes = size_t((N + 3) / 4) * 8;
-    if (ndp >= 32768 || sh.nseq >= 65535 || rk_bytes + size_t(8) * ndp > size_t(sh.scratch_bytes)) return false;
-    uint16_t* const rk = reinterpret_cast<uint16_t*>(ring);
-    ushort4* const acc = reinterpret_cast<ushort4*>(reinterpret_cast<uint8_t*>(ring) + rk_bytes);
-    for (int i = lane; i < N; i += 32) rk[i] = 0;
-    for (int i = lane; i < ndp; i += 32) acc[i] = make_ushort4(0, 0, 0, 0);
-    __syncwarp();
-    for (int c0 = 0; c0 < ndp; c0 += 128) {
-        int v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = c0 + 32 * u + lane;
-            v[u] = i < ndp ? order[i] : -1;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (v[u] >= 0) rk[v[u]] = uint16_t(c0 + 32 * u + lane + 1);
-    }
-    __syncwarp();
-    const int E = sh.nedges;
-    const unsigned below = (1u << lane) - 1u;
-    bool any_long = false;
-    for (int c0 = 0; c0 < E; c0 += 128) {
-        int es[4], ed[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int e = c0 + 32 * u + lane;
-            es[u] = e < E ? g.e_src[e] : -1;
-            ed[u] = e < E ? g.e_dst[e] : -1;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int src = es[u], dst = ed[u];
-            int rs = 0, rd = 0;
-            if (src >= 0) {
-                rs = rk[src] & 0x7FFF;
-                rd = rs > 0 ? rk[dst] & 0x7FFF : 0;
-            }
-            const bool q = rs > 0 && rd > 0;
-            const unsigned grp = __match_any_sync(kFull, q ? rd : -1 - lane);
-            int cnt = 0;
-            if (q) cnt = acc[rd - 1].w;
-            __syncwarp();
-            if (q) {
-                rk[src] = uint16_t(rs | 0x8000);  // every writer stores the same value
-                const int pos = cnt + __popc(grp & below);
-                uint16_t* a4 = reinterpret_cast<uint16_t*>(&acc[rd - 1]);
-                if (pos < 3) a4[pos] = uint16_t(rs);
-                if ((grp & below) == 0) {
-                    const int tot = cnt + __popc(grp);
-                    a4[3] = uint16_t(tot);
-                    any_long |= tot > 3;
-                }
-            }
-            __syncwarp();
-        }
-    }
-    any_long = __any_sync(kFull, any_long);
-    int list_base = 0, preds = 0;
-    for (int c0 = 0; c0 < ndp; c0 += 128) {
-        int v[4], code[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = c0 + 32 * u + lane;
-            v[u] = i < ndp ? order[i] : 0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) code[u] = c0 + 32 * u + lane < ndp ? g.code[v[u]] : 0;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            if (c0 + 32 * u >= ndp) break;
-            const int i = c0 + 32 * u + lane;
-            const ushort4 dd = i < ndp ? acc[i] : make_ushort4(0, 0, 0, 0);
-            const int np = dd.w;
-            preds += np;
-            int off = 0;
-            if (any_long) {
-                int tot = 0;
-                const int cntl = (i < ndp && np > 3) ? np : 0;
-                off = list_base + warp_excl(cntl, lane, tot);
-                list_base += tot;
-                if (cntl) g.bpred[v[u]] = off;  // list cursor of the node
-            }
-            if (i < ndp) {
-                const bool sink = (rk[v[u]] & 0x8000) == 0;
-                g.sink[i] = sink ? 1 : 0;
-                // long rows: x = list offset, y = first predecessor
-                g.rowdesc[i] = make_int4(np > 3 ? off : dd.x, np > 3 ? dd.x : dd.y, dd.z,
-                                         int(uint32_t(np) | (uint32_t(sink) << 17) | (uint32_t(code[u]) << 24)));
-            }
-        }
-    }
-    preds = __reduce_add_sync(kFull, preds);
-    if (lane == 0) sh.preds = preds;
-    __syncwarp();
-    if (any_long) {
-        for (int c0 = 0; c0 < E; c0 += 32) {
-            const int e = c0 + lane;
-            int rs = 0, dst = 0;
-            bool q = false;
-            if (e < E) {
-                dst = g.e_dst[e];
-                const int rd = rk[dst] & 0x7FFF;
-                if (rd > 0 && acc[rd - 1].w > 3) {
-                    rs = rk[g.e_src[e]] & 0x7FFF;
-                    q = rs > 0;
-                }
-            }
-            const unsigned grp = __match_any_sync(kFull, q ? dst : -1 - lane);
-            int cur = 0;
-            if (q) cur = g.bpred[dst];
-            __syncwarp();
-            if (q) {
-                g.pred_idx[cur + __popc(grp & below)] = rs;
-                if ((grp & below) == 0) g.bpred[dst] = cur + __popc(grp);
-            }
-            __syncwarp();
-        }
-    }
-    __syncwarp();
-    return true;
-}
-
-// Heaviest bundle (g_heaviest_bundle) with the scores in shared memory: per
-// node an int32 score and a uint16 predecessor, and for each chunk of 32 ranks
-// the in-edges (source, weight) staged by the lanes in parallel, so the
-// serial pass of lane 0 touches no global memory. Scores are bounded by
-// sequences x 186 x nodes (two Phred values per sequence and edge, summed
-// along a path), checked against int32. When branch completion is needed, or
-// the graph does not fit, the global form finishes or does the work.
-// Warp-collective; returns the path length (-1 on failure) on every lane.
-__device__ int heaviest_bundle_warp(const Graph& g, PoaShared& sh, int lane, int4* ring) {
-    constexpr int D = 8;  // staged in-edges per node
-    const int N = sh.nnodes, R = sh.nranks;
-    uint8_t* base = reinterpret_cast<uint8_t*>(ring);
-    int* const bs = reinterpret_cast<int*>(base);                             // [N]
-    uint16_t* const bp = reinterpret_cast<uint16_t*>(base + 4 * size_t(N));   // [N], 0xFFFF = none
-    const size_t st_off = (6 * size_t(N) + 15) & ~size_t(15);
-    int* const sw = reinterpret_cast<int*>(base + st_off);                    // [32][D] weights
-    uint16_t* const su = reinterpret_cast<uint16_t*>(sw + 32 * D);            // [32][D] sources
-    int* const sv = reinterpret_cast<int*>(su + 32 * D);                      // [32] node
-    int* const sd = sv + 32;                                                  // [32] degree, D + 1 = more
-    const size_t need = st_off + 32 * D * 6 + 32 * 8;
-    const bool fits = N < 65535 && need <= size_t(sh.scratch_bytes) &&
-                      double(sh.nseq + 1) * 186.0 * double(N + 1) < 2.0e9;
-    if (!fits) {
-        int len = 0;
-        if (lane == 0) len = g_heaviest_bundle(g, sh);
-        return __shfl_sync(0xffffffffu, len, 0);
-    }
-    for (int i = lane; i < N; i += 32) {
-        bs[i] = -1;
-        bp[i] = 0xFFFF;
-    }
-    __syncwarp();
-    int best_id = 0;
-    for (int r0 = 0; r0 < R; r0 += 32) {
-        const int r = r0 + lane;
-        if (r < R) {
-            const int v = g.rank_to_node[r];
-            int deg = 0;
-            for (int e = g.in_head[v]; e != -1; e = g.e_next_in[e]) {
-                if (deg == D) {
-                    deg = D + 1;
-                    break;
-                }
-                su[lane * D + deg] = uint16_t(g.e_src[e]);
-                sw[lane * D + deg] = g.e_w[e];
-                ++deg;
-            }
-            sv[lane] = v;
-            sd[lane] = deg;
-        }
-        __syncwarp();
-        if (lane == 0) {
-            const int cnt = min(32, R - r0);
-            for (int t = 0; t < cnt; ++t) {
-                const int v = sv[t];
-                const int deg = sd[t];
-                int sv_ = bs[v], pv_ = bp[v] == 0xFFFF ? -1 : int(bp[v]);
-                auto consider = [&](int u, int w) {
-                    if (sv_ < w || (sv_ == w && pv_ != -1 && bs[pv_] <= bs[u])) {
-                        sv_ = w;
-                        pv_ = u;
-                    }
-                };
-                if (deg <= D) {
-                    for (int q = 0; q < deg; ++q) consider(su[t * D + q], sw[t * D + q]);
-                } else {
-                    for (int e = g.in_head[v]; e != -1; e = g.e_next_in[e]) consider(g.e_src[e], g.e_w[e]);
-                }
-                if (pv_ != -1) sv_ += bs[pv_];
-                bs[v] = sv_;
-                bp[v] = pv_ < 0 ? uint16_t(0xFFFF) : uint16_t(pv_);
-                if (bs[best_id] < sv_) best_id = v;
-            }
-        }
-        __syncwarp();
-    }
-    best_id = __shfl_sync(0xffffffffu, best_id, 0);
-    const bool complete = g.out_head[best_id] != -1;
-    if (complete) {
-        // branch completion works on the global arrays
-        for (int i = lane; i < N; i += 32) {
-            g.bscore[i] = bs[i];
-            g.bpred[i] = bp[i] == 0xFFFF ? -1 : int(bp[i]);
-        }
-        __syncwarp();
-        int len = 0;
-        if (lane == 0) {
-            for (int r = 0; r < R; ++r) g.node_rank[g.rank_to_node[r]] = r;
-            int guard = 0;
-            len = 1;
-            while (g.out_head[best_id] != -1) {
-                best_id = g_branch_completion(g, sh, g.node_rank[best_id]);
-                if (++guard > N + 1) {
-                    len = -1;
-                    break;
-                }
-            }
-            if (len > 0) {
-                len = 0;
-                while (g.bpred[best_id] != -1) {
-                    g.cons[len++] = best_id;
-                    best_id = g.bpred[best_id];
-                    if (len > N) {
-                        len = -1;
-                        break;
-                    }
-                }
-                if (len >= 0) g.cons[len++] = best_id;
-            }
-            for (int i = 0, j = len - 1; i < j; ++i, --j) {
-                const int t = g.cons[i];
-                g.cons[i] = g.cons[j];
-                g.cons[j] = t;
-            }
-        }
-        return __shfl_sync(0xffffffffu, len, 0);
-    }
-    int len = 0;
-    if (lane == 0) {
-        int v = best_id;
-        while (bp[v] != 0xFFFF) {
-            g.cons[len++] = v;
-            v = bp[v];
-            if (len > N) {
-                len = -1;
-                break;
-            }
-        }
-        if (len >= 0) {
-            g.cons[len++] = v;
-            for (int i = 0, j = len - 1; i < j; ++i, --j) {
-                const int t = g.cons[i];
-                g.cons[i] = g.cons[j];
-                g.cons[j] = t;
-            }
-        }
-    }
-    return __shfl_sync(0xffffffffu, len, 0);
-}
-
-// Rows of one layer's DP (warp): marks the subgraph of a partial layer, lists
-// its rows (the incremental order, restricted to the subgraph) and builds
-// their descriptors. sh.ndp rows, or sh.fail.
-__device__ void layer_rows(const Graph& g, PoaShared& sh, const int* order, bool full, int begin, int end, int lane,
-                           int4* ring) {
-    const int N = sh.nnodes;
-    for (int i = lane; i < N; i += 32) g.member[i] = full ? 1 : 0;
-    __syncwarp();
-    if (!full && !mark_subgraph_warp(g, sh, begin, end, lane, ring) && lane == 0) sh.fail = kOverflow;
-    __syncwarp();
-    if (sh.fail) return;
-            // DP rows: the incremental order, restricted to the subgraph for a
-            // partial layer (any topological order gives the same DP values)
-            int ndp = N;
-                    if (!full) {
-                // compaction of the member nodes in order; the loads of four
-                // 32-entry chunks go out together
-                int base = 0;
-                for (int c4 = 0; c4 < N; c4 += 128) {
-                    int vv[4];
-                    bool in[4];
-    #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int r = c4 + 32 * u + lane;
-                        vv[u] = r < N ? g.ord[r] : 0;
-                    }
-    #pragma unroll
-                    for (int u = 0; u < 4; ++u) in[u] = c4 + 32 * u + lane < N && g.member[vv[u]];
-    #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const unsigned m = __ballot_sync(0xffffffffu, in[u]);
-                        if (in[u]) g.dporder[base + __popc(m & ((1u << lane) - 1u))] = vv[u];
-                        base += __popc(m);
-                    }
-                }
-                ndp = base;
-                        __syncwarp();
-            }
-            // Row descriptors: shared-memory accumulators when the graph fits,
-            // else the global form below.
-            if (!descriptors_smem(g, sh, order, N, ndp, lane, ring)) {
-                // Row descriptors. DP ranks of the nodes live in shared memory (the
-                // row ring is free until the DP) when they fit, else in global
-                // scratch; bit 31 marks a node with a successor among the rows.
-                int* const dpr = 4 * N <= sh.scratch_bytes ? reinterpret_cast<int*>(ring) : g.dprank;
-                for (int i = lane; i < N; i += 32) dpr[i] = 0;
-                __syncwarp();
-                for (int i = lane; i < ndp; i += 32) dpr[order[i]] = i + 1;
-                __syncwarp();
-                // Predecessors by one pass over the edges in id order. A node's
-                // in-edge list is in edge-id order (each layer adds at most one edge
-                // into a node, with a fresh, larger id), which is spoa's predecessor
-                // order. Lanes take 32 consecutive edges; edges into the same row
-                // are ranked by lane, so the order is deterministic. rowdesc[r - 1]
-                // collects the first three predecessor ranks (x, y, z) and the count
-                // (w) of row r; bit 31 of dpr marks a node with a successor row.
-                for (int i = lane; i < ndp; i += 32) g.rowdesc[i] = make_int4(0, 0, 0, 0);
-                __syncwarp();
-                const int E = sh.nedges;
-                const unsigned below = (1u << lane) - 1u;
-                bool any_long = false;
-                for (int c0 = 0; c0 < E; c0 += 32) {
-                    const int e = c0 + lane;
-                    int rs = 0, rd = 0, src = 0;
-                    if (e < E) {
-                        src = g.e_src[e];
-                        const int dst = g.e_dst[e];
-                        rs = dpr[src] & 0x7FFFFFFF;
-                        rd = rs > 0 ? dpr[dst] & 0x7FFFFFFF : 0;
-                    }
-                    const bool q = rs > 0 && rd > 0;
-                    const unsigned grp = __match_any_sync(0xffffffffu, q ? rd : -1 - lane);
-                    int cnt = 0;
-                    if (q) {
-                        atomicOr(reinterpret_cast<unsigned*>(&dpr[src]), 0x80000000u);
-                        cnt = g.rowdesc[rd - 1].w;
-                    }
-                    __syncwarp();
-                    if (q) {
-                        const int pos = cnt + __popc(grp & below);
-                        int* rdw = reinterpret_cast<int*>(&g.rowdesc[rd - 1]);
-                        if (pos < 3) rdw[pos] = rs;
-                        if ((grp & below) == 0) {
-                            const int tot = cnt + __popc(grp);
-                            rdw[3] = tot;
-                            any_long |= tot > 3;
-                        }
-                    }
-                    __syncwarp();
-                }
-                any_long = __any_sync(0xffffffffu, any_long);
-                // final descriptors; rows with more than three predecessors get their
-                // full list in pred_idx at an offset from a warp prefix of the counts
-                int list_base = 0, preds = 0;
-                for (int c0 = 0; c0 < ndp; c0 += 32) {
-                    const int i = c0 + lane;
-                    int4 dd = i < ndp ? g.rowdesc[i] : make_int4(0, 0, 0, 0);
-                    const int v = i < ndp ? order[i] : 0;
-                    int off = 0;
-                preds += dd.w;
-                    if (any_long) {
-                        int tot = 0;
-                        const int cntl = (i < ndp && dd.w > 3) ? dd.w : 0;
-                        off = list_base + warp_excl(cntl, lane, tot);
-                        list_base += tot;
-                        if (cntl) g.bpred[v] = off;  // list cursor of the node
-                    }
-                    if (i < ndp) {
-                        const bool sink = (dpr[v] & 0x80000000) == 0;
-                        g.sink[i] = sink ? 1 : 0;
-                        // long rows: x = list offset, y = first predecessor
-                        g.rowdesc[i] = make_int4(dd.w > 3 ? off : dd.x, dd.w > 3 ? dd.x : dd.y, dd.z,
-                                                 int(uint32_t(dd.w) | (uint32_t(sink) << 17) | (uint32_t(g.code[v]) << 24)));
-                    }
-                }
-                preds = __reduce_add_sync(0xffffffffu, preds);
-        if (lane == 0) sh.preds = preds;
-        __syncwarp();
-                if (any_long) {
-                    // second pass over the edges for the long lists, same ranking
-                    for (int c0 = 0; c0 < E; c0 += 32) {
-                        const int e = c0 + lane;
-                        int rs = 0, dst = 0;
-                        bool q = false;
-                        if (e < E) {
-                            dst = g.e_dst[e];
-                            const int rd = dpr[dst] & 0x7FFFFFFF;
-                            if (rd > 0 && desc_np(g.rowdesc[rd - 1].w) > 3) {
-                                rs = dpr[g.e_src[e]] & 0x7FFFFFFF;
-                                q = rs > 0;
-                            }
-                        }
-                        const unsigned grp = __match_any_sync(0xffffffffu, q ? dst : -1 - lane);
-                        int cur = 0;
-                        if (q) cur = g.bpred[dst];
-                        __syncwarp();
-                        if (q) {
-                            g.pred_idx[cur + __popc(grp & below)] = rs;
-                            if ((grp & below) == 0) g.bpred[dst] = cur + __popc(grp);
-                        }
-                        __syncwarp();
-                    }
-                }
-                __syncwarp();
-            }
-    if (lane == 0) sh.ndp = ndp;
-    __syncwarp();
-}
-
-// NW end row of the layer (warp): the first sink row with the best
-// last-column score, or, when several sinks share it, spoa's first among
-// them. Sets sh.end_value.
-template <bool FAST>
-__device__ int end_row(const Graph& g, PoaShared& sh, const int* order, int ndp, int L, int lc, bool full, int lane,
-                       int4* ring) {
-    const uint8_t* const Hb = reinterpret_cast<const uint8_t*>(g.H);
-    int best = INT_MIN, iend = INT_MAX, ties = 0;
-    for (int i = 1 + lane; i <= ndp; i += 32) {
-        if (!g.sink[i - 1]) continue;
-        const int v = h_at<FAST>(Hb, i, L, lc);
-        g.lastH[i] = v;
-        ties = v > best ? 1 : ties + (v == best ? 1 : 0);
-        iend = v > best ? i : iend;
-        best = max(best, v);
-    }
-    sh.end_value = __reduce_max_sync(0xffffffffu, best);
-    __syncwarp();
-    if (best != sh.end_value) {
-        ties = 0;
-        iend = INT_MAX;
-    }
-    iend = __reduce_min_sync(0xffffffffu, iend);
-    ties = __reduce_add_sync(0xffffffffu, ties);
-    if (ties > 1) {
-                // several sinks share the best last-column value: spoa takes the
-                // first in its own topological order of the aligned (sub)graph.
-                // A sink outside every aligned group is reached by spoa's DFS
-                // only as a root (no member lists it as an in-edge tail, and
-                // aligned links are symmetric), so such sinks are ranked by node
-                // id; only a tie that involves an aligned sink needs the DFS.
-                int low_id = INT_MAX, low_i = iend;
-                bool grouped = false;
-                for (int i = 1 + lane; i <= ndp; i += 32) {
-                    if (!g.sink[i - 1] || g.lastH[i] != sh.end_value) continue;
-                    const int v = order[i - 1];
-                    grouped |= g.al_cnt[v] != 0;
-                    if (v < low_id) {
-                        low_id = v;
-                        low_i = i;
-                    }
-                }
-    #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const int ov = __shfl_xor_sync(0xffffffffu, low_id, o);
-                    const int oi = __shfl_xor_sync(0xffffffffu, low_i, o);
-                    if (ov < low_id) {
-                        low_id = ov;
-                        low_i = oi;
-                    }
-                }
-                grouped = __any_sync(0xffffffffu, grouped);
-                const int nr = grouped ? topo_sort_warp(g, sh, full, g.rank_to_node, lane, ring) : 0;
-                if (!grouped) {
-                    iend = low_i;
-                } else if (nr < 0) {
-                    if (lane == 0) sh.fail = kOverflow;
-                } else {
-                    for (int r = lane; r < nr; r += 32) g.node_rank[g.rank_to_node[r]] = r;
-                    __syncwarp();
-                    // the tied sink of lowest rank (ranks are distinct)
-                    int best = INT_MAX, bi = iend;
-                    for (int i = 1 + lane; i <= ndp; i += 32) {
-                        if (!g.sink[i - 1] || g.lastH[i] != sh.end_value) continue;
-                        const int rr = g.node_rank[order[i - 1]];
-                        if (rr < best) {
-                            best = rr;
-                            bi = i;
-                        }
-                    }
-    #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        const int ob = __shfl_xor_sync(0xffffffffu, best, o);
-                        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                        if (ob < best) {
-                            best = ob;
-                            bi = oi;
-                        }
-                    }
-                    iend = bi;
-                }
-                __syncwarp();
-            }
-    return iend;
-}
-
 // ---------------- one window (one team) ----------------
 
-// The team's warps share the set-up and the DPs; warp 0 does the graph steps
-// between them. Every thread of the team returns together.
+// Every thread of the team returns together.
 template <int NW>
-__device__ void poa_window(const PoaArgs& a, const Graph& g, PoaShared& sh, uint32_t wi, int lane, int w, int team) {
+__device__ void poa_window(const PoaArgs& a, Graph& g, PoaShared& sh, uint32_t wi, int lane, int w, int team) {
     constexpr int NT = 32 * NW;
     const int tid = 32 * w + lane;
-    int4* const ring = g_poa_smem + team * (NW * WarpMem<NW>::bytes / 16);
+    constexpr int kTeamBytes = NW * WarpMem<NW>::bytes;
+    uint8_t* const smem = reinterpret_cast<uint8_t*>(g_poa_smem) + team * kTeamBytes;
     const PoaWinDev W = a.wins[wi];
     const uint8_t* bb = a.in + W.bb_off;
     const uint8_t* bq = W.bq_off == kNoQual ? nullptr : a.in + W.bq_off;
@@ -2217,38 +1876,22 @@ __device__ void poa_window(const PoaArgs& a, const Graph& g, PoaShared& sh, uint
     for (int i = tid; i < B; i += NT) {
         g.code[i] = bb[i];
         g.cov[i] = B >= 2 ? 1u : 0u;
-        g.al_head[i] = g.al_tail[i] = -1;
-        if (i == 0) {
-            g.in_head[i] = g.in_tail[i] = -1;
-        } else {
-            const int e = i - 1;
-            g.in_head[i] = g.in_tail[i] = e;
-            const int w = (bq ? int(bq[i - 1]) - 33 : 0) + (bq ? int(bq[i]) - 33 : 0);
-            g.e_src[e] = i - 1;
-            g.e_dst[e] = i;
-            g.e_w[e] = w;
-            g.e_next_in[e] = -1;
-            g.e_next_out[e] = -1;
-        }
-        if (i == B - 1) {
-            g.out_head[i] = g.out_tail[i] = -1;
-        } else {
-            g.out_head[i] = g.out_tail[i] = i;
-        }
-        g.ord[i] = i;
-        g.my_rank[i] = i;
         g.in_cnt[i] = i > 0 ? 1 : 0;
-        g.al_cnt[i] = 0;
         g.out_cnt[i] = i + 1 < B ? 1 : 0;
+        g.al_cnt[i] = 0;
+        const int wt = i > 0 && bq ? (int(bq[i - 1]) - 33) + (int(bq[i]) - 33) : 0;
+        g.in_src[2 * size_t(i)] = make_int4(i - 1, 0, 0, 0);
+        g.in_w[2 * size_t(i)] = make_int4(wt, 0, 0, 0);
+        g.ord[i] = i;
+        g.rank[i] = i;
     }
     if (tid == 0) {
         sh.nnodes = B;
-        sh.nedges = B - 1;
+        sh.nedges = 0;
         sh.naligned = 0;
         sh.nseq = 1;
-        sh.nranks = B;
         sh.fail = 0;
-        sh.scratch_bytes = NW * WarpMem<NW>::bytes;
+        sh.scratch_bytes = kTeamBytes;
     }
     team_sync<NW>(team);
     unsigned long long cells = 0, edge_cells = 0;
@@ -2259,15 +1902,24 @@ __device__ void poa_window(const PoaArgs& a, const Graph& g, PoaShared& sh, uint
         const uint8_t* qual = Lr.qual_off == kNoQual ? nullptr : a.in + Lr.qual_off;
         const int L = int(Lr.len);
         const bool full = Lr.begin < W.offset && Lr.end > uint32_t(B) - W.offset;
-        const int* const order = full ? g.ord : g.dporder;
-        if (w == 0 && !sh.fail) {
-            // subgraph, DP rows and their descriptors
-            layer_rows(g, sh, order, full, int(Lr.begin), int(Lr.end), lane, ring);
-            if (lane == 0 && !sh.fail && row_cover(NW, L + 1) > g.lcap) sh.fail = kOverflow;
+        const int begin = full ? 0 : int(Lr.begin);
+        if (row_cover(NW, L + 1) > g.lcap) {
+            if (tid == 0) sh.fail = kOverflow;
+            break;
         }
-        team_sync<NW>(team);
-        if (sh.fail) break;
-        const int ndp = sh.ndp;
+        // DP rows: the incremental order, restricted to the subgraph for a
+        // partial layer (any topological order gives the same DP values)
+        build_rows<NW>(g, sh, g.ord, sh.nnodes, false, tid, team, smem);
+        int ndp = sh.nnodes;
+        const int* order = g.ord;
+        if (!full) {
+            if (w == 0) mark_subgraph(g, sh, begin, int(Lr.end), lane, smem);
+            team_sync<NW>(team);
+            if (sh.fail) break;
+            ndp = sh.ndp;
+            order = g.dporder;
+            build_rows<NW>(g, sh, order, ndp, true, tid, team, smem);
+        }
         bool fast = fast_scores(a.match, a.mismatch, a.gap, ndp, L);
         for (int k = lane; k < L; k += 32) fast = fast && acgt_base(seq[k]);
         fast = __all_sync(0xffffffffu, fast);
@@ -2276,88 +1928,81 @@ __device__ void poa_window(const PoaArgs& a, const Graph& g, PoaShared& sh, uint
         if (w == 0) {
             cells += (unsigned long long)ndp * (unsigned long long)L;
             edge_cells += (unsigned long long)(ndp + sh.preds) * (unsigned long long)L;
-            const int N = sh.nnodes;
-            const int off = team * (NW * WarpMem<NW>::bytes), lc = row_cover(NW, L + 1);
-            const int iend = fast ? end_row<true>(g, sh, order, ndp, L, lc, full, lane, ring)
-                                  : end_row<false>(g, sh, order, ndp, L, lc, full, lane, ring);
+            const int lc = row_cover(NW, L + 1);
+            const int iend = fast ? end_row<true>(g, sh, order, L, lc, !full, begin, B, lane, smem)
+                                  : end_row<false>(g, sh, order, L, lc, !full, begin, B, lane, smem);
             if (!sh.fail) {
                 const bool ok = fast ? traceback_warp<true>(g, order, seq, L, iend, sh.end_value, a.match, a.mismatch,
-                                                           a.gap, lane, off, lc)
-                                    : traceback_warp<false>(g, order, seq, L, iend, sh.end_value, a.match, a.mismatch,
-                                                            a.gap, lane, off, lc);
+                                                            a.gap, lane, team * kTeamBytes, lc)
+                                     : traceback_warp<false>(g, order, seq, L, iend, sh.end_value, a.match, a.mismatch,
+                                                             a.gap, lane, team * kTeamBytes, lc);
                 if (!ok && lane == 0) sh.fail = kFailed;
             }
-            __syncwarp();
-            if (!sh.fail) add_alignment_warp(g, sh, seq, qual, L, lane, ring);
-            if (!sh.fail) order_insert(g, sh, N, lane, ring);
         }
+        team_sync<NW>(team);
+        if (sh.fail) break;
+        add_layer<NW>(g, sh, seq, qual, L, lane, w, team, smem);
+        if (sh.fail) break;
+        order_insert<NW>(g, sh, lane, w, team, smem);
     }
     team_sync<NW>(team);
     if (w != 0) return;
-    // spoa's topological order of the final graph for the consensus
-    if (!sh.fail) {
-        const int nr = topo_sort_warp(g, sh, true, g.rank_to_node, lane, ring);
-        if (lane == 0) {
-            if (nr < 0) sh.fail = kOverflow;
-            sh.nranks = nr;
-        }
-        __syncwarp();
-    }
     if (lane == 0 && cells) {
         atomicAdd(a.cells, cells);
         atomicAdd(a.cells + 1, edge_cells);
     }
-    if (sh.fail) {
+    const int len = sh.fail ? 0 : heaviest_bundle_warp(g, sh, lane, smem);
+    if (sh.fail || len < 0) {
         if (lane == 0) {
-            a.flags[wi] = uint8_t(sh.fail);
+            a.flags[wi] = uint8_t(sh.fail ? sh.fail : kFailed);
             a.out_len[wi] = 0;
         }
+        __syncwarp();
         return;
     }
-    // ---- consensus ----
-    const int N = sh.nnodes;
-    for (int i = lane; i < N; i += 32) {
-        g.bscore[i] = -1;
-        g.bpred[i] = -1;
-    }
-    __syncwarp();
-    const int hb_len = heaviest_bundle_warp(g, sh, lane, ring);
-    if (lane == 0) {
-        const int len = hb_len;
-        uint8_t flags = kPolished;
-        if (len < 0) {
-            flags = kFailed;
-            a.out_len[wi] = 0;
-        } else {
-            int b = 0, e = len - 1;
-            if (W.tgs && a.trim) {
-                const uint32_t avg = W.n_layers / 2;
-                auto cov_at = [&](int k) {
-                    const int v = g.cons[k];
-                    uint32_t c = g.cov[v];
-                    for (int x = g.al_head[v]; x != -1; x = g.a_next[x]) c += g.cov[g.a_node[x]];
-                    return c;
-                };
-                for (b = 0; b < len; ++b)
-                    if (cov_at(b) >= avg) break;
-                for (e = len - 1; e >= 0; --e)
-                    if (cov_at(e) >= avg) break;
-                if (b >= e) {
-                    flags |= kChimeric;
-                    b = 0;
-                    e = len - 1;
-                }
-            }
-            const int outl = e - b + 1;
-            if (uint32_t(outl) > W.out_cap) {
-                flags = kOverflow;
-                a.out_len[wi] = 0;
-            } else {
-                for (int k = 0; k < outl; ++k) outp[k] = g.code[g.cons[b + k]];
-                a.out_len[wi] = uint32_t(outl);
-            }
+    // the path is in g.cons from its end
+    uint8_t flags = kPolished;
+    int b = 0, e = len - 1;
+    if (W.tgs && a.trim) {
+        const uint32_t avg = W.n_layers / 2;
+        auto covered = [&](int k) {
+            if (k < 0 || k >= len) return false;
+            const int v = g.cons[len - 1 - k];
+            uint32_t c = g.cov[v];
+            for_aligned(g, v, [&](int y) {
+                c += g.cov[y];
+                return true;
+            });
+            return c >= avg;
+        };
+        b = len;
+        e = -1;
+        for (int c0 = 0; c0 < len && b == len; c0 += 32) {
+            const unsigned m = __ballot_sync(0xffffffffu, covered(c0 + lane));
+            if (m) b = c0 + __ffs(m) - 1;
         }
-        a.flags[wi] = flags;
+        for (int c0 = len - 1; c0 >= 0 && e < 0; c0 -= 32) {
+            const unsigned m = __ballot_sync(0xffffffffu, covered(c0 - lane));
+            if (m) e = c0 - (__ffs(m) - 1);
+        }
+        if (b >= e) {
+            flags |= kChimeric;
+            b = 0;
+            e = len - 1;
+        }
+    }
+    const int outl = e - b + 1;
+    if (uint32_t(outl) > W.out_cap) {
+        if (lane == 0) {
+            a.flags[wi] = kOverflow;
+            a.out_len[wi] = 0;
+        }
+    } else {
+        for (int k = lane; k < outl; k += 32) outp[k] = g.code[g.cons[len - 1 - (b + k)]];
+        if (lane == 0) {
+            a.flags[wi] = flags;
+            a.out_len[wi] = uint32_t(outl);
+        }
     }
     __syncwarp();
 }
@@ -2379,7 +2024,7 @@ __global__ void __launch_bounds__(32 * cta_warps(NW), kCtasPerSm) poa_kernel(Poa
     PoaShared& sh = sh_all[team];
     const uint32_t slot = blockIdx.x * (blockDim.x / (32 * NW)) + team;
     if (w == 0 && lane == 0) g_all[team] = make_graph(a, slot);
-    const Graph& g = g_all[team];
+    Graph& g = g_all[team];
     // with a cap the CTA retires after that many windows per team, so other
     // streams' kernels get SMs between launches (the host launches enough)
     for (uint32_t done = 0; a.per_warp_cap == 0 || done < a.per_warp_cap; ++done) {
