@@ -424,98 +424,174 @@ __device__ void build_rows(const Graph& g, PoaShared& sh, const int* order, int 
 
 // spoa's subgraph of a partial layer: the nodes reached from end_node
 // backwards over in-edges and aligned links, going on only from nodes whose id
-// is not below begin_node. One sweep down the incremental order, in which
-// every aligned group is contiguous and a group's successors all come after
-// it: when the sweep reaches a group's last row, all links into the group
-// are known. The descriptors of the whole graph (just built) are staged 64
-// rows at a time and one lane sweeps them. Leaves the rows in g.dporder
-// (sh.ndp of them) and every node's DP rank (0: none) in g.sub_rank. Warp 0.
-__device__ void mark_subgraph(const Graph& g, PoaShared& sh, int begin_node, int end_node, int lane, uint8_t* smem) {
+// is not below begin_node. A sweep down the incremental order, in which every
+// aligned group is contiguous and a group's successors all come after it, 32
+// rows at a time, one per lane: within a chunk the reached rows grow to their
+// closure over the lanes' predecessor and group masks, one warp reduction a
+// step; then the chunk's rows mark their predecessors below it. A chunk ends
+// at a group's edge, so that all links into a group are known when its chunk
+// comes. (One lane following the links from row to row took 380 k cycles a
+// layer of 24 reads against 64 k.) Leaves the rows in g.dporder (sh.ndp of them) and
+// every node's DP rank (0: none) in g.sub_rank. The descriptors are those of
+// the whole graph (build_rows). By the team.
+template <int NW>
+__device__ void mark_subgraph(const Graph& g, PoaShared& sh, int begin_node, int end_node, int lane, int w, int team,
+                              uint8_t* smem) {
     constexpr unsigned kFull = 0xffffffffu;
-    constexpr int CH = 64, LOW = 8;
+    constexpr int NT = 32 * NW;
+    constexpr int kReached = 1, kInside = 2;  // flags; inside: id >= begin_node
+    const int tid = 32 * w + lane;
     const int N = sh.nnodes;
     if (end_node < 0 || end_node >= N) {
-        if (lane == 0) sh.fail = kFailed;
-        __syncwarp();
+        if (tid == 0) {
+            sh.fail = kFailed;
+            sh.ndp = 0;
+        }
+        team_sync<NW>(team);
         return;
     }
-    int4* const s_desc = reinterpret_cast<int4*>(smem);              // [CH]
-    int* const s_start = reinterpret_cast<int*>(s_desc + CH);        // [CH] first row of the row's group
-    int* const s_id = s_start + CH;                                  // [LOW + CH] node of rows base - LOW ..
-    uint8_t* const rest = reinterpret_cast<uint8_t*>(s_id + LOW + CH);
-    const size_t used = size_t(rest - smem);
-    // reached flag of every row (by rank, from 0)
-    uint8_t* const flag = used + size_t(N) <= size_t(sh.scratch_bytes) ? rest : g.flag;
-    for (int r = lane; r < N; r += 32) flag[r] = 0;
-    int top = g.rank[end_node];
-    for_aligned(g, end_node, [&](int y) {
-        top = max(top, g.rank[y]);
-        return true;
-    });
-    __syncwarp();
-    if (lane == 0) flag[g.rank[end_node]] = 1;
-    for (int base = top / CH * CH; base >= 0; base -= CH) {
-        __syncwarp();
-        for (int o = lane; o < CH + LOW; o += 32) {
-            const int r = base - LOW + o;
-            const int v = r >= 0 && r < N ? g.ord[r] : 0;
-            s_id[o] = v;
-            if (o >= LOW && r < N) {
-                s_desc[o - LOW] = g.rowdesc[r];
-                int st = r;
-                for_aligned(g, v, [&](int y) {
-                    st = min(st, g.rank[y]);
-                    return true;
-                });
-                // only a group's last row starts its check
-                bool last = true;
-                for_aligned(g, v, [&](int y) {
-                    last = last && g.rank[y] < r;
-                    return last;
-                });
-                s_start[o - LOW] = last ? st : r;
-            }
-        }
-        __syncwarp();
-        if (lane == 0) {
-            for (int r = min(top, base + CH - 1); r >= base; --r) {
-                const int st = s_start[r - base];
-                if (st < r) {
-                    bool any = false;
-                    for (int x = st; x <= r; ++x) {
-                        const int id = x >= base - LOW ? s_id[x - base + LOW] : g.ord[x];
-                        any |= flag[x] != 0 && id >= begin_node;
-                    }
-                    if (any)
-                        for (int x = st; x <= r; ++x) flag[x] = 1;
-                }
-                if (!flag[r] || s_id[r - base + LOW] < begin_node) continue;
-                const int4 d = s_desc[r - base];
-                const int np = desc_np(d.w);
-                for (int p = 0; p < np; ++p) flag[desc_pred(g.pred_idx, d, p) - 1] = 1;
-            }
-        }
-    }
-    __syncwarp();
-    // the rows, in order; the loads of four 32-row chunks go out together
-    int cnt = 0;
-    for (int c4 = 0; c4 < N; c4 += 128) {
-        int vv[4];
+    // per row (by rank, from 0): flags, rows down to its group's first and up to its last
+    const bool in_smem = 3 * size_t(N) <= size_t(sh.scratch_bytes);
+    uint8_t* const flag = in_smem ? smem : g.flag;
+    uint8_t* const down = in_smem ? smem + N : reinterpret_cast<uint8_t*>(g.shift);
+    uint8_t* const upto = in_smem ? smem + 2 * size_t(N) : down + N;
+    bool big = false;
+    for (int c0 = tid; c0 < N; c0 += 4 * NT) {
+        int v[4], ac[4];
+        int4 al[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) vv[u] = c4 + 32 * u + lane < N ? g.ord[c4 + 32 * u + lane] : -1;
+        for (int u = 0; u < 4; ++u) v[u] = c0 + u * NT < N ? g.ord[c0 + u * NT] : 0;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const int r = c4 + 32 * u + lane;
-            const bool in = vv[u] >= begin_node && flag[r] != 0;
-            const unsigned m = __ballot_sync(kFull, in && r < N);
-            const int k = cnt + __popc(m & ((1u << lane) - 1u));
-            if (vv[u] >= 0) g.sub_rank[vv[u]] = in ? k + 1 : 0;
-            if (in) g.dporder[k] = vv[u];
-            cnt += __popc(m);
+            ac[u] = g.al_cnt[v[u]];
+            al[u] = g.al4[v[u]];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int r = c0 + u * NT;
+            if (r >= N) continue;
+            int lo = r, hi = r;
+            const int ys[4] = {al[u].x, al[u].y, al[u].z, al[u].w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int ry = q < ac[u] ? g.rank[ys[q]] : r;
+                lo = min(lo, ry);
+                hi = max(hi, ry);
+            }
+            if (ac[u] > 4)
+                for_aligned(g, v[u], [&](int y) {
+                    lo = min(lo, g.rank[y]);
+                    hi = max(hi, g.rank[y]);
+                    return true;
+                });
+            big |= hi - lo >= 32;
+            flag[r] = uint8_t((v[u] == end_node ? kReached : 0) | (v[u] >= begin_node ? kInside : 0));
+            down[r] = uint8_t(min(r - lo, 255));
+            upto[r] = uint8_t(min(hi - r, 255));
         }
     }
-    if (lane == 0) sh.ndp = cnt;
-    __syncwarp();
+    if (tid == 0) sh.nlisted = 0;
+    team_sync<NW>(team);
+    if (__any_sync(kFull, big) && lane == 0) sh.nlisted = 1;  // a group of more than 32 rows
+    team_sync<NW>(team);
+    const bool chunks = sh.nlisted == 0;
+    if (w == 0) {
+        if (chunks) {
+            const int re = g.rank[end_node];
+            int hi = re + upto[re];
+            int4 next = hi - 31 + lane >= 0 ? g.rowdesc[hi - 31 + lane] : make_int4(0, 0, 0, 0);
+            while (hi >= 0) {
+                // rows [lo, hi]; lane l holds row base + l
+                const int base = hi - 31;
+                const int r = base + lane;
+                const int4 d = next;
+                const int first = max(base, 0);
+                const int dn = down[first];
+                const int lo = dn > 0 && first > 0 ? first + 1 + upto[first] : first;  // a group cut in two waits
+                const int hn = lo - 1;
+                const int rn = hn - 31 + lane;
+                next = hn >= 0 && rn >= 0 ? g.rowdesc[rn] : make_int4(0, 0, 0, 0);
+                const bool mine = r >= lo;
+                const int fl = mine ? flag[r] : 0;
+                const int np = mine ? desc_np(d.w) : 0;
+                unsigned links = 0;
+                if (mine) {
+                    const int gl = lane - int(down[r]), gh = lane + int(upto[r]);
+                    links = (0xffffffffu >> (31 - gh)) & (0xffffffffu << gl);
+                    for (int p = 0; p < np; ++p) {
+                        const int q = desc_pred(g.pred_idx, d, p) - 1 - base;
+                        if (q >= lo - base) links |= 1u << q;
+                    }
+                }
+                unsigned m = __ballot_sync(kFull, (fl & kReached) != 0);
+                if (m != 0) {
+                    const bool inside = (fl & kInside) != 0;
+                    for (;;) {
+                        const unsigned t =
+                            m | __reduce_or_sync(kFull, inside && ((m >> lane) & 1u) ? links : 0u);
+                        if (t == m) break;
+                        m = t;
+                    }
+                    if ((m >> lane) & 1u) {
+                        flag[r] = uint8_t(fl | kReached);
+                        if (inside)
+                            for (int p = 0; p < np; ++p) {
+                                const int q = desc_pred(g.pred_idx, d, p) - 1;
+                                if (q < lo) flag[q] = uint8_t(flag[q] | kReached);  // same value from every lane
+                            }
+                    }
+                    __syncwarp();
+                }
+                hi = hn;
+            }
+        } else if (lane == 0) {
+            // groups of more than 32 rows: follow the links
+            int sp = 0;
+            g.stack[sp++] = end_node;
+            flag[g.rank[end_node]] &= uint8_t(~kReached);
+            bool room = true;
+            while (sp > 0 && room) {
+                const int v = g.stack[--sp];
+                const int r = g.rank[v];
+                if ((flag[r] & kReached) || !(flag[r] & kInside)) continue;
+                flag[r] |= kReached;
+                for_in_edges(g, v, [&](int u, int) {
+                    room = sp < g.scap;
+                    if (room) g.stack[sp++] = u;
+                    return room;
+                });
+                for_aligned(g, v, [&](int y) {
+                    room = room && sp < g.scap;
+                    if (room) g.stack[sp++] = y;
+                    return room;
+                });
+            }
+            if (!room) {
+                sh.fail = kOverflow;
+                for (int r = 0; r < N; ++r) flag[r] = 0;
+            }
+        }
+        __syncwarp();
+        // the rows, in order; the loads of four 32-row chunks go out together
+        int cnt = 0;
+        for (int c4 = 0; c4 < N; c4 += 128) {
+            int vv[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) vv[u] = c4 + 32 * u + lane < N ? g.ord[c4 + 32 * u + lane] : -1;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int r = c4 + 32 * u + lane;
+                const bool in = vv[u] >= 0 && flag[r] == (kReached | kInside);
+                const unsigned m = __ballot_sync(kFull, in);
+                const int k = cnt + __popc(m & ((1u << lane) - 1u));
+                if (vv[u] >= 0) g.sub_rank[vv[u]] = in ? k + 1 : 0;
+                if (in) g.dporder[k] = vv[u];
+                cnt += __popc(m);
+            }
+        }
+        if (lane == 0) sh.ndp = cnt;
+    }
+    team_sync<NW>(team);
 }
 
 // ---------------- spoa's depth-first topological order ----------------
@@ -697,8 +773,12 @@ __device__ int topo_sort_warp(const Graph& g, PoaShared& sh, bool partial, int l
 // it); a group with a backbone node x (id below B) is reached from root x,
 // no earlier (every earlier root precedes x on the backbone, so the group is
 // none of its ancestors; B is the backbone's length); and x, the group's
-// first visited node, is listed first and then its aligned list in order. Only
-// a tied sink in a group without a backbone node needs the DFS itself.
+// first visited node, is listed first and then its aligned list in order. A
+// group without a backbone node is reached from the smallest id among its
+// members and their descendants. Only several tied sinks of one such group
+// whose root lies outside it need the DFS itself. (The DFS of 9 % of the
+// layers cost as much as 30 % of all DP at 50x.)
+constexpr int kSweepRows = 1024;
 template <bool FAST>
 __device__ int end_row(const Graph& g, PoaShared& sh, const int* order, int L, int lc, bool partial, int begin_node,
                        int B, int lane, uint8_t* smem) {
@@ -755,7 +835,96 @@ __device__ int end_row(const Graph& g, PoaShared& sh, const int* order, int L, i
             row = i;
         }
     }
-    if (!__any_sync(kFull, open)) {
+    bool sure = !__any_sync(kFull, open);
+    if (!sure && !partial) {
+        // a group without a backbone node is reached from the smallest id
+        // among its members and all that follow it: swept down to the lowest
+        // such group, from the last row (these sinks end the graph, so the
+        // sweep is short)
+        int lo = INT_MAX;
+        for (int k = lane; k < ns; k += 32) {
+            if (g.sink_h[k] != top) continue;
+            const int v = order[g.sink_rows[k] - 1];
+            int x = v, first = g.rank[v];
+            for_aligned(g, v, [&](int y) {
+                x = min(x, y);
+                first = min(first, g.rank[y]);
+                return true;
+            });
+            if (g.al_cnt[v] != 0 && x >= B) lo = min(lo, first);
+        }
+        lo = __reduce_min_sync(kFull, lo);
+        const int N = sh.nnodes;
+        if (N - lo <= kSweepRows && 4 * (N - lo) <= sh.scratch_bytes) {
+            int* const from = reinterpret_cast<int*>(smem);  // [N - lo] smallest id reached from the row
+            for (int r = lane; r < N - lo; r += 32) from[r] = g.ord[lo + r];
+            __syncwarp();
+            if (lane == 0)
+                for (int r = N - 1; r >= lo; --r) {
+                    const int v = g.ord[r];
+                    int first = r;
+                    bool last = true;
+                    for_aligned(g, v, [&](int y) {
+                        first = min(first, g.rank[y]);
+                        last = last && g.rank[y] < r;
+                        return last;
+                    });
+                    if (!last) continue;  // with its group's last row
+                    int id = INT_MAX;
+                    for (int x = max(first, lo); x <= r; ++x) id = min(id, from[x - lo]);
+                    for (int x = max(first, lo); x <= r; ++x) {
+                        from[x - lo] = id;
+                        for_in_edges(g, g.ord[x], [&](int u, int) {
+                            const int q = g.rank[u] - lo;
+                            if (q >= 0) from[q] = min(from[q], id);
+                            return true;
+                        });
+                    }
+                }
+            __syncwarp();
+            root = place = ~0u;
+            bool lost = false;  // tied sinks whose order within their root's search is not known
+            int mates = 0;
+            for (int pass = 0; pass < 2; ++pass) {
+                const unsigned r0 = __reduce_min_sync(kFull, root);
+                for (int k = lane; k < ns; k += 32) {
+                    if (g.sink_h[k] != top) continue;
+                    const int i = g.sink_rows[k];
+                    const int v = order[i - 1];
+                    int x = v;
+                    for_aligned(g, v, [&](int y) {
+                        x = min(x, y);
+                        return true;
+                    });
+                    const unsigned id = g.al_cnt[v] != 0 && x >= B ? unsigned(from[i - 1 - lo]) : unsigned(x);
+                    if (pass == 0) {
+                        root = min(root, id);
+                        continue;
+                    }
+                    if (id != r0) continue;
+                    ++mates;
+                    lost |= id != unsigned(x);  // the root is no member of the group
+                    unsigned pl = 0, at = 1;
+                    if (x != v)
+                        for_aligned(g, x, [&](int y) {
+                            if (y == v) pl = at;
+                            ++at;
+                            return y != v;
+                        });
+                    if (pl < place) {
+                        place = pl;
+                        row = i;
+                    }
+                }
+                if (pass == 1) {
+                    root = place != ~0u ? r0 : ~0u;
+                    sure = __reduce_add_sync(kFull, mates) == 1 || !__any_sync(kFull, lost);
+                }
+            }
+        }
+        __syncwarp();
+    }
+    if (sure) {
         const unsigned r0 = __reduce_min_sync(kFull, root);
         const unsigned p0 = __reduce_min_sync(kFull, root == r0 ? place : ~0u);
         return __reduce_min_sync(kFull, unsigned(root == r0 && place == p0 ? row : INT_MAX));
@@ -1725,8 +1894,9 @@ __device__ __noinline__ bool traceback_warp(const Graph& g, const int* order, co
     constexpr int kUnit = 16 / HB;               // columns per 16-byte chunk
     constexpr int kChunks = kTilePitch / 16;
     uint8_t* const tile = reinterpret_cast<uint8_t*>(g_poa_smem) + smem_off;
-    // per tile row: byte offsets of the predecessors' tile rows (-1: outside,
-    // or more than three) | base
+    // per tile row: byte offsets of the predecessors' tile rows (16-bit
+    // halves of x, y, z) | base, predecessors to test (3, 6, or 0: some lie
+    // outside the tile or in pred_idx) << 8
     int4* const w_desc = reinterpret_cast<int4*>(tile + kTileBytes);
     int4* const w_raw = w_desc + kTileRows;
     int* const w_node = reinterpret_cast<int*>(w_raw + kTileRows);
@@ -1756,18 +1926,25 @@ __device__ __noinline__ bool traceback_warp(const Graph& g, const int* order, co
                 t4[q] = *reinterpret_cast<const int4*>(Hb + (size_t(wlo + tr) * lc + clo) * HB + tc * 16);
         }
 #pragma unroll
-        for (int o = lane; o < kTileRows; o += 32) {
-            const int r = wlo + o;
+        for (int t = lane; t < kTileRows; t += 32) {
+            const int r = wlo + t;
             if (r >= 1 && r <= i) {
                 const int4 d = rowdesc[r - 1];
-                w_node[o] = order[r - 1];
-                w_raw[o] = d;
+                w_node[t] = order[r - 1];
+                w_raw[t] = d;
                 const int np = desc_np(d.w);
                 // absent predecessors repeat the first
-                const int p0 = desc_packed(d, 0), p1 = np > 1 ? desc_packed(d, 1) : p0, p2 = np > 2 ? desc_packed(d, 2) : p0;
-                const bool inside = np <= 3 && !desc_listed(d.w) && min(p0, min(p1, p2)) >= wlo;
-                w_desc[o] = make_int4(inside ? (p0 - wlo) * kTilePitch : -1, (p1 - wlo) * kTilePitch,
-                                      (p2 - wlo) * kTilePitch, int(desc_base(d.w)));
+                unsigned o[kPacked];
+                int low = r;
+#pragma unroll
+                for (int q = 0; q < kPacked; ++q) {
+                    const int pr = desc_packed(d, q < np ? q : 0);
+                    low = min(low, pr);
+                    o[q] = unsigned(pr - wlo) * kTilePitch;
+                }
+                const int n = desc_listed(d.w) || low < wlo ? 0 : np <= 3 ? 3 : 6;
+                w_desc[t] = make_int4(int(o[0] | (o[1] << 16)), int(o[2] | (o[3] << 16)), int(o[4] | (o[5] << 16)),
+                                      int(desc_base(d.w) | unsigned(n) << 8));
             }
         }
         for (int c = lane; c < kCols; c += 32) w_seq[c] = (clo + c >= 1 && clo + c <= L) ? seq[clo + c - 1] : 0;
@@ -1778,24 +1955,36 @@ __device__ __noinline__ bool traceback_warp(const Graph& g, const int* order, co
             do {
                 const int4 d = w_desc[oi / kTilePitch];
                 const int v = w_node[oi / kTilePitch];
-                const int s = uint32_t(w_seq[cj]) == uint32_t(d.w) ? dmt : dmm;
+                const int s = uint32_t(w_seq[cj]) == (uint32_t(d.w) & 0xFFu) ? dmt : dmm;
                 const bool col = cj > 0;
                 const uint8_t* const tj = tile + cj * HB;
                 const uint8_t* const tl = tile + (col ? cj - 1 : 0) * HB;
                 int no = oi, nh = score(tl + oi), node = -1;  // left
                 bool step = true;
-                if (d.x >= 0) {
-                    const int a0 = score(tl + d.x), a1 = score(tl + d.y), a2 = score(tl + d.z);
-                    const int b0 = score(tj + d.x), b1 = score(tj + d.y), b2 = score(tj + d.z);
+                // the first diagonal, else the first vertical, of K predecessors
+                auto choose = [&](const auto& o) {
+                    constexpr int K = int(sizeof(o) / sizeof(o[0]));
                     const int hd = col ? h - s : INT_MIN, hu = h - gap;
-                    const bool up = b0 == hu || b1 == hu || b2 == hu;
-                    const bool dg = a0 == hd || a1 == hd || a2 == hd;
-                    const int ou = b0 == hu ? d.x : b1 == hu ? d.y : d.z;
-                    const int od = a0 == hd ? d.x : a1 == hd ? d.y : d.z;
+                    int od = -1, ou = -1;
+#pragma unroll
+                    for (int q = K - 1; q >= 0; --q) {
+                        if (score(tl + o[q]) == hd) od = o[q];
+                        if (score(tj + o[q]) == hu) ou = o[q];
+                    }
+                    const bool dg = od >= 0, up = ou >= 0;
                     no = dg ? od : up ? ou : oi;
                     nh = dg ? hd : up ? hu : nh;
                     node = dg ? v : -1;
                     step = dg || !up;
+                };
+                const int x0 = d.x & 0xFFFF, x1 = int(unsigned(d.x) >> 16), x2 = d.y & 0xFFFF;
+                const unsigned n = (unsigned(d.w) >> 8) & 7u;
+                if (n == 3) {
+                    const int o[3] = {x0, x1, x2};
+                    choose(o);
+                } else if (n == 6) {
+                    const int o[6] = {x0, x1, x2, int(unsigned(d.y) >> 16), d.z & 0xFFFF, int(unsigned(d.z) >> 16)};
+                    choose(o);
                 } else {
                     // long list, or a predecessor above the tile: the first
                     // diagonal, else the first vertical
@@ -1913,10 +2102,12 @@ __device__ void poa_window(const PoaArgs& a, Graph& g, PoaShared& sh, uint32_t w
         int ndp = sh.nnodes;
         const int* order = g.ord;
         if (!full) {
-            if (w == 0) mark_subgraph(g, sh, begin, int(Lr.end), lane, smem);
-            team_sync<NW>(team);
-            if (sh.fail) break;
+            mark_subgraph<NW>(g, sh, begin, int(Lr.end), lane, w, team, smem);
             ndp = sh.ndp;
+            if (ndp == 0) {  // failed or overflowed
+                if (tid == 0 && sh.fail == 0) sh.fail = kFailed;
+                break;
+            }
             order = g.dporder;
             build_rows<NW>(g, sh, order, ndp, true, tid, team, smem);
         }
