@@ -115,8 +115,8 @@ struct Graph {
     int4* rowdesc;            // per DP row (build_rows)
     int* pred_idx;
     int *sink_rows, *sink_h;  // sink rows and their last-column scores
-    // per sequence position of the layer: node on its path (-1 for an
-    // inserted base), node id, order slot; order slots of the new nodes
+    // per sequence position of the layer: row, then node on its path (0, then
+    // -1 for an inserted base), node id, order slot; order slots of the new nodes
     int *path, *nid, *slot, *new_slot;
     long long* bscore;
     int *bpred, *cons;
@@ -961,8 +961,8 @@ __device__ int end_row(const Graph& g, PoaShared& sh, const int* order, int L, i
 // words), so that finding or adding an edge reads only its head. Leaves the
 // new nodes' order slots (see order_insert) in g.new_slot.
 template <int NW>
-__device__ void add_layer(const Graph& g, PoaShared& sh, const uint8_t* seq, const uint8_t* qual, int len, int lane,
-                          int w, int team, uint8_t* smem) {
+__device__ void add_layer(const Graph& g, PoaShared& sh, const int* order, const uint8_t* seq, const uint8_t* qual,
+                          int len, int lane, int w, int team, uint8_t* smem) {
     constexpr unsigned kFull = 0xffffffffu;
     constexpr int NT = 32 * NW;
     const int tid = 32 * w + lane;
@@ -970,14 +970,17 @@ __device__ void add_layer(const Graph& g, PoaShared& sh, const uint8_t* seq, con
     const bool in_smem = 8 * size_t(len) <= size_t(sh.scratch_bytes);
     int* const nid = in_smem ? reinterpret_cast<int*>(smem) : g.nid;  // node of position t, -1 until numbered
     int* const slot = in_smem ? nid + len : g.slot;                   // last rank of the position's group
-    const int* const path = g.path;
-    // 1. classify (reads only the graph as it was before this insertion)
+    int* const path = g.path;
+    // 1. classify (reads only the graph as it was before this insertion); the
+    //    path's rows become nodes
     for (int t4 = tid; t4 < len; t4 += 4 * NT) {
         int at[4], ac[4], rk[4];
         uint8_t cd[4], ch[4];
         int4 al[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) at[u] = t4 + u * NT < len ? path[t4 + u * NT] : -1;
+        for (int u = 0; u < 4; ++u) at[u] = t4 + u * NT < len ? path[t4 + u * NT] : 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) at[u] = at[u] > 0 ? order[at[u] - 1] : -1;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int v = max(at[u], 0);
@@ -1018,6 +1021,7 @@ __device__ void add_layer(const Graph& g, PoaShared& sh, const uint8_t* seq, con
                         });
                 }
             }
+            path[t] = at[u];
             nid[t] = n;
             slot[t] = sl;
         }
@@ -1877,30 +1881,36 @@ __device__ void dp_dispatch(const Graph& g, PoaShared& sh, int ndp, const uint8_
 // choosing among them without branches (votes and shuffles between lanes
 // would cost more than the whole step). A predecessor above the tile is read
 // from global memory; a step that leaves the tile ends the lane's run and
-// the warp stages the next one. Writes the node of every sequence position
-// (-1 for an inserted base) to g.path; a vertical step consumes no
-// position and adds nothing to the graph. Returns false on a broken walk.
+// the warp stages the next one, all its copies in flight at once. Writes the
+// row of every sequence position (0 for an inserted base) to g.path; a
+// vertical step consumes no position and adds nothing to the graph. Returns
+// false on a broken walk. (A step takes 290 cycles, a tile 2 k; with
+// one load after another a tile took 16 k.)
 constexpr int kTileRows = 96;
 constexpr int kTilePitch = 128;  // bytes per row: 64 int16 or 32 int32 columns
-constexpr int kTileBytes = kTileRows * kTilePitch;
-constexpr int kTileSmem = kTileBytes + kTileRows * 36 + 64;
+constexpr int kTileBytes = 16 + kTileRows * kTilePitch;  // the walk may look one column left of the first
+constexpr int kTileSmem = kTileBytes + kTileRows * 32 + 64;
 static_assert(kTileSmem <= 4 * WarpMem<4>::bytes && kTileSmem <= WarpMem<1>::bytes, "the tile fits every team's memory");
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(uint32_t(__cvta_generic_to_shared(dst))), "l"(src)
+                 : "memory");
+}
 template <bool FAST>
-__device__ __noinline__ bool traceback_warp(const Graph& g, const int* order, const uint8_t* seq, int L, int iend,
-                                            int hend, int mt, int mm, int gap, int lane, int smem_off, int lc) {
+__device__ __noinline__ bool traceback_warp(const Graph& g, const uint8_t* seq, int L, int iend, int hend, int mt,
+                                            int mm, int gap, int lane, int smem_off, int lc) {
     constexpr unsigned kFull = 0xffffffffu;
     constexpr int HB = FAST ? 2 : 4;              // bytes per score
     constexpr int kCols = kTilePitch / HB;       // tile columns
     constexpr int kUnit = 16 / HB;               // columns per 16-byte chunk
     constexpr int kChunks = kTilePitch / 16;
-    uint8_t* const tile = reinterpret_cast<uint8_t*>(g_poa_smem) + smem_off;
+    uint8_t* const smem = reinterpret_cast<uint8_t*>(g_poa_smem) + smem_off;
+    uint8_t* const tile = smem + 16;
     // per tile row: byte offsets of the predecessors' tile rows (16-bit
     // halves of x, y, z) | base, predecessors to test (3, 6, or 0: some lie
     // outside the tile or in pred_idx) << 8
-    int4* const w_desc = reinterpret_cast<int4*>(tile + kTileBytes);
+    int4* const w_desc = reinterpret_cast<int4*>(smem + kTileBytes);
     int4* const w_raw = w_desc + kTileRows;
-    int* const w_node = reinterpret_cast<int*>(w_raw + kTileRows);
-    uint8_t* const w_seq = reinterpret_cast<uint8_t*>(w_node + kTileRows);
+    uint8_t* const w_seq = reinterpret_cast<uint8_t*>(w_raw + kTileRows);
     const uint8_t* const Hb = reinterpret_cast<const uint8_t*>(g.H);
     const int4* const rowdesc = g.rowdesc;
     const int* const pred_idx = g.pred_idx;
@@ -1917,65 +1927,71 @@ __device__ __noinline__ bool traceback_warp(const Graph& g, const int* order, co
         const int wlo = max(0, i - (kTileRows - 1));
         const int clo = max(0, (j / kUnit + 1) * kUnit - kCols);
         const int rows = i - wlo + 1;
-        int4* const t4 = reinterpret_cast<int4*>(tile);
         __syncwarp();
-#pragma unroll 12
-        for (int q = lane; q < kTileRows * kChunks; q += 32) {
-            const int tr = q / kChunks, tc = q % kChunks;
-            if (tr < rows && clo + tc * kUnit < lc)
-                t4[q] = *reinterpret_cast<const int4*>(Hb + (size_t(wlo + tr) * lc + clo) * HB + tc * 16);
+        // rows past i and columns past the stride repeat others and are not read
+#pragma unroll
+        for (int u = 0; u < kTileRows * kChunks / 32; ++u) {
+            const int q = u * 32 + lane;
+            const int tr = min(q / kChunks, rows - 1), tc = min(clo + q % kChunks * kUnit, lc - kUnit);
+            copy16_async(tile + q * 16, Hb + (size_t(wlo + tr) * lc + tc) * HB);
         }
+        int4 dd[kTileRows / 32];
 #pragma unroll
-        for (int t = lane; t < kTileRows; t += 32) {
-            const int r = wlo + t;
-            if (r >= 1 && r <= i) {
-                const int4 d = rowdesc[r - 1];
-                w_node[t] = order[r - 1];
-                w_raw[t] = d;
-                const int np = desc_np(d.w);
-                // absent predecessors repeat the first
-                unsigned o[kPacked];
-                int low = r;
+        for (int u = 0; u < kTileRows / 32; ++u)
+            dd[u] = rowdesc[min(max(wlo + u * 32 + lane, 1), i) - 1];
 #pragma unroll
-                for (int q = 0; q < kPacked; ++q) {
-                    const int pr = desc_packed(d, q < np ? q : 0);
-                    low = min(low, pr);
-                    o[q] = unsigned(pr - wlo) * kTilePitch;
-                }
-                const int n = desc_listed(d.w) || low < wlo ? 0 : np <= 3 ? 3 : 6;
-                w_desc[t] = make_int4(int(o[0] | (o[1] << 16)), int(o[2] | (o[3] << 16)), int(o[4] | (o[5] << 16)),
-                                      int(desc_base(d.w) | unsigned(n) << 8));
+        for (int u = 0; u < kTileRows / 32; ++u) {
+            const int t = u * 32 + lane;
+            const int4 d = dd[u];
+            const int np = desc_np(d.w);
+            // absent predecessors repeat the first
+            unsigned o[kPacked];
+            int low = INT_MAX;
+#pragma unroll
+            for (int q = 0; q < kPacked; ++q) {
+                const int pr = desc_packed(d, q < np ? q : 0);
+                low = min(low, pr);
+                o[q] = unsigned(pr - wlo) * kTilePitch;
             }
+            const int n = desc_listed(d.w) || low < wlo ? 0 : np <= 3 ? 3 : 6;
+            w_raw[t] = d;
+            w_desc[t] = make_int4(int(o[0] | (o[1] << 16)), int(o[2] | (o[3] << 16)), int(o[4] | (o[5] << 16)),
+                                  int(desc_base(d.w) | unsigned(n) << 8));
         }
         for (int c = lane; c < kCols; c += 32) w_seq[c] = (clo + c >= 1 && clo + c <= L) ? seq[clo + c - 1] : 0;
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncwarp();
         if (lane == 0) {
             int oi = (i - wlo) * kTilePitch, cj = j - clo;  // the cell in the tile
             const int cmin = clo > 0 ? 1 : 0;               // the walk needs column cj - 1 unless it is before the first
+            const int omin = wlo == 0 ? kTilePitch : 0;     // rank 0 ends the walk
             do {
                 const int4 d = w_desc[oi / kTilePitch];
-                const int v = w_node[oi / kTilePitch];
-                const int s = uint32_t(w_seq[cj]) == (uint32_t(d.w) & 0xFFu) ? dmt : dmm;
-                const bool col = cj > 0;
                 const uint8_t* const tj = tile + cj * HB;
-                const uint8_t* const tl = tile + (col ? cj - 1 : 0) * HB;
-                int no = oi, nh = score(tl + oi), node = -1;  // left
-                bool step = true;
+                const int s = uint32_t(w_seq[cj]) == (uint32_t(d.w) & 0xFFu) ? dmt : dmm;
+                const int hd = cj > 0 ? h - s : INT_MIN, hu = h - gap;
+                int no = oi, nh = score(tj + oi - HB);  // left
+                int row = 0, step = 1;
                 // the first diagonal, else the first vertical, of K predecessors
                 auto choose = [&](const auto& o) {
                     constexpr int K = int(sizeof(o) / sizeof(o[0]));
-                    const int hd = col ? h - s : INT_MIN, hu = h - gap;
                     int od = -1, ou = -1;
 #pragma unroll
                     for (int q = K - 1; q >= 0; --q) {
-                        if (score(tl + o[q]) == hd) od = o[q];
+                        if (score(tj + o[q] - HB) == hd) od = o[q];
                         if (score(tj + o[q]) == hu) ou = o[q];
                     }
-                    const bool dg = od >= 0, up = ou >= 0;
-                    no = dg ? od : up ? ou : oi;
-                    nh = dg ? hd : up ? hu : nh;
-                    node = dg ? v : -1;
-                    step = dg || !up;
+                    if (ou >= 0) {
+                        no = ou;
+                        nh = hu;
+                        step = 0;
+                    }
+                    if (od >= 0) {
+                        no = od;
+                        nh = hd;
+                        step = 1;
+                        row = 1;
+                    }
                 };
                 const int x0 = d.x & 0xFFFF, x1 = int(unsigned(d.x) >> 16), x2 = d.y & 0xFFFF;
                 const unsigned n = (unsigned(d.w) >> 8) & 7u;
@@ -1995,29 +2011,27 @@ __device__ __noinline__ bool traceback_warp(const Graph& g, const int* order, co
                         const int r = desc_pred(pred_idx, e, p);
                         const uint8_t* const pr = r >= wlo ? tj + (r - wlo) * kTilePitch
                                                            : Hb + (size_t(r) * lc + clo + cj) * HB;  // generic address
-                        if (col && score(pr - HB) == h - s) dr = r;
-                        if (vr < 0 && score(pr) == h - gap) vr = r;
+                        if (cj > 0 && score(pr - HB) == hd) dr = r;
+                        if (vr < 0 && score(pr) == hu) vr = r;
                     }
-                    const int nr = dr >= 0 ? dr : vr;
-                    if (nr >= 0) {
-                        no = (nr - wlo) * kTilePitch;
-                        nh = dr >= 0 ? h - s : h - gap;
-                        node = dr >= 0 ? v : -1;
-                        step = dr >= 0;
+                    if (dr >= 0 || vr >= 0) {
+                        no = ((dr >= 0 ? dr : vr) - wlo) * kTilePitch;
+                        nh = dr >= 0 ? hd : hu;
+                        row = dr >= 0 ? 1 : 0;
+                        step = row;
                     }
                 }
                 if (step) {
-                    if (!col) {
+                    if (cj == 0) {
                         ok = false;
                         break;
                     }
                     --cj;
-                    path[clo + cj] = node;
+                    path[clo + cj] = row ? wlo + oi / kTilePitch : 0;
                 }
                 oi = no;
                 h = nh;
-            } while (oi >= (wlo == 0 ? kTilePitch : 0) && cj >= cmin);
-            // rank 0 (oi == 0 with wlo == 0) ends the walk
+            } while (oi >= omin && cj >= cmin);
             i = wlo + (oi >= 0 ? oi / kTilePitch : -((-oi) / kTilePitch));
             j = clo + cj;
         }
@@ -2027,7 +2041,7 @@ __device__ __noinline__ bool traceback_warp(const Graph& g, const int* order, co
         ok = __shfl_sync(kFull, ok ? 1 : 0, 0) != 0;
     }
     if (ok)
-        for (int k = lane; k < j; k += 32) path[k] = -1;
+        for (int k = lane; k < j; k += 32) path[k] = 0;
     __syncwarp();
     return ok;
 }
@@ -2123,16 +2137,16 @@ __device__ void poa_window(const PoaArgs& a, Graph& g, PoaShared& sh, uint32_t w
             const int iend = fast ? end_row<true>(g, sh, order, L, lc, !full, begin, B, lane, smem)
                                   : end_row<false>(g, sh, order, L, lc, !full, begin, B, lane, smem);
             if (!sh.fail) {
-                const bool ok = fast ? traceback_warp<true>(g, order, seq, L, iend, sh.end_value, a.match, a.mismatch,
-                                                            a.gap, lane, team * kTeamBytes, lc)
-                                     : traceback_warp<false>(g, order, seq, L, iend, sh.end_value, a.match, a.mismatch,
-                                                             a.gap, lane, team * kTeamBytes, lc);
+                const bool ok = fast ? traceback_warp<true>(g, seq, L, iend, sh.end_value, a.match, a.mismatch, a.gap,
+                                                            lane, team * kTeamBytes, lc)
+                                     : traceback_warp<false>(g, seq, L, iend, sh.end_value, a.match, a.mismatch, a.gap,
+                                                             lane, team * kTeamBytes, lc);
                 if (!ok && lane == 0) sh.fail = kFailed;
             }
         }
         team_sync<NW>(team);
         if (sh.fail) break;
-        add_layer<NW>(g, sh, seq, qual, L, lane, w, team, smem);
+        add_layer<NW>(g, sh, order, seq, qual, L, lane, w, team, smem);
         if (sh.fail) break;
         order_insert<NW>(g, sh, lane, w, team, smem);
     }
