@@ -94,7 +94,7 @@ struct PoaArgs {
 
 // Per-slot scratch view.
 constexpr int kInline = 8;  // in-edges kept with their node
-constexpr int kGraphArrays = 39;
+constexpr int kGraphArrays = 40;
 struct Graph {
     // nodes
     uint8_t *code, *flag;
@@ -114,6 +114,7 @@ struct Graph {
     int* stack;
     int4* rowdesc;            // per DP row (build_rows)
     int* pred_idx;
+    uint32_t* used;           // bit r - 1: a row other than r + 1 has row r as predecessor
     int *sink_rows, *sink_h;  // sink rows and their last-column scores
     // per sequence position of the layer: row, then node on its path (0, then
     // -1 for an inserted base), node id, order slot; order slots of the new nodes
@@ -138,7 +139,7 @@ __host__ __device__ size_t walk_layout(int ncap, int ecap, int acap, int lcap, F
         N,       N + 8,   N * 4,   N * 4,   N * 4,   N * 4,    N * 32,  N * 32,        N * 4,   N * 4,
         N * 16,  N * 4,   N * 4,   E * 4,   E * 4,   E * 4,    A * 4,   A * 4,         N * 4,   N * 4,
         N * 4,   (N + 2) * 4,      N * 4,   N * 4,   N * 4,    N * 4,   S * 4,         (N + 32) * 16,
-        (N * kInline + E + 2) * 4, N * 4,   N * 4,   (L + 2) * 4, (L + 2) * 4, (L + 2) * 4, N * 4, N * 8,
+        (N * kInline + E + 2) * 4, N / 8 + 8, N * 4, N * 4, (L + 2) * 4, (L + 2) * 4, (L + 2) * 4, N * 4, N * 8,
         N * 4,   N * 4,   (N + 1) * L * 4};
     for (int id = 0; id < kGraphArrays; ++id) {
         f(id, off);
@@ -160,7 +161,7 @@ __device__ Graph make_graph(const PoaArgs& a, uint32_t slot) {
     set(g.ov_head), set(g.ov_tail), set(g.al4), set(g.al_head), set(g.al_tail);
     set(g.e_src), set(g.e_w), set(g.e_next), set(g.a_node), set(g.a_next);
     set(g.ord), set(g.ord2), set(g.rank), set(g.shift), set(g.dporder), set(g.sub_rank), set(g.dfs), set(g.dfs_rank);
-    set(g.stack), set(g.rowdesc), set(g.pred_idx), set(g.sink_rows), set(g.sink_h);
+    set(g.stack), set(g.rowdesc), set(g.pred_idx), set(g.used), set(g.sink_rows), set(g.sink_h);
     set(g.path), set(g.nid), set(g.slot), set(g.new_slot), set(g.bscore), set(g.bpred), set(g.cons), set(g.H);
     g.ncap = a.ncap;
     g.ecap = a.ecap;
@@ -190,17 +191,20 @@ struct PoaShared {
 // the CTA's dynamic shared memory: WarpMem<NW>::bytes per warp, teams in order
 extern __shared__ int4 g_poa_smem[];
 
-// Shared memory of one warp of a team of NW: the ring of recent DP rows, the
+// Shared memory of one warp of a team of NW: the ring of DP rows, the
 // staged controls and score words of 32 rows, and the final scores at the
 // right edge of the strip to its left. Between layers the whole team's
-// memory is scratch for the graph steps. One-warp teams run 12 warps to an
-// SM, four-warp teams 24.
+// memory is scratch for the graph steps. An SM holds 12 one-warp teams or 24
+// warps of four-warp teams. (16 and 20 one-warp teams with fewer rows and
+// registers each raise the throughput of the DP alone, but finish a batch's
+// slowest windows later: 2001 windows at 50x 78.7 ms with 12, 83 with 16, 93
+// with 20.)
 constexpr int kEdgeRows = 64;
 template <int NW>
 struct WarpMem {
     static constexpr int ring_bytes = NW == 1 ? 17408 : 8064;
-    static constexpr int ctl = ring_bytes;          // uint32_t[32]
-    static constexpr int pool = ctl + 32 * 4;       // uint32_t[32]
+    static constexpr int ctl = ring_bytes;          // uint32_t[33]: a block's rows and 0
+    static constexpr int pool = ctl + 36 * 4;       // uint32_t[32]
     static constexpr int edge = pool + 32 * 4 + 16; // int[kEdgeRows]
     static constexpr int bytes = edge + kEdgeRows * 4;
 };
@@ -301,6 +305,7 @@ __device__ __forceinline__ int warp_excl(int v, int lane, int& total) {
 // from x on.
 constexpr int kPacked = 6;
 constexpr int kWide = 1 << 17;
+constexpr int kPrev = 1 << 18;  // a listed row's predecessors include the row before it
 __device__ __forceinline__ int desc_np(int w) { return w & 0x1FFFF; }
 __device__ __forceinline__ uint32_t desc_base(int w) { return uint32_t(w) >> 24; }
 __device__ __forceinline__ bool desc_listed(int w) { return desc_np(w) > kPacked || (w & kWide) != 0; }
@@ -334,6 +339,7 @@ __device__ void build_rows(const Graph& g, PoaShared& sh, const int* order, int 
     uint16_t* const rk16 = reinterpret_cast<uint16_t*>(smem);
     uint8_t* const succ = in_smem ? smem + rk_bytes : g.flag;
     const bool wide = ndp >= 65536;
+    for (int k = tid; k <= ndp / 32; k += NT) g.used[k] = 0u;
     if (in_smem)
         for (int c0 = tid; c0 < N; c0 += 4 * NT) {
             int r[4];
@@ -372,10 +378,17 @@ __device__ void build_rows(const Graph& g, PoaShared& sh, const int* order, int 
             const int i = c0 + u * NT;
             if (i >= ndp) continue;
             int np = 0;
+            bool prev = false;
             int4 d = make_int4(0, 0, 0, 0);
             auto add = [&](int src) {
                 const int r = rk(src);
                 if (r == 0) return;
+                // row i + 1's predecessor r
+                if (r == i) {
+                    prev = true;
+                } else {
+                    atomicOr(&g.used[(r - 1) >> 5], 1u << ((r - 1) & 31));
+                }
                 const int h = r << (16 * (np & 1));
                 if (np < 2) d.x |= h;
                 else if (np < 4) d.y |= h;
@@ -404,7 +417,7 @@ __device__ void build_rows(const Graph& g, PoaShared& sh, const int* order, int 
                     if (r != 0) g.pred_idx[k++] = r;
                     return true;
                 });
-                d = make_int4(off, 0, 0, wide ? kWide : 0);
+                d = make_int4(off, 0, 0, (wide ? kWide : 0) | (prev ? kPrev : 0));
             }
             d.w |= np | int(uint32_t(code[u]) << 24);
             g.rowdesc[i] = d;
@@ -1433,7 +1446,7 @@ __device__ int heaviest_bundle_warp(const Graph& g, PoaShared& sh, int lane, uin
 // largest S.
 __host__ __device__ inline int seg_cells(int nw, int wc) {
     if (nw == 4) return wc <= 256 ? 2 : wc <= 512 ? 4 : wc <= 768 ? 6 : 8;
-    return wc <= 256 ? 8 : wc <= 512 ? 16 : 24;
+    return wc <= 256 ? 8 : wc <= 512 ? 16 : wc <= 640 ? 20 : 24;
 }
 // Row stride of the score rows: whole passes.
 __host__ __device__ inline int row_cover(int nw, int wc) {
@@ -1496,15 +1509,16 @@ __device__ __forceinline__ uint32_t score_pool(uint32_t base, uint32_t mm4, uint
 // over all columns spends the fewest instructions, several side by side
 // finish a window sooner.
 //
-// The last R rows sit in a shared-memory ring, [unit][lane] and then the
+// Rows that other rows than the next one need (g.used) go to a shared-memory
+// ring of the last R such rows, [unit][lane] and then the
 // score left of each lane's segment (conflict-free, and no lane reads
-// another's words); older rows come from global memory. On this chip a vote
-// with a branch on it costs about 75 cycles, a shuffle 33, so the row is kept
-// nearly free of branches. What a row needs besides its scores is
+// another's words); what has left the ring comes from global memory. On this chip a vote
+// with a branch on it costs about 75 cycles, a warp reduction 60, a shuffle
+// 33, so the row is kept nearly free of them. (A row of 500 columns with one
+// predecessor takes 440 cycles on one warp, 400 side by side on four.) What a row needs besides its scores is
 // worked out 32 rows at a time, one row per lane: a score word, and a control
 // word with the ring slots of up to 6 predecessors besides the row just
-// computed, which is still in registers. The control goes through a warp
-// reduction, so that branches on it are uniform.
+// computed, which is still in registers.
 //
 // Per cell: the elementwise maximum M over the predecessor rows, then
 // T = max(M[j-1] + s - gap, M[j] + gap) (the substitution score comes from one
@@ -1577,28 +1591,38 @@ __device__ __noinline__ void dp_strip(const Graph& g, PoaShared& sh, int ndp_, c
 #pragma unroll
     for (int k = 0; k < S; ++k) hv[k] = 0;
     int left = j0 == 0 ? kNegInf : 0;
-    int wofs = RB;  // ring offset of the row being computed: (row % R) * RB, R >= 2
+    int wofs = 0;             // ring offset of the next row to be kept
+    unsigned kept = 0;        // rows kept before this block
+    unsigned prev_used = 0;   // the previous block's used rows
+    unsigned next_used = g.used[0];
     for (int i0 = 0; i0 < ndp; i0 += 32) {
+        const unsigned used = next_used;
         __syncwarp();
         {
-            // controls of rows i0 + 1 .. i0 + 32, one per lane
+            // controls of rows i0 + 1 .. i0 + 32, one per lane. The k-th row
+            // kept (from 0) is in slot k % R until R more have been kept;
+            // rows of this block and the previous one are looked up.
             const int r = i0 + 1 + lane;
-            const int np = desc_np(pre.w);
-            uint32_t ctl = np == 0 ? kCtlChain : 0, n = 0;
-            bool slow = desc_listed(pre.w) || (np == 0 && r > 1);
-#pragma unroll
-            for (int q = 0; q < kPacked; ++q) {
+            const int np = desc_np(pre.w), packed = desc_listed(pre.w) ? 0 : np;
+            uint32_t ctl = np == 0 || (packed != np && (pre.w & kPrev)) ? kCtlChain : 0, n = 0;
+            bool slow = packed != np || (np == 0 && r > 1);
+            const unsigned here = kept + __popc(used & ((1u << lane) - 1u));  // rows kept before r
+            const unsigned kept1 = kept - __popc(prev_used);
+#pragma unroll 1
+            for (int q = 0; q < packed; ++q) {
                 const int p = desc_packed(pre, q);
-                if (q >= np) continue;
                 if (p == r - 1) {
                     ctl |= kCtlChain;
                 } else {
-                    slow |= r - p > R;
-                    ctl |= uint32_t(p % R) << (4 + 4 * n);
+                    const unsigned bit = unsigned(p - 1) & 31u, below = (1u << bit) - 1u;
+                    const unsigned k = p > i0 ? kept + __popc(used & below) : kept1 + __popc(prev_used & below);
+                    slow |= p <= i0 - 32 || here - k > unsigned(R);
+                    ctl |= (k % R) << (4 + 4 * n);
                     ++n;
                 }
             }
-            cblk[lane] = slow ? kCtlSlow : ctl | n;
+            cblk[lane] = slow ? kCtlSlow | (r > 1 && np > 0 ? ctl & kCtlChain : 0u) : ctl | n;
+            if (lane == 0) cblk[32] = 0u;  // read (as a ring slot too) after the block's last row
             pblk[lane] = FAST ? score_pool(desc_base(pre.w), mm4, flip) : desc_base(pre.w);
             if (LEFT && w == 0 && r <= ndp) {
                 // the first strip of a later pass: the edge of the strip
@@ -1609,9 +1633,34 @@ __device__ __noinline__ void dp_strip(const Graph& g, PoaShared& sh, int ndp_, c
         __syncwarp();
         const int nx = i0 + 32 + lane;
         pre = nx < ndp ? rowdesc[nx] : make_int4(0, 0, 0, 0);
+        next_used = i0 + 32 < ndp ? g.used[(i0 >> 5) + 1] : 0u;
         const int cnt = min(32, ndp - i0);
         volatile int* const ein_b = ein + (i0 & (kEdgeRows - 1));
-        unsigned cnext = __reduce_or_sync(kFull, cblk[0]);
+        // ring row at byte offset o; returns its score left of the segment
+        auto ring_row = [&](int o, int (&dst)[S]) -> int {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                if constexpr (U == 4) {
+                    const int4 v = *reinterpret_cast<const int4*>(ring + o + q * 512);
+                    dst[4 * q] = v.x;
+                    dst[4 * q + 1] = v.y;
+                    dst[4 * q + 2] = v.z;
+                    dst[4 * q + 3] = v.w;
+                } else {
+                    const int2 v = *reinterpret_cast<const int2*>(ring + o + q * 256);
+                    dst[2 * q] = v.x;
+                    dst[2 * q + 1] = v.y;
+                }
+            }
+            return *reinterpret_cast<const int*>(ring_left + o);
+        };
+        unsigned cnext = cblk[0];
+        // four-warp teams load the row's first predecessor in the ring a row
+        // ahead (whatever that reads for a row without one is not used); wide
+        // segments would hold too many registers over the row for it
+        constexpr bool kAhead = NW > 1;
+        int t[S], tleft = 0;
+        if (kAhead) tleft = ring_row(((cnext >> 4) & 15u) * RB, t);
         uint32_t pnext = pblk[0];
         for (int b0 = 0; b0 < cnt; b0 += kGroupRows) {
         const int bend = min(b0 + kGroupRows, cnt);
@@ -1638,8 +1687,8 @@ __device__ __noinline__ void dp_strip(const Graph& g, PoaShared& sh, int ndp_, c
         for (int b = b0; b < bend; ++b) {
             unsigned ctl = cnext;
             const uint32_t pool = pnext;
-            // next row's (one past the block at its end: unused)
-            cnext = __reduce_or_sync(kFull, cblk[b + 1]);
+            // next row's
+            cnext = cblk[b + 1];
             pnext = pblk[b + 1];
             int bx = kNegInf;  // final score of this row left of the strip, at lane 0
             if (LEFT) {
@@ -1647,59 +1696,56 @@ __device__ __noinline__ void dp_strip(const Graph& g, PoaShared& sh, int ndp_, c
                 bx = lane == 0 ? e : kNegInf;
             }
             if ((ctl & 15u) != kCtlChain) {
-                // ring row at byte offset o; returns its score left of the segment
-                auto ring_row = [&](int o, int (&dst)[S]) -> int {
-#pragma unroll
-                    for (int q = 0; q < Q; ++q) {
-                        if constexpr (U == 4) {
-                            const int4 t = *reinterpret_cast<const int4*>(ring + o + q * 512);
-                            dst[4 * q] = t.x;
-                            dst[4 * q + 1] = t.y;
-                            dst[4 * q + 2] = t.z;
-                            dst[4 * q + 3] = t.w;
-                        } else {
-                            const int2 t = *reinterpret_cast<const int2*>(ring + o + q * 256);
-                            dst[2 * q] = t.x;
-                            dst[2 * q + 1] = t.y;
-                        }
-                    }
-                    return *reinterpret_cast<const int*>(ring_left + o);
-                };
-                int t[S];
                 auto merge = [&](int lft) {
 #pragma unroll
                     for (int k = 0; k < S; ++k) hv[k] = max(hv[k], t[k]);
                     left = max(left, lft);
                 };
-                if ((ctl & 7u) != kCtlSlow) {
+                if (!kAhead) tleft = ring_row(((ctl >> 4) & 15u) * RB, t);
+                if (__builtin_expect((ctl & 15u) == (kCtlChain | 1u), 1)) {
+                    merge(tleft);
+                } else
+                if (__builtin_expect((ctl & 7u) != kCtlSlow, 1)) {
                     if (!(ctl & kCtlChain)) {
-                        // the row just computed is no predecessor: start from the first
-                        left = ring_row(((ctl >> 4) & 15u) * RB, hv);
-                        ctl = ((ctl >> 4) & ~15u) | ((ctl & 7u) - 1u);
+                        // the row just computed is no predecessor
+#pragma unroll
+                        for (int k = 0; k < S; ++k) hv[k] = t[k];
+                        left = tleft;
+                    } else {
+                        merge(tleft);
                     }
 #pragma unroll 1
-                    for (unsigned n = ctl & 7u; n > 0; --n) {
+                    for (unsigned n = ctl & 7u; n > 1; --n) {
                         ctl >>= 4;
-                        merge(ring_row((ctl & 15u) * RB, t));
+                        merge(ring_row(((ctl >> 4) & 15u) * RB, t));
                     }
                 } else {
-                    // general row: any number of predecessors at any distance
+                    // general row: any number of predecessors at any distance,
+                    // from the ring or from global memory
                     const int i = i0 + 1 + b;
                     const int4 d = rowdesc[i - 1];
                     const int np = desc_np(d.w);
+                    const bool chain = (ctl & kCtlChain) != 0;  // in hv already
+                    const unsigned here = kept + __popc(used & ((1u << b) - 1u));
+                    const unsigned kept1 = kept - __popc(prev_used);
+                    if (!chain) {
 #pragma unroll
-                    for (int k = 0; k < S; ++k) hv[k] = INT_MIN;
-                    left = INT_MIN;
+                        for (int k = 0; k < S; ++k) hv[k] = INT_MIN;
+                        left = INT_MIN;
+                    }
 #pragma unroll 1
                     for (int p = 0; p < max(np, 1); ++p) {
                         const int r = desc_pred(pred_idx, d, p);
                         int lft;
-                        if (r == 0) {
+                        if (chain && r == i - 1) continue;
+                        const unsigned below = (1u << (unsigned(r - 1) & 31u)) - 1u;
+                        const unsigned k = r > i0 ? kept + __popc(used & below) : kept1 + __popc(prev_used & below);
+                        if (r > 0 && r > i0 - 32 && here - k <= unsigned(R)) {
+                            lft = ring_row((k % R) * RB, t);
+                        } else if (r == 0) {
                             lft = j0 == 0 ? kNegInf : 0;
 #pragma unroll
                             for (int k = 0; k < S; ++k) t[k] = 0;
-                        } else if (i - r <= R) {
-                            lft = ring_row((r % R) * RB, t);
                         } else {
                             const uint8_t* const src = Hb + (size_t(r) * lc + j0) * HB;
                             if constexpr (FAST) {
@@ -1756,6 +1802,7 @@ __device__ __noinline__ void dp_strip(const Graph& g, PoaShared& sh, int ndp_, c
                 if (K == 4) tot[c] = max(tot[c], hv[c * K + 3]);
                 if (c > 0) tot[c] = max(tot[c], tot[c - 1]);
             }
+            const int tnext = ((cnext >> 4) & 15u) * RB;
             // prefix maximum over the lanes by fours: three shuffles of one
             // value cost little more than one (a lane that a shuffle does not
             // reach gets its own value back)
@@ -1769,6 +1816,7 @@ __device__ __noinline__ void dp_strip(const Graph& g, PoaShared& sh, int ndp_, c
                 x = max(__vimax3_s32(x, t1, t2), t3);
                 x = max(x, __shfl_up_sync(kFull, x, 16));
             }
+            if (kAhead) tleft = ring_row(tnext, t);
             left = __shfl_up_sync(kFull, x, 1);  // final value left of the segment
             if (lane == 0) left = bx;
 #pragma unroll
@@ -1779,17 +1827,19 @@ __device__ __noinline__ void dp_strip(const Graph& g, PoaShared& sh, int ndp_, c
                 for (int c = 0; c < C; ++c) hv[c * K + k] = max(hv[c * K + k], hv[c * K + k - 1]);
             if (feed_lane)
                 reinterpret_cast<volatile int*>(mine + Mem::bytes + Mem::edge)[(i0 + b) & (kEdgeRows - 1)] = hv[S - 1];
+            if ((used >> b) & 1u) {
 #pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                if constexpr (U == 4) {
-                    *reinterpret_cast<int4*>(ring + wofs + q * 512) =
-                        make_int4(hv[4 * q], hv[4 * q + 1], hv[4 * q + 2], hv[4 * q + 3]);
-                } else {
-                    *reinterpret_cast<int2*>(ring + wofs + q * 256) = make_int2(hv[2 * q], hv[2 * q + 1]);
+                for (int q = 0; q < Q; ++q) {
+                    if constexpr (U == 4) {
+                        *reinterpret_cast<int4*>(ring + wofs + q * 512) =
+                            make_int4(hv[4 * q], hv[4 * q + 1], hv[4 * q + 2], hv[4 * q + 3]);
+                    } else {
+                        *reinterpret_cast<int2*>(ring + wofs + q * 256) = make_int2(hv[2 * q], hv[2 * q + 1]);
+                    }
                 }
+                *reinterpret_cast<int*>(ring_left + wofs) = left;
+                wofs = wofs == (R - 1) * RB ? 0 : wofs + RB;
             }
-            *reinterpret_cast<int*>(ring_left + wofs) = left;
-            wofs = wofs == (R - 1) * RB ? 0 : wofs + RB;
             // streamed: keep the graph arrays in L2
             if constexpr (FAST) {
                 uint32_t pk[S / 2];
@@ -1815,12 +1865,14 @@ __device__ __noinline__ void dp_strip(const Graph& g, PoaShared& sh, int ndp_, c
             }
             hrow += hstep;
         }
-        if (NW > 1) {
-            // lane 31 wrote the strip's edge; its stores come before the count
-            __threadfence_block();
-            if (lane == 31) sh.done[w] = tag0 + i0 + bend;
+            if (NW > 1) {
+                // lane 31 wrote the strip's edge; its stores come before the count
+                __threadfence_block();
+                if (lane == 31) sh.done[w] = tag0 + i0 + bend;
+            }
         }
-        }
+        kept += __popc(used);
+        prev_used = used;
     }
     __syncwarp();
 }
@@ -1867,6 +1919,7 @@ __device__ void dp_dispatch(const Graph& g, PoaShared& sh, int ndp, const uint8_
         switch (s) {
             case 8: return dp_layer<8, NW>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, fast);
             case 16: return dp_layer<16, NW>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, fast);
+            case 20: return dp_layer<20, NW>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, fast);
             default: return dp_layer<24, NW>(g, sh, ndp, seq, L, mt, mm, gap, lane, w, team, fast);
         }
     }
@@ -2213,7 +2266,7 @@ __device__ void poa_window(const PoaArgs& a, Graph& g, PoaShared& sh, uint32_t w
 }
 
 // Warps of a full CTA (teams of NW): three CTAs fill an SM's registers and
-// shared memory, with 12 one-warp teams or 24 warps of larger teams.
+// shared memory, with 12 one-warp teams or 24 warps of four-warp teams.
 __host__ __device__ constexpr int cta_warps(int nw) { return nw == 1 ? 4 : 8; }
 __host__ __device__ constexpr int warp_smem(int nw) { return nw == 1 ? WarpMem<1>::bytes : WarpMem<4>::bytes; }
 constexpr int kCtasPerSm = 3;
@@ -2272,8 +2325,9 @@ struct PoaSvcArgs {
 // stays free for the alignment and layer kernels of newly admitted jobs.
 constexpr int kSvcCtasPerSm = 3;
 constexpr int kSvcTeamWarps = 1;
-__global__ void __launch_bounds__(32 * cta_warps(kSvcTeamWarps), kSvcCtasPerSm) poa_service_kernel(PoaSvcArgs s) {
-    constexpr int NW = kSvcTeamWarps, T = cta_warps(NW) / NW;
+constexpr int kSvcWarps = cta_warps(kSvcTeamWarps);
+__global__ void __launch_bounds__(32 * kSvcWarps, kSvcCtasPerSm) poa_service_kernel(PoaSvcArgs s) {
+    constexpr int NW = kSvcTeamWarps, T = kSvcWarps / NW;
     __shared__ PoaShared sh_all[T];
     __shared__ Graph g_all[T];
     __shared__ PoaArgs a_all[T];
@@ -2589,9 +2643,9 @@ void PoaEngine::run_list(std::vector<uint32_t> todo, int ncap, bool plain) {
         const int ecap = 2 * ncap, acap = ncap;
         const size_t slot = walk_layout(ncap, ecap, acap, lcap, [](int, size_t) {});
         // Warps per window. Four warps side by side finish a window sooner
-        // (150 windows of 1000 bases at 20x: 55 ms against 85 ms), one warp
+        // (150 windows of 1000 bases at 20x: 27 ms against 64 ms), one warp
         // spends the fewest instructions (2001 windows of 500 bases at 50x:
-        // 139 ms against 211 ms). The line lies at four windows per SM,
+        // 79 ms against 109 ms). The line lies at four windows per SM,
         // where four-warp teams no longer all run at once.
         const int nw = plain ? kPlainWarps : todo.size() <= 4 * size_t(dev_.sm_count) ? 4 : 1;
         const size_t teams = size_t(cta_warps(nw)) / nw;  // per full CTA
@@ -2755,8 +2809,7 @@ struct PoaSvcState {
 namespace {
 cudaError_t launch_poa_service(cudaStream_t stream, void* user) {
     const PoaSvcState* S = static_cast<const PoaSvcState*>(user);
-    poa_service_kernel<<<S->grid, 32 * cta_warps(kSvcTeamWarps), cta_warps(kSvcTeamWarps) * warp_smem(kSvcTeamWarps),
-                         stream>>>(S->args);
+    poa_service_kernel<<<S->grid, 32 * kSvcWarps, kSvcWarps * warp_smem(kSvcTeamWarps), stream>>>(S->args);
     return cudaGetLastError();
 }
 }  // namespace
@@ -2772,7 +2825,7 @@ PoaService::PoaService(int device, int8_t m, int8_t x, int8_t g, uint32_t window
     // graphs over 4096 nodes) overflow and run again in the job's own engine
     const int ncap = 4096, ecap = 2 * ncap, acap = ncap;
     const int lcap = row_cover(kSvcTeamWarps, int(std::max<uint32_t>(window_length, 1)) * 3 + 1);
-    const size_t teams = cta_warps(kSvcTeamWarps) / kSvcTeamWarps;
+    const size_t teams = kSvcWarps / kSvcTeamWarps;
     const size_t slot = walk_layout(ncap, ecap, acap, lcap, [](int, size_t) {});
     const uint32_t cps = std::max<uint32_t>(1, std::min<uint32_t>(ctas_per_sm, kSvcCtasPerSm));
     size_t slots = size_t(sm_count) * cps * teams;
@@ -2795,7 +2848,7 @@ PoaService::PoaService(int device, int8_t m, int8_t x, int8_t g, uint32_t window
     A.jobs = static_cast<const PoaJobDev*>(S->ring.records());
     A.q = S->ring.queue();
     check_cuda(cudaFuncSetAttribute(poa_service_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    cta_warps(kSvcTeamWarps) * warp_smem(kSvcTeamWarps)),
+                                    kSvcWarps * warp_smem(kSvcTeamWarps)),
                "cudaFuncSetAttribute");
     prefer_max_shared(reinterpret_cast<const void*>(poa_service_kernel));
     st_ = S.release();
