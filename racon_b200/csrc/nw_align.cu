@@ -132,21 +132,25 @@ __device__ __forceinline__ int band_hi_block(const Band& B, int c) {
     return min(B.nb - 1, fdiv64(c + B.dhi));
 }
 
-__device__ __forceinline__ int myers_step(u64& pv, u64& mv, u64 eq, int hin, u64& ph_out) {
-    const u64 neg = hin < 0 ? 1ull : 0ull;
+// One column of one 64-row block (Myers 1999 / Hyyro): hin is the horizontal
+// delta above the block as bits (1: +1, 2: -1); returns the delta below it the
+// same way. ph_out: the rows' +1 bits.
+__device__ __forceinline__ unsigned myers_step(u64& pv, u64& mv, u64 eq, unsigned hin, u64& ph_out) {
+    const u64 neg = hin >> 1;
     const u64 xv = eq | mv;
     eq |= neg;
     const u64 xh = (((eq & pv) + pv) ^ pv) | eq;
     u64 ph = mv | ~(xh | pv);
     u64 mh = pv & xh;
     ph_out = ph;
-    const int hout = int(ph >> 63) - int(mh >> 63);
-    ph = (ph << 1) | (hin > 0 ? 1ull : 0ull);
+    const unsigned hout = unsigned(ph >> 63) | (unsigned(mh >> 63) << 1);
+    ph = (ph << 1) | (hin & 1u);
     mh = (mh << 1) | neg;
     pv = mh | ~(xv | ph);
     mv = ph & xv;
     return hout;
 }
+__device__ __forceinline__ int delta_of(unsigned h) { return int(h & 1u) - int(h >> 1); }
 
 // Value of row i (0..63) of a block whose last row holds `score`.
 __device__ __forceinline__ int block_value(u64 pv, u64 mv, int score, int i) {
@@ -160,8 +164,7 @@ __device__ __forceinline__ void set_status(unsigned int* counters, int code) {
 
 // Per-warp scratch layout.
 struct WarpScratch {
-    int8_t* carry_h[2];
-    int32_t* carry_s[2];
+    int8_t* carry_h[2];  // deltas below a strip, 2 bits a column
     u64* capl_pv;
     u64* capl_mv;
     int32_t* capl_sc;
@@ -188,8 +191,6 @@ __device__ WarpScratch warp_scratch(const NwDevArgs& a, uint32_t slot) {
     };
     w.carry_h[0] = reinterpret_cast<int8_t*>(take(n));
     w.carry_h[1] = reinterpret_cast<int8_t*>(take(n));
-    w.carry_s[0] = reinterpret_cast<int32_t*>(take(n * 4));
-    w.carry_s[1] = reinterpret_cast<int32_t*>(take(n * 4));
     w.capl_pv = reinterpret_cast<u64*>(take(nb * 8));
     w.capl_mv = reinterpret_cast<u64*>(take(nb * 8));
     w.capl_sc = reinterpret_cast<int32_t*>(take(nb * 4));
@@ -204,7 +205,7 @@ __device__ WarpScratch warp_scratch(const NwDevArgs& a, uint32_t slot) {
 
 size_t warp_scratch_bytes(size_t n, size_t nb) {
     auto r = [](size_t b) { return (b + 255) & ~size_t(255); };
-    return 2 * r(n) + 2 * r(n * 4) + 2 * (2 * r(nb * 8) + r(nb * 4)) + r(kLeafBytes) +
+    return 2 * r(n) + 2 * (2 * r(nb * 8) + r(nb * 4)) + r(kLeafBytes) +
            r(size_t(kMaxSymWide) * 32 * 8) + r(nb * kDiagSym * 8);
 }
 
@@ -231,12 +232,27 @@ struct SweepFail {
     int min = 0;
 };
 
-// The banded block sweep below (warp_sweep) as one diagonal wavefront over
-// all blocks instead of strips, for narrow bands. Block v runs on lane
-// v % 32 and meets column c at step c + v, so it gets the carry of block
-// v - 1 at the same column from the lane before at the previous step (lane
-// 31 to lane 0 by a rotating shuffle, no carry buffer), and a lane moves on
-// to block v + 32 when block v leaves the band. With both band edges within
+// The sweep's inner loop. Block v of the query meets target column c at step
+// c - origin + (v's place in the wavefront); the horizontal delta at the same
+// column comes from the lane before at the previous step. Between two events
+// (a block enters or leaves the band, 32 steps are over) every lane takes the
+// same straight steps, with the symbols and query masks of the following
+// columns already on their way: a lane outside its block's columns computes
+// values that nothing reads and passes on +1, the delta below cells outside
+// the band. (Testing each step for its lanes' blocks, with dependent loads of
+// symbol and mask, took 350 cycles a step; this takes 150.)
+struct SweepLane {
+    u64 pv, mv;
+    int v, ts, te;    // the lane's block, the steps at which it meets its first and last column
+    int c0;           // column at step 0
+    int score, low;   // score of the block's bottom row, its minimum so far
+    unsigned in;      // delta above the block at the lane's next column
+    bool act;
+};
+
+// Diagonal form, for narrow bands: one wavefront over all blocks, block v on
+// lane v % 32 at step c + v; a lane moves to block v + 32 when block v leaves
+// the band. With both band edges within
 // kDiagBand (< 1953) diagonals of the main one, block v + 32 starts at least
 // 32 steps after block v ends, and block v + 31 (the next block of the lane
 // before) starts only after the last step at which block v reads its carry,
@@ -247,37 +263,87 @@ struct SweepFail {
 // +1 where that block is outside the band, the block's first score from the
 // block above one column to the left), so every value, the give-up checks
 // and their rows are the strip sweep's. Query masks come from a per-block
-// table built once per sweep (at most kDiagSym symbols). A form with two
+// table built once per query (at most kDiagSym symbols). A form with two
 // blocks in flight per lane (two slots, bands up to 3900 diagonals) gave the
-// same cells but was slower than strips on the config-2 batch (18217
-// against 19101 pairs/s at 20000 pairs): the per-slot bookkeeping outweighs
-// the second chain.
+// same cells but was slower than strips on the config-2 batch: the per-slot
+// bookkeeping outweighs the second chain.
 __device__ __forceinline__ bool diag_sweep_ok(const SweepIO& io, const Band& B, const WarpScratch& ws) {
     return ws.block_peq != nullptr && io.nsym <= kDiagSym && B.dhi <= kDiagBand && B.dhi - B.dlo <= kDiagBand;
 }
 
+// Query masks of block v (rows past the query's end match anything) into
+// dst[sym * stride].
+__device__ __forceinline__ void build_block_masks(const SweepIO& io, int m, int v, u64* dst, int stride) {
+    const int r0 = 64 * v;
+    const int rows = min(64, m - r0);
+    const u64 pad = rows < 64 ? (~0ull << rows) : 0ull;
+    for (int sym = 0; sym < io.nsym; ++sym) dst[sym * stride] = pad;
+    for (int i = 0; i < rows; ++i) {
+        const int r = r0 + i;
+        const int code = io.rev ? io.q[m - 1 - r] : io.q[r];
+        dst[code * stride] |= (1ull << i);
+    }
+}
+
+// Steps [t, end] of the wavefront. STREAM: lane 0 takes its deltas from
+// `carry` (2 bits a column) instead of lane 31. Lane 31's deltas shift through `out`.
+template <int MODE, bool STREAM>
+__device__ __forceinline__ void sweep_steps(const SweepIO& io, const Band& B, SweepLane& L, int t, int end, int lane,
+                                            int src, u64& carry, u64& out) {
+    const int n1 = io.ncols - 1;
+    const uint8_t* const tb = io.rev ? io.t + (B.n - 1) : io.t;
+    const int dir = io.rev ? -1 : 1;
+    const u64* const mask = io.peq + lane;
+    auto sym = [&](int c) -> unsigned { return tb[dir * min(max(c, 0), n1)]; };
+    int c = t + L.c0;
+    u64 eq = mask[sym(c) * 32], eq1 = mask[sym(c + 1) * 32];
+    unsigned s2 = sym(c + 2);
+    const bool stream0 = STREAM && lane == 0;
+    if (stream0) L.in = unsigned(carry) & 3u;
+    const unsigned keep = L.act ? 3u : 0u, idle = L.act ? 0u : 1u;
+    const bool top = L.v == 0;
+    if (top) L.in = 1u;
+#pragma unroll 2
+    for (; t <= end; ++t, ++c) {
+        const u64 e = eq;
+        eq = eq1;
+        eq1 = mask[s2 * 32];
+        s2 = sym(c + 3);
+        u64 ph;
+        const unsigned hout = myers_step(L.pv, L.mv, e, L.in, ph) & keep;
+        L.score += delta_of(hout);
+        if (MODE == kLeaf && L.act) {
+            const int blo = band_lo_block(B, c);
+            io.leaf[size_t(c) * io.bw + (L.v - blo)] =
+                make_uint4(unsigned(L.pv), unsigned(L.pv >> 32), unsigned(ph), unsigned(ph >> 32));
+        }
+        if (MODE == kDistance) L.low = min(L.low, L.score);
+        const unsigned give = hout | idle;
+        unsigned in = __shfl_sync(kFull, give, src);
+        if (STREAM) {
+            out = (out >> 2) | (u64(give) << 62);
+            carry >>= 2;
+            if (stream0) in = unsigned(carry) & 3u;
+        }
+        L.in = top ? 1u : in;
+    }
+}
+
 template <int MODE>
 __device__ int warp_sweep_diag(const SweepIO& io, const Band& B, const WarpScratch& ws, int lane,
-                               SweepFail* fail) {
-    const int m = B.m, n = B.n, nb = B.nb, nsym = io.nsym;
+                               SweepFail* fail, bool masks_built) {
+    const int m = B.m, n = B.n, nb = B.nb;
     const int ncols = io.ncols;
     // masks of every block (lane v % 32 builds block v, and only it reads
     // them back), built in the lane's column of the shared table
-    for (int v0 = 0; v0 < nb; v0 += 32) {
-        const int v = v0 + lane;
-        if (v < nb) {
-            for (int sym = 0; sym < nsym; ++sym) io.peq[sym * 32 + lane] = 0ull;
-            const int r0 = 64 * v;
-            const int rows = min(64, m - r0);
-            for (int i = 0; i < rows; ++i) {
-                const int r = r0 + i;
-                const int code = io.rev ? io.q[m - 1 - r] : io.q[r];
-                io.peq[code * 32 + lane] |= (1ull << i);
+    if (!masks_built)
+        for (int v0 = 0; v0 < nb; v0 += 32) {
+            const int v = v0 + lane;
+            if (v < nb) {
+                build_block_masks(io, m, v, io.peq + lane, 32);
+                for (int sym = 0; sym < io.nsym; ++sym) ws.block_peq[v * kDiagSym + sym] = io.peq[sym * 32 + lane];
             }
-            const u64 pad = rows < 64 ? (~0ull << rows) : 0ull;  // rows past the query end match anything
-            for (int sym = 0; sym < nsym; ++sym) ws.block_peq[v * kDiagSym + sym] = io.peq[sym * 32 + lane] | pad;
         }
-    }
     // the last block that meets the swept columns, and the last step; a
     // distance sweep also runs to the last step of the bottom block of that
     // block's 32-block group, where the strip sweep checks the group's row
@@ -289,66 +355,61 @@ __device__ int warp_sweep_diag(const SweepIO& io, const Band& B, const WarpScrat
     int chk_v = 31;                  // next group-bottom block whose row is checked
     int chk_t = last_step(chk_v);    // ... at the end of this step
     int result = INT_MAX;
-    int v = lane;
-    int cb_lo = max(0, 64 * v - B.dhi), cb_hi = min(ncols - 1, 64 * v + 63 - B.dlo);
-    const u64* mask = ws.block_peq + v * kDiagSym;
-    u64 pv = 0, mv = 0;
-    int score = 0;
-    bool started = false;
-    int bottom_min = INT_MAX;  // kDistance, lane 31: minimum of its block's bottom row
-    int in_pack = 0;           // previous step of the lane before: (score << 3) | (processed << 2) | (hout + 1)
     const int src = (lane + 31) & 31;
-    for (int t = 0; t <= t_stop; ++t) {
-        int c = t - v;
-        if (c > cb_hi) {  // the lane's block left the band: its next block
-            v += 32;
-            c -= 32;
-            cb_lo = max(0, 64 * v - B.dhi);
-            cb_hi = min(ncols - 1, 64 * v + 63 - B.dlo);
-            mask = ws.block_peq + v * kDiagSym;
-            started = false;
-            bottom_min = INT_MAX;
+    SweepLane L;
+    auto set_block = [&](int v) {
+        L.v = v;
+        L.c0 = -v;
+        L.act = false;
+        const int lo = max(0, 64 * v - B.dhi), hi = min(ncols - 1, 64 * v + 63 - B.dlo);
+        const bool any = v < nb && lo <= hi;
+        L.ts = any ? lo + v : INT_MAX;
+        L.te = any ? hi + v : INT_MAX;
+    };
+    set_block(lane);
+    L.pv = L.mv = 0;
+    L.score = 0;
+    L.low = INT_MAX;
+    L.in = 1u;
+    bool was = false;  // the lane's block met a column at the previous step
+    u64 none = 0, none2 = 0;
+    int t = 0;
+    while (t <= t_stop) {
+        // blocks that start at this step
+        const int up_score = __shfl_sync(kFull, L.score, src);
+        const bool up_was = __shfl_sync(kFull, was ? 1 : 0, src) != 0;
+        if (L.ts == t) {
+            const int c = t + L.c0;
+            L.act = true;
+            L.pv = ~0ull;
+            L.mv = 0ull;
+            L.score = c == 0 ? 64 * (L.v + 1) : (up_was ? up_score - delta_of(L.in) : up_score) + 64;
+            L.low = INT_MAX;
+            for (int sym = 0; sym < io.nsym; ++sym)
+                io.peq[sym * 32 + lane] = ws.block_peq[L.v * kDiagSym + sym];
         }
-        const bool active = v < nb && c >= cb_lo && c <= cb_hi;
-        int hout = 0;
-        if (active) {
-            const int up_h = (in_pack & 3) - 1;
-            const bool up_proc = (in_pack >> 2) & 1;
-            const int up_score = in_pack >> 3;
-            const int hin = (v == 0 || !up_proc) ? 1 : up_h;
-            if (!started) {
-                started = true;
-                pv = ~0ull;
-                mv = 0ull;
-                score = c == 0 ? 64 * (v + 1) : (up_proc ? up_score - up_h : up_score) + 64;
-            }
-            const int tc = io.rev ? io.t[n - 1 - c] : io.t[c];
-            const u64 eq = mask[tc];
-            u64 ph;
-            hout = myers_step(pv, mv, eq, hin, ph);
-            score += hout;
-            if (MODE == kLeaf) {
-                const int blo = band_lo_block(B, c);
-                io.leaf[size_t(c) * io.bw + (v - blo)] =
-                    make_uint4(unsigned(pv), unsigned(pv >> 32), unsigned(ph), unsigned(ph >> 32));
-            }
+        // straight steps up to the next event
+        int end = L.act ? L.te : (L.ts == INT_MAX ? t_stop : L.ts - 1);
+        end = min(__reduce_min_sync(kFull, end), t_stop);
+        if (MODE == kDistance && chk_t >= t) end = min(end, chk_t);
+        sweep_steps<MODE, false>(io, B, L, t, end, lane, src, none, none2);
+        was = L.act;
+        const bool done = L.act && L.te == end;
+        if (done) {
+            const int c = end + L.c0;
             if (MODE == kCapture && c == ncols - 1) {
-                io.cap_pv[v] = pv;
-                io.cap_mv[v] = mv;
-                io.cap_sc[v] = score;
+                io.cap_pv[L.v] = L.pv;
+                io.cap_mv[L.v] = L.mv;
+                io.cap_sc[L.v] = L.score;
             }
-            if (MODE == kDistance && v == nb - 1 && c == n - 1) {
-                result = block_value(pv, mv, score, (m - 1) & 63);
-            }
-            if (MODE == kDistance && lane == 31) bottom_min = min(bottom_min, score);
+            if (MODE == kDistance && L.v == nb - 1 && c == n - 1)
+                result = block_value(L.pv, L.mv, L.score, (m - 1) & 63);
         }
-        const int pack = (score << 3) | ((active ? 1 : 0) << 2) | (hout + 1);
-        in_pack = __shfl_sync(kFull, pack, src);
-        if (MODE == kDistance && t == chk_t) {
+        if (MODE == kDistance && end == chk_t) {
             // the group whose bottom block is chk_v is done (the strip
             // sweep's check after that strip)
             if (chk_v < nb - 1) {
-                const int row_min = __shfl_sync(kFull, bottom_min, 31);
+                const int row_min = __shfl_sync(kFull, done && L.v == chk_v ? L.low : INT_MAX, 31);
                 const int R = 64 * chk_v + 63;
                 if (row_min > B.k && R + 1 > B.k) {
                     if (fail) {
@@ -362,10 +423,10 @@ __device__ int warp_sweep_diag(const SweepIO& io, const Band& B, const WarpScrat
             chk_v += 32;
             chk_t = last_step(chk_v);
         }
+        if (done) set_block(L.v + 32);
+        t = end + 1;
     }
-    if (MODE == kDistance) {
-        for (int o = 16; o > 0; o >>= 1) result = min(result, __shfl_xor_sync(kFull, result, o));
-    }
+    if (MODE == kDistance) result = __reduce_min_sync(kFull, result);
     return result;
 }
 
@@ -377,107 +438,118 @@ __device__ int warp_sweep_diag(const SweepIO& io, const Band& B, const WarpScrat
 // a computed in-band value is at most the cost of any path to it inside the
 // band, so no path of cost <= k crosses row R. (Out-of-band cells only lower
 // the minimum.) The distance of a pass that reaches the end is unchanged.
+// The deltas below a strip go to the next one as 2-bit words: the word of
+// columns 32 k - 31 .. 32 k, complete when lane 31 has met column 32 k, is
+// stored at carry[k].
 template <int MODE>
 __device__ int warp_sweep(const SweepIO& io, const Band& B, const WarpScratch& ws, int lane,
-                          unsigned int* counters, SweepFail* fail = nullptr) {
-    if (diag_sweep_ok(io, B, ws)) return warp_sweep_diag<MODE>(io, B, ws, lane, fail);
+                          unsigned int* counters, SweepFail* fail = nullptr, bool masks_built = false) {
+    if (diag_sweep_ok(io, B, ws)) return warp_sweep_diag<MODE>(io, B, ws, lane, fail, masks_built);
+    constexpr u64 kOnes = 0x5555555555555555ull;  // +1 in every column
     int result = INT_MAX;
     const int nstrips = (B.nb + 31) / 32;
     const int m = B.m, n = B.n;
+    const int ncols = io.ncols;
+    const int src = (lane + 31) & 31;
+    int edge_score = 0;  // the previous strip's bottom score in the column before this strip's first
     for (int s = 0; s < nstrips; ++s) {
         const int b = 32 * s + lane;
-        const bool lane_valid = b < B.nb;
-        const int cb_lo = max(0, 64 * b - B.dhi);
-        const int cb_hi = min(io.ncols - 1, 64 * b + 63 - B.dlo);
         const int s_lo = max(0, 64 * 32 * s - B.dhi);
         const int last_b = min(B.nb - 1, 32 * s + 31);
-        const int s_hi = min(io.ncols - 1, 64 * last_b + 63 - B.dlo);
+        const int s_hi = min(ncols - 1, 64 * last_b + 63 - B.dlo);
         if (s_lo > s_hi) break;  // the band leaves the swept columns above this strip
-        const int prev_hi = min(io.ncols - 1, 64 * 32 * s - 1 - B.dlo);
+        const int prev_hi = min(ncols - 1, 64 * 32 * s - 1 - B.dlo);
+        const u64* const carry_in = reinterpret_cast<const u64*>(ws.carry_h[(s + 1) & 1]);
+        u64* const carry_out = reinterpret_cast<u64*>(ws.carry_h[s & 1]);
+        const bool feeds = 32 * s + 31 < B.nb - 1;  // there is a next strip
+        const int next_lo = max(0, 64 * 32 * (s + 1) - B.dhi);
 
-        // query bit masks of this lane's block
-        for (int sym = 0; sym < io.nsym; ++sym) io.peq[sym * 32 + lane] = 0ull;
-        if (lane_valid) {
-            const int r0 = 64 * b;
-            const int rows = min(64, m - r0);
-            for (int i = 0; i < rows; ++i) {
-                const int r = r0 + i;
-                const int code = io.rev ? io.q[m - 1 - r] : io.q[r];
-                io.peq[code * 32 + lane] |= (1ull << i);
-            }
-            if (rows < 64) {
-                const u64 pad = ~0ull << rows;  // rows past the query end match anything
-                for (int sym = 0; sym < io.nsym; ++sym) io.peq[sym * 32 + lane] |= pad;
-            }
-        }
+        if (b < B.nb) build_block_masks(io, m, b, io.peq + lane, 32);
         __syncwarp();
 
-        u64 pv = 0, mv = 0;
-        int score = 0;
-        int bottom_min = INT_MAX;  // kDistance, lane 31: minimum of the strip's bottom row
-        bool started = false;
-        int in_pack = 0;  // previous step of lane-1: (score << 3) | (processed << 2) | (hout + 1)
-        const int steps = (s_hi - s_lo) + 32;
-        int8_t* carry_h_out = ws.carry_h[s & 1];
-        int32_t* carry_s_out = ws.carry_s[s & 1];
-        const int8_t* carry_h_in = ws.carry_h[(s + 1) & 1];
-        const int32_t* carry_s_in = ws.carry_s[(s + 1) & 1];
-        for (int st = 0; st < steps; ++st) {
-            const int c = s_lo + st - lane;
-            const bool active = lane_valid && c >= cb_lo && c <= cb_hi;
-            int hout = 0;
-            if (active) {
-                const int up_h = (in_pack & 3) - 1;
-                const bool up_proc = (in_pack >> 2) & 1;
-                const int up_score = in_pack >> 3;
-                int hin;
-                if (lane == 0) {
-                    hin = (s == 0 || c > prev_hi) ? 1 : int(carry_h_in[c]);
+        SweepLane L;
+        L.v = b;
+        L.c0 = s_lo - lane;
+        L.act = false;
+        L.pv = L.mv = 0;
+        L.score = 0;
+        L.low = INT_MAX;
+        L.in = 1u;
+        {
+            const int lo = max(0, 64 * b - B.dhi), hi = min(ncols - 1, 64 * b + 63 - B.dlo);
+            const bool any = b < B.nb && lo <= hi;
+            L.ts = any ? lo - s_lo + lane : INT_MAX;
+            L.te = any ? hi - s_lo + lane : INT_MAX;
+        }
+        const bool meets = L.ts != INT_MAX;
+        const int t_stop = __reduce_max_sync(kFull, L.te == INT_MAX ? -1 : L.te);
+        // lane 31's step at column next_lo - 1, whose score the next strip starts from
+        const int t_edge = feeds && next_lo > 0 ? next_lo - 1 - s_lo + 31 : -1;
+        const int prev_k = (prev_hi + 31) >> 5;  // last word of the strip above
+        bool was = false;
+        u64 carry = kOnes, out = 0;
+        int next_edge = 0;
+        int t = 0;
+        while (t <= t_stop) {
+            const int cz = t + s_lo;  // lane 0's column
+            // lane 0's deltas for columns cz .. up to 32 k - 1 + 32
+            if (s > 0) {
+                // columns cz.. : the rest of word k, then word k + 1
+                const int k = (cz + 31) >> 5, o = (cz + 31) & 31;
+                const u64 w0 = k <= prev_k ? __ldcg(carry_in + k) : kOnes;
+                const u64 w1 = k + 1 <= prev_k ? __ldcg(carry_in + k + 1) : kOnes;
+                carry = o == 0 ? w0 : (w0 >> (2 * o)) | (w1 << (64 - 2 * o));
+            }
+            const int up_score = __shfl_sync(kFull, L.score, src);
+            const bool up_was = __shfl_sync(kFull, was ? 1 : 0, src) != 0;
+            if (L.ts == t) {
+                const int c = t + L.c0;
+                L.act = true;
+                L.pv = ~0ull;
+                L.mv = 0ull;
+                if (c == 0) {
+                    L.score = 64 * (b + 1);
                 } else {
-                    hin = up_proc ? up_h : 1;
+                    L.score = (lane == 0 ? edge_score : up_was ? up_score - delta_of(L.in) : up_score) + 64;
                 }
-                if (!started) {
-                    started = true;
-                    pv = ~0ull;
-                    mv = 0ull;
-                    if (c == 0) {
-                        score = 64 * (b + 1);
-                    } else {
-                        const int v = (lane == 0) ? carry_s_in[c - 1]
-                                                  : (up_proc ? up_score - up_h : up_score);
-                        score = v + 64;
-                    }
+                L.low = INT_MAX;
+            }
+            int end = L.act ? L.te : (L.ts == INT_MAX ? t_stop : L.ts - 1);
+            if (end < t) end = t_stop;  // the block is done
+            end = min(__reduce_min_sync(kFull, end), t_stop);
+            end = min(end, t + 31 - (cz & 31));  // lane 0's column 32 j - 1: lane 31 has met 32 (j - 1)
+            if (t_edge >= t) end = min(end, t_edge);
+            sweep_steps<MODE, true>(io, B, L, t, end, lane, src, carry, out);
+            was = L.act;
+            if (end == t_edge) next_edge = __shfl_sync(kFull, L.score, 31);
+            const bool done = L.act && L.te == end;
+            if (done) {
+                const int c = end + L.c0;
+                if (MODE == kCapture && c == ncols - 1) {
+                    io.cap_pv[b] = L.pv;
+                    io.cap_mv[b] = L.mv;
+                    io.cap_sc[b] = L.score;
                 }
-                const int tc = io.rev ? io.t[n - 1 - c] : io.t[c];
-                const u64 eq = io.peq[tc * 32 + lane];
-                u64 ph;
-                hout = myers_step(pv, mv, eq, hin, ph);
-                score += hout;
-                if (MODE == kLeaf) {
-                    const int blo = band_lo_block(B, c);
-                    io.leaf[size_t(c) * io.bw + (b - blo)] =
-                        make_uint4(unsigned(pv), unsigned(pv >> 32), unsigned(ph), unsigned(ph >> 32));
-                }
-                if (MODE == kCapture && c == io.ncols - 1) {
-                    io.cap_pv[b] = pv;
-                    io.cap_mv[b] = mv;
-                    io.cap_sc[b] = score;
-                }
-                if (MODE == kDistance && b == B.nb - 1 && c == n - 1) {
-                    result = block_value(pv, mv, score, (m - 1) & 63);
-                }
-                if (MODE == kDistance && lane == 31) bottom_min = min(bottom_min, score);
-                if (lane == 31) {
-                    carry_h_out[c] = int8_t(hout);
-                    carry_s_out[c] = score;
+                if (MODE == kDistance && b == B.nb - 1 && c == n - 1)
+                    result = block_value(L.pv, L.mv, L.score, (m - 1) & 63);
+                L.act = false;
+            }
+            if (feeds && lane == 31 && was) {
+                const int c = end + L.c0;
+                const int k = (c + 31) >> 5, p = ((c + 31) & 31) + 1;  // p columns of word k are met
+                if (p == 32) {
+                    __stcg(carry_out + k, out);
+                } else if (done) {
+                    __stcg(carry_out + k, (out >> (64 - 2 * p)) | (kOnes << (2 * p)));
                 }
             }
-            const int pack = (score << 3) | ((active ? 1 : 0) << 2) | (hout + 1);
-            in_pack = __shfl_up_sync(kFull, pack, 1);
+            if (done) L.ts = INT_MAX;
+            t = end + 1;
         }
+        edge_score = next_edge;
         __syncwarp();
-        if (MODE == kDistance && 32 * s + 31 < B.nb - 1) {
-            const int row_min = __shfl_sync(kFull, bottom_min, 31);
+        if (MODE == kDistance && feeds) {
+            const int row_min = __shfl_sync(kFull, meets ? L.low : INT_MAX, 31);
             const int R = 64 * (32 * s + 31) + 63;
             if (row_min > B.k && R + 1 > B.k) {
                 if (fail) {
@@ -489,9 +561,7 @@ __device__ int warp_sweep(const SweepIO& io, const Band& B, const WarpScratch& w
             }
         }
     }
-    if (MODE == kDistance) {
-        for (int o = 16; o > 0; o >>= 1) result = min(result, __shfl_xor_sync(kFull, result, o));
-    }
+    if (MODE == kDistance) result = __reduce_min_sync(kFull, result);
     (void)counters;
     return result;
 }
@@ -752,11 +822,13 @@ __device__ void distance_pair(const NwDevArgs& a, uint32_t pi, const WarpScratch
     io.bw = 0;
     int k = max(64, abs(m - n));
     int d = INT_MAX;
+    bool built = false;  // the diagonal sweep's masks depend on the query alone
     while (true) {
         const Band B = make_band(m, n, k);
         SweepFail f;
-        d = warp_sweep<kDistance>(io, B, ws, lane, a.counters, &f);
+        d = warp_sweep<kDistance>(io, B, ws, lane, a.counters, &f, built);
         if (d <= k) break;
+        built = diag_sweep_ok(io, B, ws);
         k = next_k(k, f, m, n);
     }
     if (lane == 0) {
@@ -1219,10 +1291,6 @@ __global__ void __launch_bounds__(32) nw_distance_noalloc_kernel(const char* q, 
     uint8_t* p = scratch + 2 * size_t(kNoAllocMaxLen);
     ws.carry_h[0] = reinterpret_cast<int8_t*>(p);
     ws.carry_h[1] = reinterpret_cast<int8_t*>(p + kNoAllocCarry);
-    p += 2 * kNoAllocCarry;
-    p = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 255) & ~uintptr_t(255));
-    ws.carry_s[0] = reinterpret_cast<int32_t*>(p);
-    ws.carry_s[1] = reinterpret_cast<int32_t*>(p + 4 * kNoAllocCarry);
     ws.capl_pv = ws.capl_mv = ws.capr_pv = ws.capr_mv = nullptr;
     ws.capl_sc = ws.capr_sc = nullptr;
     ws.leaf = nullptr;
