@@ -64,6 +64,8 @@ constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWarpsPerBlock = 4;
 constexpr int kMaxSym = 32;        // symbols whose bit masks fit the shared-memory table
 constexpr int kMaxSymWide = 256;   // any byte alphabet: the masks then live in the warp's scratch
+// queries from which a batch may be aligned by CTAs of four and of eight warps
+constexpr uint32_t kTeamRows = 6144, kWideTeamRows = 65536;
 constexpr long long kLeafBytes = 1024 * 1024;  // edlib's traceback threshold
 // The diagonal sweep (warp_sweep_diag) handles alphabets of up to kDiagSym
 // symbols and bands whose diagonals stay within kDiagBand of the main one.
@@ -76,6 +78,7 @@ enum NwStatus : int {
     kNwTraceOutOfBand = 2,
     kNwTaskOverflow = 3,
     kNwBadSymbol = 4,
+    kNwWaitLost = 6,
 };
 
 struct NwTask {
@@ -441,26 +444,54 @@ __device__ int warp_sweep_diag(const SweepIO& io, const Band& B, const WarpScrat
 // The deltas below a strip go to the next one as 2-bit words: the word of
 // columns 32 k - 31 .. 32 k, complete when lane 31 has met column 32 k, is
 // stored at carry[k].
-template <int MODE>
-__device__ int warp_sweep(const SweepIO& io, const Band& B, const WarpScratch& ws, int lane,
-                          unsigned int* counters, SweepFail* fail = nullptr, bool masks_built = false) {
-    if (diag_sweep_ok(io, B, ws)) return warp_sweep_diag<MODE>(io, B, ws, lane, fail, masks_built);
+//
+// W > 1: the strips go round the W warps of a CTA, each strip following the
+// one above as soon as its deltas arrive, so that a wide band's strips (each
+// 2048 + k steps, starting 2048 steps apart) overlap; a pass then takes about
+// m + k steps instead of (m / 2048) * (2048 + k). A strip publishes how many
+// words it has stored; one buffer more than warps keeps a strip's words until
+// the next strip, on the next warp, has read them all.
+constexpr int kMaxTeam = 8;
+constexpr int kWaitPolls = 1 << 24;  // polls of a wait on another warp before the pass is given up
+struct TeamSweep {
+    volatile u64 met[kMaxTeam + 1];   // per buffer: strip << 32 | words stored
+    volatile int edge[kMaxTeam + 1];  // per buffer: the strip's score in the column before the next strip's first
+    volatile int stop;                // the pass is over (gave up, or a wait was lost)
+    int result, fail_row, fail_min;
+    unsigned item;
+};
+
+// Buffer b of the CTA's carry buffers (two per warp slot).
+__device__ __forceinline__ u64* carry_buffer(const NwDevArgs& a, uint32_t first_slot, int b) {
+    uint8_t* p = a.scratch + size_t(first_slot + b / 2) * a.scratch_stride;
+    return reinterpret_cast<u64*>(p + size_t(b & 1) * ((size_t(a.max_n) + 255) & ~size_t(255)));
+}
+
+template <int MODE, int W>
+__device__ int strip_sweep(const SweepIO& io, const Band& B, u64* const (&buf)[W == 1 ? 2 : W + 1], int lane, int w,
+                           TeamSweep* T, SweepFail* fail) {
     constexpr u64 kOnes = 0x5555555555555555ull;  // +1 in every column
+    constexpr int NB = W == 1 ? 2 : W + 1;
     int result = INT_MAX;
     const int nstrips = (B.nb + 31) / 32;
     const int m = B.m, n = B.n;
     const int ncols = io.ncols;
     const int src = (lane + 31) & 31;
     int edge_score = 0;  // the previous strip's bottom score in the column before this strip's first
-    for (int s = 0; s < nstrips; ++s) {
+    for (int s = w; s < nstrips; s += W) {
         const int b = 32 * s + lane;
         const int s_lo = max(0, 64 * 32 * s - B.dhi);
         const int last_b = min(B.nb - 1, 32 * s + 31);
         const int s_hi = min(ncols - 1, 64 * last_b + 63 - B.dlo);
         if (s_lo > s_hi) break;  // the band leaves the swept columns above this strip
         const int prev_hi = min(ncols - 1, 64 * 32 * s - 1 - B.dlo);
-        const u64* const carry_in = reinterpret_cast<const u64*>(ws.carry_h[(s + 1) & 1]);
-        u64* const carry_out = reinterpret_cast<u64*>(ws.carry_h[s & 1]);
+        const int bi = (s + NB - 1) % NB, bo = s % NB;
+        u64 *carry_in = buf[0], *carry_out = buf[0];
+#pragma unroll
+        for (int q = 1; q < NB; ++q) {
+            if (bi == q) carry_in = buf[q];
+            if (bo == q) carry_out = buf[q];
+        }
         const bool feeds = 32 * s + 31 < B.nb - 1;  // there is a next strip
         const int next_lo = max(0, 64 * 32 * (s + 1) - B.dhi);
 
@@ -492,10 +523,18 @@ __device__ int warp_sweep(const SweepIO& io, const Band& B, const WarpScratch& w
         int t = 0;
         while (t <= t_stop) {
             const int cz = t + s_lo;  // lane 0's column
-            // lane 0's deltas for columns cz .. up to 32 k - 1 + 32
+            // lane 0's deltas from column cz on: the rest of word k, then word k + 1
             if (s > 0) {
-                // columns cz.. : the rest of word k, then word k + 1
                 const int k = (cz + 31) >> 5, o = (cz + 31) & 31;
+                if (W > 1) {
+                    const u64 want = (u64(unsigned(s - 1)) << 32) | unsigned(min(k + 1, prev_k) + 1);
+                    bool lost = false;
+                    for (int polls = 0; T->met[bi] < want && T->stop == 0 && !lost; ++polls) lost = polls > kWaitPolls;
+                    if (lost) T->stop = 2;
+                    if (__any_sync(kFull, T->stop != 0)) return INT_MAX;
+                    __threadfence_block();
+                    edge_score = T->edge[bi];
+                }
                 const u64 w0 = k <= prev_k ? __ldcg(carry_in + k) : kOnes;
                 const u64 w1 = k + 1 <= prev_k ? __ldcg(carry_in + k + 1) : kOnes;
                 carry = o == 0 ? w0 : (w0 >> (2 * o)) | (w1 << (64 - 2 * o));
@@ -515,13 +554,15 @@ __device__ int warp_sweep(const SweepIO& io, const Band& B, const WarpScratch& w
                 L.low = INT_MAX;
             }
             int end = L.act ? L.te : (L.ts == INT_MAX ? t_stop : L.ts - 1);
-            if (end < t) end = t_stop;  // the block is done
             end = min(__reduce_min_sync(kFull, end), t_stop);
             end = min(end, t + 31 - (cz & 31));  // lane 0's column 32 j - 1: lane 31 has met 32 (j - 1)
             if (t_edge >= t) end = min(end, t_edge);
             sweep_steps<MODE, true>(io, B, L, t, end, lane, src, carry, out);
             was = L.act;
-            if (end == t_edge) next_edge = __shfl_sync(kFull, L.score, 31);
+            if (end == t_edge) {
+                next_edge = __shfl_sync(kFull, L.score, 31);
+                if (W > 1 && lane == 31) T->edge[bo] = next_edge;
+            }
             const bool done = L.act && L.te == end;
             if (done) {
                 const int c = end + L.c0;
@@ -542,6 +583,10 @@ __device__ int warp_sweep(const SweepIO& io, const Band& B, const WarpScratch& w
                 } else if (done) {
                     __stcg(carry_out + k, (out >> (64 - 2 * p)) | (kOnes << (2 * p)));
                 }
+                if (W > 1 && (p == 32 || done)) {
+                    __threadfence_block();
+                    T->met[bo] = (u64(unsigned(s)) << 32) | unsigned(k + 1);
+                }
             }
             if (done) L.ts = INT_MAX;
             t = end + 1;
@@ -552,18 +597,73 @@ __device__ int warp_sweep(const SweepIO& io, const Band& B, const WarpScratch& w
             const int row_min = __shfl_sync(kFull, meets ? L.low : INT_MAX, 31);
             const int R = 64 * (32 * s + 31) + 63;
             if (row_min > B.k && R + 1 > B.k) {
-                if (fail) {
+                if (W > 1) {
+                    // strips end in order, so this is the first that fails
+                    if (lane == 0) {
+                        T->fail_row = R;
+                        T->fail_min = row_min;
+                        __threadfence_block();
+                        T->stop = 1;
+                    }
+                } else if (fail) {
                     fail->row = R;
                     fail->min = row_min;
                 }
-                result = INT_MAX;
-                break;
+                return INT_MAX;
             }
         }
     }
     if (MODE == kDistance) result = __reduce_min_sync(kFull, result);
-    (void)counters;
     return result;
+}
+
+// One warp's sweep in the form the band asks for.
+template <int MODE>
+__device__ int warp_sweep(const SweepIO& io, const Band& B, const WarpScratch& ws, int lane,
+                          unsigned int* counters, SweepFail* fail = nullptr, bool masks_built = false) {
+    (void)counters;
+    if (diag_sweep_ok(io, B, ws)) return warp_sweep_diag<MODE>(io, B, ws, lane, fail, masks_built);
+    u64* const buf[2] = {reinterpret_cast<u64*>(ws.carry_h[0]), reinterpret_cast<u64*>(ws.carry_h[1])};
+    return strip_sweep<MODE, 1>(io, B, buf, lane, 0, nullptr, fail);
+}
+
+// The same by the W warps of a CTA: the diagonal form on the first warp, the
+// strips on all. Every thread calls it and gets the result.
+template <int MODE, int W>
+__device__ int team_sweep(const NwDevArgs& a, const SweepIO& io, const Band& B, const WarpScratch& ws, int lane,
+                          int w, uint32_t first_slot, TeamSweep& T, SweepFail* fail, bool masks_built) {
+    if (w == 0 && lane == 0) {
+        for (int q = 0; q <= W; ++q) T.met[q] = 0;
+        T.stop = 0;
+        T.result = INT_MAX;
+        T.fail_row = -1;
+    }
+    __syncthreads();
+    if (diag_sweep_ok(io, B, ws)) {
+        if (w == 0) {
+            SweepFail f;
+            const int d = warp_sweep_diag<MODE>(io, B, ws, lane, &f, masks_built);
+            if (lane == 0) {
+                T.result = d;
+                T.fail_row = f.row;
+                T.fail_min = f.min;
+            }
+        }
+    } else {
+        u64* buf[W + 1];
+#pragma unroll
+        for (int q = 0; q <= W; ++q) buf[q] = carry_buffer(a, first_slot, q);
+        const int d = strip_sweep<MODE, W>(io, B, buf, lane, w, &T, nullptr);
+        if (MODE == kDistance && lane == 0 && d != INT_MAX) T.result = d;  // one warp meets the corner
+    }
+    __syncthreads();
+    const int d = T.stop == 2 ? -1 : T.stop == 1 ? INT_MAX : T.result;
+    if (fail && T.fail_row >= 0) {
+        fail->row = T.fail_row;
+        fail->min = T.fail_min;
+    }
+    __syncthreads();
+    return d;
 }
 
 // k of the next distance pass after a pass with k failed: at least twice k;
@@ -690,12 +790,13 @@ __device__ void leaf_traceback(const NwDevArgs& a, const NwPairDev& P, const NwT
     }
 }
 
-__device__ void hirschberg_split(const NwDevArgs& a, const NwPairDev& P, const NwTask& T,
-                                 const WarpScratch& ws, u64* peq, int lane) {
+// The two halves' sweeps of a split by one warp (W = 1) or the W warps of a CTA.
+template <int W>
+__device__ bool hirschberg_sweeps(const NwDevArgs& a, const NwPairDev& P, const NwTask& T, const WarpScratch& ws,
+                                  u64* peq, int lane, int w, uint32_t first_slot, TeamSweep* team) {
     const int m = int(T.m), n = int(T.n);
-    const int best = T.score;
     const int lw = n / 2, rw = n - lw;
-    const Band B = make_band(m, n, best);
+    const Band B = make_band(m, n, T.score);
     SweepIO io;
     io.q = a.codes + P.q_off + T.qa;
     io.t = a.codes + P.t_off + T.ta;
@@ -708,15 +809,33 @@ __device__ void hirschberg_split(const NwDevArgs& a, const NwPairDev& P, const N
     io.cap_pv = ws.capl_pv;
     io.cap_mv = ws.capl_mv;
     io.cap_sc = ws.capl_sc;
-    warp_sweep<kCapture>(io, B, ws, lane, a.counters);
+    bool ok = true;
+    auto sweep = [&]() {
+        if constexpr (W == 1) {
+            warp_sweep<kCapture>(io, B, ws, lane, a.counters);
+        } else {
+            ok = team_sweep<kCapture, W>(a, io, B, ws, lane, w, first_slot, *team, nullptr, false) != -1 && ok;
+        }
+    };
+    sweep();
     io.rev = true;
     io.ncols = rw;
     io.cap_pv = ws.capr_pv;
     io.cap_mv = ws.capr_mv;
     io.cap_sc = ws.capr_sc;
-    warp_sweep<kCapture>(io, B, ws, lane, a.counters);
+    sweep();
     __syncwarp();
+    return ok;
+}
 
+// The split row of a task from its captured columns, and its two halves'
+// tasks (warp).
+__device__ void hirschberg_split(const NwDevArgs& a, const NwPairDev& P, const NwTask& T, const WarpScratch& ws,
+                                 int lane) {
+    const int m = int(T.m), n = int(T.n);
+    const int best = T.score;
+    const int lw = n / 2, rw = n - lw;
+    const Band B = make_band(m, n, best);
     const int llo = band_lo_block(B, lw - 1), lhi = band_hi_block(B, lw - 1);
     const int rlo = band_lo_block(B, rw - 1), rhi = band_hi_block(B, rw - 1);
     auto left = [&](int r) -> int {  // D(q[0..r], t[0..lw-1])
@@ -850,7 +969,8 @@ __device__ void level_task(const NwDevArgs& a, uint32_t i, const WarpScratch& ws
     if (is_leaf(T.m, T.n)) {
         leaf_traceback(a, P, T, ws, peq, lane);
     } else {
-        hirschberg_split(a, P, T, ws, peq, lane);
+        hirschberg_sweeps<1>(a, P, T, ws, peq, lane, 0, 0, nullptr);
+        hirschberg_split(a, P, T, ws, lane);
     }
 }
 
@@ -887,6 +1007,94 @@ nw_level_kernel(NwDevArgs a) {
         if (i >= a.ntasks_in) break;
         level_task(a, i, ws, peq, lane);
         __syncwarp();
+    }
+}
+
+// Distance pass and recursion level with one CTA of W warps per pair or task,
+// for batches with fewer of them than warps: the wide bands' strips of one
+// pair then run side by side. Everything else runs on the CTA's first warp.
+template <int W>
+__global__ void __launch_bounds__(32 * W) nw_distance_team_kernel(NwDevArgs a) {
+    __shared__ TeamSweep T;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t first = blockIdx.x * W;
+    u64* const peq = g_peq_smem + w * kMaxSym * 32;
+    const WarpScratch mine = warp_scratch(a, first + w);
+    WarpScratch ws = warp_scratch(a, first);  // masks of the diagonal form: the first warp's
+    for (;;) {
+        if (threadIdx.x == 0) T.item = atomicAdd(&a.counters[0], 1u);
+        __syncthreads();
+        const unsigned i = T.item;
+        __syncthreads();
+        if (i >= a.npairs) break;
+        const uint32_t pi = a.order[i];
+        const NwPairDev P = a.pairs[pi];
+        const int m = int(P.m), n = int(P.n);
+        if (m == 0 || n == 0) {
+            if (threadIdx.x == 0) a.dist[pi] = max(m, n);
+            continue;
+        }
+        SweepIO io;
+        io.q = a.codes + P.q_off;
+        io.t = a.codes + P.t_off;
+        io.rev = false;
+        io.ncols = n;
+        io.nsym = int(P.nsym);
+        io.peq = int(P.nsym) > kMaxSym ? peq_wide(mine) : peq;
+        io.leaf = nullptr;
+        io.bw = 0;
+        int k = max(64, abs(m - n));
+        int d = INT_MAX;
+        bool built = false;
+        while (true) {
+            const Band B = make_band(m, n, k);
+            SweepFail f;
+            d = team_sweep<kDistance, W>(a, io, B, ws, lane, w, first, T, &f, built);
+            if (d <= k) break;
+            built = diag_sweep_ok(io, B, ws);
+            k = next_k(k, f, m, n);
+        }
+        if (threadIdx.x == 0) {
+            if (d < 0) {
+                set_status(a.counters, kNwWaitLost);
+            } else {
+                a.dist[pi] = d;
+                const unsigned idx = atomicAdd(&a.counters[1], 1u);
+                if (idx < a.tasks_out_cap) {
+                    a.tasks_out[idx] = NwTask{pi, 0, P.m, 0, P.n, d};
+                } else {
+                    set_status(a.counters, kNwTaskOverflow);
+                }
+            }
+        }
+    }
+}
+
+template <int W>
+__global__ void __launch_bounds__(32 * W) nw_level_team_kernel(NwDevArgs a) {
+    __shared__ TeamSweep T;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t first = blockIdx.x * W;
+    u64* const peq = g_peq_smem + w * kMaxSym * 32;
+    const WarpScratch mine = warp_scratch(a, first + w);
+    WarpScratch ws = warp_scratch(a, first);  // captures, leaf store and masks: the first warp's
+    if (w > 0) ws.leaf = mine.leaf;           // (the wide alphabet's masks, behind the leaf store, are each warp's own)
+    for (;;) {
+        if (threadIdx.x == 0) T.item = atomicAdd(&a.counters[0], 1u);
+        __syncthreads();
+        const unsigned i = T.item;
+        __syncthreads();
+        if (i >= a.ntasks_in) break;
+        const NwTask K = a.tasks_in[i];
+        const NwPairDev P = a.pairs[K.pair];
+        if (is_leaf(K.m, K.n)) {
+            if (w == 0) leaf_traceback(a, P, K, ws, peq, lane);
+        } else if (hirschberg_sweeps<W>(a, P, K, ws, peq, lane, w, first, &T)) {
+            if (w == 0) hirschberg_split(a, P, K, ws, lane);
+        } else if (threadIdx.x == 0) {
+            set_status(a.counters, kNwWaitLost);
+        }
+        __syncthreads();
     }
 }
 
@@ -1417,6 +1625,10 @@ NwEngine::NwEngine(const DeviceInfo& dev, cudaStream_t stream) : dev_(dev), stre
                                     kWarpsPerBlock * kMaxSym * 32 * 8),
                "cudaFuncSetAttribute");
     const void* kernels[] = {reinterpret_cast<const void*>(nw_distance_kernel),
+                             reinterpret_cast<const void*>(nw_distance_team_kernel<4>),
+                             reinterpret_cast<const void*>(nw_distance_team_kernel<8>),
+                             reinterpret_cast<const void*>(nw_level_team_kernel<4>),
+                             reinterpret_cast<const void*>(nw_level_team_kernel<8>),
                              reinterpret_cast<const void*>(nw_level_kernel),
                              reinterpret_cast<const void*>(nw_breakpoints_kernel),
                              reinterpret_cast<const void*>(nw_cigar_kernel),
@@ -1723,9 +1935,34 @@ void NwEngine::run_own() {
         return yield_items_ ? (items + scratch_warps_ * yield_items_ - 1) / (scratch_warps_ * yield_items_)
                             : size_t(1);
     };
-    for (size_t l = launches_for(n); l > 0; --l) {
-        nw_distance_kernel<<<grid, 32 * kWarpsPerBlock, smem, stream_>>>(a);
+    // Warps per pair or task. Bands wide enough for several strips at once
+    // come with queries of several thousand bases; a CTA of four warps works
+    // on each item while there are at most four times as many as resident
+    // CTAs (600 pairs of 1-50 kb: 57 ms against 137 ms with one warp each;
+    // 2400 pairs of 1-30 kb: 74 against 78; 5000 pairs of 1-20 kb: 81 against
+    // 50), of eight warps for the longest queries on a half-empty GPU (9 pairs
+    // of 60-120 kb: 48 ms against 56; 60 of 60-100 kb: 61 against 67; 140 of
+    // 50-70 kb: 56 against 51; 60 of 8-50 kb: 27 against 26).
+    auto team_for = [&](size_t items) -> int {
+        if (yield_items_ || max_m_ < kTeamRows || scratch_warps_ < 2 * kMaxTeam) return 1;
+        if (items <= size_t(dev_.sm_count) / 2 && max_m_ >= kWideTeamRows) return 8;
+        return items <= 4 * (scratch_warps_ / 4) ? 4 : 1;
+    };
+    auto team_launch = [&](int w, size_t items, void (*k4)(NwDevArgs), void (*k8)(NwDevArgs)) {
+        const size_t bytes = size_t(w) * kMaxSym * 32 * 8;
+        check_cuda(cudaFuncSetAttribute(w == 8 ? k8 : k4, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)),
+                   "cudaFuncSetAttribute");
+        const int ctas = int(std::min(items, scratch_warps_ / size_t(w)));
+        (w == 8 ? k8 : k4)<<<ctas, 32 * w, bytes, stream_>>>(a);
         ++stats_.launches;
+    };
+    if (const int w = team_for(n); w > 1) {
+        team_launch(w, n, nw_distance_team_kernel<4>, nw_distance_team_kernel<8>);
+    } else {
+        for (size_t l = launches_for(n); l > 0; --l) {
+            nw_distance_kernel<<<grid, 32 * kWarpsPerBlock, smem, stream_>>>(a);
+            ++stats_.launches;
+        }
     }
     unsigned int h_cnt[4];
     check_cuda(cudaMemcpyAsync(h_cnt, a.counters, 16, cudaMemcpyDeviceToHost, stream_), "D2H count");
@@ -1742,9 +1979,13 @@ void NwEngine::run_own() {
         a.tasks_out = d_tasks_[cur ^ 1].as<NwTask>();
         a.tasks_out_cap = uint32_t(task_cap);
         check_cuda(cudaMemsetAsync(a.counters, 0, 8, stream_), "memset counters");
-        for (size_t l = launches_for(ntasks); l > 0; --l) {
-            nw_level_kernel<<<grid, 32 * kWarpsPerBlock, smem, stream_>>>(a);
-            ++stats_.launches;
+        if (const int w = team_for(ntasks); w > 1) {
+            team_launch(w, ntasks, nw_level_team_kernel<4>, nw_level_team_kernel<8>);
+        } else {
+            for (size_t l = launches_for(ntasks); l > 0; --l) {
+                nw_level_kernel<<<grid, 32 * kWarpsPerBlock, smem, stream_>>>(a);
+                ++stats_.launches;
+            }
         }
         check_cuda(cudaMemcpyAsync(h_cnt, a.counters, 16, cudaMemcpyDeviceToHost, stream_), "D2H count");
         check_cuda(cudaStreamSynchronize(stream_), "sync level");

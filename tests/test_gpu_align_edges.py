@@ -45,3 +45,19 @@ def test_bands(native_lib, oracle_lib, shift):
     t = "".join(rng.choice("ACGT") for _ in range(9000))
     q = _mutate(rng, t[:4000] + t[4000 + shift:], 0.05, "ACGT")
     _check(native_lib, oracle_lib, [(q, t), (t, q)])
+
+
+# Batches of few long pairs are swept by CTAs of four warps (queries from 6144
+# bases) and eight (from 65536): both sides of the two lines, strips that wrap
+# around the warps and their buffers, passes that give up, wide alphabets.
+@pytest.mark.parametrize("length,letters", [(6143, "ACGT"), (6144, "ACGT"), (8193, "ABCDEFGHIJKL"), (10240, "ACGT"),
+                                            (10241, "".join(map(chr, range(40, 80)))), (18433, "ACGT"),
+                                            (65535, "ACGT"), (65536, "ACGT")])
+def test_teams(native_lib, oracle_lib, length, letters):
+    rng = random.Random(length)
+    s = "".join(rng.choice(letters) for _ in range(length))
+    third = s[:length // 3]
+    pairs = [(s, third + s[length // 2:]), (_mutate(rng, s, 0.3, letters), s), (s, third)]
+    if length < 20000:
+        pairs += [(s[::-1], s), (third, s), ("A", s), (_mutate(rng, s, 0.05, letters), s)]
+    _check(native_lib, oracle_lib, pairs)
