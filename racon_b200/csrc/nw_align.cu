@@ -1180,63 +1180,81 @@ nw_service_kernel(NwSvcArgs s) {
     }
 }
 
-// Breaking points from mq: one window segment per floor(t / w); for each
-// segment with a match, (first match t, q) and (last match t + 1, q + 1).
 // Window breaking points of each pair from its match table, one warp per
-// pair over 32-position chunks: racon's walk (src/overlap.cpp:244-290) emits,
-// per window the target touches, the first matched (t, q) and the last
-// matched (t + 1, q + 1). A matched position opens a window segment when the
-// previous matched position (the highest matched lane below, or the carry of
-// earlier chunks) lies in another window; it writes its segment's first pair
-// and closes the previous segment's last pair.
-__global__ void __launch_bounds__(256) nw_breakpoints_kernel(NwDevArgs a) {
+// pair: racon's walk (src/overlap.cpp:244-290) emits, per window the target
+// touches, the first matched (t, q) and the last matched (t + 1, q + 1). A
+// lane takes a window and looks for both from the window's ends, where a match
+// is nearly always within a few positions; the warp finishes the search of a
+// lane that meets a gap. (A warp stepping through all positions took 1.7 ms
+// for 120 kb pairs and 0.8 ms for 700 pairs of 1-50 kb; now 0.014 and 0.011.)
+constexpr int kOwnSteps = 8;  // positions a lane looks at before the warp helps
+__global__ void __launch_bounds__(256, 6) nw_breakpoints_kernel(NwDevArgs a) {
     const int lane = threadIdx.x & 31;
     const unsigned below_mask = (1u << lane) - 1u;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < a.npairs; i += nwarps) {
         const NwPairDev P = a.pairs[i];
-        uint32_t* out = a.bp + P.bp_off;
+        uint4* const out = reinterpret_cast<uint4*>(a.bp + P.bp_off);  // four values per window from the base
         uint32_t segs = 0;
         if (P.m != 0 && P.n != 0) {
-            const int32_t* mq = a.mq + P.mq_off;
+            const int32_t* const mq = a.mq + P.mq_off;
             const uint32_t w = a.window_length;
-            uint32_t carry_sgm = 0xFFFFFFFFu, carry_t = 0, carry_q = 0;
-            for (uint32_t c0 = 0; c0 < P.n; c0 += 32) {
-                const uint32_t c = c0 + lane;
-                const int32_t v = c < P.n ? mq[c] : -1;
-                const bool matched = v >= 0;
-                const uint32_t t = P.t_begin + c;
-                const uint32_t q = P.q_offset + uint32_t(v);
-                const uint32_t sgm = t / w;
-                const unsigned mm = __ballot_sync(kFull, matched);
-                const unsigned below = mm & below_mask;
-                const int p = below ? 31 - __clz(below) : 0;
-                const uint32_t p_sgm = __shfl_sync(kFull, sgm, p);
-                const uint32_t p_t = __shfl_sync(kFull, t, p);
-                const uint32_t p_q = __shfl_sync(kFull, q, p);
-                const uint32_t prev_sgm = below ? p_sgm : carry_sgm;
-                const bool first = matched && sgm != prev_sgm;
-                const unsigned fm = __ballot_sync(kFull, first);
-                if (first) {
-                    const uint32_t idx = segs + __popc(fm & below_mask);
-                    out[4 * idx] = t;
-                    out[4 * idx + 1] = q;
-                    if (idx > 0) {
-                        out[4 * (idx - 1) + 2] = (below ? p_t : carry_t) + 1;
-                        out[4 * (idx - 1) + 3] = (below ? p_q : carry_q) + 1;
+            const uint32_t w0 = P.t_begin / w;
+            const uint32_t nw = uint32_t((u64(P.t_begin) + P.n - 1) / w) - w0 + 1;
+            for (uint32_t s0 = 0; s0 < nw; s0 += 32) {
+                const u64 ws = u64(w0) + s0 + lane;  // this lane's window
+                int lo = 0, hi = 0;                  // its positions
+                if (s0 + lane < nw) {
+                    lo = ws * w > P.t_begin ? int(ws * w - P.t_begin) : 0;
+                    hi = int(min(u64(P.n), (ws + 1) * w - P.t_begin));
+                }
+                int v0 = -1, v1 = -1;
+                for (const int stop = min(hi, lo + kOwnSteps); lo < stop; ++lo) {
+                    v0 = mq[lo];
+                    if (v0 >= 0) break;
+                }
+                for (unsigned open = __ballot_sync(kFull, v0 < 0 && lo < hi); open; open &= open - 1) {
+                    const int u = __ffs(open) - 1;
+                    const int end = __shfl_sync(kFull, hi, u);
+                    for (int x = __shfl_sync(kFull, lo, u); x < end; x += 32) {
+                        const int v = x + lane < end ? mq[x + lane] : -1;
+                        const unsigned hit = __ballot_sync(kFull, v >= 0);
+                        const int at = hit ? __ffs(hit) - 1 : 0;
+                        const int got = __shfl_sync(kFull, v, at);
+                        if (hit && lane == u) {
+                            lo = x + at;
+                            v0 = got;
+                        }
+                        if (hit) break;
                     }
                 }
-                segs += __popc(fm);
-                if (mm) {
-                    const int hl = 31 - __clz(mm);
-                    carry_sgm = __shfl_sync(kFull, sgm, hl);
-                    carry_t = __shfl_sync(kFull, t, hl);
-                    carry_q = __shfl_sync(kFull, q, hl);
+                const bool any = v0 >= 0;
+                if (!any) hi = lo;
+                for (const int stop = max(lo, hi - kOwnSteps); hi > stop; --hi) {
+                    v1 = mq[hi - 1];
+                    if (v1 >= 0) break;
                 }
-            }
-            if (segs > 0 && lane == 0) {
-                out[4 * (segs - 1) + 2] = carry_t + 1;
-                out[4 * (segs - 1) + 3] = carry_q + 1;
+                for (unsigned open = __ballot_sync(kFull, any && v1 < 0); open; open &= open - 1) {
+                    const int u = __ffs(open) - 1;
+                    const int end = __shfl_sync(kFull, lo, u);  // a match is at `end` at the latest
+                    for (int x = __shfl_sync(kFull, hi, u) - 1; x >= end; x -= 32) {
+                        const int v = x - lane >= end ? mq[x - lane] : -1;
+                        const unsigned hit = __ballot_sync(kFull, v >= 0);
+                        const int at = hit ? __ffs(hit) - 1 : 0;
+                        const int got = __shfl_sync(kFull, v, at);
+                        if (hit && lane == u) {
+                            hi = x - at + 1;
+                            v1 = got;
+                        }
+                        if (hit) break;
+                    }
+                }
+                const unsigned all = __ballot_sync(kFull, any);
+                if (any)
+                    out[segs + __popc(all & below_mask)] =
+                        make_uint4(P.t_begin + uint32_t(lo), P.q_offset + uint32_t(v0), P.t_begin + uint32_t(hi),
+                                   P.q_offset + uint32_t(v1) + 1);
+                segs += __popc(all);
             }
         }
         if (lane == 0) a.bp_count[i] = 4 * segs;
@@ -1266,93 +1284,130 @@ __device__ __forceinline__ int decimal_digits(uint32_t x) {
     return d;
 }
 
-// Standard CIGAR (M/I/D runs) of each pair from its match table, one warp
-// per pair over 32-position chunks; write = 0 counts the characters into
-// lens, write = 1 writes them at offs. The sequential walk it restates: per
+// Standard CIGAR (M/I/D runs) of each pair from its match table, by one warp
+// or by the eight of a CTA (parts), each over its share of the positions in
+// 32-position chunks; write = 0 counts the characters into lens, write = 1
+// writes them at offs. The sequential walk it restates: per
 // target position an insertion run before a matched position (the query
 // positions skipped since the previous match), then M, or D when unmatched;
 // equal neighbouring ops merge, and trailing query positions end with I.
 // An M/D run therefore starts where the op changes or an insertion comes
 // first; each such position closes the previous run and emits its own I run,
-// and a warp prefix sum of their text lengths gives every lane's offset.
-__global__ void __launch_bounds__(256) nw_cigar_kernel(NwDevArgs a, uint64_t* lens, const uint64_t* offs, char* out,
-                                                       int write) {
-    const int lane = threadIdx.x & 31;
+// and a warp prefix sum of their text lengths gives every lane's offset. A
+// part begins with what the positions before it decide: the last match, the
+// last op and where its run started, all found by looking back; with several
+// parts the write pass counts its part once more for its place in the text.
+// (700 pairs of 1-50 kb, both passes: 3.2 ms by one warp a pair, 0.66 ms by
+// eight.)
+__global__ void __launch_bounds__(256, 6) nw_cigar_kernel(NwDevArgs a, uint64_t* lens, const uint64_t* offs, char* out,
+                                                          int write, uint32_t parts) {
+    __shared__ uint32_t part_len[8];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const unsigned below_mask = (1u << lane) - 1u;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < a.npairs; i += nwarps) {
+    const uint32_t teams = gridDim.x * (8 / parts);
+    const uint32_t part = uint32_t(wib) % parts;
+    for (uint32_t i = blockIdx.x * (8 / parts) + uint32_t(wib) / parts; i < a.npairs; i += teams) {
         const NwPairDev P = a.pairs[i];
         if (P.m == 0 || P.n == 0) {
-            if (!write && lane == 0) lens[i] = 0;
+            if (!write && lane == 0 && part == 0) lens[i] = 0;
             continue;
         }
         const int32_t* mq = a.mq + P.mq_off;
         char* dst = write ? out + offs[i] : nullptr;
         const uint32_t n = P.n;
-        uint64_t pos = 0;           // characters before this chunk
-        int carry_v = -1;           // last matched query position so far
-        int carry_op = -1;          // op of the position before the chunk (0 = M, 1 = D)
-        uint32_t run_start = 0;     // first position of the open M/D run
-        int run_op = -1;            // its op (-1: none yet)
-        for (uint32_t c0 = 0; c0 < n; c0 += 32) {
-            const uint32_t c = c0 + lane;
-            const bool valid = c < n;
-            const int v = valid ? mq[c] : -1;
-            const bool matched = v >= 0;
-            const int op = matched ? 0 : 1;
-            const unsigned mm = __ballot_sync(kFull, matched);
-            const unsigned mbelow = mm & below_mask;
-            const int p_v = __shfl_sync(kFull, v, mbelow ? 31 - __clz(mbelow) : 0);
-            const int prev_v = mbelow ? p_v : carry_v;
-            const int ins = matched ? v - prev_v - 1 : 0;
-            const int up_op = __shfl_up_sync(kFull, op, 1);
-            const int prev_op = lane > 0 ? up_op : carry_op;
-            const bool start = valid && (c == 0 || op != prev_op || ins > 0);
-            const unsigned sm = __ballot_sync(kFull, start);
-            const unsigned sbelow = sm & below_mask;
-            const int ps = sbelow ? 31 - __clz(sbelow) : 0;
-            const int ps_op = __shfl_sync(kFull, op, ps);
-            const uint32_t prev_start = sbelow ? c0 + uint32_t(ps) : run_start;
-            const int prev_run_op = sbelow ? ps_op : run_op;
-            const bool close_prev = start && prev_run_op >= 0;
-            const uint32_t close_len = c - prev_start;
-            int tl = 0;
-            if (close_prev) tl += decimal_digits(close_len) + 1;
-            if (start && ins > 0) tl += decimal_digits(uint32_t(ins)) + 1;
-            int x = tl;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int y = __shfl_up_sync(kFull, x, d);
-                if (lane >= d) x += y;
+        const uint32_t share = (n + 32 * parts - 1) / (32 * parts) * 32;
+        const uint32_t begin = min(n, part * share), end = min(n, begin + share);
+        const bool last = begin < end && end == n;
+        int first_v = -1, first_op = -1;  // before the part: last matched query position, last op (0 = M, 1 = D)
+        uint32_t first_run = 0;           // and the first position of its run
+        if (begin > 0 && begin < end) {
+            bool run_found = false;
+            for (uint32_t x = begin; x > 0 && (first_v < 0 || !run_found); x = x > 32 ? x - 32 : 0) {
+                const int c = int(x) - 1 - lane;
+                const int v = c >= 0 ? mq[c] : -1, before = c > 0 ? mq[c - 1] : -1;
+                const unsigned mm = __ballot_sync(kFull, v >= 0);
+                const unsigned sm = __ballot_sync(
+                    kFull, c == 0 || (c > 0 && ((v >= 0) != (before >= 0) || (v >= 0 && v != before + 1))));
+                if (x == begin) first_op = (mm & 1u) ? 0 : 1;
+                if (first_v < 0 && mm) first_v = __shfl_sync(kFull, v, __ffs(mm) - 1);
+                if (!run_found && sm) {
+                    run_found = true;
+                    first_run = x - uint32_t(__ffs(sm));
+                }
             }
-            const int total = __shfl_sync(kFull, x, 31);
-            if (write && tl) {
-                int at = int(pos) + x - tl;
-                if (close_prev) at = put_run(dst, at, true, int(close_len), prev_run_op ? 'D' : 'M');
-                if (ins > 0) put_run(dst, at, true, ins, 'I');
-            }
-            pos += uint64_t(total);
-            if (sm) {
-                const int hs = 31 - __clz(sm);
-                run_start = c0 + uint32_t(hs);
-                run_op = __shfl_sync(kFull, op, hs);
-            }
-            const int last_lane = int(min(31u, n - 1 - c0));
-            carry_op = __shfl_sync(kFull, op, last_lane);
-            if (mm) carry_v = __shfl_sync(kFull, v, 31 - __clz(mm));
         }
-        // the open run, then the query positions after the last match
-        const uint32_t last_len = n - run_start;
-        const int tail = int(P.m) - 1 - carry_v;
-        uint64_t end = pos + decimal_digits(last_len) + 1;
-        if (tail > 0) end += decimal_digits(uint32_t(tail)) + 1;
-        if (lane == 0) {
-            if (write) {
-                const int at = put_run(dst, int(pos), true, int(last_len), run_op ? 'D' : 'M');
-                if (tail > 0) put_run(dst, at, true, tail, 'I');
-            } else {
-                lens[i] = end;
+        uint64_t pos = 0;  // characters before this chunk
+        for (int pass = write && parts == 1 ? 1 : 0; pass <= write; ++pass) {
+            int carry_v = first_v;           // last matched query position so far
+            int carry_op = first_op;         // op of the position before the chunk
+            uint32_t run_start = first_run;  // first position of the open M/D run
+            int run_op = first_op;           // its op (-1: none yet)
+            for (uint32_t c0 = begin; c0 < end; c0 += 32) {
+                const uint32_t c = c0 + lane;
+                const bool valid = c < end;
+                const int v = valid ? mq[c] : -1;
+                const bool matched = v >= 0;
+                const int op = matched ? 0 : 1;
+                const unsigned mm = __ballot_sync(kFull, matched);
+                const unsigned mbelow = mm & below_mask;
+                const int p_v = __shfl_sync(kFull, v, mbelow ? 31 - __clz(mbelow) : 0);
+                const int prev_v = mbelow ? p_v : carry_v;
+                const int ins = matched ? v - prev_v - 1 : 0;
+                const int up_op = __shfl_up_sync(kFull, op, 1);
+                const int prev_op = lane > 0 ? up_op : carry_op;
+                const bool start = valid && (c == 0 || op != prev_op || ins > 0);
+                const unsigned sm = __ballot_sync(kFull, start);
+                const unsigned sbelow = sm & below_mask;
+                const int ps = sbelow ? 31 - __clz(sbelow) : 0;
+                const int ps_op = __shfl_sync(kFull, op, ps);
+                const uint32_t prev_start = sbelow ? c0 + uint32_t(ps) : run_start;
+                const int prev_run_op = sbelow ? ps_op : run_op;
+                const bool close_prev = start && prev_run_op >= 0;
+                const uint32_t close_len = c - prev_start;
+                int tl = 0;
+                if (close_prev) tl += decimal_digits(close_len) + 1;
+                if (start && ins > 0) tl += decimal_digits(uint32_t(ins)) + 1;
+                int x = tl;
+    #pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int y = __shfl_up_sync(kFull, x, d);
+                    if (lane >= d) x += y;
+                }
+                const int total = __shfl_sync(kFull, x, 31);
+                if (pass && tl) {
+                    int at = int(pos) + x - tl;
+                    if (close_prev) at = put_run(dst, at, true, int(close_len), prev_run_op ? 'D' : 'M');
+                    if (ins > 0) put_run(dst, at, true, ins, 'I');
+                }
+                pos += uint64_t(total);
+                if (sm) {
+                    const int hs = 31 - __clz(sm);
+                    run_start = c0 + uint32_t(hs);
+                    run_op = __shfl_sync(kFull, op, hs);
+                }
+                const int last_lane = int(min(31u, end - 1 - c0));
+                carry_op = __shfl_sync(kFull, op, last_lane);
+                if (mm) carry_v = __shfl_sync(kFull, v, 31 - __clz(mm));
             }
+            if (last) {
+                // the open run, then the query positions after the last match
+                const uint32_t last_len = n - run_start;
+                const int tail = int(P.m) - 1 - carry_v;
+                if (pass && lane == 0) {
+                    const int at = put_run(dst, int(pos), true, int(last_len), run_op ? 'D' : 'M');
+                    if (tail > 0) put_run(dst, at, true, tail, 'I');
+                }
+                pos += decimal_digits(last_len) + 1;
+                if (tail > 0) pos += decimal_digits(uint32_t(tail)) + 1;
+            }
+            if (pass == 0 && parts > 1) {
+                if (lane == 0) part_len[wib] = uint32_t(pos);
+                __syncthreads();
+                pos = 0;
+                for (uint32_t q = 0; q < (write ? part : parts); ++q) pos += part_len[q];
+                __syncthreads();
+            }
+            if (!write && lane == 0 && part == 0) lens[i] = pos;
         }
     }
 }
@@ -1564,52 +1619,85 @@ struct NwStoreSrc {
 // come from one pass over 32-byte chunks in order: the lowest lane holding a
 // byte value not seen before records its position. A pair with more than
 // kMaxSymWide distinct bytes (impossible for bytes) sets status[0] = 1.
-__global__ void __launch_bounds__(256) nw_encode_kernel(const uint8_t* store, const NwStoreSrc* src,
-                                                        NwPairDev* pairs, uint8_t* codes, uint32_t n,
-                                                        unsigned int* status) {
+// One warp or the eight of a CTA (parts) take a pair. A symbol's first
+// position is a minimum over all positions, and after the first few hundred
+// bases a look at the table is all a position costs (a warp grouping its
+// bytes by __match_any_sync took 3.7 ms for 120 kb pairs, 1.9 ms for 700 pairs
+// of 1-50 kb and 0.23 ms for 4600 of 4 kb; now 0.19, 0.10 and 0.08).
+__global__ void __launch_bounds__(256, 6) nw_encode_kernel(const uint8_t* store, const NwStoreSrc* src,
+                                                           NwPairDev* pairs, uint8_t* codes, uint32_t n,
+                                                           unsigned int* status, uint32_t parts) {
     __shared__ uint32_t first_pos[8][256];
     __shared__ uint8_t code[8][256];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    uint32_t* fp = first_pos[wib];
-    uint8_t* cd = code[wib];
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nwarps) {
+    __shared__ int count[8];
+    const uint32_t wib = threadIdx.x >> 5, team = wib / parts;
+    const uint32_t size = 32 * parts, tid = threadIdx.x % size;
+    uint32_t* fp = first_pos[team];
+    uint8_t* cd = code[team];
+    const uint32_t teams = gridDim.x * (8 / parts);
+    auto sync = [&]() {
+        if (parts > 1) __syncthreads();
+        else __syncwarp();
+    };
+    for (uint32_t i = blockIdx.x * (8 / parts) + team; i < n; i += teams) {
         const NwStoreSrc sp = src[i];
         const uint32_t m = pairs[i].m, nt = pairs[i].n;
         const uint64_t q_off = pairs[i].q_off, t_off = pairs[i].t_off;
-        for (int v = lane; v < 256; v += 32) fp[v] = 0xFFFFFFFFu;
-        __syncwarp();
-        const uint32_t total = m + nt;
-        for (uint32_t k0 = 0; k0 < total; k0 += 32) {
-            const uint32_t k = k0 + lane;
-            uint32_t c = 0x100u + uint32_t(lane);  // matches no byte value
-            if (k < total) c = k < m ? store[sp.q_src + k] : store[sp.t_src + (k - m)];
-            const unsigned same = __match_any_sync(0xffffffffu, c);
-            if (c < 0x100u && __ffs(same) - 1 == lane && fp[c] == 0xFFFFFFFFu) fp[c] = k;
-            __syncwarp();
-        }
-        int present = 0;
-        for (int v = lane; v < 256; v += 32) {
+        for (uint32_t v = tid; v < 256; v += size) fp[v] = 0xFFFFFFFFu;
+        if (tid == 0) count[team] = 0;
+        sync();
+        auto find = [&](const uint8_t* s, uint32_t len, uint32_t at) {
+            for (uint32_t k0 = tid; k0 < len; k0 += 4 * size) {
+                uint32_t c[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) c[j] = s[min(k0 + j * size, len - 1)];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t k = at + min(k0 + j * size, len - 1);
+                    if (*(volatile uint32_t*)(fp + c[j]) > k) atomicMin(fp + c[j], k);
+                }
+            }
+        };
+        find(store + sp.q_src, m, 0);
+        find(store + sp.t_src, nt, m);
+        sync();
+        for (uint32_t v = tid; v < 256; v += size) {
             const uint32_t p = fp[v];
             if (p == 0xFFFFFFFFu) continue;
             int r = 0;
             for (int u = 0; u < 256; ++u) r += fp[u] < p ? 1 : 0;
             cd[v] = uint8_t(r);
-            ++present;
+            atomicAdd(&count[team], 1);
         }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) present += __shfl_xor_sync(0xffffffffu, present, d);
-        __syncwarp();
+        sync();
+        const int present = count[team];
         if (present > kMaxSymWide) {  // cannot happen for byte symbols; kept as a guard
-            if (lane == 0) status[0] = 1u;
-            continue;
+            if (tid == 0) status[0] = 1u;
+        } else {
+            // the codes may replace the bytes they are made from
+            auto put = [&](const uint8_t* s, uint8_t* d, uint32_t len) {
+                for (uint32_t k0 = tid; k0 < len; k0 += 4 * size) {
+                    uint8_t c[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (k0 + j * size < len) c[j] = s[k0 + j * size];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (k0 + j * size < len) d[k0 + j * size] = cd[c[j]];
+                }
+            };
+            put(store + sp.q_src, codes + q_off, m);
+            put(store + sp.t_src, codes + t_off, nt);
+            if (tid == 0) pairs[i].nsym = uint32_t(max(present, 1));
         }
-        for (uint32_t k = lane; k < m; k += 32) codes[q_off + k] = cd[store[sp.q_src + k]];
-        for (uint32_t k = lane; k < nt; k += 32) codes[t_off + k] = cd[store[sp.t_src + k]];
-        if (lane == 0) pairs[i].nsym = uint32_t(max(present, 1));
-        __syncwarp();
+        sync();
     }
 }
+
+// Warps per pair of the kernels that read or write all of a pair's bases
+// (codes, CIGARs): a CTA's eight while there are too few pairs to give every
+// warp one, else one.
+uint32_t pair_parts(size_t n, int sm_count) { return n <= 16 * size_t(sm_count) ? 8 : 1; }
 
 }  // namespace
 
@@ -1747,10 +1835,11 @@ void NwEngine::stage(const rb_pair* pairs, size_t n, int want_cigar, uint32_t wi
         check_cuda(cudaMemcpyAsync(d_src_.ptr, src, n * sizeof(NwStoreSrc), cudaMemcpyHostToDevice, stream_),
                    "H2D pair sources");
         check_cuda(cudaMemsetAsync(d_misc_.ptr, 0, 64, stream_), "memset status");
-        const int grid = int(std::max<size_t>(1, std::min<size_t>((n + 7) / 8, size_t(dev_.sm_count) * 8)));
+        const uint32_t parts = pair_parts(n, dev_.sm_count);
+        const int grid = int(std::min<size_t>((n * parts + 7) / 8, size_t(dev_.sm_count) * 8));
         nw_encode_kernel<<<grid, 256, 0, stream_>>>(d_codes_.as<uint8_t>(), d_src_.as<NwStoreSrc>(),
                                                     d_pairs_.as<NwPairDev>(), d_codes_.as<uint8_t>(), uint32_t(n),
-                                                    d_misc_.as<unsigned int>());
+                                                    d_misc_.as<unsigned int>(), parts);
         check_cuda(cudaGetLastError(), "nw_encode_kernel");
         check_cuda(cudaMemcpyAsync(&status, d_misc_.ptr, 4, cudaMemcpyDeviceToHost, stream_), "D2H status");
     }
@@ -1838,9 +1927,11 @@ void NwEngine::stage_store(const rb_store_pair* pairs, size_t n, int want_cigar,
         check_cuda(cudaMemcpyAsync(d_order_.ptr, order, n * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_),
                    "H2D order");
         check_cuda(cudaMemsetAsync(d_misc_.ptr, 0, 64, stream_), "memset status");
-        const int grid = int(std::max<size_t>(1, std::min<size_t>((n + 7) / 8, size_t(dev_.sm_count) * 8)));
+        const uint32_t parts = pair_parts(n, dev_.sm_count);
+        const int grid = int(std::min<size_t>((n * parts + 7) / 8, size_t(dev_.sm_count) * 8));
         nw_encode_kernel<<<grid, 256, 0, stream_>>>(st.bytes, d_src_.as<NwStoreSrc>(), d_pairs_.as<NwPairDev>(),
-                                                    d_codes_.as<uint8_t>(), uint32_t(n), d_misc_.as<unsigned int>());
+                                                    d_codes_.as<uint8_t>(), uint32_t(n), d_misc_.as<unsigned int>(),
+                                                    parts);
         check_cuda(cudaGetLastError(), "nw_encode_kernel");
     }
     check_cuda(cudaEventRecord(ev1_, stream_), "cudaEventRecord");
@@ -2069,7 +2160,7 @@ void NwEngine::run_shared() {
 }
 
 // Breaking points, and with want_cigar the CIGAR strings, of the aligned
-// pairs: warp-per-pair kernels on this engine's stream.
+// pairs, on this engine's stream.
 void NwEngine::finish_outputs(const void* args) {
     const NwDevArgs& a = *static_cast<const NwDevArgs*>(args);
     const size_t n = npairs_;
@@ -2079,8 +2170,9 @@ void NwEngine::finish_outputs(const void* args) {
     if (want_cigar_) {
         d_ciglen_.reserve((n + 1) * sizeof(uint64_t));
         d_cigoff_.reserve((n + 1) * sizeof(uint64_t));
-        nw_cigar_kernel<<<warp_grid, 256, 0, stream_>>>(a, d_ciglen_.as<uint64_t>(), nullptr,
-                                                                   nullptr, 0);
+        const uint32_t parts = pair_parts(n, dev_.sm_count);
+        const int cigar_grid = int(std::max<size_t>(1, std::min<size_t>((n * parts + 7) / 8, size_t(dev_.sm_count) * 16)));
+        nw_cigar_kernel<<<cigar_grid, 256, 0, stream_>>>(a, d_ciglen_.as<uint64_t>(), nullptr, nullptr, 0, parts);
         exclusive_scan_kernel<<<1, 256, 0, stream_>>>(d_ciglen_.as<uint64_t>(), d_cigoff_.as<uint64_t>(),
                                                        uint32_t(n));
         uint64_t total = 0;
@@ -2088,8 +2180,8 @@ void NwEngine::finish_outputs(const void* args) {
                    "D2H cigar total");
         check_cuda(cudaStreamSynchronize(stream_), "sync cigar");
         d_cig_.reserve(std::max<uint64_t>(total, 1));
-        nw_cigar_kernel<<<warp_grid, 256, 0, stream_>>>(a, d_ciglen_.as<uint64_t>(),
-                                                                   d_cigoff_.as<uint64_t>(), d_cig_.as<char>(), 1);
+        nw_cigar_kernel<<<cigar_grid, 256, 0, stream_>>>(a, d_ciglen_.as<uint64_t>(), d_cigoff_.as<uint64_t>(),
+                                                         d_cig_.as<char>(), 1, parts);
         stats_.launches += 3;
     }
 }
