@@ -60,9 +60,9 @@ POA_DRAM_BYTES_PER_CELL = (2.199457e9 + 12.164103e9) / 5838774640
 L2_FLUSH_BYTES = 512 << 20
 # DRAM bytes (read + write) of nw_distance_kernel per nominal cell (query x
 # target span) from one ncu capture of the first 500 pairs of the config-2
-# batch (31.4 MB read + 104.8 MB written over 421.3 G nominal cells); the
+# batch (31.3 MB read + 1.1 MB written over 421.3 G nominal cells); the
 # strip carry buffers grow with the swept cells
-NWD_DRAM_BYTES_PER_CELL = (31.4e6 + 104.8e6) / 421325730898
+NWD_DRAM_BYTES_PER_CELL = (31.252e6 + 1.092e6) / 421325730898
 
 
 def _args():

@@ -666,6 +666,17 @@ __device__ int team_sweep(const NwDevArgs& a, const SweepIO& io, const Band& B, 
     return d;
 }
 
+// k of the first distance pass: the widest band of the diagonal sweep where the
+// pair takes that form, whose steps do not depend on k, else edlib's 64. From
+// 64, short pairs swept twice and long ones gave up three times on the way to
+// their distance: 20000 pairs of 0.5-3 kb 15.3 ms, now 11.4; 700 of 1-50 kb
+// 48.4, now 40.2; 5000 of 3-8 kb at 3 % error 15.4, now 13.4.
+__device__ __forceinline__ int first_k(const SweepIO& io, const WarpScratch& ws, int m, int n) {
+    const int k = max(64, abs(m - n));
+    const int wide = max(k, kDiagBand);
+    return diag_sweep_ok(io, make_band(m, n, wide), ws) ? wide : k;
+}
+
 // k of the next distance pass after a pass with k failed: at least twice k;
 // when the pass gave up at row f.row with minimum cost f.min, the cost per
 // row so far projected over the longer side (x 1.1), up to 8k. Any k gives
@@ -931,7 +942,7 @@ __device__ void distance_pair(const NwDevArgs& a, uint32_t pi, const WarpScratch
     io.peq = int(P.nsym) > kMaxSym ? peq_wide(ws) : peq;
     io.leaf = nullptr;
     io.bw = 0;
-    int k = max(64, abs(m - n));
+    int k = first_k(io, ws, m, n);
     int d = INT_MAX;
     bool built = false;  // the diagonal sweep's masks depend on the query alone
     while (true) {
@@ -1035,7 +1046,7 @@ __global__ void __launch_bounds__(32 * W) nw_distance_team_kernel(NwDevArgs a) {
         io.peq = int(P.nsym) > kMaxSym ? peq_wide(mine) : peq;
         io.leaf = nullptr;
         io.bw = 0;
-        int k = max(64, abs(m - n));
+        int k = first_k(io, ws, m, n);
         int d = INT_MAX;
         bool built = false;
         while (true) {
