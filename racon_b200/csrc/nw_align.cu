@@ -20,7 +20,7 @@
 //   is an upper bound and every cell on an optimal path is exact. Therefore
 //   the edit distance, the Hirschberg split row and every traceback decision
 //   equal those of the unbanded dynamic program.
-// * Distance. k doubles from max(64, |m - n|) until the band holds the corner
+// * Distance. k grows from first_k until the band holds the corner
 //   (the first k >= distance returns the exact distance).
 // * Path. edlib's recursion is followed exactly: a subproblem is traced back
 //   from stored columns when (2*8+4) * ceil(m/64) * n < 1 MiB, else it is
@@ -923,7 +923,7 @@ __device__ __forceinline__ bool is_leaf(uint32_t m, uint32_t n) {
 
 extern __shared__ u64 g_peq_smem[];
 
-// Edit distance of pair pi by one warp (k doubling from max(64, |m - n|)),
+// Edit distance of pair pi by one warp (k growing from first_k),
 // and, from lane 0, the pair's root task of the path recursion when both
 // sides are non-empty (edlib returns no alignment for an empty side).
 __device__ void distance_pair(const NwDevArgs& a, uint32_t pi, const WarpScratch& ws, u64* peq, int lane) {
