@@ -43,6 +43,7 @@
 
 #include "rb_internal.hpp"
 #include "ring_queue.cuh"
+#include "score_rows.hpp"
 
 namespace rb {
 
@@ -1454,24 +1455,10 @@ __host__ __device__ inline int row_cover(int nw, int wc) {
     return ((wc + ch - 1) / ch) * ch;
 }
 
-// Scores are kept slanted: H'[i][j] = H[i][j] - j * gap. A gap along the row
-// is then free (H'[i][j] = max(T'[i][j], H'[i][j-1])), so the in-row term is
-// a plain running maximum, the diagonal step adds s - gap, the vertical step
-// gap, and the empty prefix row is 0. Cells of one column compare as before.
-//
-// The fast form of a layer's DP stores int16 rows and permutes bytes for the
-// substitution scores. It needs a gap not above 0, s - gap in a signed
-// byte, bases A, C, G, T only, and slanted scores that provably fit: H lies
-// between gap x (row + column) (the all-gap path, which the maximum
-// includes) and max(match, 0) x column, so H' lies between gap x row and
-// (max(match, 0) - gap) x column. Other layers take the general form: int32
-// rows, characters compared. The DP is int32 in registers and in the ring
-// either way.
-__device__ __forceinline__ bool fast_scores(int mt, int mm, int gap, int ndp, int L) {
-    return gap <= 0 && max(mt, mm) - gap <= 127 && min(mt, mm) - gap >= -128 &&
-           (long long)ndp * (long long)(-gap) <= 32767 &&
-           ((long long)max(mt, 0) - gap) * (long long)L <= 32767;
-}
+// Scores are slanted (score_rows.hpp). Layers of bases A, C, G, T only whose
+// scores fit (fast_scores) take the fast form, int16 rows; other layers the
+// general form: int32 rows, characters compared. The DP is int32 in registers
+// and in the ring either way.
 __device__ __forceinline__ bool acgt_base(uint32_t c) {
     return ((0x47544341u >> (8 * ((c >> 1) & 3u))) & 0xFFu) == c;
 }
