@@ -57,5 +57,7 @@ def test_refused(fast):
     assert not fast(3, -5, 1, 10, 10)         # a gap that gains
     assert not fast(100, -100, -90, 10, 10)   # s - gap leaves a signed byte
     assert not fast(5, 60, -60, 500, 500)
+    assert not fast(-1, 20, -40, 100, 100)    # mismatch above match
+    assert not fast(5, -4, -8, 3100, 1000)    # the all-gap path itself, (rows + columns) x gap, leaves 16 bits
     assert not fast(-1, 20, -40, 700, 700)
     assert fast(3, -5, -4, 2000, 600)
