@@ -1061,8 +1061,9 @@ __device__ void add_layer(const Graph& g, PoaShared& sh, const int* order, const
                     return true;
                 });
                 carry = st - 1;
-                // bases inserted so far were given the slot "before" below
-                for (int k = lane; k < nnew; k += 32) g.new_slot[k] = carry;
+                // bases inserted so far were given the slot "before" below,
+                // as many as the slot has room for
+                for (int k = lane; k < min(nnew, g.ncap - nold); k += 32) g.new_slot[k] = carry;
             }
             const unsigned bn = __ballot_sync(kFull, on && n < 0);
             const unsigned upto = ba & (0xffffffffu >> (31 - lane));
