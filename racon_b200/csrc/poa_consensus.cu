@@ -744,6 +744,7 @@ __device__ int topo_sort_warp(const Graph& g, PoaShared& sh, bool partial, int l
         // members of a group outside the subgraph were listed with it
         if (partial) {
             nr = __shfl_sync(kFull, nr, 0);
+            __syncwarp();  // lane 0's list (a shuffle orders no memory)
             int k = 0;
             for (int c0 = 0; c0 < nr; c0 += 32) {
                 const int v = c0 + lane < nr ? g.dfs[c0 + lane] : -1;
@@ -1062,7 +1063,8 @@ __device__ void add_layer(const Graph& g, PoaShared& sh, const int* order, const
                 });
                 carry = st - 1;
                 // bases inserted so far were given the slot "before" below,
-                // as many as the slot has room for
+                // as many as the slot has room for, by other lanes
+                __syncwarp();
                 for (int k = lane; k < min(nnew, g.ncap - nold); k += 32) g.new_slot[k] = carry;
             }
             const unsigned bn = __ballot_sync(kFull, on && n < 0);
