@@ -91,6 +91,7 @@ struct PoaArgs {
     unsigned int* counters;      // [0] window cursor, [1] status
     unsigned long long* cells;   // [0] DP cells computed, [1] edge-cells
     uint32_t per_warp_cap;       // windows a warp takes per launch (0: until the queue is empty)
+    int wait_polls;              // polls of a wait between a team's warps before the window is given up
 };
 
 // Per-slot scratch view.
@@ -185,6 +186,7 @@ struct PoaShared {
     int scratch_bytes;     // the team's shared memory, scratch between the DPs
     uint32_t next;         // queue position the team took
     volatile int done[4];  // per warp: rows it has finished (counting on from pass to pass)
+    volatile int wait_polls;  // limit of the waits on done, 0 once one of them ran out
 };
 
 // ---------------- team memory ----------------
@@ -211,9 +213,23 @@ struct WarpMem {
 };
 // rows between two looks at the neighbouring warps' progress
 constexpr int kGroupRows = 8;
-// polls of a wait on another warp of the team (about a second) before the
-// window is given up as failed
-constexpr int kWaitPolls = 1 << 26;
+// Polls of a wait on another warp of the team before the window is given up as
+// failed: a poll takes 75 cycles or more, so the wait at least 0.15 s, where
+// the rows waited for take microseconds.
+constexpr int kWaitPolls = 1 << 22;
+
+// Waits until `done` reaches `want`. When that takes too long the window is
+// given up, and the team waits no more: its warps run through their rows (whose
+// scores nothing reads), every further wait a single poll. (Leaving the strip
+// instead cost every row 5 %.)
+__device__ __forceinline__ void wait_rows(PoaShared& sh, const volatile int& done, int want) {
+    for (int left = sh.wait_polls; __any_sync(0xffffffffu, done < want); --left)
+        if (left <= 0) {
+            sh.fail = kFailed;
+            sh.wait_polls = 0;
+            break;
+        }
+}
 
 // Barrier of the NW warps of one team (hardware barrier team + 1).
 template <int NW>
@@ -1658,20 +1674,10 @@ __device__ __noinline__ void dp_strip(const Graph& g, PoaShared& sh, int ndp_, c
             // the left neighbour is past these rows; the right one is at
             // most the edge ring behind
             if (waits) {
-                for (int polls = 0; __any_sync(kFull, sh.done[w - 1] < tag0 + i0 + bend); ++polls)
-                    if (polls > kWaitPolls) {
-                        sh.fail = kFailed;
-                        break;
-                    }
+                wait_rows(sh, sh.done[w - 1], tag0 + i0 + bend);
                 __threadfence_block();
             }
-            if (feeds) {
-                for (int polls = 0; __any_sync(kFull, sh.done[w + 1] < tag0 + i0 + bend - kEdgeRows); ++polls)
-                    if (polls > kWaitPolls) {
-                        sh.fail = kFailed;
-                        break;
-                    }
-            }
+            if (feeds) wait_rows(sh, sh.done[w + 1], tag0 + i0 + bend - kEdgeRows);
         }
 #pragma unroll 1
         for (int b = b0; b < bend; ++b) {
@@ -2138,6 +2144,7 @@ __device__ void poa_window(const PoaArgs& a, Graph& g, PoaShared& sh, uint32_t w
         sh.nseq = 1;
         sh.fail = 0;
         sh.scratch_bytes = kTeamBytes;
+        sh.wait_polls = a.wait_polls;
     }
     team_sync<NW>(team);
     unsigned long long cells = 0, edge_cells = 0;
@@ -2173,7 +2180,7 @@ __device__ void poa_window(const PoaArgs& a, Graph& g, PoaShared& sh, uint32_t w
         fast = __all_sync(0xffffffffu, fast);
         dp_dispatch<NW>(g, sh, ndp, seq, L, a.match, a.mismatch, a.gap, lane, w, team, fast);
         team_sync<NW>(team);
-        if (w == 0) {
+        if (w == 0 && !sh.fail) {
             cells += (unsigned long long)ndp * (unsigned long long)L;
             edge_cells += (unsigned long long)(ndp + sh.preds) * (unsigned long long)L;
             const int lc = row_cover(NW, L + 1);
@@ -2685,6 +2692,9 @@ void PoaEngine::run_list(std::vector<uint32_t> todo, int ncap, bool plain) {
         a.trim = trim_;
         a.counters = d_misc_.as<unsigned int>();
         a.cells = reinterpret_cast<unsigned long long*>(d_misc_.as<unsigned int>() + 8);
+        // RB_POA_WAIT_POLLS shortens the limit (tests of a wait that runs out)
+        a.wait_polls = kWaitPolls;
+        if (const char* e = getenv("RB_POA_WAIT_POLLS")) a.wait_polls = std::max(0, std::min(kWaitPolls, atoi(e)));
         check_cuda(cudaMemsetAsync(d_misc_.ptr, 0, 64, stream_), "memset counters");
         check_cuda(cudaEventRecord(ev0_, stream_), "cudaEventRecord");
         if (plain) {
@@ -2834,6 +2844,7 @@ PoaService::PoaService(int device, int8_t m, int8_t x, int8_t g, uint32_t window
     A.base.match = m;
     A.base.mismatch = x;
     A.base.gap = g;
+    A.base.wait_polls = kWaitPolls;
     S->ring.set_large_first_every(large_first_every);
     A.jobs = static_cast<const PoaJobDev*>(S->ring.records());
     A.q = S->ring.queue();
