@@ -3,7 +3,9 @@
 Outputs (git-ignored, shipped with the working tree):
   racon_b200/lib/libracon_b200.so   CUDA kernels + C ABI + racon C++ API
   racon_b200/bin/racon_b200         command-line front end
-Objects go to racon_b200/_build/. Rebuilds only what changed.
+Objects go to racon_b200/_build/, each kernel source's resource usage (registers,
+shared memory, as the assembler reports them) beside its object. Rebuilds only
+what changed.
 """
 import os
 import subprocess
@@ -43,6 +45,10 @@ def _run(cmd):
     return r.stdout
 
 
+def usage_file(src):
+    return os.path.join(BUILD, src.replace("/", "_") + ".usage")
+
+
 def build(verbose=False):
     os.makedirs(BUILD, exist_ok=True)
     os.makedirs(os.path.dirname(LIB), exist_ok=True)
@@ -52,8 +58,10 @@ def build(verbose=False):
     for src in CU_SOURCES:
         s = os.path.join(CSRC, src)
         o = os.path.join(BUILD, src.replace("/", "_") + ".o")
-        if _newer(o, [s] + headers):
-            out = _run([NVCC] + CU_FLAGS + ["-c", s, "-o", o])
+        if _newer(o, [s] + headers) or _newer(usage_file(src), [s] + headers):
+            out = _run([NVCC] + CU_FLAGS + ["-Xptxas", "-v", "-c", s, "-o", o])
+            with open(usage_file(src), "w") as f:
+                f.write(out)
             if verbose and out:
                 print(out)
         objs.append(o)

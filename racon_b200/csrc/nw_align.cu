@@ -2039,7 +2039,8 @@ void NwEngine::run_own() {
     // 50-70 kb: 56 against 51; 60 of 8-50 kb: 27 against 26).
     auto team_for = [&](size_t items) -> int {
         if (yield_items_ || max_m_ < kTeamRows || scratch_warps_ < 2 * kMaxTeam) return 1;
-        if (items <= size_t(dev_.sm_count) / 2 && max_m_ >= kWideTeamRows) return 8;
+        // (a CTA of eight does not fit on an SM beside the services' kernels)
+        if (items <= size_t(dev_.sm_count) / 2 && max_m_ >= kWideTeamRows && !svc_) return 8;
         return items <= 4 * (scratch_warps_ / 4) ? 4 : 1;
     };
     auto team_launch = [&](int w, size_t items, void (*k4)(NwDevArgs), void (*k8)(NwDevArgs)) {

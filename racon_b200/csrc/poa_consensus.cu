@@ -2319,11 +2319,17 @@ struct PoaSvcArgs {
 // Persistent consensus over the shared queue: each team owns one scratch
 // slot and takes windows of any job until the queue stays empty. Sized for
 // at most kSvcCtasPerSm resident CTAs per SM, so that the rest of each SM
-// stays free for the alignment and layer kernels of newly admitted jobs.
+// stays free for the alignment and layer kernels of newly admitted jobs. Held
+// to 160 registers: two of its CTAs take 10240 of an SM sub-partition's 16384,
+// one of the alignment service 3072, which leaves the 3072 of a warp of
+// nw_level_kernel. With 168 a job whose spans exceed the alignment service's
+// scratch could not run its own levels until a service closed for lack of
+// work. (Four jobs at once 91 ms either way; taking the registers from the
+// alignment service instead, 80 or 88 for 96, 93 ms.)
 constexpr int kSvcCtasPerSm = 3;
 constexpr int kSvcTeamWarps = 1;
 constexpr int kSvcWarps = cta_warps(kSvcTeamWarps);
-__global__ void __launch_bounds__(32 * kSvcWarps, kSvcCtasPerSm) poa_service_kernel(PoaSvcArgs s) {
+__global__ void __maxnreg__(160) poa_service_kernel(PoaSvcArgs s) {
     constexpr int NW = kSvcTeamWarps, T = kSvcWarps / NW;
     __shared__ PoaShared sh_all[T];
     __shared__ Graph g_all[T];
