@@ -46,6 +46,7 @@
 #include <climits>
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <mutex>
@@ -110,6 +111,7 @@ struct NwDevArgs {
     NwTask* tasks_out;
     uint32_t tasks_out_cap;
     uint32_t per_warp_cap;   // pairs / tasks a warp takes per launch (0: until the queue is empty)
+    int wait_polls;          // polls of a wait between a team's warps before the pass is given up
 };
 
 __device__ __forceinline__ int fdiv64(int a) { return a >= 0 ? a / 64 : -((-a + 63) / 64); }
@@ -452,12 +454,13 @@ __device__ int warp_sweep_diag(const SweepIO& io, const Band& B, const WarpScrat
 // words it has stored; one buffer more than warps keeps a strip's words until
 // the next strip, on the next warp, has read them all.
 constexpr int kMaxTeam = 8;
-constexpr int kWaitPolls = 1 << 24;  // polls of a wait on another warp before the pass is given up
+constexpr int kWaitPolls = 1 << 24;  // the usual limit of a wait on another warp (half a second or more)
 struct TeamSweep {
     volatile u64 met[kMaxTeam + 1];   // per buffer: strip << 32 | words stored
     volatile int edge[kMaxTeam + 1];  // per buffer: the strip's score in the column before the next strip's first
     volatile int stop;                // the pass is over (gave up, or a wait was lost)
     int result, fail_row, fail_min;
+    int wait_polls;
     unsigned item;
 };
 
@@ -529,7 +532,7 @@ __device__ int strip_sweep(const SweepIO& io, const Band& B, u64* const (&buf)[W
                 if (W > 1) {
                     const u64 want = (u64(unsigned(s - 1)) << 32) | unsigned(min(k + 1, prev_k) + 1);
                     bool lost = false;
-                    for (int polls = 0; T->met[bi] < want && T->stop == 0 && !lost; ++polls) lost = polls > kWaitPolls;
+                    for (int polls = 0; T->met[bi] < want && T->stop == 0 && !lost; ++polls) lost = polls >= T->wait_polls;
                     if (lost) T->stop = 2;
                     if (__any_sync(kFull, T->stop != 0)) return INT_MAX;
                     __threadfence_block();
@@ -637,6 +640,7 @@ __device__ int team_sweep(const NwDevArgs& a, const SweepIO& io, const Band& B, 
         T.stop = 0;
         T.result = INT_MAX;
         T.fail_row = -1;
+        T.wait_polls = a.wait_polls;
     }
     __syncthreads();
     if (diag_sweep_ok(io, B, ws)) {
@@ -2025,6 +2029,9 @@ void NwEngine::run_own() {
     // persistent by default; with a per-warp cap, enough launches back to
     // back that every pair (task) is taken
     a.per_warp_cap = yield_items_;
+    // RB_NW_WAIT_POLLS shortens the limit (tests of a wait that runs out)
+    a.wait_polls = kWaitPolls;
+    if (const char* e = getenv("RB_NW_WAIT_POLLS")) a.wait_polls = std::max(1, std::min(kWaitPolls, atoi(e)));
     auto launches_for = [&](size_t items) {
         return yield_items_ ? (items + scratch_warps_ * yield_items_ - 1) / (scratch_warps_ * yield_items_)
                             : size_t(1);
