@@ -475,7 +475,7 @@ void rb_server_destroy(rb_server* server);
  * synchronise the device (cudaMalloc and cudaFree can wait for all work on
  * it), and code running under a fixed device-memory budget that has already
  * been handed out (a failed allocation there would end the job). Scratch lives in one static device array of about
- * 1.6 MB per device, so each sequence is limited to 131072 bytes; longer
+ * 0.3 MB per device, so each sequence is limited to 131072 bytes; longer
  * inputs return RB_ERR_ARG with that message. The pair must have at most 32
  * distinct byte values, else *distance is set to -1.
  *

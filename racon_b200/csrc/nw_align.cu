@@ -3,15 +3,18 @@
 //   src/overlap.cpp:205-224  edlibAlign(NW, PATH, k = -1) + standard CIGAR
 //   src/overlap.cpp:226-292  find_breaking_points_from_cigar
 //
-// Design (B200, sm_100a). One warp owns one subproblem at a time; warps are
-// persistent and pull work from an atomic queue (pairs sorted by size).
+// Design (B200, sm_100a). One warp owns one subproblem at a time, or the four
+// or eight of a CTA where a batch has few and long ones; warps are persistent
+// and pull work from an atomic queue (pairs sorted by size).
 //
 // * Block sweep. The query is cut into 64-row blocks (one uint64 of vertical
-//   +1/-1 delta bits per block, Myers 1999 / Hyyro). Blocks are grouped into
-//   strips of 32, one block per lane; a strip is swept as a diagonal wavefront
-//   (lane l works on column c - l), the horizontal carry of each column moves
-//   one lane down per step through a warp shuffle, and the bottom lane's carry
-//   is kept in a per-warp column buffer for the next strip.
+//   +1/-1 delta bits per block, Myers 1999 / Hyyro), one per lane. A narrow
+//   band is swept as one diagonal wavefront over all blocks, lanes going round
+//   (warp_sweep_diag); a wider one in strips of 32 blocks (strip_sweep), whose
+//   bottom deltas go to the next strip as 2-bit words, or on to the next warp
+//   of the CTA while the strip is still swept. The horizontal delta of each
+//   column moves one lane down per step through a warp shuffle; between two
+//   band events all lanes take the same straight steps (sweep_steps).
 // * Band. Only blocks that meet the Ukkonen band of the subproblem are
 //   computed: a cell (r, c) can lie on a path of cost <= k only if
 //   |r - c| + |(m - n) - (r - c)| <= k, i.e. r - c in
@@ -33,8 +36,9 @@
 //   +1 bits after the step and the horizontal +1 bits of the step. At a cell
 //   the walk moves up (query base inserted) if the vertical bit is set, left
 //   (target base deleted) if the horizontal bit is set, else diagonally -
-//   edlib's preference order. The 32 lanes prefetch 32 columns; the row is
-//   passed lane to lane.
+//   edlib's preference order. 32 columns at a time, a lane each: the lane's
+//   bits of the 64 rows below the entry row go out to all lanes, which take
+//   every step together.
 // * Output. The path is recorded as mq[t] = matched query position or -1 for
 //   every target position. An optimal alignment never has an insertion next
 //   to a deletion (a diagonal step is cheaper), so the op string, the CIGAR
@@ -623,8 +627,7 @@ __device__ int strip_sweep(const SweepIO& io, const Band& B, u64* const (&buf)[W
 // One warp's sweep in the form the band asks for.
 template <int MODE>
 __device__ int warp_sweep(const SweepIO& io, const Band& B, const WarpScratch& ws, int lane,
-                          unsigned int* counters, SweepFail* fail = nullptr, bool masks_built = false) {
-    (void)counters;
+                          SweepFail* fail = nullptr, bool masks_built = false) {
     if (diag_sweep_ok(io, B, ws)) return warp_sweep_diag<MODE>(io, B, ws, lane, fail, masks_built);
     u64* const buf[2] = {reinterpret_cast<u64*>(ws.carry_h[0]), reinterpret_cast<u64*>(ws.carry_h[1])};
     return strip_sweep<MODE, 1>(io, B, buf, lane, 0, nullptr, fail);
@@ -715,7 +718,7 @@ __device__ void leaf_traceback(const NwDevArgs& a, const NwPairDev& P, const NwT
     io.peq = int(P.nsym) <= kMaxSym ? peq : peq_wide(ws);
     io.leaf = ws.leaf;
     io.bw = bw;
-    warp_sweep<kLeaf>(io, B, ws, lane, a.counters);
+    warp_sweep<kLeaf>(io, B, ws, lane);
     __syncwarp();
 
     // 32 columns at a time, a lane each: the lane's vertical and horizontal
@@ -819,7 +822,7 @@ __device__ bool hirschberg_sweeps(const NwDevArgs& a, const NwPairDev& P, const 
     bool ok = true;
     auto sweep = [&]() {
         if constexpr (W == 1) {
-            warp_sweep<kCapture>(io, B, ws, lane, a.counters);
+            warp_sweep<kCapture>(io, B, ws, lane);
         } else {
             ok = team_sweep<kCapture, W>(a, io, B, ws, lane, w, first_slot, *team, nullptr, false) != -1 && ok;
         }
@@ -952,7 +955,7 @@ __device__ void distance_pair(const NwDevArgs& a, uint32_t pi, const WarpScratch
     while (true) {
         const Band B = make_band(m, n, k);
         SweepFail f;
-        d = warp_sweep<kDistance>(io, B, ws, lane, a.counters, &f, built);
+        d = warp_sweep<kDistance>(io, B, ws, lane, &f, built);
         if (d <= k) break;
         built = diag_sweep_ok(io, B, ws);
         k = next_k(k, f, m, n);
@@ -1533,17 +1536,17 @@ __global__ void cigar_breakpoints_kernel(const char* cig, const CigarOvlDev* ov,
 
 
 // ---------------------------------------------------------------------------
-// Allocation-free edit distance (rb_nw_distance_noalloc). Same banded block
-// sweep and k doubling as nw_distance_kernel, for one pair, with every byte of
+// Allocation-free edit distance (rb_nw_distance_noalloc). The strip sweep and
+// the growth of k of nw_distance_kernel for one pair, the first k as edlib's
+// (strips pay for a wide one), with every byte of
 // scratch (symbol-coded sequences, the two strip carry buffers) in one
 // file-scope device array instead of cudaMalloc'd memory. Every call on a
 // device uses the same array: it keeps the last call's contents, nothing in it
 // has to start at zero (each call writes every byte it later reads), and two
 // calls whose kernels overlap in time race on it.
 constexpr uint32_t kNoAllocMaxLen = 1u << 17;  // per sequence
-constexpr size_t kNoAllocCarry = size_t(kNoAllocMaxLen) + 64;
-constexpr size_t kNoAllocScratchBytes =
-    2 * size_t(kNoAllocMaxLen) + 2 * kNoAllocCarry + 2 * 4 * kNoAllocCarry + 4096;
+constexpr size_t kNoAllocCarry = size_t(kNoAllocMaxLen) / 4 + 64;  // 2 bits a column, whole words
+constexpr size_t kNoAllocScratchBytes = 2 * size_t(kNoAllocMaxLen) + 2 * kNoAllocCarry;
 static __device__ __align__(256) uint8_t g_noalloc_scratch[kNoAllocScratchBytes];
 
 __global__ void __launch_bounds__(32) nw_distance_noalloc_kernel(const char* q, uint32_t m, const char* t,
@@ -1608,7 +1611,7 @@ __global__ void __launch_bounds__(32) nw_distance_noalloc_kernel(const char* q, 
     while (true) {
         const Band B = make_band(int(m), int(n), k);
         SweepFail f;
-        d = warp_sweep<kDistance>(io, B, ws, lane, nullptr, &f);
+        d = warp_sweep<kDistance>(io, B, ws, lane, &f);
         if (d <= k) break;
         k = next_k(k, f, int(m), int(n));
     }
@@ -1621,11 +1624,8 @@ struct NwStoreSrc {
 };
 
 // Symbol codes of pairs cut from the staged sequence table: bytes are
-// numbered by first appearance in the query, then the target (the numbering
-// NwEngine::stage gives on the host), one warp per pair. First appearances
-// come from one pass over 32-byte chunks in order: the lowest lane holding a
-// byte value not seen before records its position. A pair with more than
-// kMaxSymWide distinct bytes (impossible for bytes) sets status[0] = 1.
+// numbered by first appearance in the query, then the target. A pair with more
+// than kMaxSymWide distinct bytes (impossible for bytes) sets status[0] = 1.
 // One warp or the eight of a CTA (parts) take a pair. A symbol's first
 // position is a minimum over all positions, and after the first few hundred
 // bases a look at the table is all a position costs (a warp grouping its
@@ -2043,7 +2043,13 @@ void NwEngine::run_own() {
     // 2400 pairs of 1-30 kb: 74 against 78; 5000 pairs of 1-20 kb: 81 against
     // 50), of eight warps for the longest queries on a half-empty GPU (9 pairs
     // of 60-120 kb: 48 ms against 56; 60 of 60-100 kb: 61 against 67; 140 of
-    // 50-70 kb: 56 against 51; 60 of 8-50 kb: 27 against 26).
+    // 50-70 kb: 56 against 51; 60 of 8-50 kb: 27 against 26). The longest
+    // query decides for the batch. With a polishing job's overlaps that costs
+    // little where few are long, as the heaviest pairs start first, and pays
+    // where those take strips (kernel times, CTAs of four against one warp
+    // each: 2000 pairs of 0.5-8 kb 5.7 ms against 5.7, with ten of 40 kb 20
+    // against 33; 600 of 0.5-8 kb 3.2 against 3.4; 2300 of 1-3 kb and one of
+    // 6.3 kb 3.0 against 2.8; 2300 of 3-12 kb 11.0 against 10.9).
     auto team_for = [&](size_t items) -> int {
         if (yield_items_ || max_m_ < kTeamRows || scratch_warps_ < 2 * kMaxTeam) return 1;
         // (a CTA of eight does not fit on an SM beside the services' kernels)

@@ -13,8 +13,9 @@
 // * Per layer: the subgraph of a partial layer, row descriptors (predecessor
 //   ranks, count, base), the DP, the end cell, the traceback and the insertion
 //   of the aligned layer. Per-node and per-position steps run on the whole
-//   team with four entries per thread in flight; the few serial ones (subgraph
-//   sweep, DFS, bundle scores) run on one lane over shared memory.
+//   team with four entries per thread in flight; the subgraph sweep runs on
+//   one warp, 32 rows at a time, and the few serial steps (DFS, bundle scores)
+//   on one lane, over shared memory.
 // * The DP runs one row (graph node in a valid topological order kept
 //   incrementally) at a time, the team's warps side by side on strips of its
 //   columns (dp_strip), on slanted scores H - column * gap, so that the
@@ -1516,14 +1517,15 @@ __device__ __forceinline__ uint32_t score_pool(uint32_t base, uint32_t mm4, uint
 // finish a window sooner.
 //
 // Rows that other rows than the next one need (g.used) go to a shared-memory
-// ring of the last R such rows, [unit][lane] and then the
-// score left of each lane's segment (conflict-free, and no lane reads
-// another's words); what has left the ring comes from global memory. On this chip a vote
-// with a branch on it costs about 75 cycles, a warp reduction 60, a shuffle
-// 33, so the row is kept nearly free of them. (A row of 500 columns with one
-// predecessor takes 440 cycles on one warp, 400 side by side on four.) What a row needs besides its scores is
-// worked out 32 rows at a time, one row per lane: a score word, and a control
-// word with the ring slots of up to 6 predecessors besides the row just
+// ring of the last R such rows, [unit][lane] and then the score left of each
+// lane's segment (conflict-free, and no lane reads another's words); what has
+// left the ring comes from global memory. On this chip a vote with a branch on
+// it costs about 75 cycles, a warp reduction 60, a shuffle 33, so the row is
+// kept nearly free of them. (Whole layers, cycles a row with one warp and with
+// four: 615 and 540 for layers of 500 bases, 1500 and 690 for 1000; with every
+// SM full of teams 835 and 830, 1880 and 1350.) What a row needs besides its
+// scores is worked out 32 rows at a time, one row per lane: a score word, and a
+// control word with the ring slots of up to 6 predecessors besides the row just
 // computed, which is still in registers.
 //
 // Per cell: the elementwise maximum M over the predecessor rows, then
@@ -1933,8 +1935,9 @@ __device__ void dp_dispatch(const Graph& g, PoaShared& sh, int ndp, const uint8_
 // the warp stages the next one, all its copies in flight at once. Writes the
 // row of every sequence position (0 for an inserted base) to g.path; a
 // vertical step consumes no position and adds nothing to the graph. Returns
-// false on a broken walk. (A step takes 290 cycles, a tile 2 k; with
-// one load after another a tile took 16 k.)
+// false on a broken walk. (The walk takes about 335
+// cycles a base with its tiles, 530 where every SM is full; with one load after
+// another a tile took 16 k cycles, now 2 k.)
 constexpr int kTileRows = 96;
 constexpr int kTilePitch = 128;  // bytes per row: 64 int16 or 32 int32 columns
 constexpr int kTileBytes = 16 + kTileRows * kTilePitch;  // the walk may look one column left of the first
@@ -2648,8 +2651,12 @@ void PoaEngine::run_list(std::vector<uint32_t> todo, int ncap, bool plain) {
         // Warps per window. Four warps side by side finish a window sooner
         // (150 windows of 1000 bases at 20x: 27 ms against 64 ms), one warp
         // spends the fewest instructions (2001 windows of 500 bases at 50x:
-        // 79 ms against 109 ms). The line lies at four windows per SM,
-        // where four-warp teams no longer all run at once.
+        // 79 ms against 109 ms). The line lies at four windows per SM, where
+        // the two meet for windows of 500 bases (30x, kernel ms with one and
+        // with four warps: 300 windows 24.0 / 20.4, 592 27.2 / 26.0, 600 24.8 /
+        // 25.2, 888 26.3 / 30.7, 1776 31.6 / 42.9). Windows of 200 meet a
+        // little before it (300: 8.7 / 8.2, 592: 9.8 / 10.0), windows of 1000
+        // past the resident teams (888: 107 / 76, 1776: 162 / 115).
         const int nw = plain ? kPlainWarps : todo.size() <= 4 * size_t(dev_.sm_count) ? 4 : 1;
         const size_t teams = size_t(cta_warps(nw)) / nw;  // per full CTA
         // resident windows (one team each): enough to fill the SMs, bounded by
