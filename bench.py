@@ -48,21 +48,21 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0}
-# Thread instructions the consensus executes per DP cell with one warp a
-# window (poa_plain_kernel: the same per-window code), from one ncu capture of
-# config 1 at 0.1 genome scale (smsp__inst_executed.sum x threads per
-# instruction / DP cells: 3.44 G x 26.11 / 5.84 G)
-POA_THREAD_INST_PER_CELL = 3443240049 * 26.11 / 5838774640
-# DRAM bytes (read + write) per DP cell, from the same capture (2.199 GB read +
-# 12.164 GB written over 5.839 G cells); traffic grows with the cells, so a
-# full launch's traffic is this times its cells
-POA_DRAM_BYTES_PER_CELL = (2.199457e9 + 12.164103e9) / 5838774640
+# Thread instructions poa_kernel<1> (one warp a window, the form that config 1
+# takes) executes per DP cell, from one ncu capture of config 1 at 0.3 genome
+# scale (smsp__inst_executed.sum x threads per instruction / DP cells: 10.03 G
+# x 26.07 / 17.12 G)
+POA_THREAD_INST_PER_CELL = 10027705487 * 26.07 / 17119442071
+# DRAM bytes (read + write) of poa_kernel<1> per DP cell, from a one-pass ncu
+# capture of the full config 1 launch (44.23 GB read + 127.65 GB written over
+# 58.01 G cells)
+POA_DRAM_BYTES_PER_CELL = (44.23e9 + 127.65e9) / 58012556627
 L2_FLUSH_BYTES = 512 << 20
-# DRAM bytes (read + write) of nw_distance_kernel per nominal cell (query x
-# target span) from one ncu capture of the first 500 pairs of the config-2
-# batch (31.3 MB read + 1.1 MB written over 421.3 G nominal cells); the
-# strip carry buffers grow with the swept cells
-NWD_DRAM_BYTES_PER_CELL = (31.252e6 + 1.092e6) / 421325730898
+# DRAM bytes (read + write) of nw_distance_kernel (one warp a pair, the form
+# that large batches take) per nominal cell (query x target span), from a
+# one-pass ncu capture of a 2400-pair config-2 batch (213.5 MB read + 43.6 MB
+# written over 2.052 T nominal cells); an estimate for other batch sizes
+NWD_DRAM_BYTES_PER_CELL = (213.45e6 + 43.62e6) / 2051963804375
 
 
 def _args():
@@ -483,7 +483,7 @@ def run_align(args, local, world, rank):
                         "achieved": achieved_gbs, "peak": peaks.get("hbm_gbs", 6650.0), "unit": "GB/s",
                         "frac": achieved_gbs / peaks.get("hbm_gbs", 6650.0),
                         "traffic": nominal * NWD_DRAM_BYTES_PER_CELL,
-                        "traffic_source": "nw_distance_kernel DRAM bytes per nominal cell from a 500-pair ncu "
+                        "traffic_source": "estimate: nw_distance_kernel DRAM bytes per nominal cell of a 2400-pair ncu "
                                           "capture, times this step's nominal cells",
                         "note": "algorithmic bytes = sequences in + CIGAR and breakpoints out; the sweep is "
                                 "integer-issue bound, see compute"},
@@ -754,7 +754,7 @@ def main():
                      "peak": peaks.get("hbm_gbs", 6650.0), "unit": "GB/s",
                      "frac": achieved_gbs / peaks.get("hbm_gbs", 6650.0),
                      "traffic": cells / max(1, launches) * POA_DRAM_BYTES_PER_CELL,
-                     "traffic_source": "ncu dram bytes of a 0.1-scale capture, scaled by DP cells per launch",
+                     "traffic_source": "ncu dram bytes per DP cell of a full config 1 launch, times DP cells per launch",
                      "peak_source": peak_kind,
                      "note": "algorithmic bytes = bases+qualities in + consensus out; the DP is integer-issue "
                              "bound, see compute"},
