@@ -224,12 +224,15 @@ constexpr int kWaitPolls = 1 << 22;
 // scores nothing reads), every further wait a single poll. (Leaving the strip
 // instead cost every row 5 %.)
 __device__ __forceinline__ void wait_rows(PoaShared& sh, const volatile int& done, int want) {
-    for (int left = sh.wait_polls; __any_sync(0xffffffffu, done < want); --left)
-        if (left <= 0) {
+    if (!__any_sync(0xffffffffu, done < want)) return;
+    int left = sh.wait_polls;
+    do {
+        if (left-- <= 0) {
             sh.fail = kFailed;
             sh.wait_polls = 0;
             break;
         }
+    } while (__any_sync(0xffffffffu, done < want));
 }
 
 // Barrier of the NW warps of one team (hardware barrier team + 1).
