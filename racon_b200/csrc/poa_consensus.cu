@@ -1068,6 +1068,7 @@ __device__ void add_layer(const Graph& g, PoaShared& sh, const int* order, const
     //    path), those before the first anchor in front of its group
     if (w == 0) {
         int nnew = 0, carry = INT_MIN;
+        const int room = g.ncap - nold;
         for (int c0 = 0; c0 < len; c0 += 32) {
             const int t = c0 + lane;
             const bool on = t < len;
@@ -1085,23 +1086,23 @@ __device__ void add_layer(const Graph& g, PoaShared& sh, const int* order, const
                 // bases inserted so far were given the slot "before" below,
                 // as many as the slot has room for, by other lanes
                 __syncwarp();
-                for (int k = lane; k < min(nnew, g.ncap - nold); k += 32) g.new_slot[k] = carry;
+                for (int k = lane; k < min(nnew, room); k += 32) g.new_slot[k] = carry;
             }
             const unsigned bn = __ballot_sync(kFull, on && n < 0);
             const unsigned upto = ba & (0xffffffffu >> (31 - lane));
             const int sl = __shfl_sync(kFull, s, upto ? 31 - __clz(upto) : 0);
             if (on && n < 0) {
                 const int k = nnew + __popc(bn & ((1u << lane) - 1u));
-                if (nold + k < g.ncap) g.new_slot[k] = upto ? sl : carry == INT_MIN ? nold - 1 : carry;
+                if (k < room) g.new_slot[k] = upto ? sl : carry == INT_MIN ? nold - 1 : carry;
                 nid[t] = nold + k;
             }
             if (ba) carry = __shfl_sync(kFull, s, 31 - __clz(ba));
             nnew += __popc(bn);
         }
         if (lane == 0) {
-            const bool room = nold + nnew <= g.ncap;
-            sh.nnew = room ? nnew : -1;
-            if (!room) sh.fail = kOverflow;
+            const bool fits = nnew <= room;
+            sh.nnew = fits ? nnew : -1;
+            if (!fits) sh.fail = kOverflow;
         }
         __syncwarp();
     }
@@ -2261,7 +2262,7 @@ __device__ void poa_window(const PoaArgs& a, Graph& g, PoaShared& sh, uint32_t w
         fast = __all_sync(0xffffffffu, fast);
         dp_dispatch<NW>(g, sh, ndp, seq, L, a.match, a.mismatch, a.gap, lane, w, team, fast);
         team_sync<NW>(team);
-        if (w == 0 && !sh.fail) {
+        if (w == 0 && (NW == 1 || !sh.fail)) {
             cells += (unsigned long long)ndp * (unsigned long long)L;
             edge_cells += (unsigned long long)(ndp + sh.preds) * (unsigned long long)L;
             const int lc = row_cover(NW, L + 1);
