@@ -21,7 +21,7 @@ BIN = os.path.join(HERE, "bin", "racon_b200")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CU_FLAGS = ARCH + ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
-                   "-Wno-deprecated-gpu-targets"]
+                   "-Wno-deprecated-gpu-targets", "--no-compress"]
 CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-Wall", "-Wextra", "-pthread",
              "-I/usr/local/cuda/include"]
 
